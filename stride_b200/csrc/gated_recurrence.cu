@@ -6,14 +6,11 @@
 // The kernel takes q, g, k, v as columns of one float32 row per token, so whatever makes them is a kernel in front.
 // HGRN2 is one such maker (`hgrn2_activate_kernel`): q = silu(W_q x), g = l + (1 - l) sigmoid(W_f x + b) with a lower
 // bound l per channel, k = 1 - g (the gate's complement is the key: what a channel does not keep, it takes in), v = W_v x.
-// Everything here is 32-bit. A CTA owns (request of the step, head, 32 value columns) and walks the request's tokens of
-// this step in order with the state in registers; it reads the state the step before left (or starts from zero at
-// position 0) and writes it back at the end. The D sums of an output are cut into parts of 16 consecutive elements, each
-// one chain of fused multiply-adds in ascending order, and the parts are added in ascending order; neither depends on the
-// step, so a token's output has the same bits in a prompt, in a portion and decoded alone.
+// Everything here is 32-bit; the recurrence is linear_scan.cuh's, whose outputs have the same bits in a prompt, in a portion and decoded alone.
 //
 // `group_rmsnorm_kernel` is what follows: every head's output RMS-normed on its own with one gain vector for all heads.
 #include "common.cuh"
+#include "linear_scan.cuh"
 #include "step_ops.h"
 
 SB_DEFINE_LAST_ERROR()
@@ -22,8 +19,6 @@ namespace {
 
 using bf16 = __nv_bfloat16;
 constexpr int kInFlight = 8;
-constexpr int R = 16;        // elements of a state column a thread holds
-constexpr int kChunk = 16;   // tokens staged in shared memory at a time
 
 __device__ __forceinline__ float folded(const float* p, int n_partials, int64_t stride) {
   float part[kInFlight];
@@ -66,120 +61,27 @@ __global__ void hgrn2_activate_kernel(const float* __restrict__ proj, int n_part
   }
 }
 
-struct ScanParams {
-  const float* act;         // [n][width]
-  int width;
-  int q_off, g_off, k_off, v_off;
-  const int32_t* meta;      // [4][meta_stride]: slot, first row, length, first position of every entry
-  int meta_stride;
-  float* state;             // [slots][H][D][V]
-  float* out;               // [n][H V]
-  int H, D, V;
-};
-
-__device__ __forceinline__ void copy_async4(float* dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copy_async16(float* dst, const float* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
-}
-
-// The q, g, k rows and the CTA's 32 value columns of a chunk of kChunk tokens reach shared memory by asynchronous copies, a chunk
-// ahead of the one being walked (two staging buffers). VEC = 4: every size and offset is a multiple of four floats, 16 bytes a copy.
-template <int VEC>
-__global__ void __launch_bounds__(512) gated_scan_kernel(const ScanParams p) {
+// Steps in which every entry brings one token.
+template <int DL>
+__global__ void __launch_bounds__(DL * 64, 1024 / (DL * 64)) gated_step_kernel(const sbscan::Params p) {
   extern __shared__ __align__(16) float smem[];
   sb::grid_launch_dependents();
   const int e = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * 32;
-  const int parts = blockDim.x >> 5, Dp = parts * R;
-  const int part = threadIdx.x >> 5, cl = threadIdx.x & 31;
-  const int stage = kChunk * (3 * Dp + 32);       // floats of a staging buffer: q, g, k [kChunk][Dp], v [kChunk][32]
-  float* so = smem + 2 * stage;                    // [parts][kChunk][32]
-  const int slot = p.meta[e], row0 = p.meta[p.meta_stride + e], len = p.meta[2 * p.meta_stride + e], pos0 = p.meta[3 * p.meta_stride + e];
-  const bool live = c0 + cl < p.V;
-  const int vn = min(32, p.V - c0);
-  const int dn = min(R, p.D - part * R);
-  float* st = p.state + ((static_cast<int64_t>(slot) * p.H + h) * p.D + part * R) * p.V + c0 + cl;
-  // nothing copies into the cells beyond D and beyond the CTA's existing columns: they are zero for good
-  if (Dp != p.D || vn != 32)
-    for (int i = threadIdx.x; i < 2 * stage; i += blockDim.x) smem[i] = 0.0f;
+  const int slot = p.meta[e], row = p.meta[p.meta_stride + e], pos0 = p.meta[3 * p.meta_stride + e];
   sb::grid_dependency_wait();
-  __syncthreads();
-  float S[R];
-#pragma unroll
-  for (int i = 0; i < R; ++i) S[i] = (pos0 > 0 && live && i < dn) ? st[static_cast<int64_t>(i) * p.V] : 0.0f;
-  const int du = p.D / VEC, vu = vn / VEC, per_token = 3 * du + vu;
-  auto request = [&](int chunk) {
-    float* sq = smem + (chunk & 1) * stage;
-    const int nt = min(kChunk, len - chunk * kChunk);
-    for (int i = threadIdx.x; i < nt * per_token; i += blockDim.x) {
-      const int t = i / per_token, j = i % per_token;
-      const float* src = p.act + static_cast<int64_t>(row0 + chunk * kChunk + t) * p.width;
-      float* dst;
-      if (j < 3 * du) {
-        const int which = j / du, u = j % du;
-        src += (which == 0 ? p.q_off : which == 1 ? p.g_off : p.k_off) + h * p.D + u * VEC;
-        dst = sq + which * kChunk * Dp + t * Dp + u * VEC;
-      } else {
-        const int u = j - 3 * du;
-        src += p.v_off + h * p.V + c0 + u * VEC;
-        dst = sq + 3 * kChunk * Dp + t * 32 + u * VEC;
+  sbscan::step_core<DL, true>(p, smem, slot, row, pos0, [&](float* to, int Dp) {
+    const float* src = p.rows + static_cast<int64_t>(row) * p.width;
+    for (int j = threadIdx.x; j < 3 * Dp + 32; j += blockDim.x) {
+      float v = 0.0f;
+      if (j < 3 * Dp) {
+        const int which = j / Dp, d = j - which * Dp;          // q, k, g
+        if (d < p.D) v = src[(which == 0 ? p.q_off : which == 1 ? p.k_off : p.g_off) + h * p.D + d];
+      } else if (c0 + j - 3 * Dp < p.V) {
+        v = src[p.v_off + h * p.V + c0 + j - 3 * Dp];
       }
-      if (VEC == 4) copy_async16(dst, src);
-      else copy_async4(dst, src);
+      to[j] = v;
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  const int chunks = (len + kChunk - 1) / kChunk;
-  request(0);
-  for (int chunk = 0; chunk < chunks; ++chunk) {
-    if (chunk + 1 < chunks) {
-      request(chunk + 1);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
-    __syncthreads();
-    const int nt = min(kChunk, len - chunk * kChunk);
-    const float* sq = smem + (chunk & 1) * stage;
-    const float* sg = sq + kChunk * Dp;
-    const float* sk = sg + kChunk * Dp;
-    const float* sv = sk + kChunk * Dp;
-    for (int t = 0; t < nt; ++t) {
-      const float4* q4 = reinterpret_cast<const float4*>(sq + t * Dp + part * R);
-      const float4* g4 = reinterpret_cast<const float4*>(sg + t * Dp + part * R);
-      const float4* k4 = reinterpret_cast<const float4*>(sk + t * Dp + part * R);
-      const float x = sv[t * 32 + cl];
-      float acc = 0.0f;
-#pragma unroll
-      for (int i = 0; i < R / 4; ++i) {
-        const float4 q = q4[i], g = g4[i], k = k4[i];
-        S[4 * i] = fmaf(g.x, S[4 * i], __fmul_rn(k.x, x));
-        acc = fmaf(S[4 * i], q.x, acc);
-        S[4 * i + 1] = fmaf(g.y, S[4 * i + 1], __fmul_rn(k.y, x));
-        acc = fmaf(S[4 * i + 1], q.y, acc);
-        S[4 * i + 2] = fmaf(g.z, S[4 * i + 2], __fmul_rn(k.z, x));
-        acc = fmaf(S[4 * i + 2], q.z, acc);
-        S[4 * i + 3] = fmaf(g.w, S[4 * i + 3], __fmul_rn(k.w, x));
-        acc = fmaf(S[4 * i + 3], q.w, acc);
-      }
-      so[(part * kChunk + t) * 32 + cl] = acc;
-    }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < nt * 32; idx += blockDim.x) {
-      const int t = idx >> 5, c = idx & 31;
-      if (c0 + c < p.V) {
-        float sum = so[t * 32 + c];
-        for (int q = 1; q < parts; ++q) sum += so[(q * kChunk + t) * 32 + c];
-        p.out[static_cast<int64_t>(row0 + chunk * kChunk + t) * p.H * p.V + h * p.V + c0 + c] = sum;
-      }
-    }
-  }
-  if (live) {
-#pragma unroll
-    for (int i = 0; i < R; ++i)
-      if (i < dn) st[static_cast<int64_t>(i) * p.V] = S[i];
-  }
+  });
 }
 
 // out[r, h V + j] = o[r, h V + j] / sqrt(mean_j(o[r, h V + :]^2) + eps) * gain[j]: a warp per (row, head).
@@ -221,25 +123,18 @@ SB_EXPORT int sb_hgrn2_activate(const float* proj, int n_partials, int64_t parti
   return sb::check_launch("sb_hgrn2_activate");
 }
 
+// n: the step's tokens
 SB_EXPORT int sb_gated_scan(const float* act, int width, int q_off, int g_off, int k_off, int v_off, const int32_t* meta, int meta_stride,
-                            int entries, float* state, float* out, int H, int D, int V, cudaStream_t stream) {
+                            int entries, int n, float* state, float* out, int H, int D, int V, cudaStream_t stream) {
   if (entries <= 0) return 0;
   if (H <= 0 || D <= 0 || V <= 0 || D > 256) return sb::fail("sb_gated_scan: heads %d, key size %d (at most 256), value size %d", H, D, V);
-  const int parts = (D + R - 1) / R, Dp = parts * R;
-  ScanParams p{act, width, q_off, g_off, k_off, v_off, meta, meta_stride, state, out, H, D, V};
-  const size_t smem = sizeof(float) * (static_cast<size_t>(2) * kChunk * (3 * Dp + 32) + static_cast<size_t>(parts) * kChunk * 32);
-  if (smem > 200 * 1024) return sb::fail("sb_gated_scan: key size %d does not fit shared memory", D);
-  const bool vec = D % 4 == 0 && V % 4 == 0 && width % 4 == 0 && q_off % 4 == 0 && g_off % 4 == 0 && k_off % 4 == 0 && v_off % 4 == 0 &&
-                   (reinterpret_cast<uintptr_t>(act) & 15) == 0;
-  static sb::DeviceOnce once;
-  if (once.needed()) {
-    cudaFuncSetAttribute(gated_scan_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(gated_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    once.done();
+  sbscan::Params p{act, width, q_off, k_off, v_off, g_off, meta, meta_stride, nullptr, state, out, H, D, V};
+  if (n == entries) {
+    const auto kernel = sbscan::lane_elements(D) == 2 ? gated_step_kernel<2> : sbscan::lane_elements(D) == 4 ? gated_step_kernel<4> : gated_step_kernel<8>;
+    sb::launch_pdl(kernel, dim3(entries, H, (V + 31) / 32), dim3(sbscan::step_threads(D)), sbscan::step_smem(D, true), stream, p);
+    return sb::check_launch("sb_gated_scan");
   }
-  if (vec) sb::launch_pdl(gated_scan_kernel<4>, dim3(entries, H, (V + 31) / 32), dim3(parts * 32), smem, stream, p);
-  else sb::launch_pdl(gated_scan_kernel<1>, dim3(entries, H, (V + 31) / 32), dim3(parts * 32), smem, stream, p);
-  return sb::check_launch("sb_gated_scan");
+  return sbscan::launch_scan<true>(p, entries, "sb_gated_scan", stream);
 }
 
 SB_EXPORT int sb_group_rmsnorm(const float* o, const void* gain, int gain_dtype, void* out, int out_dtype, int n, int H, int V, float eps,
@@ -273,7 +168,7 @@ SB_EXPORT int sb_op_gated_scan(const SbOp* op, const SbStep* s, void* stream) {
   using namespace sbstep;
   if (s->n <= 0) return SB_OP_SKIPPED;
   return sb_gated_scan(ptr<const float>(op->i[0]), (int)op->i[1], (int)op->i[2], (int)op->i[3], (int)op->i[4], (int)op->i[5], entry_meta(s),
-                       s->max_rows, s->entries, ptr<float>(op->i[6]), ptr<float>(op->i[7]), (int)op->i[8], (int)op->i[9], (int)op->i[10],
+                       s->max_rows, s->entries, s->n, ptr<float>(op->i[6]), ptr<float>(op->i[7]), (int)op->i[8], (int)op->i[9], (int)op->i[10],
                        static_cast<cudaStream_t>(stream));
 }
 

@@ -1,0 +1,344 @@
+// The recurrence of linear attention over a state kept per request, with one decay a head (lightning attention, retention) or a gate per
+// key channel and token (HGRN2):
+//
+//   S_t = a_t S_(t-1) + k_t v_t^T        S: [D, V] float32 per head; a_t: a constant of the head, or diag(g_t)
+//   o_t = S_t^T q_t
+//
+// Everything is 32-bit. A column of the state depends on no other column, so the value columns may be spread over CTAs and threads in any
+// way. The D sums of an output are cut into 32 parts of DL consecutive elements (DL = 2, 4 or 8 by the key size alone; elements beyond D are
+// zero), each two chains of fused multiply-adds (even and odd elements, ascending, then added), and the parts are added as a binary tree of
+// neighbours (part 2i + part 2i + 1, and so on). None of it depends on the step, so a token's output has the same bits however the sequence
+// was cut into steps, whichever of the two kernels below ran, and whatever else the batch holds.
+//
+// `scan_kernel` is for steps in which an entry brings several tokens; `step_core` is the work of a token for steps of single tokens.
+#pragma once
+
+#include <type_traits>
+
+#include "common.cuh"
+#include "step_ops.h"
+
+namespace sbscan {
+
+constexpr int kLanes = 32;       // parts of the D sums
+constexpr int kWarps = 4;        // computing warps of scan_kernel
+constexpr int kChunk = 16;       // tokens staged in shared memory at a time
+constexpr int kStages = 3;       // staging buffers of scan_kernel
+
+inline int lane_elements(int D) { return D <= 64 ? 2 : D <= 128 ? 4 : 8; }
+
+struct Params {
+  const float* rows;        // [n][width], float32: the tokens' q, k, v (and gates)
+  int width;                // elements of a token's row
+  int q_off, k_off, v_off, g_off;
+  const int32_t* meta;      // [4][meta_stride]: slot, first row, length, first position of every entry
+  int meta_stride;
+  const float* decay;       // [H]; unused with gates
+  float* state;             // [slots][H][D][V]
+  float* out;               // [n][H V]
+  int H, D, V;
+};
+
+// Asynchronous copies from global to shared memory and the wait for all but the newest N groups of a thread's own.
+template <int FLOATS>
+__device__ __forceinline__ void copy_async(float* dst, const float* src) {
+  const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  if constexpr (FLOATS == 4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(src) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Two float32 operations in one instruction (sm_100): each half rounds as the scalar one does.
+__device__ __forceinline__ uint64_t bits2(float2 a) { return *reinterpret_cast<const uint64_t*>(&a); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(bits2(a)), "l"(bits2(b)), "l"(bits2(c)));
+  return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(bits2(a)), "l"(bits2(b)));
+  return *reinterpret_cast<float2*>(&d);
+}
+
+// A token's keys, queries and gates of DL elements, as pairs.
+template <int DL, bool GATED>
+struct Part {
+  float2 k[DL / 2], q[DL / 2], g[GATED ? DL / 2 : 1];
+  static __device__ __forceinline__ void fetch(float2 (&to)[DL / 2], const float* from) {
+    if constexpr (DL == 2) {
+      to[0] = *reinterpret_cast<const float2*>(from);
+    } else {
+#pragma unroll
+      for (int i = 0; i < DL / 4; ++i) {
+        const float4 v = reinterpret_cast<const float4*>(from)[i];
+        to[2 * i] = make_float2(v.x, v.y);
+        to[2 * i + 1] = make_float2(v.z, v.w);
+      }
+    }
+  }
+  __device__ __forceinline__ void load(const float* sq, const float* sk, const float* sg) {
+    fetch(k, sk);
+    fetch(q, sq);
+    if constexpr (GATED) fetch(g, sg);
+  }
+};
+
+// One token for one part of one column: S <- a S + k v; the part's share of the output.
+template <int DL, bool GATED>
+__device__ __forceinline__ float token(float2 (&S)[DL / 2], const Part<DL, GATED>& x, float v, float decay) {
+  const float2 v2 = make_float2(v, v), d2 = make_float2(decay, decay);
+  float2 acc;
+#pragma unroll
+  for (int i = 0; i < DL / 2; ++i) {
+    S[i] = fma2(GATED ? x.g[GATED ? i : 0] : d2, S[i], mul2(x.k[i], v2));
+    acc = i == 0 ? mul2(S[0], x.q[0]) : fma2(S[i], x.q[i], acc);
+  }
+  return acc.x + acc.y;
+}
+
+template <int N>
+__device__ __forceinline__ void put(float2 (&S)[N], int i, float v) {
+  if (i & 1) S[i / 2].y = v;
+  else S[i / 2].x = v;
+}
+template <int N>
+__device__ __forceinline__ float get(const float2 (&S)[N], int i) { return i & 1 ? S[i / 2].y : S[i / 2].x; }
+
+// Every lane holds its part of 32 sums; lane i returns the whole of sum i: 31 exchanges instead of 32 times 5.
+__device__ __forceinline__ float transpose_add(float (&a)[32], int lane) {
+#pragma unroll
+  for (int m = 1; m < 32; m <<= 1) {
+    const bool up = lane & m;
+#pragma unroll
+    for (int i = 0; i < 32; i += 2 * m) {
+      const float give = up ? a[i] : a[i + m], keep = up ? a[i + m] : a[i];
+      a[i] = keep + __shfl_xor_sync(0xffffffffu, give, m);
+    }
+  }
+  return a[0];
+}
+
+// Named barriers of scan_kernel (id 0 is __syncthreads): one per buffer and direction.
+enum { kBarFull = 1, kBarEmpty = 1 + kStages };
+__device__ __forceinline__ void bar_sync(int id, int count) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int count) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory"); }
+
+// A CTA owns (entry, head, 4 PER value columns) and walks the entry's tokens of this step in order. A computing warp owns PER columns, a
+// lane one part of each: a token's keys and queries are read from shared memory once a warp, every lane its own, and serve PER columns. The
+// parts of 32 / PER tokens' outputs are added up together by exchanges between lanes, so that no part goes through shared memory. One more
+// warp keeps the rows of the next two chunks of tokens on their way into the staging buffers; it announces a chunk before it requests
+// another, since a request waits until its buffer is free. What bounds the kernel is the chain of a token's dependent operations in the one
+// computing warp that a scheduler has (without the loads and the exchanges 155 of its 220 us are left).
+// Measured (16 heads of 128 x 128, one entry of 2,048 tokens / eight): eight warps of one column a thread, the outputs' parts through shared
+// memory, 611 / 1,600 us; PER = 4 220 / 721 us, PER = 2 193 / 828 us.
+template <int DL, int PER, bool GATED, int VEC>
+__global__ void __launch_bounds__(kWarps * 32 + 32) scan_kernel(const Params p) {
+  extern __shared__ __align__(16) float smem[];
+  sb::grid_launch_dependents();
+  constexpr int kCols = kWarps * PER, kGroup = 32 / PER;       // a group: the tokens whose outputs a warp adds up together
+  constexpr int Dp = kLanes * DL, NC = kWarps * 32, NQ = GATED ? 3 : 2, stage = kChunk * (NQ * Dp + kCols);
+  const int e = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * kCols, vn = min(kCols, p.V - c0);
+  const int slot = p.meta[e], row0 = p.meta[p.meta_stride + e], len = p.meta[2 * p.meta_stride + e], pos0 = p.meta[3 * p.meta_stride + e];
+  const int chunks = (len + kChunk - 1) / kChunk;
+  // nothing copies into the cells beyond D and beyond the CTA's existing columns: they are zero for good
+  if (Dp != p.D || vn != kCols)
+    for (int i = threadIdx.x; i < kStages * stage; i += blockDim.x) smem[i] = 0.0f;
+  sb::grid_dependency_wait();
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp < kWarps) {
+    // ---------------------------------------------------------------- the recurrence
+    const float decay = GATED ? 0.0f : p.decay[h];
+    const int cl = warp * PER, dn = min(DL, p.D - lane * DL);
+    float* st = p.state + ((static_cast<int64_t>(slot) * p.H + h) * p.D + lane * DL) * p.V + c0 + cl;
+    float2 S[PER][DL / 2];
+#pragma unroll
+    for (int i = 0; i < DL; ++i)
+#pragma unroll
+      for (int c = 0; c < PER; ++c) put(S[c], i, pos0 > 0 && cl + c < vn && i < dn ? st[static_cast<int64_t>(i) * p.V + c] : 0.0f);
+    float* out = p.out + static_cast<int64_t>(row0) * p.H * p.V + h * p.V + c0 + cl + (lane & (PER - 1));
+    const bool live = cl + (lane & (PER - 1)) < vn;
+    for (int c = 0, b = 0; c < chunks; ++c, b = b + 1 == kStages ? 0 : b + 1) {
+      const float* sq = smem + b * stage + lane * DL;
+      const float* sv = smem + b * stage + NQ * kChunk * Dp + cl;
+      bar_sync(kBarFull + b, NC + 32);
+#pragma unroll 1
+      for (int t0 = 0; t0 < kChunk; t0 += kGroup) {
+        const int nt = min(kGroup, len - c * kChunk - t0);
+        if (nt <= 0) break;
+        float sums[32];
+        // the next token's operands are on their way while a token is computed; a whole group runs without a test between its tokens, which
+        // would keep one token's operations from filling another's waits (320 us in place of 220)
+        auto walk = [&](auto whole) {
+          Part<DL, GATED> x[2];
+          float v[2][PER];
+          auto load = [&](int t, int at) {
+            const float* row = sq + (t0 + t) * Dp;
+            x[at].load(row, row + kChunk * Dp, row + (GATED ? 2 : 0) * kChunk * Dp);
+            const float* from = sv + (t0 + t) * kCols;
+            if constexpr (PER == 4) {
+              const float4 w = *reinterpret_cast<const float4*>(from);
+              v[at][0] = w.x, v[at][1] = w.y, v[at][2] = w.z, v[at][3] = w.w;
+            } else {
+              const float2 w = *reinterpret_cast<const float2*>(from);
+              v[at][0] = w.x, v[at][1] = w.y;
+            }
+          };
+          load(0, 0);
+#pragma unroll
+          for (int t = 0; t < kGroup; ++t) {
+            if (t + 1 < kGroup) load(t + 1, (t + 1) & 1);        // (a row beyond the chunk's tokens holds old values, which nothing uses)
+            if (decltype(whole)::value || t < nt) {
+#pragma unroll
+              for (int j = 0; j < PER; ++j) sums[t * PER + j] = token<DL, GATED>(S[j], x[t & 1], v[t & 1][j], decay);
+            } else {
+#pragma unroll
+              for (int j = 0; j < PER; ++j) sums[t * PER + j] = 0.0f;
+            }
+          }
+        };
+        if (nt == kGroup) walk(std::true_type{});
+        else walk(std::false_type{});
+        if (t0 + kGroup >= min(kChunk, len - c * kChunk) && c + kStages < chunks) bar_arrive(kBarEmpty + b, NC + 32);
+        const float sum = transpose_add(sums, lane);
+        const int t = lane / PER;
+        if (live && t < nt) out[static_cast<int64_t>(c * kChunk + t0 + t) * p.H * p.V] = sum;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < DL; ++i)
+#pragma unroll
+      for (int c = 0; c < PER; ++c)
+        if (cl + c < vn && i < dn) st[static_cast<int64_t>(i) * p.V + c] = get(S[c], i);
+  } else {
+    // ---------------------------------------------------------------- the loads
+    const int du = p.D / VEC, vu = vn / VEC;      // (VEC == 4 only when every size and offset is a multiple of four)
+    const float* src0 = p.rows + static_cast<int64_t>(row0) * p.width;
+    auto request = [&](int c, int b) {
+      const int nt = min(kChunk, len - c * kChunk);
+      float* to = smem + b * stage;
+      const float* from = src0 + static_cast<int64_t>(c) * kChunk * p.width;
+      for (int u = lane; u < du; u += 32) {
+        const float* src = from + h * p.D + u * VEC;
+        float* dst = to + u * VEC;
+#pragma unroll 4
+        for (int t = 0; t < nt; ++t, src += p.width, dst += Dp) {
+          copy_async<VEC>(dst, src + p.q_off);
+          copy_async<VEC>(dst + kChunk * Dp, src + p.k_off);
+          if constexpr (GATED) copy_async<VEC>(dst + 2 * kChunk * Dp, src + p.g_off);
+        }
+      }
+      constexpr int kPieces = kCols / VEC;
+      for (int i = lane; i < nt * kPieces; i += 32) {
+        const int t = i / kPieces, u = i % kPieces;
+        if (u < vu)
+          copy_async<VEC>(to + NQ * kChunk * Dp + t * kCols + u * VEC, from + static_cast<int64_t>(t) * p.width + p.v_off + h * p.V + c0 + u * VEC);
+      }
+      copy_async_commit();
+    };
+    constexpr int ahead = kStages - 1;
+    for (int c = 0; c < ahead && c < chunks; ++c) request(c, c);
+    for (int c = 0, b = 0; c < chunks; ++c, b = b + 1 == kStages ? 0 : b + 1) {
+      if (c + 1 < chunks) copy_async_wait<ahead - 1>();
+      else copy_async_wait<0>();
+      bar_arrive(kBarFull + b, NC + 32);
+      if (c + ahead < chunks) {
+        const int rb = b == 0 ? kStages - 1 : b - 1;
+        if (c + ahead >= kStages) bar_sync(kBarEmpty + rb, NC + 32);
+        request(c + ahead, rb);
+      }
+    }
+  }
+}
+
+template <int DL, int PER, bool GATED>
+int launch_scan_of(const Params& p, int entries, const char* who, cudaStream_t stream) {
+  constexpr int kCols = kWarps * PER;
+  constexpr size_t smem = sizeof(float) * kStages * kChunk * ((GATED ? 3 : 2) * kLanes * DL + kCols);
+  static_assert(smem <= 200 * 1024, "staging buffers");
+  const bool vec = p.D % 4 == 0 && p.V % 4 == 0 && p.width % 4 == 0 && p.q_off % 4 == 0 && p.k_off % 4 == 0 && p.v_off % 4 == 0 &&
+                   (!GATED || p.g_off % 4 == 0) && (reinterpret_cast<uintptr_t>(p.rows) & 15) == 0;
+  static sb::DeviceOnce once;
+  if (once.needed()) {
+    cudaFuncSetAttribute(scan_kernel<DL, PER, GATED, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(scan_kernel<DL, PER, GATED, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    once.done();
+  }
+  const dim3 grid(entries, p.H, (p.V + kCols - 1) / kCols), block(kWarps * 32 + 32);
+  if (vec) sb::launch_pdl(scan_kernel<DL, PER, GATED, 4>, grid, block, smem, stream, p);
+  else sb::launch_pdl(scan_kernel<DL, PER, GATED, 1>, grid, block, smem, stream, p);
+  return sb::check_launch(who);
+}
+
+// Launches scan_kernel for the key size (at most 256). Four columns a warp make fewer reads a column; two make twice the CTAs, which is the
+// faster way while they all run at once (193 against 220 us for 128 CTAs of four; 828 against 721 us for 1,024).
+template <bool GATED>
+int launch_scan(const Params& p, int entries, const char* who, cudaStream_t stream) {
+  const bool few = static_cast<int64_t>(entries) * p.H * ((p.V + 15) / 16) <= sb::sm_count();
+#define SB_SCAN_OF(DL) (few ? launch_scan_of<DL, 2, GATED>(p, entries, who, stream) : launch_scan_of<DL, 4, GATED>(p, entries, who, stream))
+  switch (lane_elements(p.D)) {
+    case 2: return SB_SCAN_OF(2);
+    case 4: return SB_SCAN_OF(4);
+    default: return SB_SCAN_OF(8);
+  }
+#undef SB_SCAN_OF
+}
+
+// Steps in which every entry brings one token: a CTA is (entry, head, 32 value columns), a thread kRows elements of one column (what a
+// warp reads of the state is whole 128-byte rows). The state's loads are requested first; `fill(smem, Dp)` writes the token's q, k, (g,) v
+// into shared memory meanwhile: q, k, g [Dp] each, zero beyond D, v [32]. The same operations in the same order as scan_kernel: a thread
+// adds its own neighbouring parts, the warps' sums are the upper levels of the tree.
+constexpr int kRows = 16;
+template <int DL, bool GATED, class Fill>
+__device__ __forceinline__ void step_core(const Params& p, float* smem, int slot, int row, int pos0, Fill fill) {
+  constexpr int Dp = kLanes * DL, kParts = kRows / DL, warps = Dp / kRows;
+  const int h = blockIdx.y, c0 = blockIdx.z * 32, warp = threadIdx.x >> 5, cl = threadIdx.x & 31;
+  float* sv = smem + (GATED ? 3 : 2) * Dp;
+  float* so = sv + 32;         // [warps][32]
+  const bool live = c0 + cl < p.V;
+  const int d0 = warp * kRows, dn = min(kRows, p.D - d0);
+  float* st = p.state + ((static_cast<int64_t>(slot) * p.H + h) * p.D + d0) * p.V + c0 + cl;
+  float2 S[kParts][DL / 2];
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) put(S[i / DL], i % DL, pos0 > 0 && live && i < dn ? st[static_cast<int64_t>(i) * p.V] : 0.0f);
+  fill(smem, Dp);
+  __syncthreads();
+  const float decay = GATED ? 0.0f : p.decay[h];
+  float a[kParts];
+#pragma unroll
+  for (int j = 0; j < kParts; ++j) {
+    const float* sq = smem + d0 + j * DL;
+    Part<DL, GATED> x;
+    x.load(sq, sq + Dp, sq + (GATED ? 2 : 0) * Dp);
+    a[j] = token<DL, GATED>(S[j], x, sv[cl], decay);
+  }
+#pragma unroll
+  for (int m = 1; m < kParts; m <<= 1)
+#pragma unroll
+    for (int j = 0; j < kParts; j += 2 * m) a[j] = a[j] + a[j + m];
+  so[warp * 32 + cl] = a[0];
+  if (live) {
+#pragma unroll
+    for (int i = 0; i < kRows; ++i)
+      if (i < dn) st[static_cast<int64_t>(i) * p.V] = get(S[i / DL], i % DL);
+  }
+  __syncthreads();
+  if (warp == 0 && live) {
+    float w[warps];
+#pragma unroll
+    for (int q = 0; q < warps; ++q) w[q] = so[q * 32 + cl];
+#pragma unroll
+    for (int m = 1; m < warps; m <<= 1)
+#pragma unroll
+      for (int q = 0; q < warps; q += 2 * m) w[q] = w[q] + w[q + m];
+    p.out[static_cast<int64_t>(row) * p.H * p.V + h * p.V + c0 + cl] = w[0];
+  }
+}
+
+inline int step_threads(int D) { return kLanes * lane_elements(D) / kRows * 32; }
+inline size_t step_smem(int D, bool gated) { return sizeof(float) * ((gated ? 3 : 2) * kLanes * lane_elements(D) + 32 + step_threads(D)); }
+
+}  // namespace sbscan

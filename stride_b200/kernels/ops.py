@@ -571,10 +571,10 @@ def gated_scan(act: torch.Tensor, q_off: int, g_off: int, k_off: int, v_off: int
                out: torch.Tensor, heads: int, key_dim: int, value_dim: int) -> None:
     """S <- diag(g) S + k v^T, o = S^T q for every entry of the step, token by token; state [slots, heads, key_dim, value_dim] float32."""
     _cuda(act, entry_meta, state, out)
-    lib, fn = _fn("gated_recurrence", "sb_gated_scan", [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p,
+    lib, fn = _fn("gated_recurrence", "sb_gated_scan", [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
                                                          c_int, c_int, c_int, c_void_p])
-    _check(lib, fn(_ptr(act), act.stride(0), q_off, g_off, k_off, v_off, _ptr(entry_meta), entry_meta.stride(0), entries, _ptr(state), _ptr(out),
-                   heads, key_dim, value_dim, _stream()))
+    _check(lib, fn(_ptr(act), act.stride(0), q_off, g_off, k_off, v_off, _ptr(entry_meta), entry_meta.stride(0), entries, act.shape[0], _ptr(state),
+                   _ptr(out), heads, key_dim, value_dim, _stream()))
 
 
 def group_rmsnorm(o: torch.Tensor, gain: torch.Tensor, eps: float, out: torch.Tensor, heads: int, value_dim: int) -> None:
