@@ -33,32 +33,64 @@ __device__ __forceinline__ float folded(const float* p, int n_partials, int64_t 
   return sum;
 }
 
-// proj [P][n][2 HD + HV]: columns q | f | v. act [n][3 HD + HV]: columns q | g | k | v.
-template <class TW>
-__global__ void hgrn2_activate_kernel(const float* __restrict__ proj, int n_partials, int64_t partial_stride, const TW* __restrict__ f_bias,
-                                      const TW* __restrict__ lower, float* __restrict__ act, int n, int HD, int HV) {
+__device__ __forceinline__ float4 folded4(const float* p, int n_partials, int64_t stride) {      // four neighbouring elements, 16-byte aligned
+  float4 part[kInFlight];
+#pragma unroll
+  for (int s = 0; s < kInFlight; ++s)
+    if (s < n_partials) part[s] = *reinterpret_cast<const float4*>(p + s * stride);
+  float4 sum = part[0];
+  auto add = [&](float4 a) { sum.x += a.x, sum.y += a.y, sum.z += a.z, sum.w += a.w; };
+#pragma unroll
+  for (int s = 1; s < kInFlight; ++s)
+    if (s < n_partials) add(part[s]);
+  for (int s = kInFlight; s < n_partials; ++s) add(*reinterpret_cast<const float4*>(p + s * stride));
+  return sum;
+}
+
+// proj [P][n][2 HD + HV]: columns q | f | v. act [n][3 HD + HV]: columns q | g | k | v. grid: (rows, pieces of a row). VE = 4: four elements
+// an access where the sizes and buffers allow it. Bound by memory: 1,250 rows of 16 heads of 128 | 128 18 us, 37 us with one element and a
+// 64-bit division a thread and round.
+template <class TW, int VE>
+__global__ void __launch_bounds__(128) hgrn2_activate_kernel(const float* __restrict__ proj, int n_partials, int64_t partial_stride,
+                                                             const TW* __restrict__ f_bias, const TW* __restrict__ lower, float* __restrict__ act, int HD, int HV) {
   sb::grid_launch_dependents();
-  sb::grid_dependency_wait();
-  const int in_w = 2 * HD + HV, out_w = 3 * HD + HV;
-  const int64_t total = static_cast<int64_t>(n) * in_w;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t r = i / in_w;
-    const int j = static_cast<int>(i % in_w);
-    const float z = folded(proj + i, n_partials, partial_stride);
-    float* row = act + r * out_w;
-    if (j < HD) {
-      row[j] = z / (1.0f + expf(-z));
-    } else if (j < 2 * HD) {
-      const int c = j - HD;
-      const float l = sb::widen(lower[c]);
-      const float s = 1.0f / (1.0f + expf(-(z + sb::widen(f_bias[c]))));
-      const float g = fmaf(1.0f - l, s, l);
-      row[HD + c] = g;
-      row[2 * HD + c] = 1.0f - g;
-    } else {
-      row[3 * HD + (j - 2 * HD)] = z;
-    }
+  const int in_w = 2 * HD + HV, j = (blockIdx.y * blockDim.x + threadIdx.x) * VE;
+  if (j >= in_w) return;
+  const bool gate = j >= HD && j < 2 * HD;
+  float l[VE], fb[VE], z[VE], g[VE];
+  if (gate) {
+#pragma unroll
+    for (int i = 0; i < VE; ++i) l[i] = sb::widen(lower[j - HD + i]), fb[i] = sb::widen(f_bias[j - HD + i]);
   }
+  sb::grid_dependency_wait();
+  const float* src = proj + static_cast<int64_t>(blockIdx.x) * in_w + j;
+  if constexpr (VE == 4) {
+    const float4 v = folded4(src, n_partials, partial_stride);
+    z[0] = v.x, z[1] = v.y, z[2] = v.z, z[3] = v.w;
+  } else {
+    z[0] = folded(src, n_partials, partial_stride);
+  }
+  auto store = [&](float* to, const float (&v)[VE]) {
+    if constexpr (VE == 4) *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]);
+    else to[0] = v[0];
+  };
+  float* row = act + static_cast<int64_t>(blockIdx.x) * (3 * HD + HV);
+  if (gate) {
+#pragma unroll
+    for (int i = 0; i < VE; ++i) {
+      const float s = 1.0f / (1.0f + expf(-(z[i] + fb[i])));
+      g[i] = fmaf(1.0f - l[i], s, l[i]);
+      z[i] = 1.0f - g[i];
+    }
+    store(row + j, g);
+    store(row + HD + j, z);
+    return;
+  }
+  if (j < HD) {
+#pragma unroll
+    for (int i = 0; i < VE; ++i) z[i] = z[i] / (1.0f + expf(-z[i]));
+  }
+  store(row + (j < HD ? j : HD + j), z);
 }
 
 // Steps in which every entry brings one token.
@@ -100,26 +132,27 @@ __global__ void group_rmsnorm_kernel(const float* __restrict__ o, const TW* __re
   for (int j = lane; j < V; j += 32) out[gidx * V + j] = sb::narrow<TO>(src[j] * scale * sb::widen(gain[j]));
 }
 
-inline int grid_for(int64_t total) {
-  const int64_t blocks = (total + 255) / 256, most = static_cast<int64_t>(sb::sm_count()) * 16;
-  return static_cast<int>(blocks < most ? blocks : most);
-}
-
 }  // namespace
 
 SB_EXPORT int sb_hgrn2_activate(const float* proj, int n_partials, int64_t partial_stride, const void* f_bias, const void* lower, int w_dtype,
                                 float* act, int n, int HD, int HV, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (n_partials < 1) return sb::fail("sb_hgrn2_activate: n_partials must be >= 1");
-  const int64_t total = static_cast<int64_t>(n) * (2 * HD + HV);
-  if (w_dtype == 0)
-    sb::launch_pdl(hgrn2_activate_kernel<float>, dim3(grid_for(total)), dim3(256), 0, stream, proj, n_partials, partial_stride,
-                   static_cast<const float*>(f_bias), static_cast<const float*>(lower), act, n, HD, HV);
-  else if (w_dtype == 1)
-    sb::launch_pdl(hgrn2_activate_kernel<bf16>, dim3(grid_for(total)), dim3(256), 0, stream, proj, n_partials, partial_stride,
-                   static_cast<const bf16*>(f_bias), static_cast<const bf16*>(lower), act, n, HD, HV);
-  else
+  const bool vec = HD % 4 == 0 && HV % 4 == 0 && partial_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(act)) & 15) == 0;
+  const dim3 grid(n, ((2 * HD + HV) / (vec ? 4 : 1) + 127) / 128);
+#define SB_ACT(TW, VE) \
+  sb::launch_pdl(hgrn2_activate_kernel<TW, VE>, grid, dim3(128), 0, stream, proj, n_partials, partial_stride, static_cast<const TW*>(f_bias), \
+                 static_cast<const TW*>(lower), act, HD, HV)
+  if (w_dtype == 0) {
+    if (vec) SB_ACT(float, 4);
+    else SB_ACT(float, 1);
+  } else if (w_dtype == 1) {
+    if (vec) SB_ACT(bf16, 4);
+    else SB_ACT(bf16, 1);
+  } else {
     return sb::fail("sb_hgrn2_activate: unsupported dtype %d", w_dtype);
+  }
+#undef SB_ACT
   return sb::check_launch("sb_hgrn2_activate");
 }
 

@@ -186,50 +186,83 @@ __global__ void __launch_bounds__(64) rmsnorm_rows_kernel(float* __restrict__ h,
 }
 
 // ------------------------------------------------------------------ layer norm
-// One block per row: x = h + (partial_0 + partial_1 + ...) as in rmsnorm_kernel (written back to h when partials are
-// given); mean = sum(x) / H; var = sum((x - mean)^2) / H, the deviations taken from the row kept in shared memory;
-// out = (x - mean) / sqrt(var + eps) * w + b. Both sums in the order of sb::block_sum, which the width alone decides.
-template <class TW, class TO>
-__global__ void __launch_bounds__(1024) layernorm_kernel(float* __restrict__ h, const float* __restrict__ partials, int n_partials,
+// One block per row: x = h + (partial_0 + partial_1 + ...) as in rmsnorm_kernel (written back to h when partials are given);
+// mean = sum(x) / H; var = sum((x - mean)^2) / H; out = (x - mean) / sqrt(var + eps) * w + b. Both sums in the order of sb::block_sum.
+// VEC = 4: four elements an access where the width and every buffer allow it; which form runs depends on the width and the buffers alone,
+// never on the rows, so a row's result does not either. A thread keeps its first kKeep pieces in registers through both sums; wider rows are
+// read again. Bound by memory: 2,048 rows of 2,048 with one partial buffer 22 us, single elements in shared memory 24 us.
+template <class TW, class TO, int VEC, int MAXT>     // MAXT: the most threads of a block, as in rmsnorm_kernel
+__global__ void __launch_bounds__(MAXT) layernorm_kernel(float* __restrict__ h, const float* __restrict__ partials, int n_partials,
                                                          int64_t partial_stride, const TW* __restrict__ weight,
                                                          const TW* __restrict__ bias, TO* __restrict__ out, int H, float eps) {
-  extern __shared__ __align__(16) float row[];
+  using V = typename VecF<VEC>::type;
+  constexpr int kKeep = 2;
   __shared__ float red[32];
   sb::grid_launch_dependents();
   sb::grid_dependency_wait();
   const int64_t r = blockIdx.x;
-  float* hr = h + r * H;
-  float sum = 0.0f;
-  for (int i = threadIdx.x; i < H; i += blockDim.x) {
-    float v = hr[i];
+  const int units = H / VEC;
+  V* hr = reinterpret_cast<V*>(h + r * H);
+  auto fetch = [&](int i) {
+    V v = hr[i];
     if (n_partials > 0) {
       constexpr int kInFlight = 8;
-      const float* p = partials + r * H + i;
-      float part[kInFlight];
+      const V* p = reinterpret_cast<const V*>(partials + r * H) + i;
+      const int64_t ps = partial_stride / VEC;
+      V part[kInFlight];
 #pragma unroll
       for (int s = 0; s < kInFlight; ++s)
-        if (s < n_partials) part[s] = p[s * partial_stride];
-      float ps = part[0];
+        if (s < n_partials) part[s] = p[s * ps];
+      V sum = part[0];
 #pragma unroll
       for (int s = 1; s < kInFlight; ++s)
-        if (s < n_partials) ps += part[s];
-      for (int s = kInFlight; s < n_partials; ++s) ps += p[s * partial_stride];
-      v += ps;
+        if (s < n_partials) sum = add4(sum, part[s]);
+      for (int s = kInFlight; s < n_partials; ++s) sum = add4(sum, p[s * ps]);
+      v = add4(v, sum);
       hr[i] = v;
     }
-    row[i] = v;
-    sum += v;
-  }
+    return v;
+  };
+  auto total = [](V v) {
+    if constexpr (VEC == 4) return ((v.x + v.y) + v.z) + v.w;
+    else return v;
+  };
+  auto apart = [](V v, float mean, float sq) {
+    if constexpr (VEC == 4) {
+      const float x = v.x - mean, y = v.y - mean, z = v.z - mean, w = v.w - mean;
+      return fmaf(w, w, fmaf(z, z, fmaf(y, y, fmaf(x, x, sq))));
+    } else {
+      return fmaf(v - mean, v - mean, sq);
+    }
+  };
+  const int beyond = kKeep * blockDim.x + threadIdx.x;
+  V keep[kKeep];
+  float sum = 0.0f;
+#pragma unroll
+  for (int j = 0; j < kKeep; ++j)
+    if (threadIdx.x + j * blockDim.x < units) sum += total(keep[j] = fetch(threadIdx.x + j * blockDim.x));
+  for (int i = beyond; i < units; i += blockDim.x) sum += total(fetch(i));
   const float mean = sb::block_sum(sum, red) / static_cast<float>(H);
   float sq = 0.0f;
-  for (int i = threadIdx.x; i < H; i += blockDim.x) {
-    const float d = row[i] - mean;
-    sq = fmaf(d, d, sq);
-  }
+#pragma unroll
+  for (int j = 0; j < kKeep; ++j)
+    if (threadIdx.x + j * blockDim.x < units) sq = apart(keep[j], mean, sq);
+  for (int i = beyond; i < units; i += blockDim.x) sq = apart(hr[i], mean, sq);
   const float scale = 1.0f / sqrtf(sb::block_sum(sq, red) / static_cast<float>(H) + eps);
-  TO* o = out + r * H;
-  for (int i = threadIdx.x; i < H; i += blockDim.x)
-    o[i] = sb::narrow<TO>(fmaf((row[i] - mean) * scale, sb::widen(weight[i]), bias != nullptr ? sb::widen(bias[i]) : 0.0f));
+  auto write = [&](int i, V v) {
+    if constexpr (VEC == 4) {
+      const float4 w = load_gain4(weight, sizeof(TW) == 2, 4 * i), b = bias != nullptr ? load_gain4(bias, sizeof(TW) == 2, 4 * i) : make_float4(0, 0, 0, 0);
+      const float4 o = make_float4(fmaf((v.x - mean) * scale, w.x, b.x), fmaf((v.y - mean) * scale, w.y, b.y), fmaf((v.z - mean) * scale, w.z, b.z),
+                                   fmaf((v.w - mean) * scale, w.w, b.w));
+      store_normed4<TO>(out + r * H + 4 * i, o, make_float4(1, 1, 1, 1), 1.0f);
+    } else {
+      out[r * H + i] = sb::narrow<TO>(fmaf((v - mean) * scale, sb::widen(weight[i]), bias != nullptr ? sb::widen(bias[i]) : 0.0f));
+    }
+  };
+#pragma unroll
+  for (int j = 0; j < kKeep; ++j)
+    if (threadIdx.x + j * blockDim.x < units) write(threadIdx.x + j * blockDim.x, keep[j]);
+  for (int i = beyond; i < units; i += blockDim.x) write(i, hr[i]);
 }
 
 }  // namespace
@@ -238,14 +271,18 @@ __global__ void __launch_bounds__(1024) layernorm_kernel(float* __restrict__ h, 
 SB_EXPORT int sb_layernorm(float* h, const float* partials, int n_partials, int64_t partial_stride, const void* weight,
                            const void* bias, int weight_dtype, void* out, int out_dtype, int n, int H, float eps, cudaStream_t stream) {
   if (n <= 0) return 0;
-  const size_t smem = static_cast<size_t>(H) * sizeof(float);
-  if (smem > 200 * 1024) return sb::fail("sb_layernorm: width %d does not fit the row buffer (max 51200)", H);
-  const int threads = H >= 4096 ? 1024 : H >= 2048 ? 512 : H >= 512 ? 256 : 128;
-#define SB_LN(TW, TO)                                                                                                       \
-  do {                                                                                                                      \
-    if (smem > 48 * 1024) cudaFuncSetAttribute(layernorm_kernel<TW, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    sb::launch_pdl(layernorm_kernel<TW, TO>, n, threads, smem, stream, h, partials, n_partials, partial_stride,             \
-                   static_cast<const TW*>(weight), static_cast<const TW*>(bias), static_cast<TO*>(out), H, eps);            \
+  if (H > 50 * 1024) return sb::fail("sb_layernorm: width %d does not fit the row buffer (max 51200)", H);
+  auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  const bool vec = H % 4 == 0 && aligned(h) && aligned(partials) && aligned(weight) && aligned(bias) && aligned(out) && partial_stride % 4 == 0;
+  const int units = vec ? H / 4 : H, threads = units > 1024 ? 1024 : units > 512 ? 512 : units > 256 ? 256 : 128;
+#define SB_LN_V(TW, TO, VEC, MAXT)                                                                                            \
+  sb::launch_pdl(layernorm_kernel<TW, TO, VEC, MAXT>, n, threads, 0, stream, h, partials, n_partials, partial_stride,         \
+                 static_cast<const TW*>(weight), static_cast<const TW*>(bias), static_cast<TO*>(out), H, eps)
+#define SB_LN(TW, TO)                                  \
+  do {                                                 \
+    if (vec && threads <= 512) SB_LN_V(TW, TO, 4, 512); \
+    else if (vec) SB_LN_V(TW, TO, 4, 1024);            \
+    else SB_LN_V(TW, TO, 1, 1024);                     \
   } while (0)
   if (weight_dtype == 0 && out_dtype == 0) SB_LN(float, float);
   else if (weight_dtype == 0 && out_dtype == 1) SB_LN(float, bf16);
@@ -253,6 +290,7 @@ SB_EXPORT int sb_layernorm(float* h, const float* partials, int n_partials, int6
   else if (weight_dtype == 1 && out_dtype == 1) SB_LN(bf16, bf16);
   else return sb::fail("sb_layernorm: unsupported dtypes weight=%d out=%d", weight_dtype, out_dtype);
 #undef SB_LN
+#undef SB_LN_V
   return sb::check_launch("sb_layernorm");
 }
 

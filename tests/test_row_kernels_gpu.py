@@ -1,0 +1,93 @@
+"""Edges of the kernels that walk a step's rows: sizes at which a thread holds its whole share in registers and just beyond, sizes without
+16-byte accesses, and the numbers of tokens at which another form of a kernel takes over (equal bits: a token does not show its step)."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("H", [4, 127, 2048, 2052, 8192, 8196, 10240, 2050])
+def test_layer_norm_at_the_edges_of_a_thread(H):
+    """Against 64 bits. The bound is 2e-6 of the largest value: sixteen roundings of a 32-bit result (three partial sums, two means, the scale)."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(H)
+    h, parts = torch.randn(5, H, generator=g) * 2 + 0.5, torch.randn(3, 5, H, generator=g)
+    w, b = torch.randn(H, generator=g), torch.randn(H, generator=g)
+    out, hd = torch.empty(5, H, device=DEV), h.to(DEV)
+    ops.layernorm(hd, w.to(DEV), b.to(DEV), 1e-5, out, partials=parts.to(DEV))
+    x = h.double() + parts.double().sum(0)
+    d = x - x.mean(-1, keepdim=True)
+    want = d / torch.sqrt((d * d).mean(-1, keepdim=True) + 1e-5) * w.double() + b.double()
+    assert (out.cpu().double() - want).abs().max() <= 2e-6 * float(want.abs().max())
+    assert (hd.cpu().double() - x).abs().max() <= 1e-6 * float(x.abs().max())
+    alone = torch.empty(1, H, device=DEV)
+    ops.layernorm(h[3:4].to(DEV), w.to(DEV), b.to(DEV), 1e-5, alone, partials=parts[:, 3:4].contiguous().to(DEV))
+    assert torch.equal(alone[0], out[3])
+
+
+@pytest.mark.parametrize("F", [5, 1020, 8192, 8196, 9001, 12288])
+def test_polynorm_at_the_edges_of_a_thread(F):
+    """Against 64 bits, within 4e-6 of the largest value (six partial sums, cubed: their roundings three times over, a mean, the result's own)."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(F)
+    up = torch.randn(6, 4, F, generator=g) * 0.4                     # (more partial buffers than are requested together)
+    a, b, c, e = 0.7, -0.3, 0.2, 0.05
+    out = torch.empty(4, F, device=DEV)
+    ops.polynorm(up.to(DEV), out, (a, b, c, e), 1e-5)
+    z = up.double().sum(0)
+    n = lambda y: y / torch.sqrt((y * y).mean(-1, keepdim=True) + 1e-5)
+    want = a * n(z) + b * n(z ** 2) + c * n(z ** 3) + e
+    assert (out.cpu().double() - want).abs().max() <= 4e-6 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("bw,B", [(128, 2), (100, 3), (10, 2), (33, 1), (260, 1)])
+def test_gates_do_not_show_the_number_of_tokens(bw, B):
+    """Both kernels of the gates, and one and four rows a block of the convolution: the bits of 1 to 257 tokens in those of 300."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(bw)
+    C, n, K = bw * B, 300, 4
+    dev = lambda *s, k=0.3: (torch.randn(*s, generator=g) * k).to(DEV)
+    proj = dev(2, n, 2 * C)
+    xb, yb, rb, ib, lam, taps, cb = dev(C), dev(C), dev(C), dev(C), dev(C) - 3.0, dev(C, K), dev(C)
+    gate_w = dev(B, bw, 2 * bw).bfloat16()
+    pos, slot = torch.arange(n, dtype=torch.int32, device=DEV), torch.zeros(n, dtype=torch.int32, device=DEV)
+    state = torch.zeros(1, K, C, device=DEV)
+
+    def run(m):
+        p = proj[:, :m].contiguous()
+        u, a, d, y = (torch.empty(m, C, device=DEV) for _ in range(4))
+        ops.rglru_conv(p, xb, taps, cb, pos[:m], slot[:m], state, u)
+        ops.rglru_gates(gate_w, rb, ib, lam, yb, u, p, a, d, y)
+        return u, a, d, y
+
+    whole = run(n)
+    for m in (1, 8, 128, 129, 257):
+        for x, w in zip(run(m), whole):
+            assert torch.equal(x, w[:m]), m
+
+
+@pytest.mark.parametrize("D,rot", [(64, 32), (64, 8), (24, 8), (64, 64), (20, 4), (64, 0)])
+def test_rotation_of_a_part_of_the_head(D, rot):
+    """The 16-byte form (head and rotated part multiples of eight) and the single-element one against the rotation itself, in 32 bits."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(D + rot)
+    n, Hq, Hkv, page = 7, 5, 2, 16
+    qk = torch.randn(2, n, (Hq + Hkv) * D, generator=g)
+    pos = torch.arange(3, 3 + n, dtype=torch.int32)
+    angle = pos.float()[:, None] * torch.rand(max(rot // 2, 1), generator=g)[None]
+    table = torch.zeros(16, max(rot // 2, 1), 2)
+    table[3:3 + n] = torch.stack([angle.cos(), angle.sin()], -1)
+    q_out = torch.empty(n, Hq * D, device=DEV)
+    cache = torch.zeros(2, 2, Hkv, page, D, device=DEV)
+    ops.rope_append(qk.to(DEV), pos.to(DEV), torch.zeros(n, dtype=torch.int32, device=DEV), table.to(DEV), rot, q_out, cache,
+                    torch.tensor([[1]], dtype=torch.int32, device=DEV), Hq, Hkv, D, values_from_keys=True)
+    x = qk.sum(0).view(n, Hq + Hkv, D)
+    c, s = angle.cos()[:, None, :rot // 2], angle.sin()[:, None, :rot // 2]
+    u, v = x[..., :rot // 2], x[..., rot // 2:rot]
+    turned = torch.cat([u * c - v * s, v * c + u * s, x[..., rot:]], -1)
+    assert (q_out.cpu() - turned[:, :Hq].reshape(n, -1)).abs().max() <= 1e-5
+    assert (cache[1, 0, :, 3:3 + n].cpu().transpose(0, 1) - turned[:, Hq:]).abs().max() <= 1e-5
+    assert torch.equal(cache[1, 1, :, 3:3 + n].cpu().transpose(0, 1), x[:, Hq:])
