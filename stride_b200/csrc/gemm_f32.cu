@@ -7,9 +7,9 @@
 // class is one chain of fused multiply-adds over its elements in ascending k (from zero), and the 32 classes are added
 // by the butterfly of a warp (xor 16, 8, 4, 2, 1). A warp computes TM features by TN tokens; lane c is class c: it reads
 // its pieces of the weight rows (16 bytes of bfloat16 at once, the 32 lanes 512 consecutive bytes) and of the tokens.
-// One token is then a stream over the weights (gemv_f32_kernel below). With one dependent chain per output, the order
+// A few tokens are then a stream over the weights (gemv_f32_kernel below). With one dependent chain per output, the order
 // before this one, the latency of K fused multiply-adds bounded it: 5 ms a decoded token at the sizes of Llama 3.2 1B,
-// 1.07 ms now.
+// 0.90 ms now.
 //
 // Counterparts in arhaamatiq/stride: gemm_partial and its users GemmResidual,
 // Mlp13, LmFull of the exact path (src/kernels.cu:63-94, 294-325, 329-363, 427-452), which add 32 interleaved
@@ -139,162 +139,172 @@ void launch(const void* x, int64_t ldx, const void* w, int64_t ldw, float* out, 
                  static_cast<const TW*>(w), ldw, out, ldo, n, M, K, accumulate);
 }
 
-// Eight consecutive values as they lie in memory (16 bytes of bfloat16, 32 of float32), widened when they are used:
-// what a lane keeps in flight of a weight row costs half the registers for bfloat16.
-template <class T>
-struct Raw8;
-template <>
-struct Raw8<bf16> {
-  uint4 v;
-  __device__ __forceinline__ void load(const bf16* p) { v = *reinterpret_cast<const uint4*>(p); }
-  __device__ __forceinline__ void widen(float* f) const {
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+// Eight consecutive weights in shared memory (16 bytes of bfloat16, 32 of float32), widened.
+__device__ __forceinline__ void widen8(const bf16* p, float* f) {
+  const uint4 v = *reinterpret_cast<const uint4*>(p);
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) f[2 * i] = __uint_as_float(w[i] << 16), f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-  }
-};
-template <>
-struct Raw8<float> {
-  float4 a, b;
-  __device__ __forceinline__ void load(const float* p) { a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4); }
-  __device__ __forceinline__ void widen(float* f) const {
-    f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
-  }
-};
+  for (int i = 0; i < 4; ++i) f[2 * i] = __uint_as_float(w[i] << 16), f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+}
+__device__ __forceinline__ void copy16_async(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
+}
 
-// One token (a decoded token's linear layers): the token lies in shared memory and the weights are one stream. As many
-// blocks as the GPU holds at once; warp g of all G takes the features g, g + G, g + 2G, ... and keeps NG groups of
-// P pieces of their rows requested (a group is requested again as soon as it has been multiplied), across the end of
-// a row into the next one, so that the requests in flight do not drain at every feature. The additions of a feature are those of the kernel above. K is a multiple of 8, rows 16-byte aligned.
-template <class TX, class TW, int TM, int NG, int P>
-__global__ void __launch_bounds__(kWarps * 32) gemv_f32_kernel(const TX* __restrict__ x, const TW* __restrict__ w, int64_t ldw,
-                                                                float* __restrict__ out, int M, int K, int accumulate) {
-  // The token, piece by piece: a piece's first four values of all 32 lanes, then its last four (a lane reads its
-  // eight with two requests of 16 bytes, each of them consecutive over the lanes). Padded to whole pieces of 256.
+// A few tokens (a decoded token's linear layers): the tokens lie in shared memory and the weights are one stream. Blocks of sixteen
+// warps; warp g of all G takes the features g, g + G, g + 2G, ... and keeps STAGES groups of kPieces pieces of their rows on their way into a
+// ring of its own in shared memory (asynchronous copies: a lane copies what it will multiply, so that no lane waits for another), across the
+// end of a row into the next one; a group's place is requested again as soon as it has been multiplied. The additions of a feature are those
+// of the kernel above. K is a multiple of 8, rows 16-byte aligned.
+//
+// The bound is HBM: what is in flight has to cover its latency, 128 to 192 KB an SM here, requested before the wait for the kernel in front.
+// In registers a warp kept half as much, drained at every wait, and a second kernel's requests began only when the first had ended. Measured
+// with bfloat16 weights, one token, before -> now: 16384 x 2048 17.0 -> 13.6 us, 128256 x 2048 106 -> 88,
+// 2048 x 8192 13.8 -> 10.2; within a step of the 1B sizes 17.1 -> 14.7 and 13.7 -> 8.6.
+constexpr int kStreamWarps = 16, kPieces = 4;
+template <class TX, class TW, int NT, int STAGES>
+__global__ void __launch_bounds__(kStreamWarps * 32) gemv_f32_kernel(const TX* __restrict__ x, int64_t ldx, const TW* __restrict__ w, int64_t ldw,
+                                                                      float* __restrict__ out, int64_t ldo, int n, int M, int K, int accumulate) {
+  // The tokens, piece by piece: a piece's first four values of all 32 lanes, then its last four (a lane reads its
+  // eight with two requests of 16 bytes, each of them consecutive over the lanes). Padded to whole pieces of 256. Behind them the rings.
   extern __shared__ __align__(16) float xs[];
+  constexpr int kLane = 8 * sizeof(TW);                // bytes of a lane's share of a piece
   sb::grid_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = blockIdx.x * kWarps + warp, G = gridDim.x * kWarps;
-  const int pieces = (K + 255) >> 8;  // of a row, for a lane (the last may lie beyond K for the upper lanes)
-  const int groups = (M + TM - 1) / TM;  // of TM features; warp g takes the groups g, g + G, ...
-  const int mine = g < groups ? (groups - g + G - 1) / G : 0;
-  const int total = mine * pieces;
-  const int kl = lane * 8;
-
-  Raw8<TW> ring[NG][P][TM];
-  int next_group = 0, next_piece = 0;  // the piece that is requested next
+  const int g = warp * gridDim.x + blockIdx.x, G = gridDim.x * kStreamWarps;      // (the first features spread over all SMs)
+  const int pieces = (K + 255) >> 8;                   // of a row, for a lane (the last may lie beyond K for the upper lanes)
+  const int mine = g < M ? (M - g + G - 1) / G : 0, total = mine * pieces;
+  const int kl = lane * 8, Kp = pieces * 256;
+  char* ring = reinterpret_cast<char*>(xs + NT * Kp) + warp * (STAGES * kPieces * 32 * kLane);
+  int next_row = 0, next_piece = 0;                    // the piece that is requested next
   auto request = [&](int h) {
 #pragma unroll
-    for (int s = 0; s < P; ++s)
-      if (next_group < mine) {
+    for (int s = 0; s < kPieces; ++s)
+      if (next_row < mine) {
         const int k = kl + 256 * next_piece;
         if (k < K) {
-          const int m = (g + next_group * G) * TM;
-#pragma unroll
-          for (int i = 0; i < TM; ++i) ring[h][s][i].load(w + static_cast<int64_t>(min(m + i, M - 1)) * ldw + k);  // beyond M: read, not stored
+          const TW* src = w + static_cast<int64_t>(g + next_row * G) * ldw + k;
+          char* dst = ring + (h * kPieces + s) * 32 * kLane + lane * 16;
+          copy16_async(dst, src);
+          if constexpr (kLane == 32) copy16_async(dst + 512, src + 4);
         }
-        if (++next_piece == pieces) next_piece = 0, ++next_group;
+        if (++next_piece == pieces) next_piece = 0, ++next_row;
       }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
   // the weights do not depend on the kernels before this one
 #pragma unroll
-  for (int h = 0; h < NG; ++h) request(h);
+  for (int h = 0; h < STAGES; ++h) request(h);
   sb::grid_dependency_wait();
-#pragma unroll 4
-  for (int k = threadIdx.x * 8; k < K; k += kWarps * 32 * 8) {
-    float v[8];
-    load8<true>(x + k, 8, v);
-    float* at = xs + (k & ~255) + ((k >> 3) & 31) * 4;
-    *reinterpret_cast<float4*>(at) = make_float4(v[0], v[1], v[2], v[3]);
-    *reinterpret_cast<float4*>(at + 128) = make_float4(v[4], v[5], v[6], v[7]);
-  }
+#pragma unroll
+  for (int t = 0; t < NT; ++t)
+    for (int k = threadIdx.x * 8; k < K; k += kStreamWarps * 32 * 8) {
+      float v[8];
+      load8<true>(x + min(t, n - 1) * ldx + k, 8, v);
+      float* at = xs + t * Kp + (k & ~255) + ((k >> 3) & 31) * 4;
+      *reinterpret_cast<float4*>(at) = make_float4(v[0], v[1], v[2], v[3]);
+      *reinterpret_cast<float4*>(at + 128) = make_float4(v[4], v[5], v[6], v[7]);
+    }
   __syncthreads();
 
-  float acc[TM];
+  float acc[NT];
 #pragma unroll
-  for (int i = 0; i < TM; ++i) acc[i] = 0.0f;
-  int group = 0, piece = 0;  // the piece that is multiplied next
-  for (int q = 0; q < total; q += NG * P) {
+  for (int t = 0; t < NT; ++t) acc[t] = 0.0f;
+  int m = g, piece = 0, h = 0;                         // the piece that is multiplied next
+  for (int q = 0; q < total; q += kPieces) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
 #pragma unroll
-    for (int h = 0; h < NG; ++h) {
-#pragma unroll
-      for (int s = 0; s < P; ++s) {
-        if (q + h * P + s < total) {
-          if (kl + 256 * piece < K) {
-            const float4 xa = *reinterpret_cast<const float4*>(xs + 256 * piece + lane * 4);
-            const float4 xb = *reinterpret_cast<const float4*>(xs + 256 * piece + 128 + lane * 4);
-            const float xv[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-            float wv[TM][8];
-#pragma unroll
-            for (int i = 0; i < TM; ++i) ring[h][s][i].widen(wv[i]);
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-#pragma unroll
-              for (int i = 0; i < TM; ++i) acc[i] = fmaf(xv[e], wv[i][e], acc[i]);
+    for (int s = 0; s < kPieces; ++s)
+      if (q + s < total) {
+        if (kl + 256 * piece < K) {
+          const char* at = ring + (h * kPieces + s) * 32 * kLane + lane * 16;
+          float wv[8];
+          if constexpr (kLane == 16) {
+            widen8(reinterpret_cast<const bf16*>(at), wv);
+          } else {
+            const float4 a = *reinterpret_cast<const float4*>(at), b = *reinterpret_cast<const float4*>(at + 512);
+            wv[0] = a.x, wv[1] = a.y, wv[2] = a.z, wv[3] = a.w, wv[4] = b.x, wv[5] = b.y, wv[6] = b.z, wv[7] = b.w;
           }
-          if (++piece == pieces) {
-            const int m = (g + group * G) * TM;
 #pragma unroll
-            for (int i = 0; i < TM; ++i) {
-              float v = acc[i];
+          for (int t = 0; t < NT; ++t) {
+            const float* xt = xs + t * Kp + 256 * piece + lane * 4;
+            const float4 a = *reinterpret_cast<const float4*>(xt), b = *reinterpret_cast<const float4*>(xt + 128);
+            const float xv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-              for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-              if (lane == i && m + i < M) out[m + i] = accumulate ? (out[m + i] + v) : v;
-              acc[i] = 0.0f;
-            }
-            piece = 0, ++group;
+            for (int e = 0; e < 8; ++e) acc[t] = fmaf(xv[e], wv[e], acc[t]);
           }
         }
+        if (++piece == pieces) {
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            float v = acc[t];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == t && t < n) {
+              float* dst = out + static_cast<int64_t>(t) * ldo + m;
+              *dst = accumulate ? (*dst + v) : v;
+            }
+            acc[t] = 0.0f;
+          }
+          piece = 0, m += G;
+        }
       }
-      request(h);
-    }
+    request(h);
+    h = h + 1 == STAGES ? 0 : h + 1;
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-constexpr int kGemvFeatures = 1, kGemvPieces = 4;
-constexpr size_t kGemvMaxShared = 200 * 1024;
-inline size_t gemv_shared(int K) { return static_cast<size_t>((K + 255) / 256) * 256 * sizeof(float); }
+constexpr size_t kStreamMaxShared = 224 * 1024;
+template <class TW>
+inline size_t stream_shared(int tokens, int K, int stages) {
+  return static_cast<size_t>(tokens) * ((K + 255) / 256) * 256 * sizeof(float) + static_cast<size_t>(kStreamWarps) * stages * kPieces * 32 * 8 * sizeof(TW);
+}
 
-template <class TX, class TW, int NG>
-void launch_gemv_groups(const void* x, const void* w, int64_t ldw, float* out, int M, int K, int accumulate, cudaStream_t stream) {
-  auto kernel = gemv_f32_kernel<TX, TW, kGemvFeatures, NG, kGemvPieces>;
-  const size_t smem = gemv_shared(K);
+template <class TX, class TW, int NT, int STAGES>
+void launch_stream_of(const void* x, int64_t ldx, const void* w, int64_t ldw, float* out, int64_t ldo, int n, int M, int K, int accumulate, int blocks, cudaStream_t stream) {
+  auto kernel = gemv_f32_kernel<TX, TW, NT, STAGES>;
   static sb::DeviceOnce once;
   if (once.needed()) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemvMaxShared));
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kStreamMaxShared));
     once.done();
   }
-  int resident = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kWarps * 32, smem) != cudaSuccess || resident < 1) resident = 1;
-  const int per_block = kWarps * kGemvFeatures;
-  const int blocks = std::min((M + per_block - 1) / per_block, resident * sb::sm_count());
-  sb::launch_pdl(kernel, dim3(blocks), dim3(kWarps * 32), smem, stream, static_cast<const TX*>(x), static_cast<const TW*>(w), ldw, out, M, K,
-                 accumulate);
+  sb::launch_pdl(kernel, dim3(std::min(M, blocks)), dim3(kStreamWarps * 32), stream_shared<TW>(NT, K, STAGES), stream, static_cast<const TX*>(x), ldx,
+                 static_cast<const TW*>(w), ldw, out, ldo, n, M, K, accumulate);
 }
 
-// Measured on a B200 with bfloat16 weights, microseconds. A feature per warp and two groups: 16384 x 2048 17.8,
-// 128256 x 2048 106, 2048 x 8192 16.5. Four groups: 20.6, 155, 13.9: with few features (fewer warps than the GPU holds)
-// every warp has to keep more requested; with many, more warps do better than more requests a warp. Two features a
-// warp (fewer instructions a byte, half the warps): 19.2, 137, 22.8.
-template <class TX, class TW>
-void launch_gemv(const void* x, const void* w, int64_t ldw, float* out, int M, int K, int accumulate, cudaStream_t stream) {
-  if ((M + kWarps - 1) / kWarps < 4 * sb::sm_count()) launch_gemv_groups<TX, TW, 4>(x, w, ldw, out, M, K, accumulate, stream);
-  else launch_gemv_groups<TX, TW, 2>(x, w, ldw, out, M, K, accumulate, stream);
+// Up to a feature a warp: one block an SM whose warps keep five groups requested (most of a row). More features: two blocks an SM, that is
+// 32 warps and 192 KB on their way, where the tokens leave the room (one block of 16 warps: 23 us for 16384 x 2048 within a step; two blocks
+// with two groups a warp 18.5; with three 13.9). Blocks of more than half an SM are launched once an SM.
+template <class TX, class TW, int NT>
+bool launch_stream(const void* x, int64_t ldx, const void* w, int64_t ldw, float* out, int64_t ldo, int n, int M, int K, int accumulate, cudaStream_t stream) {
+  const int sms = sb::sm_count();
+  auto fits = [&](int stages, int kilobytes) { return stream_shared<TW>(NT, K, stages) <= static_cast<size_t>(kilobytes) * 1024; };
+#define SB_STREAM(STAGES, BLOCKS) launch_stream_of<TX, TW, NT, STAGES>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, BLOCKS, stream)
+  if (M <= kStreamWarps * sms && fits(5, 200)) SB_STREAM(5, sms);
+  else if (fits(3, 108)) SB_STREAM(3, 2 * sms);
+  else if (fits(2, 108)) SB_STREAM(2, 2 * sms);
+  else if (fits(3, 200)) SB_STREAM(3, sms);
+  else if (stream_shared<TW>(NT, K, 2) <= kStreamMaxShared) SB_STREAM(2, sms);
+  else return false;
+#undef SB_STREAM
+  return true;
 }
 
-// The warp's tile by the number of tokens: one token is a stream over the weights with a feature per warp (the most
-// warps, the most bytes in flight); a few tokens share the weights a warp reads; many tokens also share the tokens' pieces
-// among four features. Every shape adds in the same order.
+// The warp's tile by the number of tokens: up to four are a stream over the weights with a feature per warp; more tokens share the weights
+// a warp reads, many also the tokens' pieces among four features. Every shape adds in the same order.
 template <class TX, class TW, bool VEC>
 void dispatch(const void* x, int64_t ldx, const void* w, int64_t ldw, float* out, int64_t ldo, int n, int M, int K, int accumulate,
               cudaStream_t stream) {
   if (!VEC) return launch<TX, TW, false, 1, 4, 1>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream);
-  if (n == 1 && gemv_shared(K) <= kGemvMaxShared) return launch_gemv<TX, TW>(x, w, ldw, out, M, K, accumulate, stream);
+  if (n == 1 && launch_stream<TX, TW, 1>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream)) return;
   if (n == 1) return launch<TX, TW, true, 1, 1, 4>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream);
   // few outputs (a router's product): as many warps as there are outputs, or a quarter of that, rather than a few that share operands
   // (9 x 2048, 8 and 64 tokens: 30 and 21 us with the shapes below)
   const long long outputs = static_cast<long long>(M) * n, sms = sb::sm_count();
   if (outputs < 16 * sms) return launch<TX, TW, true, 1, 1, 4>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream);
+  // (16384 x 2048, four tokens: 26 us as a stream, 45 with the tile below, which reads the tokens again for every piece)
+  if (n == 2 && launch_stream<TX, TW, 2>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream)) return;
+  if ((n == 3 || n == 4) && launch_stream<TX, TW, 4>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream)) return;
   if (n <= 4 || outputs < 64 * sms) return launch<TX, TW, true, 1, 4, 2>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream);
   if (n <= 16) return launch<TX, TW, true, 2, 8, 1>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream);
   return launch<TX, TW, true, 4, 8, 1>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream);

@@ -91,3 +91,23 @@ def test_rotation_of_a_part_of_the_head(D, rot):
     assert (q_out.cpu() - turned[:, :Hq].reshape(n, -1)).abs().max() <= 1e-5
     assert (cache[1, 0, :, 3:3 + n].cpu().transpose(0, 1) - turned[:, Hq:]).abs().max() <= 1e-5
     assert torch.equal(cache[1, 1, :, 3:3 + n].cpu().transpose(0, 1), x[:, Hq:])
+
+
+@pytest.mark.parametrize("M,K", [(1, 8), (149, 264), (2369, 248), (5000, 2056), (4737, 8192), (40, 12288)])
+@pytest.mark.parametrize("wdtype", [torch.bfloat16, torch.float32])
+def test_a_few_tokens_as_a_stream_over_the_weights(M, K, wdtype):
+    """One to four tokens, features around the number of warps, rows that end within a piece: the bits of the tiles that many tokens take, and
+    64 bits within K roundings of the sum of the products' magnitudes."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(M + K)
+    w, x = (torch.randn(M, K, generator=g) * 0.1).to(wdtype).to(DEV), torch.randn(40, K, generator=g).to(DEV)
+    tiles = torch.empty(40, M, device=DEV)
+    ops.gemm_f32(x, w, tiles)
+    for n in (1, 2, 3, 4):
+        out = torch.full((n, M), 0.5, device=DEV)
+        ops.gemm_f32(x[:n].contiguous(), w, out)
+        assert torch.equal(out, tiles[:n])
+        ops.gemm_f32(x[:n].contiguous(), w, out, accumulate=True)
+        assert torch.equal(out, tiles[:n] + tiles[:n])
+    xd, wd = x[:4].double(), w.double()
+    assert ((tiles[:4].double() - xd @ wd.T).abs() <= (K / 32 + 40) * 2.0 ** -24 * (xd.abs() @ wd.abs().T)).all()
