@@ -152,14 +152,15 @@ struct GateParams {
   int n, C, bw;
 };
 
-__device__ __forceinline__ void gate_outputs(const GateParams& p, int t, int c, float sr, float si, float ut, float rb, float ib, float softplus, float yb) {
-  const int64_t i = static_cast<int64_t>(t) * p.C + c;
+struct GateValues {
+  float a, d, y;
+};
+// z: the y projection's sum (no bias yet)
+__device__ __forceinline__ GateValues gate_values(float sr, float si, float ut, float z, float rb, float ib, float softplus, float yb) {
   const float rg = 1.0f / (1.0f + expf(-(sr + rb)));
   const float ig = 1.0f / (1.0f + expf(-(si + ib)));
   const float log_a = -8.0f * rg * softplus;
-  p.a[i] = expf(log_a);
-  p.d[i] = sqrtf(-expm1f(2.0f * log_a)) * (ig * ut);
-  p.y[i] = gelu_tanh(folded(p.proj.p + static_cast<int64_t>(t) * 2 * p.C + c, p.proj.n_partials, p.proj.stride) + yb);
+  return {expf(log_a), sqrtf(-expm1f(2.0f * log_a)) * (ig * ut), gelu_tanh(z + yb)};
 }
 __device__ __forceinline__ float softplus_of(float l) { return l > 20.0f ? l : log1pf(expf(l)); }
 
@@ -219,15 +220,20 @@ __global__ void __launch_bounds__(kQuarters * 2 * kFewOutputs) rglru_gates_few_k
   float sr = red[0][0][ct][lane], si = red[0][1][ct][lane];
 #pragma unroll
   for (int q = 1; q < kQuarters; ++q) sr += red[q][0][ct][lane], si += red[q][1][ct][lane];
-  gate_outputs(p, t0 + ct, c, sr, si, us[j * kFewTokens + ct], rb, ib, softplus, yb);
+  const float z = folded(p.proj.p + static_cast<int64_t>(t0 + ct) * 2 * p.C + c, p.proj.n_partials, p.proj.stride);
+  const GateValues v = gate_values(sr, si, us[j * kFewTokens + ct], z, rb, ib, softplus, yb);
+  const int64_t i = static_cast<int64_t>(t0 + ct) * p.C + c;
+  p.a[i] = v.a, p.d[i] = v.d, p.y[i] = v.y;
 }
 
 // Many tokens: a CTA is (32 tokens, block of channels, 64 of its channels), a warp four tokens, a lane two channels with both gates: 16
-// sums a thread for one read of the tokens' inputs and two of the weights a k, both staged in shared memory 32 inputs at a time. A thread
-// has whole sums (quarter after quarter) and so makes its outputs without an exchange. 1,250 tokens of 16 blocks of 128: 131 us, 167 us as
-// one channel of 16 tokens a thread with its weights from global memory.
+// sums a thread for one read of the tokens' inputs and two of the weights a k, both staged in shared memory 32 inputs at a time, the next
+// tile's on their way in registers meanwhile. A thread has whole sums (quarter after quarter) and so makes its outputs without an exchange,
+// its inputs requested together in front of them. VEC: 16-byte requests (blocks of a multiple of 16 channels, aligned buffers).
+// 1,250 tokens of 16 blocks of 128: 59 us; 167 us as one channel of 16 tokens a thread with its weights from global memory, 131 us as
+// here but with single-element requests that nothing overlapped.
 constexpr int kManyTokens = 32, kManyOutputs = 64, kManyInputs = 32;
-template <class TG>
+template <class TG, bool VEC>
 __global__ void __launch_bounds__(256) rglru_gates_kernel(const TG* __restrict__ gate_w, GateParams p) {
   __shared__ __align__(16) float ws[kManyInputs][2][kManyOutputs];
   __shared__ __align__(16) float us[kManyInputs][kManyTokens + 4];     // (rows of 16-byte pieces that start at different banks)
@@ -236,11 +242,54 @@ __global__ void __launch_bounds__(256) rglru_gates_kernel(const TG* __restrict__
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tg = warp * 4;
   const int per = (bw + kQuarters - 1) / kQuarters;
   const TG* w = gate_w + static_cast<int64_t>(b) * bw * 2 * bw;
+  const float* u = p.u + b * bw;
+  constexpr int kN = VEC ? 16 / sizeof(TG) : 1;                        // weights a request
+  constexpr int kW = kManyInputs * 2 * kManyOutputs / kN / 256;        // requests a thread and tile
+  struct __align__(sizeof(TG) * kN) Weights { TG v[kN]; };
+  Weights wr[VEC ? kW : 1];
+  float ur[4];
+  auto request = [&](int k0, int nk) {                                 // (VEC)
+#pragma unroll
+    for (int i = 0; i < kW; ++i) {
+      const int at = (threadIdx.x + 256 * i) * kN, k = at / (2 * kManyOutputs), g = at / kManyOutputs % 2, o = at % kManyOutputs;
+      if (k < nk && j0 + o < bw)
+        *reinterpret_cast<uint4*>(&wr[i]) = *reinterpret_cast<const uint4*>(w + static_cast<int64_t>(k0 + k) * 2 * bw + g * bw + j0 + o);
+      else
+        *reinterpret_cast<uint4*>(&wr[i]) = make_uint4(0, 0, 0, 0);
+    }
+    const int t = threadIdx.x / 8, k = threadIdx.x % 8 * 4;
+    const float4 x = t0 + t < p.n && k < nk ? *reinterpret_cast<const float4*>(u + static_cast<int64_t>(t0 + t) * p.C + k0 + k) : make_float4(0, 0, 0, 0);
+    ur[0] = x.x, ur[1] = x.y, ur[2] = x.z, ur[3] = x.w;
+  };
+  auto stage = [&](int k0, int nk) {
+    if constexpr (VEC) {
+#pragma unroll
+      for (int i = 0; i < kW; ++i) {
+        const int at = (threadIdx.x + 256 * i) * kN;
+        float* to = &ws[0][0][0] + at;
+#pragma unroll
+        for (int e = 0; e < kN; e += 4)
+          *reinterpret_cast<float4*>(to + e) = make_float4(sb::widen(wr[i].v[e]), sb::widen(wr[i].v[e + 1]), sb::widen(wr[i].v[e + 2]), sb::widen(wr[i].v[e + 3]));
+      }
+      const int t = threadIdx.x / 8, k = threadIdx.x % 8 * 4;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) us[k + e][t] = ur[e];
+    } else {
+      for (int i = threadIdx.x; i < nk * 2 * kManyOutputs; i += 256) {
+        const int k = i / (2 * kManyOutputs), g = i / kManyOutputs % 2, o = i % kManyOutputs;
+        ws[k][g][o] = j0 + o < bw ? sb::widen(w[static_cast<int64_t>(k0 + k) * 2 * bw + g * bw + j0 + o]) : 0.0f;
+      }
+      for (int i = threadIdx.x; i < kManyInputs * kManyTokens; i += 256) {
+        const int t = i / kManyInputs, k = i % kManyInputs;
+        if (k < nk) us[k][t] = t0 + t < p.n ? u[static_cast<int64_t>(t0 + t) * p.C + k0 + k] : 0.0f;
+      }
+    }
+  };
   sb::grid_dependency_wait();
-  float sum[2][4][2];                                  // gate, token, channel
+  if constexpr (VEC) request(0, min(kManyInputs, min(bw, per)));
+  float sum[2][4][2], acc[2][4][2];                    // gate, token, channel
   for (int q = 0; q < kQuarters; ++q) {
     const int k_begin = min(bw, q * per), k_end = min(bw, k_begin + per);
-    float acc[2][4][2];
 #pragma unroll
     for (int g = 0; g < 2; ++g)
 #pragma unroll
@@ -248,15 +297,13 @@ __global__ void __launch_bounds__(256) rglru_gates_kernel(const TG* __restrict__
     for (int k0 = k_begin; k0 < k_end; k0 += kManyInputs) {
       const int nk = min(kManyInputs, k_end - k0);
       __syncthreads();
-      for (int i = threadIdx.x; i < nk * 2 * kManyOutputs; i += blockDim.x) {
-        const int k = i / (2 * kManyOutputs), g = i / kManyOutputs % 2, o = i % kManyOutputs;
-        ws[k][g][o] = j0 + o < bw ? sb::widen(w[static_cast<int64_t>(k0 + k) * 2 * bw + g * bw + j0 + o]) : 0.0f;
-      }
-      for (int i = threadIdx.x; i < kManyInputs * kManyTokens; i += blockDim.x) {
-        const int t = i / kManyInputs, k = i % kManyInputs;
-        if (k < nk) us[k][t] = t0 + t < p.n ? p.u[static_cast<int64_t>(t0 + t) * p.C + b * bw + k0 + k] : 0.0f;
-      }
+      stage(k0, nk);
       __syncthreads();
+      if constexpr (VEC) {
+        const bool same = k0 + kManyInputs < k_end;    // the next tile, of this quarter or of the next one (blocks of 16 channels and more fill all four)
+        const int next = same ? k0 + kManyInputs : k_end, end = same ? k_end : min(bw, k_end + per);
+        if (next < end) request(next, min(kManyInputs, end - next));
+      }
       auto one = [&](int k) {
         const float4 x = *reinterpret_cast<const float4*>(&us[k][tg]);
         const float xs[4] = {x.x, x.y, x.z, x.w};
@@ -281,15 +328,51 @@ __global__ void __launch_bounds__(256) rglru_gates_kernel(const TG* __restrict__
 #pragma unroll
         for (int o = 0; o < 2; ++o) sum[g][t][o] = q == 0 ? acc[g][t][o] : sum[g][t][o] + acc[g][t][o];
   }
+  const int j = j0 + 2 * lane, c = b * bw + j;
+  if (j >= bw) return;
+  const bool two = j + 1 < bw;
+  float rb[2], ib[2], softplus[2], yb[2], ut[4][2], z[4][2];
 #pragma unroll
-  for (int o = 0; o < 2; ++o) {
-    const int j = j0 + 2 * lane + o, c = b * bw + j;
-    if (j >= bw) break;
-    const float rb = p.r_bias[c], ib = p.i_bias[c], softplus = softplus_of(p.lam[c]), yb = p.y_bias[c];
+  for (int o = 0; o < 2; ++o)
+    if (o == 0 || two) rb[o] = p.r_bias[c + o], ib[o] = p.i_bias[c + o], softplus[o] = softplus_of(p.lam[c + o]), yb[o] = p.y_bias[c + o];
 #pragma unroll
-    for (int t = 0; t < 4; ++t)
-      if (t0 + tg + t < p.n)
-        gate_outputs(p, t0 + tg + t, c, sum[0][t][o], sum[1][t][o], p.u[static_cast<int64_t>(t0 + tg + t) * p.C + c], rb, ib, softplus, yb);
+  for (int t = 0; t < 4; ++t) {
+    const int row = t0 + tg + t;
+    if (row >= p.n) break;
+    const float* zs = p.proj.p + static_cast<int64_t>(row) * 2 * p.C + c;
+    if constexpr (VEC) {
+      const float2 x = *reinterpret_cast<const float2*>(p.u + static_cast<int64_t>(row) * p.C + c);
+      ut[t][0] = x.x, ut[t][1] = x.y;
+      float2 f = *reinterpret_cast<const float2*>(zs);
+      for (int k = 1; k < p.proj.n_partials; ++k) {
+        const float2 more = *reinterpret_cast<const float2*>(zs + k * p.proj.stride);
+        f.x += more.x, f.y += more.y;
+      }
+      z[t][0] = f.x, z[t][1] = f.y;
+    } else {
+#pragma unroll
+      for (int o = 0; o < 2; ++o)
+        if (o == 0 || two) ut[t][o] = p.u[static_cast<int64_t>(row) * p.C + c + o], z[t][o] = folded(zs + o, p.proj.n_partials, p.proj.stride);
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const int row = t0 + tg + t;
+    if (row >= p.n) break;
+    GateValues v[2];
+#pragma unroll
+    for (int o = 0; o < 2; ++o)
+      if (o == 0 || two) v[o] = gate_values(sum[0][t][o], sum[1][t][o], ut[t][o], z[t][o], rb[o], ib[o], softplus[o], yb[o]);
+    const int64_t i = static_cast<int64_t>(row) * p.C + c;
+    if constexpr (VEC) {
+      *reinterpret_cast<float2*>(p.a + i) = make_float2(v[0].a, v[1].a);
+      *reinterpret_cast<float2*>(p.d + i) = make_float2(v[0].d, v[1].d);
+      *reinterpret_cast<float2*>(p.y + i) = make_float2(v[0].y, v[1].y);
+    } else {
+#pragma unroll
+      for (int o = 0; o < 2; ++o)
+        if (o == 0 || two) p.a[i + o] = v[o].a, p.d[i + o] = v[o].d, p.y[i + o] = v[o].y;
+    }
   }
 }
 
@@ -411,11 +494,14 @@ SB_EXPORT int sb_rglru_gates(const void* gate_w, int gate_dtype, const void* r_b
   const dim3 few_grid((n + kFewTokens - 1) / kFewTokens, blocks, (bw + kFewOutputs - 1) / kFewOutputs);
   const dim3 grid((n + kManyTokens - 1) / kManyTokens, blocks, (bw + kManyOutputs - 1) / kManyOutputs);
   const size_t smem = sizeof(float) * kFewTokens * bw;
+  auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  const bool vec = bw % 16 == 0 && partial_stride % 4 == 0 && aligned(gate_w) && aligned(u) && aligned(proj) && aligned(a) && aligned(d) && aligned(y);
 #define SB_GATES(TG)                                                                                                                            \
   do {                                                                                                                                          \
     if (few && smem > 16 * 1024) cudaFuncSetAttribute(rglru_gates_few_kernel<TG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);      \
     if (few) sb::launch_pdl(rglru_gates_few_kernel<TG>, few_grid, dim3(kQuarters * 2 * kFewOutputs), smem, stream, static_cast<const TG*>(gate_w), p); \
-    else sb::launch_pdl(rglru_gates_kernel<TG>, grid, dim3(256), 0, stream, static_cast<const TG*>(gate_w), p);                                 \
+    else if (vec) sb::launch_pdl(rglru_gates_kernel<TG, true>, grid, dim3(256), 0, stream, static_cast<const TG*>(gate_w), p);                  \
+    else sb::launch_pdl(rglru_gates_kernel<TG, false>, grid, dim3(256), 0, stream, static_cast<const TG*>(gate_w), p);                          \
   } while (0)
   if (gate_dtype == 0) SB_GATES(float);
   else if (gate_dtype == 1) SB_GATES(bf16);

@@ -43,7 +43,7 @@ def test_polynorm_at_the_edges_of_a_thread(F):
     assert (out.cpu().double() - want).abs().max() <= 4e-6 * float(want.abs().max())
 
 
-@pytest.mark.parametrize("bw,B", [(128, 2), (100, 3), (10, 2), (33, 1), (260, 1)])
+@pytest.mark.parametrize("bw,B", [(128, 2), (100, 3), (10, 2), (33, 1), (260, 1), (16, 3), (272, 1)])
 def test_gates_do_not_show_the_number_of_tokens(bw, B):
     """Both kernels of the gates, and one and four rows a block of the convolution: the bits of 1 to 257 tokens in those of 300."""
     from stride_b200.kernels import ops
