@@ -139,6 +139,7 @@ class CacheManager:
         self.entry_group: dict = {}     # schedule entry -> (group index) for page needs
         self.entry_shared: dict = {}    # schedule entry -> entry whose cache it reads
         self.states: dict = {}          # schedule entry -> state arena
+        self._zeroed: list = []         # those of them that a new request finds zeroed
         # One slot and one page per group beyond those handed out: padding rows of a fixed-size batch
         # (a step recorded as a CUDA graph) write their key and value there.
         self.pad_slot = max_slots
@@ -165,6 +166,8 @@ class CacheManager:
                 continue
             if need.kind == "state":
                 self.states[i] = torch.zeros((max_slots + 1, *need.state_shape), dtype=need.state_dtype, device=self.device)
+                if getattr(need, "zeroed", True):
+                    self._zeroed.append(self.states[i])
                 continue
             if need.kind != "pages":
                 raise CacheError(f"unknown cache need kind '{need.kind}'")
@@ -229,10 +232,10 @@ class CacheManager:
 
     # ------------------------------------------------------------------ slots
     def acquire_slot(self) -> int:
-        """A free slot id, its state records zeroed; -1 when every slot is taken."""
+        """A free slot id, its state records zeroed (where the mixers ask for it: `CacheNeed.zeroed`); -1 when every slot is taken."""
         slot = self._lib.sb_pool_acquire_slot(self._pool)
         if slot >= 0:
-            for arena in self.states.values():
+            for arena in self._zeroed:
                 arena[slot].zero_()
         return slot
 
@@ -291,11 +294,17 @@ class CacheManager:
         n = self._lib.sb_pool_take_dirty(self._pool, self._dirty.ctypes.data_as(_I32P), len(self._dirty))
         if n < 0:
             raise CacheError("more block-table rows changed than there are")
-        for gi, slot in self._dirty[:n].tolist():
+        rows = sorted(self._dirty[:n].tolist())
+        at = 0
+        while at < n:                                   # neighbouring rows in one copy
+            (gi, slot), end = rows[at], at + 1
+            while end < n and rows[end] == [gi, slot + end - at]:
+                end += 1
             g = self.groups[gi]
             # From pinned memory and without waiting: a row that changes again before the copy runs only delivers
             # the later content early, which adds pages that no token of an earlier step looks at.
-            g.table_device[slot].copy_(g.table_pinned[slot], non_blocking=True)
+            g.table_device[slot:slot + end - at].copy_(g.table_pinned[slot:slot + end - at], non_blocking=True)
+            at = end
 
     # ------------------------------------------------------------------ views
     def layer_cache(self, entry) -> LayerCache:

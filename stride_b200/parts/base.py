@@ -79,7 +79,8 @@ class CacheNeed:
     and layer (`planes` is 2, keys and values, unless the mixer keeps one row per token that serves as both: 1);
     `window` > 0 means only the last `window` tokens are ever read, so older pages may be given back, except those of a request's first
     `keep_first` tokens, which stay seen. kind "state": `state_shape` elements of `state_dtype` per
-    request, zeroed when a request takes its slot.
+    request, zeroed when a request takes its slot unless `zeroed` is False (mixers whose kernels start from zeros at position 0 whatever
+    the record holds).
     """
     kind: str
     kv_heads: int = 0
@@ -90,6 +91,7 @@ class CacheNeed:
     state_dtype: torch.dtype = torch.float32
     planes: int = 2
     keep_first: int = 0
+    zeroed: bool = True
 
 
 class Part:

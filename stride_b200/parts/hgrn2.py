@@ -54,7 +54,7 @@ class HGRN2Mixer(Mixer):
         return self.proj.weight_bytes() + self.o.weight_bytes()
 
     def cache_need(self):
-        return CacheNeed("state", state_shape=(self.num_heads, self.key_dim, self.value_dim), state_dtype=torch.float32)
+        return CacheNeed("state", state_shape=(self.num_heads, self.key_dim, self.value_dim), state_dtype=torch.float32, zeroed=False)
 
     def kernel_libraries(self):
         return {"gated_recurrence", "gemm_tc" if self.env.compute_dtype == torch.bfloat16 else "gemm_f32"}

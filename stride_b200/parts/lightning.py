@@ -64,7 +64,7 @@ class LightningMixer(Mixer):
         return self.proj.weight_bytes() + self.o.weight_bytes() + self.gain.numel() * self.gain.element_size()
 
     def cache_need(self):
-        return CacheNeed("state", state_shape=(self.num_heads, self.key_dim, self.value_dim), state_dtype=torch.float32)
+        return CacheNeed("state", state_shape=(self.num_heads, self.key_dim, self.value_dim), state_dtype=torch.float32, zeroed=False)
 
     def kernel_libraries(self):
         return {"lightning", "gemm_tc" if self.env.compute_dtype == torch.bfloat16 else "gemm_f32"}

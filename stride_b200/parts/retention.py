@@ -66,7 +66,7 @@ class RetentionMixer(Mixer):
         return self.proj.weight_bytes() + self.o.weight_bytes()
 
     def cache_need(self):
-        return CacheNeed("state", state_shape=(self.H, self.D, self.V), state_dtype=torch.float32)
+        return CacheNeed("state", state_shape=(self.H, self.D, self.V), state_dtype=torch.float32, zeroed=False)
 
     def kernel_libraries(self):
         return {"lightning", "gemm_tc" if self.env.compute_dtype == torch.bfloat16 else "gemm_f32"}

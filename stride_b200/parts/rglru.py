@@ -63,7 +63,7 @@ class RGLRUMixer(Mixer):
         return self.proj.weight_bytes() + self.o.weight_bytes() + self.gate_weights.numel() * self.gate_weights.element_size()
 
     def cache_need(self):
-        return CacheNeed("state", state_shape=(self.taps, self.width), state_dtype=torch.float32)
+        return CacheNeed("state", state_shape=(self.taps, self.width), state_dtype=torch.float32, zeroed=False)
 
     def kernel_libraries(self):
         return {"rglru", "gemm_tc" if self.env.compute_dtype == torch.bfloat16 else "gemm_f32"}
