@@ -574,9 +574,10 @@ __device__ __forceinline__ float soft_cap(float s, float c, float two_over_c) {
 
 constexpr int KT = 64, NK = KT / 16;
 
-// NVW: value column groups of 16 a warp owns (value sizes up to 64 NVW).
-template <int NVW>
-__global__ void __launch_bounds__(128) masked_attention_tile_kernel(TileParams p) {
+// NVW: value column groups of 16 a warp owns (value sizes up to 64 NVW). RG: row groups of a CTA, four warps and 16 rows each, which share
+// the staged keys and values. A tile that only another group's rows see is masked for a row: its sums stay as they are, bit for bit.
+template <int NVW, int RG>
+__global__ void __launch_bounds__(128 * RG) masked_attention_tile_kernel(TileParams p) {
   extern __shared__ __align__(16) unsigned char raw[];
   sb::grid_launch_dependents();
   const int Hg = p.H / p.G, Ht = min(Hg, 16), PT = 16 / Ht;
@@ -585,41 +586,45 @@ __global__ void __launch_bounds__(128) masked_attention_tile_kernel(TileParams p
   const bool own_values = p.v_offset != 0;                      // values staged apart from the keys
   const int ldk = p.D + 8, ldv = own_values ? p.Dv + 8 : ldk;   // padded rows: ldmatrix without bank conflicts
   const bf16** rowptr = reinterpret_cast<const bf16**>(raw);    // [2][KT]: where a tile's key rows lie (null: a row nobody sees)
-  uint32_t* Ps = reinterpret_cast<uint32_t*>(raw + 2 * KT * sizeof(void*));   // [2 parts][NK steps][4 registers][32 lanes]
-  float* tmax = reinterpret_cast<float*>(Ps + 2 * NK * 4 * 32);               // [4 warps][16 rows]
-  bf16* Qs = reinterpret_cast<bf16*>(tmax + 4 * 16);            // [16][ldk]
-  bf16* stage0 = Qs + 16 * ldk;
+  const int group = threadIdx.x / 128, g_pos = group * PT;      // (this thread's row group and its first position within the CTA's)
+  uint32_t* Ps0 = reinterpret_cast<uint32_t*>(raw + 2 * KT * sizeof(void*));  // per group: [2 parts][NK steps][4 registers][32 lanes]
+  float* tmax0 = reinterpret_cast<float*>(Ps0 + RG * 2 * NK * 4 * 32);        // per group: [4 warps][16 rows]
+  bf16* Qs0 = reinterpret_cast<bf16*>(tmax0 + RG * 4 * 16);     // [RG 16][ldk]
+  bf16* stage0 = Qs0 + RG * 16 * ldk;
+  uint32_t* Ps = Ps0 + group * (2 * NK * 4 * 32);
+  float* tmax = tmax0 + group * 4 * 16;
+  const bf16* Qs = Qs0 + group * 16 * ldk;
   const int stage_elems = KT * (ldk + (own_values ? ldv : 0));
   // the blocks that start first take the last tiles: the last positions of an entry see the most keys (a full window, the end of a chunk),
   // and a launch that ends with its longest blocks leaves SMs idle behind them
   int e = 0, tile = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x), len = 0;
   for (; e < p.entries; ++e) {
     len = p.meta[2 * p.meta_stride + e];
-    const int tiles = (len + PT - 1) / PT;
+    const int tiles = (len + RG * PT - 1) / (RG * PT);
     if (tile < tiles) break;
     tile -= tiles;
   }
   if (e >= p.entries) return;
   const int slot = p.meta[e], row0 = p.meta[p.meta_stride + e], pos0 = p.meta[3 * p.meta_stride + e];
-  const int t0 = tile * PT, nt = min(PT, len - t0);            // positions pos0 + t0 .. + nt - 1
+  const int t0 = tile * RG * PT, nt = min(RG * PT, len - t0);  // positions pos0 + t0 .. + nt - 1
   const int first_pos = pos0 + t0, last_pos = first_pos + nt - 1;
   const int first_key = max(p.window > 0 ? max(0, first_pos - p.window + 1) : 0, p.chunk > 0 ? first_pos / p.chunk * p.chunk : 0);
   const int kept = p.window > 0 ? p.keep_first : 0;
   const int kt_first = first_key / KT, kt_last = last_pos / KT;
   const int kt_keep = kept > 0 ? min((kept - 1) / KT, kt_last) : -1;          // the last tile with kept tokens
   const int32_t* table = p.block_table + static_cast<int64_t>(slot) * p.max_pages;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;      // (the warp of its group)
   sb::grid_dependency_wait();
   const int dchunks = p.D / 8, vchunks = own_values ? p.Dv / 8 : 0, cpr = dchunks + vchunks;
-  for (int i = threadIdx.x; i < 16 * dchunks; i += blockDim.x) {
-    const int r = i / dchunks, c = i % dchunks, t = r / Ht;
+  for (int i = threadIdx.x; i < RG * 16 * dchunks; i += blockDim.x) {
+    const int r = i / dchunks, c = i % dchunks, t = r / 16 * PT + r % 16 / Ht;
     uint4 v = make_uint4(0, 0, 0, 0);
-    if (t < nt) v = *reinterpret_cast<const uint4*>(p.q + (static_cast<int64_t>(row0 + t0 + t) * p.H + head0 + r % Ht) * p.D + c * 8);
-    *reinterpret_cast<uint4*>(Qs + r * ldk + c * 8) = v;
+    if (t < nt) v = *reinterpret_cast<const uint4*>(p.q + (static_cast<int64_t>(row0 + t0 + t) * p.H + head0 + r % 16 % Ht) * p.D + c * 8);
+    *reinterpret_cast<uint4*>(Qs0 + r * ldk + c * 8) = v;
   }
   const float two_over_cap = p.cap > 0.0f ? 2.0f / p.cap : 0.0f;
   const int r_lo = lane >> 2, r_hi = r_lo + 8;
-  const int p_lo = r_lo / Ht < nt ? first_pos + r_lo / Ht : -1, p_hi = r_hi / Ht < nt ? first_pos + r_hi / Ht : -1;
+  const int p_lo = g_pos + r_lo / Ht < nt ? first_pos + g_pos + r_lo / Ht : -1, p_hi = g_pos + r_hi / Ht < nt ? first_pos + g_pos + r_hi / Ht : -1;
   const int h_lo = head0 + r_lo % Ht, h_hi = head0 + r_hi % Ht;
   const float s_lo = p.slopes != nullptr ? p.slopes[h_lo] : 0.0f, s_hi = p.slopes != nullptr ? p.slopes[h_hi] : 0.0f;
   float o[2 * NVW][4];
@@ -816,9 +821,9 @@ __global__ void __launch_bounds__(128) masked_attention_tile_kernel(TileParams p
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
     const int r = half ? r_hi : r_lo;
-    if (r / Ht >= nt) continue;
+    if (g_pos + r / Ht >= nt) continue;
     const float inv = 1.0f / (half ? t_hi : t_lo);
-    const int64_t at = (static_cast<int64_t>(row0 + t0 + r / Ht) * p.H + head0 + r % Ht) * p.Dv + (lane & 3) * 2;
+    const int64_t at = (static_cast<int64_t>(row0 + t0 + g_pos + r / Ht) * p.H + head0 + r % Ht) * p.Dv + (lane & 3) * 2;
     bf16* dst = p.out + at;
     float* dst32 = reinterpret_cast<float*>(p.out) + at;
 #pragma unroll
@@ -835,6 +840,26 @@ __global__ void __launch_bounds__(128) masked_attention_tile_kernel(TileParams p
   }
 }
 
+// Two row groups a CTA for long value rows (NVW = 8: 246 registers a thread leave room for eight warps on an SM either way) once they are
+// enough to fill the SMs: the two share a double-buffered tile of keys, where two CTAs of one group each had a single buffer and a copy of
+// their own (16 heads over latents of 512, window 1,024, prompts of 333, 584 and 1,025 tokens: 282 us a layer, 310 so).
+template <int NVW>
+int launch_pairs(const TileParams& p, int n, int y, int PT, size_t stage, cudaStream_t stream, bool* done) {
+  const size_t smem = 2 * KT * sizeof(void*) + 2 * (2 * NK * 4 * 32 * sizeof(uint32_t) + 4 * 16 * sizeof(float) + sizeof(bf16) * 16 * (p.D + 8)) + 2 * stage;
+  const dim3 grid((n + 2 * PT - 1) / (2 * PT) + p.entries, y);
+  *done = smem <= 220 * 1024 && static_cast<int64_t>((n + 2 * PT - 1) / (2 * PT)) * y >= sb::sm_count();
+  if (!*done) return 0;
+  TileParams q = p;
+  q.stages = 2;
+  static sb::DeviceOnce once;
+  if (once.needed()) {
+    cudaFuncSetAttribute(masked_attention_tile_kernel<NVW, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    once.done();
+  }
+  sb::launch_pdl(masked_attention_tile_kernel<NVW, 2>, grid, dim3(256), smem, stream, q);
+  return sb::check_launch("sb_masked_attention_tiles");
+}
+
 template <int NVW>
 int launch_tiles(const TileParams& p, int n, cudaStream_t stream) {
   const int Hg = p.H / p.G, Ht = Hg < 16 ? Hg : 16, PT = 16 / Ht;
@@ -844,6 +869,11 @@ int launch_tiles(const TileParams& p, int n, cudaStream_t stream) {
   size_t smem = fixed + 2 * stage;
   if (smem > 220 * 1024) return sb::fail("sb_masked_attention_tiles: key size %d and value size %d need %zu bytes of shared memory", p.D, p.Dv, smem);
   const dim3 grid((n + PT - 1) / PT + p.entries, p.G * (Hg / Ht));
+  if constexpr (NVW == 8) {
+    bool done = false;
+    const int rc = launch_pairs<NVW>(p, n, static_cast<int>(grid.y), PT, stage, stream, &done);
+    if (done) return rc;
+  }
   TileParams q = p;
   q.stages = 2;
   // rows so long that two stages leave room for one CTA on an SM: with CTAs enough for two on every SM, one stage each and two CTAs that
@@ -855,11 +885,11 @@ int launch_tiles(const TileParams& p, int n, cudaStream_t stream) {
   }
   static sb::DeviceOnce once;
   if (once.needed()) {
-    cudaFuncSetAttribute(masked_attention_tile_kernel<NVW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    cudaFuncSetAttribute(masked_attention_tile_kernel<NVW, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     once.done();
   }
-  sb::prefer_max_shared(reinterpret_cast<const void*>(masked_attention_tile_kernel<NVW>));
-  sb::launch_pdl(masked_attention_tile_kernel<NVW>, grid, dim3(128), smem, stream, q);
+  sb::prefer_max_shared(reinterpret_cast<const void*>(masked_attention_tile_kernel<NVW, 1>));
+  sb::launch_pdl(masked_attention_tile_kernel<NVW, 1>, grid, dim3(128), smem, stream, q);
   return sb::check_launch("sb_masked_attention_tiles");
 }
 
