@@ -144,7 +144,7 @@ __global__ void rope_append_kernel(RopeAppendParams p) {
 
 // The common case (head size and rotated part multiples of eight): one thread per (head, four adjacent rotation pairs, or eight adjacent
 // elements that are not rotated), 16-byte loads of both halves and of cos/sin, 8- or 16-byte stores. Same arithmetic as rope_append_kernel
-// (32 + 8 heads of 64 of which 32 elements are rotated, 2,048 tokens: 17 us, there 36).
+// (32 + 8 heads of 64 of which 32 elements are rotated, 2,048 tokens: 8 us, there 36).
 template <class T>
 __device__ __forceinline__ void store4(T* dst, float a, float b, float c, float d);
 template <>
@@ -160,7 +160,8 @@ __device__ __forceinline__ void store4<bf16>(bf16* dst, float a, float b, float 
   *reinterpret_cast<uint2*>(dst) = packed;
 }
 
-template <class TQ, class TKV>
+// ONE: one partial buffer: without the registers for eight of them more blocks live on an SM (2,048 tokens of 32 + 2 x 8 heads of 64: 16.4 -> 8.0 us).
+template <class TQ, class TKV, bool ONE>
 __global__ void rope_append_vec_kernel(RopeAppendParams p) {
   sb::grid_launch_dependents();
   const int row = blockIdx.x;
@@ -188,7 +189,7 @@ __global__ void rope_append_vec_kernel(RopeAppendParams p) {
   const float* src = p.qkv + static_cast<int64_t>(row) * (p.v_from_k ? p.Hq + p.Hkv : heads) * D +
                      static_cast<int64_t>(is_v && p.v_from_k ? head - p.Hkv : head) * D;
   // the K ranges' sums are added in ascending order; up to kInFlight of them are requested at once
-  constexpr int kInFlight = 8;
+  constexpr int kInFlight = ONE ? 1 : 8;
   float4 pa[kInFlight], pb[kInFlight];
 #pragma unroll
   for (int s = 0; s < kInFlight; ++s) {
@@ -205,7 +206,7 @@ __global__ void rope_append_vec_kernel(RopeAppendParams p) {
       b = add4(b, pb[s]);
     }
   }
-  for (int s = kInFlight; s < p.n_partials; ++s) {
+  for (int s = kInFlight; !ONE && s < p.n_partials; ++s) {
     a = add4(a, *reinterpret_cast<const float4*>(src + s * p.partial_stride + d0));
     b = add4(b, *reinterpret_cast<const float4*>(src + s * p.partial_stride + d1));
   }
@@ -351,11 +352,17 @@ SB_EXPORT int sb_rope_append(const float* qkv, int n_partials, int64_t partial_s
   if (rotary_dim % 8 == 0 && D % 8 == 0 && aligned && partial_stride % 4 == 0 && page_stride % 8 == 0 && v_offset % 8 == 0 &&
       head_stride % 8 == 0) {
     const dim3 vgrid(n, ((Hq + 2 * Hkv) * (D / 8) + threads - 1) / threads);
-    if (q_dtype == 0 && kv_dtype == 0) sb::launch_pdl(rope_append_vec_kernel<float, float>, vgrid, threads, 0, stream, p);
-    else if (q_dtype == 1 && kv_dtype == 1) sb::launch_pdl(rope_append_vec_kernel<bf16, bf16>, vgrid, threads, 0, stream, p);
-    else if (q_dtype == 0 && kv_dtype == 1) sb::launch_pdl(rope_append_vec_kernel<float, bf16>, vgrid, threads, 0, stream, p);
-    else if (q_dtype == 1 && kv_dtype == 0) sb::launch_pdl(rope_append_vec_kernel<bf16, float>, vgrid, threads, 0, stream, p);
+#define SB_ROPE(TQ, TKV)                                                                                                 \
+  do {                                                                                                                   \
+    if (n_partials == 1) sb::launch_pdl(rope_append_vec_kernel<TQ, TKV, true>, vgrid, threads, 0, stream, p);            \
+    else sb::launch_pdl(rope_append_vec_kernel<TQ, TKV, false>, vgrid, threads, 0, stream, p);                           \
+  } while (0)
+    if (q_dtype == 0 && kv_dtype == 0) SB_ROPE(float, float);
+    else if (q_dtype == 1 && kv_dtype == 1) SB_ROPE(bf16, bf16);
+    else if (q_dtype == 0 && kv_dtype == 1) SB_ROPE(float, bf16);
+    else if (q_dtype == 1 && kv_dtype == 0) SB_ROPE(bf16, float);
     else return sb::fail("sb_rope_append: unsupported dtypes q=%d kv=%d", q_dtype, kv_dtype);
+#undef SB_ROPE
     return sb::check_launch("sb_rope_append");
   }
   const dim3 grid(n, ((Hq + 2 * Hkv) * (D / 2) + threads - 1) / threads);

@@ -36,8 +36,10 @@ __device__ __forceinline__ float folded(const float* p, int n_partials, int64_t 
   return sum;
 }
 
+template <bool ONE>
 __device__ __forceinline__ float4 folded4(const float* p, int n_partials, int64_t stride) {      // four neighbouring elements, 16-byte aligned
   constexpr int kTogether = 4;      // (64 registers a thread hold no more)
+  if constexpr (ONE) return *reinterpret_cast<const float4*>(p);      // (without the registers for more, more blocks live on an SM)
   float4 part[kTogether];
 #pragma unroll
   for (int s = 0; s < kTogether; ++s)
@@ -55,7 +57,7 @@ __device__ __forceinline__ float4 folded4(const float* p, int n_partials, int64_
 // in registers between the sums and the stores; what lies beyond is folded again. The three sums share one barrier, each warp adding
 // up the warps' sums by exchanges: a fixed order. Bound by memory: 1,250 rows of 8,192 26 us, 64 us with single elements, a row in shared
 // memory and three block sums one after the other (8 rows: 5 us, 13).
-template <class TO, int VE>
+template <class TO, int VE, bool ONE>
 __global__ void __launch_bounds__(1024) polynorm_kernel(const float* __restrict__ up, int n_partials, int64_t partial_stride, TO* __restrict__ out,
                                                          int F, float a, float b, float c, float e, float eps) {
   using V = typename std::conditional<VE == 4, float4, float>::type;
@@ -67,7 +69,7 @@ __global__ void __launch_bounds__(1024) polynorm_kernel(const float* __restrict_
   const int units = F / VE, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const float* src = up + r * F;
   auto fetch = [&](int i) {
-    if constexpr (VE == 4) return folded4(src + 4 * i, n_partials, partial_stride);
+    if constexpr (VE == 4) return folded4<ONE>(src + 4 * i, n_partials, partial_stride);
     else return folded(src + i, n_partials, partial_stride);
   };
   float s[3] = {0.0f, 0.0f, 0.0f};
@@ -242,14 +244,16 @@ SB_EXPORT int sb_polynorm(const float* up, int n_partials, int64_t partial_strid
   if (F > 50 * 1024) return sb::fail("sb_polynorm: a row of %d elements does not fit the row buffer", F);
   const bool vec = F % 4 == 0 && partial_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   const int units = vec ? F / 4 : F, threads = units > 1024 ? 1024 : units > 512 ? 512 : units > 256 ? 256 : 128;
-#define SB_POLY(TO, VE) \
-  sb::launch_pdl(polynorm_kernel<TO, VE>, dim3(n), dim3(threads), 0, stream, up, n_partials, partial_stride, static_cast<TO*>(out), F, a, b, c, e, eps)
+#define SB_POLY(TO, VE, ONE) \
+  sb::launch_pdl(polynorm_kernel<TO, VE, ONE>, dim3(n), dim3(threads), 0, stream, up, n_partials, partial_stride, static_cast<TO*>(out), F, a, b, c, e, eps)
   if (out_dtype == 0) {
-    if (vec) SB_POLY(float, 4);
-    else SB_POLY(float, 1);
+    if (vec && n_partials == 1) SB_POLY(float, 4, true);
+    else if (vec) SB_POLY(float, 4, false);
+    else SB_POLY(float, 1, false);
   } else if (out_dtype == 1) {
-    if (vec) SB_POLY(bf16, 4);
-    else SB_POLY(bf16, 1);
+    if (vec && n_partials == 1) SB_POLY(bf16, 4, true);
+    else if (vec) SB_POLY(bf16, 4, false);
+    else SB_POLY(bf16, 1, false);
   } else {
     return sb::fail("sb_polynorm: unsupported output dtype %d", out_dtype);
   }

@@ -33,7 +33,9 @@ __device__ __forceinline__ float folded(const float* p, int n_partials, int64_t 
   return sum;
 }
 
+template <bool ONE>
 __device__ __forceinline__ float4 folded4(const float* p, int n_partials, int64_t stride) {      // four neighbouring elements, 16-byte aligned
+  if constexpr (ONE) return *reinterpret_cast<const float4*>(p);      // (without the registers for more, more blocks live on an SM)
   float4 part[kInFlight];
 #pragma unroll
   for (int s = 0; s < kInFlight; ++s)
@@ -50,7 +52,7 @@ __device__ __forceinline__ float4 folded4(const float* p, int n_partials, int64_
 // proj [P][n][2 HD + HV]: columns q | f | v. act [n][3 HD + HV]: columns q | g | k | v. grid: (rows, pieces of a row). VE = 4: four elements
 // an access where the sizes and buffers allow it. Bound by memory: 1,250 rows of 16 heads of 128 | 128 18 us, 37 us with one element and a
 // 64-bit division a thread and round.
-template <class TW, int VE>
+template <class TW, int VE, bool ONE>
 __global__ void __launch_bounds__(128) hgrn2_activate_kernel(const float* __restrict__ proj, int n_partials, int64_t partial_stride,
                                                              const TW* __restrict__ f_bias, const TW* __restrict__ lower, float* __restrict__ act, int HD, int HV) {
   sb::grid_launch_dependents();
@@ -65,7 +67,7 @@ __global__ void __launch_bounds__(128) hgrn2_activate_kernel(const float* __rest
   sb::grid_dependency_wait();
   const float* src = proj + static_cast<int64_t>(blockIdx.x) * in_w + j;
   if constexpr (VE == 4) {
-    const float4 v = folded4(src, n_partials, partial_stride);
+    const float4 v = folded4<ONE>(src, n_partials, partial_stride);
     z[0] = v.x, z[1] = v.y, z[2] = v.z, z[3] = v.w;
   } else {
     z[0] = folded(src, n_partials, partial_stride);
@@ -140,15 +142,17 @@ SB_EXPORT int sb_hgrn2_activate(const float* proj, int n_partials, int64_t parti
   if (n_partials < 1) return sb::fail("sb_hgrn2_activate: n_partials must be >= 1");
   const bool vec = HD % 4 == 0 && HV % 4 == 0 && partial_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(act)) & 15) == 0;
   const dim3 grid(n, ((2 * HD + HV) / (vec ? 4 : 1) + 127) / 128);
-#define SB_ACT(TW, VE) \
-  sb::launch_pdl(hgrn2_activate_kernel<TW, VE>, grid, dim3(128), 0, stream, proj, n_partials, partial_stride, static_cast<const TW*>(f_bias), \
+#define SB_ACT(TW, VE, ONE) \
+  sb::launch_pdl(hgrn2_activate_kernel<TW, VE, ONE>, grid, dim3(128), 0, stream, proj, n_partials, partial_stride, static_cast<const TW*>(f_bias), \
                  static_cast<const TW*>(lower), act, HD, HV)
   if (w_dtype == 0) {
-    if (vec) SB_ACT(float, 4);
-    else SB_ACT(float, 1);
+    if (vec && n_partials == 1) SB_ACT(float, 4, true);
+    else if (vec) SB_ACT(float, 4, false);
+    else SB_ACT(float, 1, false);
   } else if (w_dtype == 1) {
-    if (vec) SB_ACT(bf16, 4);
-    else SB_ACT(bf16, 1);
+    if (vec && n_partials == 1) SB_ACT(bf16, 4, true);
+    else if (vec) SB_ACT(bf16, 4, false);
+    else SB_ACT(bf16, 1, false);
   } else {
     return sb::fail("sb_hgrn2_activate: unsupported dtype %d", w_dtype);
   }

@@ -39,7 +39,9 @@ __device__ __forceinline__ float folded(const float* p, int n_partials, int64_t 
 }
 
 // The same over four neighbouring elements (p and the stride 16-byte aligned).
+template <bool ONE>
 __device__ __forceinline__ float4 folded4(const float* p, int n_partials, int64_t stride) {
+  if constexpr (ONE) return *reinterpret_cast<const float4*>(p);      // (without the registers for more, more blocks live on an SM)
   float4 part[kInFlight];
 #pragma unroll
   for (int s = 0; s < kInFlight; ++s)
@@ -85,8 +87,8 @@ __global__ void __launch_bounds__(DL * 64, 768 / (DL * 64)) lightning_step_kerne
 // act[r, j] = silu(sum of the partial buffers at [r, j]) for the first `cols` columns of every row: what the recurrence
 // reads, made once for all of a long step's tokens instead of by every CTA that needs a token's keys and queries.
 // VE: 4 where the columns and buffers allow 16-byte accesses, else 1. grid: (rows, pieces of a row). Bound by memory: 2,048 rows of 6,144
-// columns (101 MB) 22 us, 48 us with one element and a 64-bit division a thread and round.
-template <int VE>
+// columns (101 MB) 17 us, 48 us with one element and a 64-bit division a thread and round.
+template <int VE, bool ONE>
 __global__ void __launch_bounds__(256) lightning_activate_kernel(const float* __restrict__ proj, int n_partials, int64_t partial_stride, int width,
                                                                  float* __restrict__ act, int cols) {
   sb::grid_launch_dependents();
@@ -95,7 +97,7 @@ __global__ void __launch_bounds__(256) lightning_activate_kernel(const float* __
   float* dst = act + static_cast<int64_t>(blockIdx.x) * cols;
   for (int i = (blockIdx.y * blockDim.x + threadIdx.x) * VE; i < cols; i += gridDim.y * blockDim.x * VE) {
     if constexpr (VE == 4) {
-      const float4 v = folded4(src + i, n_partials, partial_stride);
+      const float4 v = folded4<ONE>(src + i, n_partials, partial_stride);
       *reinterpret_cast<float4*>(dst + i) = make_float4(silu(v.x), silu(v.y), silu(v.z), silu(v.w));
     } else {
       dst[i] = silu(folded(src + i, n_partials, partial_stride));
@@ -106,8 +108,8 @@ __global__ void __launch_bounds__(256) lightning_activate_kernel(const float* __
 // out[r, j] = o[r, j] / sqrt(mean_j(o[r, :]^2) + eps) * gain[j] * sigmoid(gate[r, j]); the gate is a column range of the
 // projection's partial sums. One block per row. VE: 4 where the width and every buffer allow 16-byte accesses, else 1; which one depends on
 // the width and the buffers alone, never on the rows. A thread keeps up to kKeep pieces of o and of the gate in registers, requested before
-// the block's sum; what lies beyond is read again behind it. 2,048 rows of 2,048: 15 us, 24 us with single elements and the gate behind the sum.
-template <class TW, class TO, int VE>
+// the block's sum; what lies beyond is read again behind it. 2,048 rows of 2,048: 11.6 us, 24 us with single elements and the gate behind the sum.
+template <class TW, class TO, int VE, bool ONE>
 __global__ void __launch_bounds__(1024) gated_rmsnorm_kernel(const float* __restrict__ o, const float* __restrict__ proj, int n_partials,
                                                               int64_t partial_stride, int width, int g_off,
                                                               const TW* __restrict__ gain, TO* __restrict__ out, int W, float eps) {
@@ -121,7 +123,7 @@ __global__ void __launch_bounds__(1024) gated_rmsnorm_kernel(const float* __rest
   const V* src = reinterpret_cast<const V*>(o + r * W);
   const float* gate = proj + r * width + g_off;
   auto gate_at = [&](int i) {
-    if constexpr (VE == 4) return folded4(gate + 4 * i, n_partials, partial_stride);
+    if constexpr (VE == 4) return folded4<ONE>(gate + 4 * i, n_partials, partial_stride);
     else return folded(gate + i, n_partials, partial_stride);
   };
   V v[kKeep], g[kKeep];
@@ -196,8 +198,10 @@ SB_EXPORT int sb_lightning_scan_ex(const float* proj, int n_partials, int64_t pa
   if (act == nullptr) return sb::fail("sb_lightning_scan: a step with an entry of several tokens needs the scratch for the activated sums");
   const int cols = max(max(q_off + H * D, k_off + H * D), v_off + H * V);
   const bool vec = cols % 4 == 0 && width % 4 == 0 && partial_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(act)) & 15) == 0;
-  if (vec) sb::launch_pdl(lightning_activate_kernel<4>, dim3(n, (cols / 4 + 255) / 256), dim3(256), 0, stream, proj, n_partials, partial_stride, width, act, cols);
-  else sb::launch_pdl(lightning_activate_kernel<1>, dim3(n, (cols + 1023) / 1024), dim3(256), 0, stream, proj, n_partials, partial_stride, width, act, cols);
+  const dim3 vgrid(n, (cols / 4 + 255) / 256);
+  if (vec && n_partials == 1) sb::launch_pdl(lightning_activate_kernel<4, true>, vgrid, dim3(256), 0, stream, proj, n_partials, partial_stride, width, act, cols);
+  else if (vec) sb::launch_pdl(lightning_activate_kernel<4, false>, vgrid, dim3(256), 0, stream, proj, n_partials, partial_stride, width, act, cols);
+  else sb::launch_pdl(lightning_activate_kernel<1, false>, dim3(n, (cols + 1023) / 1024), dim3(256), 0, stream, proj, n_partials, partial_stride, width, act, cols);
   p.rows = act;
   p.width = cols;
   return sbscan::launch_scan<false>(p, entries, "sb_lightning_scan", stream);
@@ -221,11 +225,14 @@ SB_EXPORT int sb_gated_rmsnorm(const float* o, const float* proj, int n_partials
   const int units = vec ? W / 4 : W, threads = units > 1024 ? 1024 : units > 512 ? 512 : units > 256 ? 256 : 128;
 #define SB_GN(TW, TO)                                                                                                           \
   do {                                                                                                                          \
-    if (vec)                                                                                                                    \
-      sb::launch_pdl(gated_rmsnorm_kernel<TW, TO, 4>, n, threads, 0, stream, o, proj, n_partials, partial_stride, width, g_off, \
+    if (vec && n_partials == 1)                                                                                                 \
+      sb::launch_pdl(gated_rmsnorm_kernel<TW, TO, 4, true>, n, threads, 0, stream, o, proj, n_partials, partial_stride, width, g_off, \
+                     static_cast<const TW*>(gain), static_cast<TO*>(out), W, eps);                                              \
+    else if (vec)                                                                                                               \
+      sb::launch_pdl(gated_rmsnorm_kernel<TW, TO, 4, false>, n, threads, 0, stream, o, proj, n_partials, partial_stride, width, g_off, \
                      static_cast<const TW*>(gain), static_cast<TO*>(out), W, eps);                                              \
     else                                                                                                                        \
-      sb::launch_pdl(gated_rmsnorm_kernel<TW, TO, 1>, n, threads, 0, stream, o, proj, n_partials, partial_stride, width, g_off, \
+      sb::launch_pdl(gated_rmsnorm_kernel<TW, TO, 1, false>, n, threads, 0, stream, o, proj, n_partials, partial_stride, width, g_off, \
                      static_cast<const TW*>(gain), static_cast<TO*>(out), W, eps);                                              \
   } while (0)
   if (gain_dtype == 0 && out_dtype == 0) SB_GN(float, float);

@@ -10,7 +10,6 @@ SB_DEFINE_LAST_ERROR()
 namespace {
 
 using bf16 = __nv_bfloat16;
-constexpr int kRowsKernelMin = 1536;   // more rows than this, and no partial sums: the warp-per-row kernel
 
 // ------------------------------------------------------------------ rmsnorm
 // One block per row. The row is h + (partial_0 + partial_1 + ...), the partials summed left to
@@ -28,8 +27,10 @@ struct VecF<1> { using type = float; };
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 __device__ __forceinline__ float add4(float a, float b) { return a + b; }
 
-template <class TW, class TO, int VEC, int MAXT>     // MAXT: the most threads of a block (1024, or 512 with more registers each)
-__global__ void __launch_bounds__(MAXT) rmsnorm_kernel(float* __restrict__ h, const float* __restrict__ partials, int n_partials,
+// FLIGHT: the partial sums requested together. With few rows 12: every one is a round trip to L2. With more rows than SMs 6: two blocks an SM
+// instead of one (256 rows of 2,048 behind nine buffers 5.4 us, 7.1 with 12). The additions are the same: equal bits.
+template <class TW, class TO, int VEC, int MAXT, int FLIGHT>     // MAXT: the most threads of a block
+__global__ void __launch_bounds__(MAXT, FLIGHT == 6 ? 2 : 1) rmsnorm_kernel(float* __restrict__ h, const float* __restrict__ partials, int n_partials,
                                int64_t partial_stride, const TW* __restrict__ weight, TO* __restrict__ out,
                                int H, float eps) {
   using V = typename VecF<VEC>::type;
@@ -50,9 +51,7 @@ __global__ void __launch_bounds__(MAXT) rmsnorm_kernel(float* __restrict__ h, co
   for (int i = threadIdx.x; i < units; i += blockDim.x) {
     V v = hr[i];
     if (n_partials > 0) {
-      // up to kInFlight partial sums are requested at once (every load of a few tokens' row is a round trip to L2,
-      // and they are what this kernel's time consists of), then added left to right
-      constexpr int kInFlight = MAXT > 512 ? 8 : 12;
+      constexpr int kInFlight = FLIGHT;
       const V* p = reinterpret_cast<const V*>(partials + static_cast<int64_t>(r) * H) + i;
       const int64_t ps = partial_stride / VEC;
       V part[kInFlight];
@@ -63,7 +62,8 @@ __global__ void __launch_bounds__(MAXT) rmsnorm_kernel(float* __restrict__ h, co
 #pragma unroll
       for (int s = 1; s < kInFlight; ++s)
         if (s < n_partials) sum = add4(sum, part[s]);
-      for (int s = kInFlight; s < n_partials; ++s) sum = add4(sum, p[s * ps]);
+      if constexpr (FLIGHT > 1)
+        for (int s = kInFlight; s < n_partials; ++s) sum = add4(sum, p[s * ps]);
       v = add4(v, sum);
       hr[i] = v;
     }
@@ -89,14 +89,6 @@ __global__ void __launch_bounds__(MAXT) rmsnorm_kernel(float* __restrict__ h, co
   }
 }
 
-// Many rows (a prompt portion): one warp per row, two rows per block (small blocks spread evenly over the SMs), no shared memory and no block barrier.
-// Pass 1 folds the partials (written back to h) and sums the squares; pass 2 re-reads the row (it is in L2) and
-// writes the normed values. H % 4 == 0. The squares are added in the order of rmsnorm_kernel with 32 W threads, so
-// that a row's result has the same bits whichever kernel the size of the step selects: lane l stands for that
-// kernel's threads l, l + 32, .., one chain of fused multiply-adds each, the 32 chains of a warp are combined by
-// xor shuffles and the W warps' sums are added in ascending order.
-// JT > 0: the row has at most JT rounds of 32 W pieces and stays in registers between the passes; 0: any width,
-// pass 2 re-reads it.
 // Four gains from element i of a bfloat16 or float32 vector (the widening is exact).
 __device__ __forceinline__ float4 load_gain4(const void* w, bool is_bf16, int i) {
   if (is_bf16) {
@@ -120,68 +112,57 @@ __device__ __forceinline__ void store_normed4(TO* o, float4 v, float4 w, float s
   }
 }
 
-template <class TO, int W, int JT>
-__global__ void __launch_bounds__(64) rmsnorm_rows_kernel(float* __restrict__ h, const float* __restrict__ partials,
-                                                           int n_partials, int64_t partial_stride,
-                                                           const void* __restrict__ weight, bool weight_bf16,
-                                                           TO* __restrict__ out, int n, int H, float eps) {
+// At most one partial buffer (prompts, whose projections fold their K ranges themselves; the 32-bit path): half as many threads as
+// rmsnorm_kernel has for the width, each with the shares of two of its threads, t and t + blockDim.x, so that twice as much is in flight a
+// thread and no register is kept for partial buffers that do not exist. The squares are added in rmsnorm_kernel's order (a warp stands for
+// two of its warps): equal bits. 2,048 rows of 2,048: 11.8 us; 17 us as a warp a row, 19 with rmsnorm_kernel's threads.
+template <class TW, class TO>
+__global__ void __launch_bounds__(512) rmsnorm_pairs_kernel(float* __restrict__ h, const float* __restrict__ partial, const TW* __restrict__ weight,
+                                                            TO* __restrict__ out, int H, float eps) {
+  __shared__ float red[32];
   sb::grid_launch_dependents();
   sb::grid_dependency_wait();
-  const int r = blockIdx.x * 2 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (r >= n) return;
-  float4* hr = reinterpret_cast<float4*>(h + static_cast<int64_t>(r) * H);
-  const int units = H / 4;
-  const int64_t ps = partial_stride / 4;
-  float chain[W];
-  float4 keep[JT > 0 ? JT * W : 1];
+  const int64_t r = blockIdx.x;
+  const int units = H / 4, half = blockDim.x, warps = half >> 5;
+  float4* hr = reinterpret_cast<float4*>(h + r * H);
+  const float4* pr = reinterpret_cast<const float4*>(partial + r * H);
+  auto square = [](float4 v, float ss) { return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, fmaf(v.x, v.x, ss)))); };
+  float4 keep[2], add[2];
+  float ss[2] = {0.0f, 0.0f};
 #pragma unroll
-  for (int w = 0; w < W; ++w) chain[w] = 0.0f;
-  auto round = [&](int i0, int jt) {
-#pragma unroll
-    for (int w = 0; w < W; ++w) {
-      const int i = i0 + 32 * w + lane;
-      if (i < units) {
-        float4 v = hr[i];
-        if (n_partials > 0) {
-          const float4* p = reinterpret_cast<const float4*>(partials + static_cast<int64_t>(r) * H) + i;
-          float4 sum = p[0];
-          for (int s = 1; s < n_partials; ++s) sum = add4(sum, p[s * ps]);
-          v = add4(v, sum);
-          hr[i] = v;
-        }
-        if (JT > 0) keep[jt * W + w] = v;
-        chain[w] = fmaf(v.x, v.x, chain[w]);
-        chain[w] = fmaf(v.y, v.y, chain[w]);
-        chain[w] = fmaf(v.z, v.z, chain[w]);
-        chain[w] = fmaf(v.w, v.w, chain[w]);
-      }
+  for (int j = 0; j < 2; ++j) {
+    const int i = threadIdx.x + j * half;
+    if (i < units) {
+      keep[j] = hr[i];
+      if (partial != nullptr) add[j] = pr[i];
     }
-  };
-  if constexpr (JT > 0) {
-#pragma unroll
-    for (int jt = 0; jt < JT; ++jt) round(jt * 32 * W, jt);
-  } else {
-    for (int i0 = 0; i0 < units; i0 += 32 * W) round(i0, 0);
   }
-  float ss = 0.0f;
 #pragma unroll
-  for (int w = 0; w < W; ++w) {
-    float c = chain[w];
+  for (int j = 0; j < 2; ++j) {
+    const int i = threadIdx.x + j * half;
+    if (i < units) {
+      if (partial != nullptr) hr[i] = keep[j] = add4(keep[j], add[j]);
+      ss[j] = square(keep[j], 0.0f);
+    }
+    for (int k = i + 2 * half; k < units; k += 2 * half) {      // wider rows are read again behind the sum
+      float4 v = hr[k];
+      if (partial != nullptr) hr[k] = v = add4(v, pr[k]);
+      ss[j] = square(v, ss[j]);
+    }
+    float c = ss[j];
     for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    ss = w == 0 ? c : ss + c;
+    if ((threadIdx.x & 31) == 0) red[j * warps + (threadIdx.x >> 5)] = c;
   }
-  const float scale = 1.0f / sqrtf(ss / static_cast<float>(H) + eps);
-  TO* o = out + static_cast<int64_t>(r) * H;
-  if constexpr (JT > 0) {
+  __syncthreads();
+  float total = red[0];
+  for (int i = 1; i < 2 * warps; ++i) total += red[i];
+  const float scale = 1.0f / sqrtf(total / static_cast<float>(H) + eps);
+  TO* o = out + r * H;
 #pragma unroll
-    for (int jt = 0; jt < JT; ++jt)
-#pragma unroll
-      for (int w = 0; w < W; ++w) {
-        const int i = jt * 32 * W + 32 * w + lane;
-        if (i < units) store_normed4<TO>(o + 4 * i, keep[jt * W + w], load_gain4(weight, weight_bf16, 4 * i), scale);
-      }
-  } else {
-    for (int i = lane; i < units; i += 32) store_normed4<TO>(o + 4 * i, hr[i], load_gain4(weight, weight_bf16, 4 * i), scale);
+  for (int j = 0; j < 2; ++j) {
+    const int i = threadIdx.x + j * half;
+    if (i < units) store_normed4<TO>(o + 4 * i, keep[j], load_gain4(weight, sizeof(TW) == 2, 4 * i), scale);
+    for (int k = i + 2 * half; k < units; k += 2 * half) store_normed4<TO>(o + 4 * k, hr[k], load_gain4(weight, sizeof(TW) == 2, 4 * k), scale);
   }
 }
 
@@ -190,8 +171,9 @@ __global__ void __launch_bounds__(64) rmsnorm_rows_kernel(float* __restrict__ h,
 // mean = sum(x) / H; var = sum((x - mean)^2) / H; out = (x - mean) / sqrt(var + eps) * w + b. Both sums in the order of sb::block_sum.
 // VEC = 4: four elements an access where the width and every buffer allow it; which form runs depends on the width and the buffers alone,
 // never on the rows, so a row's result does not either. A thread keeps its first kKeep pieces in registers through both sums; wider rows are
-// read again. Bound by memory: 2,048 rows of 2,048 with one partial buffer 22 us, single elements in shared memory 24 us.
-template <class TW, class TO, int VEC, int MAXT>     // MAXT: the most threads of a block, as in rmsnorm_kernel
+// read again. Bound by memory: 2,048 rows of 2,048 with one partial buffer 10.5 us (22 with the
+// registers for eight partial buffers), single elements in shared memory 24 us.
+template <class TW, class TO, int VEC, int MAXT, bool ONE>     // MAXT: the most threads of a block, ONE: at most one partial buffer, as in rmsnorm_kernel
 __global__ void __launch_bounds__(MAXT) layernorm_kernel(float* __restrict__ h, const float* __restrict__ partials, int n_partials,
                                                          int64_t partial_stride, const TW* __restrict__ weight,
                                                          const TW* __restrict__ bias, TO* __restrict__ out, int H, float eps) {
@@ -206,7 +188,7 @@ __global__ void __launch_bounds__(MAXT) layernorm_kernel(float* __restrict__ h, 
   auto fetch = [&](int i) {
     V v = hr[i];
     if (n_partials > 0) {
-      constexpr int kInFlight = 8;
+      constexpr int kInFlight = ONE ? 1 : 8;
       const V* p = reinterpret_cast<const V*>(partials + r * H) + i;
       const int64_t ps = partial_stride / VEC;
       V part[kInFlight];
@@ -217,7 +199,8 @@ __global__ void __launch_bounds__(MAXT) layernorm_kernel(float* __restrict__ h, 
 #pragma unroll
       for (int s = 1; s < kInFlight; ++s)
         if (s < n_partials) sum = add4(sum, part[s]);
-      for (int s = kInFlight; s < n_partials; ++s) sum = add4(sum, p[s * ps]);
+      if constexpr (!ONE)
+        for (int s = kInFlight; s < n_partials; ++s) sum = add4(sum, p[s * ps]);
       v = add4(v, sum);
       hr[i] = v;
     }
@@ -275,14 +258,15 @@ SB_EXPORT int sb_layernorm(float* h, const float* partials, int n_partials, int6
   auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   const bool vec = H % 4 == 0 && aligned(h) && aligned(partials) && aligned(weight) && aligned(bias) && aligned(out) && partial_stride % 4 == 0;
   const int units = vec ? H / 4 : H, threads = units > 1024 ? 1024 : units > 512 ? 512 : units > 256 ? 256 : 128;
-#define SB_LN_V(TW, TO, VEC, MAXT)                                                                                            \
-  sb::launch_pdl(layernorm_kernel<TW, TO, VEC, MAXT>, n, threads, 0, stream, h, partials, n_partials, partial_stride,         \
+#define SB_LN_V(TW, TO, VEC, MAXT, ONE)                                                                                       \
+  sb::launch_pdl(layernorm_kernel<TW, TO, VEC, MAXT, ONE>, n, threads, 0, stream, h, partials, n_partials, partial_stride,    \
                  static_cast<const TW*>(weight), static_cast<const TW*>(bias), static_cast<TO*>(out), H, eps)
-#define SB_LN(TW, TO)                                  \
-  do {                                                 \
-    if (vec && threads <= 512) SB_LN_V(TW, TO, 4, 512); \
-    else if (vec) SB_LN_V(TW, TO, 4, 1024);            \
-    else SB_LN_V(TW, TO, 1, 1024);                     \
+#define SB_LN(TW, TO)                                                              \
+  do {                                                                             \
+    if (vec && threads <= 512 && n_partials <= 1) SB_LN_V(TW, TO, 4, 512, true);   \
+    else if (vec && threads <= 512) SB_LN_V(TW, TO, 4, 512, false);                \
+    else if (vec) SB_LN_V(TW, TO, 4, 1024, false);                                 \
+    else SB_LN_V(TW, TO, 1, 1024, false);                                          \
   } while (0)
   if (weight_dtype == 0 && out_dtype == 0) SB_LN(float, float);
   else if (weight_dtype == 0 && out_dtype == 1) SB_LN(float, bf16);
@@ -303,53 +287,23 @@ SB_EXPORT int sb_rmsnorm(float* h, const float* partials, int n_partials, int64_
   const bool vec = H % 4 == 0 && partial_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(partials)) & 15) == 0;
   const int units = vec ? H / 4 : H;
   const int threads = units >= 1024 ? 1024 : units >= 512 ? 512 : units >= 256 ? 256 : 128;
-  // (a block per row is the faster of the two up to about 1,500 rows, and whenever partial sums are to be added:
-  // measured at H = 2048, 256 rows: 2.9 us against 9.7 us; 2,048 rows: 19.4 against 18.7)
-  if (vec && n > kRowsKernelMin && n_partials <= 1 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(weight)) & 15) == 0) {
-    // the warp-per-row kernel adds the squares in the order of the block-per-row kernel with `threads` threads
-    const dim3 grid((n + 1) / 2);
-#define SB_ROWS_J(TO, W, JT) \
-  sb::launch_pdl(rmsnorm_rows_kernel<TO, W, JT>, grid, dim3(64), 0, stream, h, partials, n_partials, partial_stride, \
-                 weight, weight_dtype == 1, static_cast<TO*>(out), n, H, eps)
-  // the row stays in registers between the passes while it has at most 16 pieces a lane; wider rows are read again from
-  // L2 in the second pass (measured: 32 pieces in registers leave too few warps an SM: width 4096 58 -> 38 us for 2,048
-  // rows, width 3072 48 -> 30; at width 2048, 16 pieces, registers are the faster way, 17 us against 21)
-#define SB_ROWS(TO)                                                      \
-  do {                                                                   \
-    if (threads == 1024) SB_ROWS_J(TO, 32, 0);                           \
-    else if (threads == 512 && units <= 512) SB_ROWS_J(TO, 16, 1);   \
-    else if (threads == 512) SB_ROWS_J(TO, 16, 0);                   \
-    else if (threads == 256 && units <= 256) SB_ROWS_J(TO, 8, 1);    \
-    else if (threads == 256) SB_ROWS_J(TO, 8, 2);                    \
-    else if (units <= 128) SB_ROWS_J(TO, 4, 1);                      \
-    else SB_ROWS_J(TO, 4, 2);                                        \
-  } while (0)
-    if ((weight_dtype != 0 && weight_dtype != 1) || (out_dtype != 0 && out_dtype != 1))
-      return sb::fail("sb_rmsnorm: unsupported dtypes weight=%d out=%d", weight_dtype, out_dtype);
-    if (out_dtype == 0) SB_ROWS(float);
-    else SB_ROWS(bf16);
-#undef SB_ROWS
-#undef SB_ROWS_J
-    return sb::check_launch("sb_rmsnorm");
-  }
-#define SB_NORM_V(TW, TO, VEC)                                                                                   \
+#define SB_NORM_V(TW, TO, VEC, MAXT, FLIGHT)                                                                     \
   do {                                                                                                           \
-    if (threads > 512) {                                                                                         \
-      if (smem > 48 * 1024)                                                                                      \
-        cudaFuncSetAttribute(rmsnorm_kernel<TW, TO, VEC, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-      sb::launch_pdl(rmsnorm_kernel<TW, TO, VEC, 1024>, n, threads, smem, stream, h, partials, n_partials, partial_stride, \
-                     static_cast<const TW*>(weight), static_cast<TO*>(out), H, eps);                            \
-    } else {                                                                                                     \
-      if (smem > 48 * 1024)                                                                                      \
-        cudaFuncSetAttribute(rmsnorm_kernel<TW, TO, VEC, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-      sb::launch_pdl(rmsnorm_kernel<TW, TO, VEC, 512>, n, threads, smem, stream, h, partials, n_partials, partial_stride, \
-                     static_cast<const TW*>(weight), static_cast<TO*>(out), H, eps);                            \
-    }                                                                                                            \
+    if (smem > 48 * 1024)                                                                                        \
+      cudaFuncSetAttribute(rmsnorm_kernel<TW, TO, VEC, MAXT, FLIGHT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    sb::launch_pdl(rmsnorm_kernel<TW, TO, VEC, MAXT, FLIGHT>, n, threads, smem, stream, h, partials, n_partials, partial_stride, \
+                   static_cast<const TW*>(weight), static_cast<TO*>(out), H, eps);                               \
   } while (0)
-#define SB_NORM(TW, TO)          \
-  do {                           \
-    if (vec) SB_NORM_V(TW, TO, 4); \
-    else SB_NORM_V(TW, TO, 1);   \
+#define SB_NORM(TW, TO)                                                                                                         \
+  do {                                                                                                                          \
+    if (vec && n_partials <= 1 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(weight)) & 15) == 0)         \
+      sb::launch_pdl(rmsnorm_pairs_kernel<TW, TO>, dim3(n), dim3(threads / 2), 0, stream, h, n_partials == 1 ? partials : nullptr, \
+                     static_cast<const TW*>(weight), static_cast<TO*>(out), H, eps);                                            \
+    else if (vec && threads > 512) SB_NORM_V(TW, TO, 4, 1024, 8);                                                               \
+    else if (vec && n > sb::sm_count()) SB_NORM_V(TW, TO, 4, 512, 6);                                                           \
+    else if (vec) SB_NORM_V(TW, TO, 4, 512, 12);                                                                                \
+    else if (threads > 512) SB_NORM_V(TW, TO, 1, 1024, 8);                                                                      \
+    else SB_NORM_V(TW, TO, 1, 512, 12);                                                                                         \
   } while (0)
   if (weight_dtype == 0 && out_dtype == 0) SB_NORM(float, float);
   else if (weight_dtype == 0 && out_dtype == 1) SB_NORM(float, bf16);
