@@ -169,6 +169,8 @@ __global__ void __launch_bounds__(128) attn_chunk_kernel(const AttnTcParams p) {
 // holds their position (no rotation kernel runs).
 struct BlockEnv {
   static constexpr bool kFoldAhead = true;    // the next group of chunk records is requested while one is folded
+  // a CTA without keys leaves its place without a wait (every entry has a CTA that waits, so the launch ends behind the kernels in front all the same)
+  static constexpr bool kLeavesEarly = true;
   __device__ __forceinline__ void sync() { __syncthreads(); }
   __device__ __forceinline__ void wait_inputs() { sb::grid_dependency_wait(); }
 };
@@ -182,7 +184,10 @@ __global__ void __launch_bounds__(128, FUSED ? 3 : (D == 64 ? kDecodeCtas64 : 3)
   // cluster is the grid's z extent, so the rank is the chunk)
   static_assert((4 * 16 * (D + 2) + decode_record_floats<D>()) * sizeof(float) <= 4 * 64 * D * sizeof(bf16), "the record must fit over the tiles");
   float* record = CLUSTER ? reinterpret_cast<float*>(smem_tiles) + 4 * 16 * (D + 2) : nullptr;
-  decode_unit<D, FUSED, CLUSTER, EXTRA>(p, blockIdx.x, blockIdx.y, blockIdx.z, smem_tiles, &is_last_s, threadIdx.x, env, record);
+  // The last chunks start first: a recorded step's grid reaches to the longest context it may meet, so they are the sparse ones, and the
+  // entries with the most chunks to fold are not what the launch ends with.
+  const int chunk = CLUSTER ? blockIdx.z : gridDim.z - 1 - blockIdx.z;
+  decode_unit<D, FUSED, CLUSTER, EXTRA>(p, blockIdx.x, blockIdx.y, chunk, smem_tiles, &is_last_s, threadIdx.x, env, record);
 }
 
 template <int D>

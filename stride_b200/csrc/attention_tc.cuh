@@ -465,7 +465,7 @@ __device__ __forceinline__ void decode_unit(const AttnTcParams& p, int item, int
     sb::cluster_sync();
   };
   if (chunk * kChunk > pos_hi || chunk * kChunk + kChunk - 1 < key_lo) {   // no key of this chunk is visible
-    env.wait_inputs();
+    if (CLUSTER || !Env::kLeavesEarly) env.wait_inputs();
     if (CLUSTER) cluster_fold();
     return;
   }
