@@ -112,6 +112,60 @@ __device__ __forceinline__ void store_normed4(TO* o, float4 v, float4 w, float s
   }
 }
 
+// Few rows behind several partial buffers (decoding): a row's ten reads of 8 KB are more than one SM takes in during a round trip to L2, so a
+// row is a cluster of four blocks, each with a quarter of rmsnorm_kernel's threads and their shares; the warps' sums of squares go to all four
+// blocks' shared memory and are added in rmsnorm_kernel's order: equal bits. One to 64 rows of 2,048 behind nine buffers, within a decode
+// step: 3.5 to 3.8 us, 4.1 to 4.5 as a block a row.
+__device__ __forceinline__ void cluster_store(const float* p, uint32_t rank, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(sb::cluster_peer_address(p, rank)), "f"(v) : "memory");
+}
+constexpr int kRowBlocks = 4;
+template <class TW, class TO>
+__global__ void __launch_bounds__(256) rmsnorm_cluster_kernel(float* __restrict__ h, const float* __restrict__ partials, int n_partials,
+                                                              int64_t partial_stride, const TW* __restrict__ weight, TO* __restrict__ out, int H, float eps) {
+  __shared__ float red[32];
+  sb::grid_launch_dependents();
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");     // (all four blocks have begun: waited for below)
+  const int64_t r = blockIdx.x / kRowBlocks;
+  const int rank = blockIdx.x % kRowBlocks, units = H / 4, threads = kRowBlocks * blockDim.x, t = rank * blockDim.x + threadIdx.x;
+  float4 w_first = make_float4(0, 0, 0, 0);
+  if (t < units) w_first = load_gain4(weight, sizeof(TW) == 2, 4 * t);
+  sb::grid_dependency_wait();
+  float4* hr = reinterpret_cast<float4*>(h + r * H);
+  const int64_t ps = partial_stride / 4;
+  float4 first = make_float4(0, 0, 0, 0);
+  float ss = 0.0f;
+  for (int i = t; i < units; i += threads) {
+    constexpr int kInFlight = 12;
+    const float4* p = reinterpret_cast<const float4*>(partials + r * H) + i;
+    float4 v = hr[i], part[kInFlight];
+#pragma unroll
+    for (int s = 0; s < kInFlight; ++s)
+      if (s < n_partials) part[s] = p[s * ps];
+    float4 sum = part[0];
+#pragma unroll
+    for (int s = 1; s < kInFlight; ++s)
+      if (s < n_partials) sum = add4(sum, part[s]);
+    for (int s = kInFlight; s < n_partials; ++s) sum = add4(sum, p[s * ps]);
+    v = add4(v, sum);
+    hr[i] = v;
+    if (i == t) first = v;
+    ss = fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, fmaf(v.x, v.x, ss))));
+  }
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  const int lane = threadIdx.x & 31;
+  if (lane < kRowBlocks) cluster_store(&red[t >> 5], lane, ss);
+  __syncwarp();
+  sb::cluster_sync();
+  float total = red[0];
+  for (int i = 1; i < threads >> 5; ++i) total += red[i];
+  const float scale = 1.0f / sqrtf(total / static_cast<float>(H) + eps);
+  TO* o = out + r * H;
+  if (t < units) store_normed4<TO>(o + 4 * t, first, w_first, scale);
+  for (int i = t + threads; i < units; i += threads) store_normed4<TO>(o + 4 * i, hr[i], load_gain4(weight, sizeof(TW) == 2, 4 * i), scale);
+}
+
 // At most one partial buffer (prompts, whose projections fold their K ranges themselves; the 32-bit path): half as many threads as
 // rmsnorm_kernel has for the width, each with the shares of two of its threads, t and t + blockDim.x, so that twice as much is in flight a
 // thread and no register is kept for partial buffers that do not exist. The squares are added in rmsnorm_kernel's order (a warp stands for
@@ -299,6 +353,9 @@ SB_EXPORT int sb_rmsnorm(float* h, const float* partials, int n_partials, int64_
     if (vec && n_partials <= 1 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(weight)) & 15) == 0)         \
       sb::launch_pdl(rmsnorm_pairs_kernel<TW, TO>, dim3(n), dim3(threads / 2), 0, stream, h, n_partials == 1 ? partials : nullptr, \
                      static_cast<const TW*>(weight), static_cast<TO*>(out), H, eps);                                            \
+    else if (vec && n <= 64 && threads >= 512 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(weight)) & 15) == 0) \
+      sb::launch_pdl_cluster(rmsnorm_cluster_kernel<TW, TO>, dim3(n * kRowBlocks), dim3(threads / kRowBlocks), 0, stream, dim3(kRowBlocks), h, partials, \
+                             n_partials, partial_stride, static_cast<const TW*>(weight), static_cast<TO*>(out), H, eps);        \
     else if (vec && threads > 512) SB_NORM_V(TW, TO, 4, 1024, 8);                                                               \
     else if (vec && n > sb::sm_count()) SB_NORM_V(TW, TO, 4, 512, 6);                                                           \
     else if (vec) SB_NORM_V(TW, TO, 4, 512, 12);                                                                                \

@@ -111,3 +111,71 @@ def test_a_few_tokens_as_a_stream_over_the_weights(M, K, wdtype):
         assert torch.equal(out, tiles[:n] + tiles[:n])
     xd, wd = x[:4].double(), w.double()
     assert ((tiles[:4].double() - xd @ wd.T).abs() <= (K / 32 + 40) * 2.0 ** -24 * (xd.abs() @ wd.abs().T)).all()
+
+
+@pytest.mark.parametrize("window,keep,sinks", [(0, 0, False), (100, 0, True), (64, 5, True), (1, 0, False)])
+def test_masked_attention_of_two_row_groups_a_block(window, keep, sinks):
+    """Latent rows of 512 and 16 heads: a step of 410 tokens (two tokens a block; entries of odd lengths, one of which continues) in the bits
+    of the same tokens in steps of at most 99 (a token a block), and the rows against the sum in 64 bits."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(window + keep)
+    H, D, page, scale = 16, 512, 32, 0.05
+    old, new = [0, 70], [333, 77]                                    # cached tokens in front, tokens of the step
+    pages = (torch.randn(2 * 16, 1, 1, page, D, generator=g) * 0.5).bfloat16().to(DEV)
+    table = torch.randperm(32, generator=g).view(2, 16).int().to(DEV)
+    q = torch.randn(sum(new), H * D, generator=g).bfloat16().to(DEV)
+    sink = torch.randn(H, generator=g).to(DEV) if sinks else None
+
+    def run(rows, entries):
+        meta = torch.tensor([[e[k] for e in entries] for k in range(4)], dtype=torch.int32, device=DEV)
+        out = torch.empty(rows.shape[0], H * D, dtype=torch.bfloat16, device=DEV)
+        ops.masked_attention_tiles(rows, out, pages, table, meta, len(entries), None, sink, H, 1, D, D, window, keep, scale)
+        return out
+
+    whole = run(q, [(0, 0, new[0], old[0]), (1, new[0], new[1], old[1])])
+    first = 0
+    for slot in (0, 1):
+        keys = pages[table[slot].long(), 0, 0].reshape(-1, D).double()
+        for a in range(0, new[slot], 99):
+            n = min(99, new[slot] - a)
+            part = run(q[first + a:first + a + n].contiguous(), [(slot, 0, n, old[slot] + a)])
+            assert torch.equal(part, whole[first + a:first + a + n])
+        i, j = torch.arange(new[slot], device=DEV)[:, None] + old[slot], torch.arange(keys.shape[0], device=DEV)[None]
+        seen = (j <= i) & ((i - j < window) | (j < keep)) if window else j <= i
+        s = torch.einsum("ihd,jd->hij", q[first:first + new[slot]].double().view(-1, H, D), keys) * scale
+        s = s.masked_fill(~seen, float("-inf"))
+        if sink is not None:
+            s = torch.cat([s, sink.double().view(H, 1, 1).expand(H, new[slot], 1)], -1)
+        want = torch.einsum("hij,jd->ihd", torch.softmax(s, -1)[..., :keys.shape[0]], keys).reshape(new[slot], -1)
+        # half a step of bfloat16 of the largest value, and what the 32-bit exponentials leave
+        assert (whole[first:first + new[slot]].double() - want).abs().max() <= 2.0 ** -8 * float(want.abs().max())
+        first += new[slot]
+
+
+@pytest.mark.parametrize("H", [2048, 2052, 4096, 8192, 8200, 1024, 516])
+def test_rms_norm_does_not_show_its_form(H):
+    """Four blocks a row (up to 64 rows behind several partial buffers), a block a row with twelve and with six buffers requested together, and
+    half the threads for a row behind one buffer (here as two, the second zero, in the other forms): the same bits."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(H)
+    n, w = 200, (1 + 0.1 * torch.randn(H, generator=g)).bfloat16().to(DEV)
+    h, parts = torch.randn(n, H, generator=g).to(DEV), torch.randn(9, n, H, generator=g).to(DEV)
+    zero = torch.zeros(1, n, H, device=DEV)
+    for partials, alone in ((parts, None), (torch.cat([parts[:1], zero]), parts[:1])):
+        def run(m, p, dtype):
+            hd, out = h[:m].clone(), torch.empty(m, H, dtype=dtype, device=DEV)
+            ops.rmsnorm(hd, w, 1e-5, out, partials=p[:, :m].contiguous())
+            return hd, out
+        for dtype in (torch.bfloat16, torch.float32):
+            whole = run(n, partials, dtype)
+            for m in (1, 64, 65, 148):
+                for x, y in zip(run(m, partials, dtype), whole):
+                    assert torch.equal(x, y[:m]), m
+            if alone is not None:
+                for x, y in zip(run(n, alone, dtype), whole):
+                    assert torch.equal(x, y)
+    x = h.double() + parts.double().sum(0)
+    want = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5) * w.double()
+    out = torch.empty(64, H, device=DEV)
+    ops.rmsnorm(h[:64].clone(), w, 1e-5, out, partials=parts[:, :64].contiguous())
+    assert (out.double() - want[:64]).abs().max() <= 2e-6 * float(want.abs().max())      # sixteen roundings of a 32-bit result
