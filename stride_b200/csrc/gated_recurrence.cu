@@ -50,7 +50,7 @@ __device__ __forceinline__ float4 folded4(const float* p, int n_partials, int64_
 }
 
 // proj [P][n][2 HD + HV]: columns q | f | v. act [n][3 HD + HV]: columns q | g | k | v. grid: (rows, pieces of a row). VE = 4: four elements
-// an access where the sizes and buffers allow it. Bound by memory: 1,250 rows of 16 heads of 128 | 128 18 us, 37 us with one element and a
+// an access where the sizes and buffers allow it. Bound by memory: 1,250 rows of 16 heads of 128 | 128 15.5 us, 37 us with one element and a
 // 64-bit division a thread and round.
 template <class TW, int VE, bool ONE>
 __global__ void __launch_bounds__(128) hgrn2_activate_kernel(const float* __restrict__ proj, int n_partials, int64_t partial_stride,
