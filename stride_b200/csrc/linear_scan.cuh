@@ -130,8 +130,8 @@ __device__ __forceinline__ void bar_arrive(int id, int count) { asm volatile("ba
 // lane one part of each: a token's keys and queries are read from shared memory once a warp, every lane its own, and serve PER columns. The
 // parts of 32 / PER tokens' outputs are added up together by exchanges between lanes, so that no part goes through shared memory. One more
 // warp keeps the rows of the next two chunks of tokens on their way into the staging buffers; it announces a chunk before it requests
-// another, since a request waits until its buffer is free. What bounds the kernel is the chain of a token's dependent operations in the one
-// computing warp that a scheduler has (without the loads and the exchanges 155 of its 220 us are left).
+// another, since a request waits until its buffer is free. What bounds the kernel is each warp's wait for its own reads and exchanges, with one
+// or two computing warps a scheduler (issue slots 47% busy; without the loads and the exchanges 155 of its 220 us are left).
 // Measured (16 heads of 128 x 128, one entry of 2,048 tokens / eight): eight warps of one column a thread, the outputs' parts through shared
 // memory, 611 / 1,600 us; PER = 4 220 / 721 us, PER = 2 193 / 828 us.
 template <int DL, int PER, bool GATED, int VEC>
