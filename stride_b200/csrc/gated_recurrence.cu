@@ -101,9 +101,9 @@ __global__ void __launch_bounds__(DL * 64, 1024 / (DL * 64)) gated_step_kernel(c
   extern __shared__ __align__(16) float smem[];
   sb::grid_launch_dependents();
   const int e = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * 32;
-  const int slot = p.meta[e], row = p.meta[p.meta_stride + e], pos0 = p.meta[3 * p.meta_stride + e];
+  const int slot = p.meta[e], row0 = p.meta[p.meta_stride + e], len = p.meta[2 * p.meta_stride + e], pos0 = p.meta[3 * p.meta_stride + e];
   sb::grid_dependency_wait();
-  sbscan::step_core<DL, true>(p, smem, slot, row, pos0, [&](float* to, int Dp) {
+  sbscan::step_core<DL, true>(p, smem, slot, row0, len, pos0, [&](float* to, int Dp, int row) {
     const float* src = p.rows + static_cast<int64_t>(row) * p.width;
     for (int j = threadIdx.x; j < 3 * Dp + 32; j += blockDim.x) {
       float v = 0.0f;

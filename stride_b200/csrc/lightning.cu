@@ -55,15 +55,15 @@ __device__ __forceinline__ float4 folded4(const float* p, int n_partials, int64_
   return sum;
 }
 
-// Steps in which every entry brings one token (decoding): the partial sums folded (and activated) inside.
+// Steps with as many tokens as entries (decoding): the partial sums folded (and activated) inside.
 template <int DL>
 __global__ void __launch_bounds__(DL * 64, 768 / (DL * 64)) lightning_step_kernel(const sbscan::Params p, int n_partials, int64_t partial_stride, int activated) {
   extern __shared__ __align__(16) float smem[];
   sb::grid_launch_dependents();
   const int e = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * 32;
-  const int slot = p.meta[e], row = p.meta[p.meta_stride + e], pos0 = p.meta[3 * p.meta_stride + e];
+  const int slot = p.meta[e], row0 = p.meta[p.meta_stride + e], len = p.meta[2 * p.meta_stride + e], pos0 = p.meta[3 * p.meta_stride + e];
   sb::grid_dependency_wait();
-  sbscan::step_core<DL, false>(p, smem, slot, row, pos0, [&](float* to, int Dp) {
+  sbscan::step_core<DL, false>(p, smem, slot, row0, len, pos0, [&](float* to, int Dp, int row) {
     const float* src = p.rows + static_cast<int64_t>(row) * p.width;
 #pragma unroll 1
     for (int j = threadIdx.x; j < 2 * Dp + 32; j += blockDim.x) {

@@ -287,26 +287,26 @@ int launch_scan(const Params& p, int entries, const char* who, cudaStream_t stre
 #undef SB_SCAN_OF
 }
 
-// Steps in which every entry brings one token: a CTA is (entry, head, 32 value columns), a thread kRows elements of one column (what a
-// warp reads of the state is whole 128-byte rows). The state's loads are requested first; `fill(smem, Dp)` writes the token's q, k, (g,) v
-// into shared memory meanwhile: q, k, g [Dp] each, zero beyond D, v [32]. The same operations in the same order as scan_kernel: a thread
-// adds its own neighbouring parts, the warps' sums are the upper levels of the tree.
+// Steps with as many tokens as entries: a CTA is (entry, head, 32 value columns), a thread kRows elements of one column (what a warp reads of
+// the state is whole 128-byte rows). The state's loads are requested first; `fill(smem, Dp, row)` writes the token's q, k, (g,) v into shared
+// memory meanwhile: q, k, g [Dp] each, zero beyond D, v [32]. The same operations in the same order as scan_kernel: a thread adds its own
+// neighbouring parts, the warps' sums are the upper levels of the tree.
 constexpr int kRows = 16;
 template <int DL, bool GATED, class Fill>
-__device__ __forceinline__ void step_core(const Params& p, float* smem, int slot, int row, int pos0, Fill fill) {
+__device__ __forceinline__ void step_token(const Params& p, float* smem, int slot, int row, int pos, int V, Fill fill) {
   constexpr int Dp = kLanes * DL, kParts = kRows / DL, warps = Dp / kRows;
   const int h = blockIdx.y, c0 = blockIdx.z * 32, warp = threadIdx.x >> 5, cl = threadIdx.x & 31;
   float* sv = smem + (GATED ? 3 : 2) * Dp;
   float* so = sv + 32;         // [warps][32]
-  const bool live = c0 + cl < p.V;
+  const bool live = c0 + cl < V;
   const int d0 = warp * kRows, dn = min(kRows, p.D - d0);
-  float* st = p.state + ((static_cast<int64_t>(slot) * p.H + h) * p.D + d0) * p.V + c0 + cl;
+  const float decay = GATED ? 0.0f : p.decay[h];
+  float* st = p.state + ((static_cast<int64_t>(slot) * p.H + h) * p.D + d0) * V + c0 + cl;
   float2 S[kParts][DL / 2];
 #pragma unroll
-  for (int i = 0; i < kRows; ++i) put(S[i / DL], i % DL, pos0 > 0 && live && i < dn ? st[static_cast<int64_t>(i) * p.V] : 0.0f);
-  fill(smem, Dp);
+  for (int i = 0; i < kRows; ++i) put(S[i / DL], i % DL, pos > 0 && live && i < dn ? st[static_cast<int64_t>(i) * V] : 0.0f);
+  fill(smem, Dp, row);
   __syncthreads();
-  const float decay = GATED ? 0.0f : p.decay[h];
   float a[kParts];
 #pragma unroll
   for (int j = 0; j < kParts; ++j) {
@@ -323,7 +323,7 @@ __device__ __forceinline__ void step_core(const Params& p, float* smem, int slot
   if (live) {
 #pragma unroll
     for (int i = 0; i < kRows; ++i)
-      if (i < dn) st[static_cast<int64_t>(i) * p.V] = get(S[i / DL], i % DL);
+      if (i < dn) st[static_cast<int64_t>(i) * V] = get(S[i / DL], i % DL);
   }
   __syncthreads();
   if (warp == 0 && live) {
@@ -334,7 +334,22 @@ __device__ __forceinline__ void step_core(const Params& p, float* smem, int slot
     for (int m = 1; m < warps; m <<= 1)
 #pragma unroll
       for (int q = 0; q < warps; q += 2 * m) w[q] = w[q] + w[q + m];
-    p.out[static_cast<int64_t>(row) * p.H * p.V + h * p.V + c0 + cl] = w[0];
+    p.out[static_cast<int64_t>(row) * p.H * V + h * V + c0 + cl] = w[0];
+  }
+}
+template <int DL, bool GATED, class Fill>
+__device__ __forceinline__ void step_core(const Params& p, float* smem, int slot, int row0, int len, int pos0, Fill fill) {
+  if (len == 1) {
+    step_token<DL, GATED>(p, smem, slot, row0, pos0, p.V, fill);
+    return;
+  }
+  // no token, or several: one after the other, the state through memory (a thread reads what it wrote; the token in front has been read when
+  // every warp has passed the second barrier)
+#pragma unroll 1
+  for (int t = 0; t < len; ++t) {
+    int V = p.V;
+    asm volatile("" : "+r"(V));      // (sixteen addresses kept from one token to the next would cost the usual case its registers)
+    step_token<DL, GATED>(p, smem, slot, row0 + t, pos0 + t, V, fill);
   }
 }
 

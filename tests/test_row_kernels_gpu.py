@@ -179,3 +179,33 @@ def test_rms_norm_does_not_show_its_form(H):
     out = torch.empty(64, H, device=DEV)
     ops.rmsnorm(h[:64].clone(), w, 1e-5, out, partials=parts[:, :64].contiguous())
     assert (out.double() - want[:64]).abs().max() <= 2e-6 * float(want.abs().max())      # sixteen roundings of a 32-bit result
+
+
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("lengths", [[2, 0], [1, 3, 0, 0], [1, 1, 1]])
+def test_recurrence_with_as_many_tokens_as_entries(gated, lengths):
+    """The kernel of single tokens is chosen by the number of tokens and entries alone: entries without a token and entries of several give
+    the bits of each entry's tokens in a step of their own."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(len(lengths))
+    H, D, V, E, n = 2, 40, 36, len(lengths), len(lengths)
+    rows, width = [sum(lengths[:i]) for i in range(E)], 3 * H * D + H * V
+    act = torch.rand(n, width, generator=g).to(DEV)
+    before = torch.randn(E, H, D, V, generator=g).to(DEV)
+
+    def run(x, entries, state):
+        meta = torch.tensor([[e[k] for e in entries] for k in range(4)], dtype=torch.int32, device=DEV)
+        out = torch.zeros(x.shape[0], H * V, device=DEV)
+        if gated:
+            ops.gated_scan(x, 0, H * D, 2 * H * D, 3 * H * D, meta, len(entries), state, out, H, D, V)
+        else:
+            ops.lightning_scan(x, 0, H * D, 3 * H * D, meta, len(entries), torch.tensor([0.9, 0.99], device=DEV), state, out, H, D, V, torch.empty_like(x))
+        return out
+
+    state, alone = before.clone(), before.clone()
+    out = run(act, [(i, rows[i], lengths[i], 5) for i in range(E)], state)
+    for i in range(E):
+        for t in range(lengths[i]):
+            r = rows[i] + t
+            assert torch.equal(run(act[r:r + 1].contiguous(), [(i, 0, 1, 5 + t)], alone)[0], out[r])
+    assert torch.equal(state, alone)
