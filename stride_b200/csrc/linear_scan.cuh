@@ -5,10 +5,11 @@
 //   o_t = S_t^T q_t
 //
 // Everything is 32-bit. A column of the state depends on no other column, so the value columns may be spread over CTAs and threads in any
-// way. The D sums of an output are cut into 32 parts of DL consecutive elements (DL = 2, 4 or 8 by the key size alone; elements beyond D are
-// zero), each two chains of fused multiply-adds (even and odd elements, ascending, then added), and the parts are added as a binary tree of
-// neighbours (part 2i + part 2i + 1, and so on). None of it depends on the step, so a token's output has the same bits however the sequence
-// was cut into steps, whichever of the two kernels below ran, and whatever else the batch holds.
+// way. The D sums of an output are cut into 32 parts of DL consecutive elements (DL = 2, 4 or 8 by the key size alone; elements beyond D
+// are zero, and a part that lies wholly beyond D adds zeros whatever the values, which may be infinite), each two chains of fused multiply-adds
+// (even and odd elements, ascending, then added), and the parts are added as a binary tree of neighbours (part 2i + part 2i + 1, and so on).
+// None of it depends on the step, so a token's output has the same bits however the sequence was cut into steps, whichever of the two kernels
+// below ran, and whatever else the batch holds.
 //
 // `scan_kernel` is for steps in which an entry brings several tokens; `step_core` is the work of a token for steps of single tokens.
 #pragma once
@@ -203,6 +204,10 @@ __global__ void __launch_bounds__(kWarps * 32 + 32) scan_kernel(const Params p) 
         if (nt == kGroup) walk(std::true_type{});
         else walk(std::false_type{});
         if (t0 + kGroup >= min(kChunk, len - c * kChunk) && c + kStages < chunks) bar_arrive(kBarEmpty + b, NC + 32);
+        if (dn <= 0) {      // a part beyond D: zeros, whatever 0 times an infinite value is
+#pragma unroll
+          for (int i = 0; i < 32; ++i) sums[i] = 0.0f;
+        }
         const float sum = transpose_add(sums, lane);
         const int t = lane / PER;
         if (live && t < nt) out[static_cast<int64_t>(c * kChunk + t0 + t) * p.H * p.V] = sum;
@@ -313,7 +318,7 @@ __device__ __forceinline__ void step_token(const Params& p, float* smem, int slo
     const float* sq = smem + d0 + j * DL;
     Part<DL, GATED> x;
     x.load(sq, sq + Dp, sq + (GATED ? 2 : 0) * Dp);
-    a[j] = token<DL, GATED>(S[j], x, sv[cl], decay);
+    a[j] = token<DL, GATED>(S[j], x, j * DL < dn ? sv[cl] : 0.0f, decay);
   }
 #pragma unroll
   for (int m = 1; m < kParts; m <<= 1)

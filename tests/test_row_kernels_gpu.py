@@ -209,3 +209,27 @@ def test_recurrence_with_as_many_tokens_as_entries(gated, lengths):
             r = rows[i] + t
             assert torch.equal(run(act[r:r + 1].contiguous(), [(i, 0, 1, 5 + t)], alone)[0], out[r])
     assert torch.equal(state, alone)
+
+
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("D,tokens", [(144, 40), (144, 1), (40, 40), (40, 1), (16, 20)])
+def test_recurrence_with_an_infinite_value(D, tokens, gated):
+    """Key sizes that do not fill the lanes: an infinite value makes its own column infinite from its token on (all keys, queries and states
+    are positive here) and nothing else; the elements that pad the keys add zeros."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(D)
+    H, V = 2, 36
+    act = 0.1 + torch.rand(tokens, 3 * H * D + H * V, generator=g)
+    at, column = tokens // 2, 7
+    act[at, 3 * H * D + column] = float("inf")
+    meta = torch.tensor([[0], [0], [tokens], [3]], dtype=torch.int32, device=DEV)
+    state, out = torch.rand(1, H, D, V, generator=g).to(DEV), torch.zeros(tokens, H * V, device=DEV)
+    if gated:
+        ops.gated_scan(act.to(DEV), 0, H * D, 2 * H * D, 3 * H * D, meta, 1, state, out, H, D, V)
+    else:
+        ops.lightning_scan(act.to(DEV), 0, H * D, 3 * H * D, meta, 1, torch.tensor([0.9, 0.99], device=DEV), state, out, H, D, V,
+                           torch.empty_like(act).to(DEV))
+    infinite = torch.zeros(tokens, H * V, dtype=torch.bool)
+    infinite[at:, column] = True
+    assert torch.equal(torch.isinf(out.cpu()), infinite) and not torch.isnan(out).any()
+    assert torch.isinf(state[0, 0, :, column]).all() and torch.isinf(state).sum() == D and not torch.isnan(state).any()
