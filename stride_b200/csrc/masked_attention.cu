@@ -575,7 +575,8 @@ __device__ __forceinline__ float soft_cap(float s, float c, float two_over_c) {
 constexpr int KT = 64, NK = KT / 16;
 
 // NVW: value column groups of 16 a warp owns (value sizes up to 64 NVW). RG: row groups of a CTA, four warps and 16 rows each, which share
-// the staged keys and values. A tile that only another group's rows see is masked for a row: its sums stay as they are, bit for bit.
+// the staged keys and values. A key that only the other group's rows see is masked for a row, and its value is read as zeros: what lies
+// there, an infinity or a NaN too, never meets the row, whose bits do not depend on what it shares a CTA with.
 template <int NVW, int RG>
 __global__ void __launch_bounds__(128 * RG) masked_attention_tile_kernel(TileParams p) {
   extern __shared__ __align__(16) unsigned char raw[];
@@ -595,6 +596,7 @@ __global__ void __launch_bounds__(128 * RG) masked_attention_tile_kernel(TilePar
   float* tmax = tmax0 + group * 4 * 16;
   const bf16* Qs = Qs0 + group * 16 * ldk;
   const int stage_elems = KT * (ldk + (own_values ? ldv : 0));
+  bf16* zeros = stage0 + p.stages * stage_elems;                // (RG > 1: a value row of zeros, [ldv])
   // the blocks that start first take the last tiles: the last positions of an entry see the most keys (a full window, the end of a chunk),
   // and a launch that ends with its longest blocks leaves SMs idle behind them
   int e = 0, tile = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x), len = 0;
@@ -622,6 +624,11 @@ __global__ void __launch_bounds__(128 * RG) masked_attention_tile_kernel(TilePar
     if (t < nt) v = *reinterpret_cast<const uint4*>(p.q + (static_cast<int64_t>(row0 + t0 + t) * p.H + head0 + r % 16 % Ht) * p.D + c * 8);
     *reinterpret_cast<uint4*>(Qs0 + r * ldk + c * 8) = v;
   }
+  // the keys that any row of this group may see: up to g_last, from g_first on or below `kept`
+  const int g_pos0 = first_pos + g_pos, g_last = min(g_pos0 + PT - 1, last_pos);
+  const int g_first = max(p.window > 0 ? g_pos0 - p.window + 1 : 0, p.chunk > 0 ? g_pos0 / p.chunk * p.chunk : 0);
+  if constexpr (RG > 1)
+    for (int i = threadIdx.x; i < ldv / 8; i += blockDim.x) *reinterpret_cast<uint4*>(zeros + i * 8) = make_uint4(0, 0, 0, 0);
   const float two_over_cap = p.cap > 0.0f ? 2.0f / p.cap : 0.0f;
   const int r_lo = lane >> 2, r_hi = r_lo + 8;
   const int p_lo = g_pos + r_lo / Ht < nt ? first_pos + g_pos + r_lo / Ht : -1, p_hi = g_pos + r_hi / Ht < nt ? first_pos + g_pos + r_hi / Ht : -1;
@@ -777,6 +784,18 @@ __global__ void __launch_bounds__(128 * RG) masked_attention_tile_kernel(TilePar
     for (int i = 0; i < 2 * NVW; ++i) o[i][0] *= f_lo, o[i][1] *= f_lo, o[i][2] *= f_hi, o[i][3] *= f_hi;
     __syncthreads();
     // O += hi V + lo V for this warp's value columns, the tile's steps in ascending order
+    // the value rows that this lane's fragments come from: zeros for keys that the group does not see
+    const int v_row0 = (lane & 7) + ((lane >> 3) & 1) * 8;
+    const bf16* v_rows[NK];
+#pragma unroll
+    for (int kk = 0; kk < NK; ++kk) v_rows[kk] = Vs + (kk * 16 + v_row0) * ldv + (lane >> 4) * 8;
+    if (RG > 1 && (kt * KT + KT - 1 > g_last || (kt * KT < g_first && kt * KT + KT > kept))) {
+#pragma unroll
+      for (int kk = 0; kk < NK; ++kk) {
+        const int key = kt * KT + kk * 16 + v_row0;
+        if (key > g_last || (key < g_first && key >= kept)) v_rows[kk] = zeros + (lane >> 4) * 8;
+      }
+    }
 #pragma unroll
     for (int kk = 0; kk < NK; ++kk) {
       uint32_t hi[4], lo[4];
@@ -788,7 +807,7 @@ __global__ void __launch_bounds__(128 * RG) masked_attention_tile_kernel(TilePar
       // the step's value fragments first, then the products of the first parts for every column group, then those of the second parts:
       // a column's sum takes its terms in the same order (hi, then lo), with the other columns' products between the two
       uint32_t b[NVW][4];
-      const bf16* v_at = Vs + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * ldv + (lane >> 4) * 8;
+      const bf16* v_at = RG > 1 ? v_rows[kk] : Vs + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * ldv + (lane >> 4) * 8;
 #pragma unroll
       for (int i = 0; i < NVW; ++i)
         if (warp + 4 * i < NV) ldmatrix_x4_trans(b[i], v_at + (warp + 4 * i) * 16);
@@ -845,7 +864,8 @@ __global__ void __launch_bounds__(128 * RG) masked_attention_tile_kernel(TilePar
 // their own (16 heads over latents of 512, window 1,024, prompts of 333, 584 and 1,025 tokens: 282 us a layer, 310 so).
 template <int NVW>
 int launch_pairs(const TileParams& p, int n, int y, int PT, size_t stage, cudaStream_t stream, bool* done) {
-  const size_t smem = 2 * KT * sizeof(void*) + 2 * (2 * NK * 4 * 32 * sizeof(uint32_t) + 4 * 16 * sizeof(float) + sizeof(bf16) * 16 * (p.D + 8)) + 2 * stage;
+  const size_t smem = 2 * KT * sizeof(void*) + 2 * (2 * NK * 4 * 32 * sizeof(uint32_t) + 4 * 16 * sizeof(float) + sizeof(bf16) * 16 * (p.D + 8)) + 2 * stage +
+                      sizeof(bf16) * ((p.v_offset != 0 ? p.Dv : p.D) + 8);
   const dim3 grid((n + 2 * PT - 1) / (2 * PT) + p.entries, y);
   *done = smem <= 220 * 1024 && static_cast<int64_t>((n + 2 * PT - 1) / (2 * PT)) * y >= sb::sm_count();
   if (!*done) return 0;

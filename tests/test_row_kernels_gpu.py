@@ -233,3 +233,32 @@ def test_recurrence_with_an_infinite_value(D, tokens, gated):
     infinite[at:, column] = True
     assert torch.equal(torch.isinf(out.cpu()), infinite) and not torch.isnan(out).any()
     assert torch.isinf(state[0, 0, :, column]).all() and torch.isinf(state).sum() == D and not torch.isnan(state).any()
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("window,keep", [(0, 0), (64, 5)])
+def test_rows_never_meet_keys_they_do_not_see(bad, window, keep):
+    """Two tokens a block share staged keys: the one in front does not see the other's latent, the other has one key less at the window's
+    start. Latents that are no numbers change no row that does not see them, alone in a block or as one of two."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(window)
+    H, D, page, n = 16, 512, 32, 400
+    pages = (torch.randn(13, 1, 1, page, D, generator=g) * 0.5).bfloat16().to(DEV)
+    table = torch.arange(13, dtype=torch.int32, device=DEV)[None]
+    q = torch.randn(n, H * D, generator=g).bfloat16().to(DEV)
+
+    def run(cache, first, count):
+        meta = torch.tensor([[0], [0], [count], [first]], dtype=torch.int32, device=DEV)
+        out = torch.empty(count, H * D, dtype=torch.bfloat16, device=DEV)
+        ops.masked_attention_tiles(q[first:first + count].contiguous(), out, cache, table, meta, 1, None, None, H, 1, D, D, window, keep, 0.05)
+        return out
+
+    i = torch.arange(n, device=DEV)
+    for key in (101, 154, 399):                     # the second and the first token of a block, the last of all
+        damaged = pages.clone()
+        damaged[key // page, 0, 0, key % page] = bad
+        sees = (i >= key) & ((i - key < window) | (key < keep)) if window else i >= key
+        for first, count in ((0, n), (90, 99), (301, 99)):
+            clean, got, seen = run(pages, first, count), run(damaged, first, count), sees[first:first + count]
+            assert torch.equal(got[~seen], clean[~seen]) and torch.isfinite(clean).all()
+            assert not torch.isfinite(got[seen].float()).all() or not seen.any()
