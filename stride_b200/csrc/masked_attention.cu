@@ -861,13 +861,16 @@ __global__ void __launch_bounds__(128 * RG) masked_attention_tile_kernel(TilePar
 
 // Two row groups a CTA for long value rows (NVW = 8: 246 registers a thread leave room for eight warps on an SM either way) once they are
 // enough to fill the SMs: the two share a double-buffered tile of keys, where two CTAs of one group each had a single buffer and a copy of
-// their own (16 heads over latents of 512, window 1,024, prompts of 333, 584 and 1,025 tokens: 282 us a layer, 310 so).
+// their own. Only where the entries are long: an entry whose tokens are an odd number of groups leaves half a CTA idle, and one token is all
+// of it (a group an SM then, two otherwise). Latents of 512, microseconds, pairs / single: 16 heads, a prompt of 2,048 tokens 667 / 735,
+// 1,500 tokens beside 64 entries of one (24 groups an entry) 650 / 699, 300 entries of one 181 / 130; 64 heads, 40 entries of nine tokens
+// 204 / 192, 301 tokens beside 99 of one (four groups an entry) 320 / 300.
 template <int NVW>
 int launch_pairs(const TileParams& p, int n, int y, int PT, size_t stage, cudaStream_t stream, bool* done) {
   const size_t smem = 2 * KT * sizeof(void*) + 2 * (2 * NK * 4 * 32 * sizeof(uint32_t) + 4 * 16 * sizeof(float) + sizeof(bf16) * 16 * (p.D + 8)) + 2 * stage +
                       sizeof(bf16) * ((p.v_offset != 0 ? p.Dv : p.D) + 8);
   const dim3 grid((n + 2 * PT - 1) / (2 * PT) + p.entries, y);
-  *done = smem <= 220 * 1024 && static_cast<int64_t>((n + 2 * PT - 1) / (2 * PT)) * y >= sb::sm_count();
+  *done = smem <= 220 * 1024 && static_cast<int64_t>((n + 2 * PT - 1) / (2 * PT)) * y >= sb::sm_count() && n >= 12 * PT * p.entries;
   if (!*done) return 0;
   TileParams q = p;
   q.stages = 2;
