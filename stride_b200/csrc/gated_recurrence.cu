@@ -103,18 +103,24 @@ __global__ void __launch_bounds__(DL * 64, 1024 / (DL * 64)) gated_step_kernel(c
   const int e = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * 32;
   const int slot = p.meta[e], row0 = p.meta[p.meta_stride + e], len = p.meta[2 * p.meta_stride + e], pos0 = p.meta[3 * p.meta_stride + e];
   sb::grid_dependency_wait();
-  sbscan::step_core<DL, true>(p, smem, slot, row0, len, pos0, [&](float* to, int Dp, int row) {
+  sbscan::step_core<DL, true>(p, smem, slot, row0, len, pos0, [&](float* to, int Ds, int row) {
+    // up to three values a thread, requested together (2 Ds threads, 3 Ds + 32 values, Ds >= 16)
     const float* src = p.rows + static_cast<int64_t>(row) * p.width;
-    for (int j = threadIdx.x; j < 3 * Dp + 32; j += blockDim.x) {
-      float v = 0.0f;
-      if (j < 3 * Dp) {
-        const int which = j / Dp, d = j - which * Dp;          // q, k, g
-        if (d < p.D) v = src[(which == 0 ? p.q_off : which == 1 ? p.k_off : p.g_off) + h * p.D + d];
-      } else if (c0 + j - 3 * Dp < p.V) {
-        v = src[p.v_off + h * p.V + c0 + j - 3 * Dp];
+    float v[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int j = threadIdx.x + k * blockDim.x;
+      v[k] = 0.0f;
+      if (j < 3 * Ds) {
+        const int which = j / Ds, d = j - which * Ds;          // q, k, g
+        if (d < p.D) v[k] = src[(which == 0 ? p.q_off : which == 1 ? p.k_off : p.g_off) + h * p.D + d];
+      } else if (j < 3 * Ds + 32 && c0 + j - 3 * Ds < p.V) {
+        v[k] = src[p.v_off + h * p.V + c0 + j - 3 * Ds];
       }
-      to[j] = v;
     }
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      if (threadIdx.x + k * blockDim.x < 3 * Ds + 32) to[threadIdx.x + k * blockDim.x] = v[k];
   });
 }
 

@@ -57,22 +57,22 @@ __device__ __forceinline__ float4 folded4(const float* p, int n_partials, int64_
 
 // Steps with as many tokens as entries (decoding): the partial sums folded (and activated) inside.
 template <int DL>
-__global__ void __launch_bounds__(DL * 64, 768 / (DL * 64)) lightning_step_kernel(const sbscan::Params p, int n_partials, int64_t partial_stride, int activated) {
+__global__ void __launch_bounds__(DL * 64, DL == 2 ? 7 : 1024 / (DL * 64)) lightning_step_kernel(const sbscan::Params p, int n_partials, int64_t partial_stride, int activated) {
   extern __shared__ __align__(16) float smem[];
   sb::grid_launch_dependents();
   const int e = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * 32;
   const int slot = p.meta[e], row0 = p.meta[p.meta_stride + e], len = p.meta[2 * p.meta_stride + e], pos0 = p.meta[3 * p.meta_stride + e];
   sb::grid_dependency_wait();
-  sbscan::step_core<DL, false>(p, smem, slot, row0, len, pos0, [&](float* to, int Dp, int row) {
+  sbscan::step_core<DL, false>(p, smem, slot, row0, len, pos0, [&](float* to, int Ds, int row) {
     const float* src = p.rows + static_cast<int64_t>(row) * p.width;
 #pragma unroll 1
-    for (int j = threadIdx.x; j < 2 * Dp + 32; j += blockDim.x) {
-      const int d = j >= Dp ? j - Dp : j;
+    for (int j = threadIdx.x; j < 2 * Ds + 32; j += blockDim.x) {
+      const int d = j >= Ds ? j - Ds : j;
       const float* at = nullptr;
-      if (j < 2 * Dp) {
-        if (d < p.D) at = src + (j >= Dp ? p.k_off : p.q_off) + h * p.D + d;
-      } else if (c0 + j - 2 * Dp < p.V) {
-        at = src + p.v_off + h * p.V + c0 + j - 2 * Dp;
+      if (j < 2 * Ds) {
+        if (d < p.D) at = src + (j >= Ds ? p.k_off : p.q_off) + h * p.D + d;
+      } else if (c0 + j - 2 * Ds < p.V) {
+        at = src + p.v_off + h * p.V + c0 + j - 2 * Ds;
       }
       float v = 0.0f;
       if (at != nullptr) {

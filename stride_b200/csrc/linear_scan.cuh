@@ -24,7 +24,7 @@ namespace sbscan {
 constexpr int kLanes = 32;       // parts of the D sums
 constexpr int kWarps = 4;        // computing warps of scan_kernel
 constexpr int kChunk = 16;       // tokens staged in shared memory at a time
-constexpr int kStages = 3;       // staging buffers of scan_kernel
+constexpr int kMaxStages = 3;    // staging buffers of scan_kernel, at most
 
 inline int lane_elements(int D) { return D <= 64 ? 2 : D <= 128 ? 4 : 8; }
 
@@ -68,22 +68,25 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
 template <int DL, bool GATED>
 struct Part {
   float2 k[DL / 2], q[DL / 2], g[GATED ? DL / 2 : 1];
+  // GAP: floats from one of the part's pieces of four elements to the next
+  template <int GAP>
   static __device__ __forceinline__ void fetch(float2 (&to)[DL / 2], const float* from) {
     if constexpr (DL == 2) {
       to[0] = *reinterpret_cast<const float2*>(from);
     } else {
 #pragma unroll
       for (int i = 0; i < DL / 4; ++i) {
-        const float4 v = reinterpret_cast<const float4*>(from)[i];
+        const float4 v = *reinterpret_cast<const float4*>(from + i * GAP);
         to[2 * i] = make_float2(v.x, v.y);
         to[2 * i + 1] = make_float2(v.z, v.w);
       }
     }
   }
+  template <int GAP>
   __device__ __forceinline__ void load(const float* sq, const float* sk, const float* sg) {
-    fetch(k, sk);
-    fetch(q, sq);
-    if constexpr (GATED) fetch(g, sg);
+    fetch<GAP>(k, sk);
+    fetch<GAP>(q, sq);
+    if constexpr (GATED) fetch<GAP>(g, sg);
   }
 };
 
@@ -123,7 +126,7 @@ __device__ __forceinline__ float transpose_add(float (&a)[32], int lane) {
 }
 
 // Named barriers of scan_kernel (id 0 is __syncthreads): one per buffer and direction.
-enum { kBarFull = 1, kBarEmpty = 1 + kStages };
+enum { kBarFull = 1, kBarEmpty = 1 + kMaxStages };
 __device__ __forceinline__ void bar_sync(int id, int count) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int count) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory"); }
 
@@ -135,35 +138,64 @@ __device__ __forceinline__ void bar_arrive(int id, int count) { asm volatile("ba
 // or two computing warps a scheduler (issue slots 47% busy; without the loads and the exchanges 155 of its 220 us are left).
 // Measured (16 heads of 128 x 128, one entry of 2,048 tokens / eight): eight warps of one column a thread, the outputs' parts through shared
 // memory, 611 / 1,600 us; PER = 4 220 / 721 us, PER = 2 193 / 828 us.
-template <int DL, int PER, bool GATED, int VEC>
-__global__ void __launch_bounds__(kWarps * 32 + 32) scan_kernel(const Params p) {
+// With eight elements a lane: the row's pieces of four lie the even ones first, then the odd ones, so that the lanes' 16-byte reads take
+// neighbouring places (side by side they would meet in half the banks), and with gates two staging buffers, which leaves two CTAs an SM.
+template <int DL, bool GATED>
+__host__ __device__ constexpr int stages_of() { return DL == 8 && GATED ? 2 : kMaxStages; }
+template <int DL>
+__device__ __forceinline__ int staged_at(int d) { return DL == 8 ? (d >> 2 & 1) * (kLanes * 4) + (d >> 3) * 4 + (d & 3) : d; }
+
+template <int DL, int PER, bool GATED, int VEC, bool PAD>      // PAD: the key size is less than the lanes' elements
+__global__ void __launch_bounds__(kWarps * 32 + 32, DL == 8 ? 2 : DL == 4 && PER == 4 ? 3 : 0) scan_kernel(const Params p) {
   extern __shared__ __align__(16) float smem[];
   sb::grid_launch_dependents();
+  constexpr int kStages = stages_of<DL, GATED>(), kGap = DL == 8 ? kLanes * 4 : 4;
   constexpr int kCols = kWarps * PER, kGroup = 32 / PER;       // a group: the tokens whose outputs a warp adds up together
   constexpr int Dp = kLanes * DL, NC = kWarps * 32, NQ = GATED ? 3 : 2, stage = kChunk * (NQ * Dp + kCols);
   const int e = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * kCols, vn = min(kCols, p.V - c0);
   const int slot = p.meta[e], row0 = p.meta[p.meta_stride + e], len = p.meta[2 * p.meta_stride + e], pos0 = p.meta[3 * p.meta_stride + e];
   const int chunks = (len + kChunk - 1) / kChunk;
   // nothing copies into the cells beyond D and beyond the CTA's existing columns: they are zero for good
-  if (Dp != p.D || vn != kCols)
-    for (int i = threadIdx.x; i < kStages * stage; i += blockDim.x) smem[i] = 0.0f;
+  if (PAD || vn != kCols) {
+    auto clear = [](float* at, int floats) {
+      for (int i = threadIdx.x * 4; i < floats; i += (kWarps + 1) * 128) *reinterpret_cast<float4*>(at + i) = make_float4(0, 0, 0, 0);
+    };
+    for (int b = 0; b < kStages; ++b) {
+      const int rows = min(kChunk, len - b * kChunk);            // that tokens will use
+      if (rows <= 0) break;
+      for (int k = 0; k < NQ; ++k) clear(smem + b * stage + k * kChunk * Dp, rows * Dp);
+      clear(smem + b * stage + NQ * kChunk * Dp, rows * kCols);
+    }
+  }
   sb::grid_dependency_wait();
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (warp < kWarps) {
     // ---------------------------------------------------------------- the recurrence
     const float decay = GATED ? 0.0f : p.decay[h];
-    const int cl = warp * PER, dn = min(DL, p.D - lane * DL);
+    const int cl = warp * PER, dn = PAD ? min(DL, p.D - lane * DL) : DL;
     float* st = p.state + ((static_cast<int64_t>(slot) * p.H + h) * p.D + lane * DL) * p.V + c0 + cl;
     float2 S[PER][DL / 2];
+    using Columns = typename std::conditional<PER == 4, float4, float2>::type;      // (VEC == 4: a warp's columns all exist, or none)
 #pragma unroll
-    for (int i = 0; i < DL; ++i)
+    for (int i = 0; i < DL; ++i) {
+      alignas(16) float row[PER];
 #pragma unroll
-      for (int c = 0; c < PER; ++c) put(S[c], i, pos0 > 0 && cl + c < vn && i < dn ? st[static_cast<int64_t>(i) * p.V + c] : 0.0f);
+      for (int c = 0; c < PER; ++c) row[c] = 0.0f;
+      if constexpr (VEC == 4) {
+        if (pos0 > 0 && cl < vn && i < dn) *reinterpret_cast<Columns*>(row) = *reinterpret_cast<const Columns*>(st + static_cast<int64_t>(i) * p.V);
+      } else {
+#pragma unroll
+        for (int c = 0; c < PER; ++c)
+          if (pos0 > 0 && cl + c < vn && i < dn) row[c] = st[static_cast<int64_t>(i) * p.V + c];
+      }
+#pragma unroll
+      for (int c = 0; c < PER; ++c) put(S[c], i, row[c]);
+    }
     float* out = p.out + static_cast<int64_t>(row0) * p.H * p.V + h * p.V + c0 + cl + (lane & (PER - 1));
     const bool live = cl + (lane & (PER - 1)) < vn;
     for (int c = 0, b = 0; c < chunks; ++c, b = b + 1 == kStages ? 0 : b + 1) {
-      const float* sq = smem + b * stage + lane * DL;
+      const float* sq = smem + b * stage + lane * min(DL, 4);
       const float* sv = smem + b * stage + NQ * kChunk * Dp + cl;
       bar_sync(kBarFull + b, NC + 32);
 #pragma unroll 1
@@ -178,7 +210,7 @@ __global__ void __launch_bounds__(kWarps * 32 + 32) scan_kernel(const Params p) 
           float v[2][PER];
           auto load = [&](int t, int at) {
             const float* row = sq + (t0 + t) * Dp;
-            x[at].load(row, row + kChunk * Dp, row + (GATED ? 2 : 0) * kChunk * Dp);
+            x[at].template load<kGap>(row, row + kChunk * Dp, row + (GATED ? 2 : 0) * kChunk * Dp);
             const float* from = sv + (t0 + t) * kCols;
             if constexpr (PER == 4) {
               const float4 w = *reinterpret_cast<const float4*>(from);
@@ -204,7 +236,7 @@ __global__ void __launch_bounds__(kWarps * 32 + 32) scan_kernel(const Params p) 
         if (nt == kGroup) walk(std::true_type{});
         else walk(std::false_type{});
         if (t0 + kGroup >= min(kChunk, len - c * kChunk) && c + kStages < chunks) bar_arrive(kBarEmpty + b, NC + 32);
-        if (dn <= 0) {      // a part beyond D: zeros, whatever 0 times an infinite value is
+        if (PAD && dn <= 0) {      // a part beyond D: zeros, whatever 0 times an infinite value is
 #pragma unroll
           for (int i = 0; i < 32; ++i) sums[i] = 0.0f;
         }
@@ -214,10 +246,18 @@ __global__ void __launch_bounds__(kWarps * 32 + 32) scan_kernel(const Params p) 
       }
     }
 #pragma unroll
-    for (int i = 0; i < DL; ++i)
+    for (int i = 0; i < DL; ++i) {
+      alignas(16) float row[PER];
 #pragma unroll
-      for (int c = 0; c < PER; ++c)
-        if (cl + c < vn && i < dn) st[static_cast<int64_t>(i) * p.V + c] = get(S[c], i);
+      for (int c = 0; c < PER; ++c) row[c] = get(S[c], i);
+      if constexpr (VEC == 4) {
+        if (cl < vn && i < dn) *reinterpret_cast<Columns*>(st + static_cast<int64_t>(i) * p.V) = *reinterpret_cast<const Columns*>(row);
+      } else {
+#pragma unroll
+        for (int c = 0; c < PER; ++c)
+          if (cl + c < vn && i < dn) st[static_cast<int64_t>(i) * p.V + c] = row[c];
+      }
+    }
   } else {
     // ---------------------------------------------------------------- the loads
     const int du = p.D / VEC, vu = vn / VEC;      // (VEC == 4 only when every size and offset is a multiple of four)
@@ -228,7 +268,7 @@ __global__ void __launch_bounds__(kWarps * 32 + 32) scan_kernel(const Params p) 
       const float* from = src0 + static_cast<int64_t>(c) * kChunk * p.width;
       for (int u = lane; u < du; u += 32) {
         const float* src = from + h * p.D + u * VEC;
-        float* dst = to + u * VEC;
+        float* dst = to + staged_at<DL>(u * VEC);
 #pragma unroll 4
         for (int t = 0; t < nt; ++t, src += p.width, dst += Dp) {
           copy_async<VEC>(dst, src + p.q_off);
@@ -262,19 +302,22 @@ __global__ void __launch_bounds__(kWarps * 32 + 32) scan_kernel(const Params p) 
 template <int DL, int PER, bool GATED>
 int launch_scan_of(const Params& p, int entries, const char* who, cudaStream_t stream) {
   constexpr int kCols = kWarps * PER;
-  constexpr size_t smem = sizeof(float) * kStages * kChunk * ((GATED ? 3 : 2) * kLanes * DL + kCols);
+  constexpr size_t smem = sizeof(float) * stages_of<DL, GATED>() * kChunk * ((GATED ? 3 : 2) * kLanes * DL + kCols);
   static_assert(smem <= 200 * 1024, "staging buffers");
   const bool vec = p.D % 4 == 0 && p.V % 4 == 0 && p.width % 4 == 0 && p.q_off % 4 == 0 && p.k_off % 4 == 0 && p.v_off % 4 == 0 &&
-                   (!GATED || p.g_off % 4 == 0) && (reinterpret_cast<uintptr_t>(p.rows) & 15) == 0;
+                   (!GATED || p.g_off % 4 == 0) &&
+                   ((reinterpret_cast<uintptr_t>(p.rows) | reinterpret_cast<uintptr_t>(p.state)) & 15) == 0;
+  // (without gates and with two columns a warp the form that looks at the lanes' sizes is the faster one also where they are full: one entry of
+  // 2,048 tokens, 16 heads of 128 x 128, 154 us and 178)
+  const bool pad = p.D != kLanes * DL || (!GATED && DL == 4 && PER == 2);
+  const auto kernel = !vec ? scan_kernel<DL, PER, GATED, 1, true> : pad ? scan_kernel<DL, PER, GATED, 4, true> : scan_kernel<DL, PER, GATED, 4, false>;
   static sb::DeviceOnce once;
   if (once.needed()) {
-    cudaFuncSetAttribute(scan_kernel<DL, PER, GATED, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(scan_kernel<DL, PER, GATED, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    for (const auto k : {scan_kernel<DL, PER, GATED, 1, true>, scan_kernel<DL, PER, GATED, 4, true>, scan_kernel<DL, PER, GATED, 4, false>})
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     once.done();
   }
-  const dim3 grid(entries, p.H, (p.V + kCols - 1) / kCols), block(kWarps * 32 + 32);
-  if (vec) sb::launch_pdl(scan_kernel<DL, PER, GATED, 4>, grid, block, smem, stream, p);
-  else sb::launch_pdl(scan_kernel<DL, PER, GATED, 1>, grid, block, smem, stream, p);
+  sb::launch_pdl(kernel, dim3(entries, p.H, (p.V + kCols - 1) / kCols), dim3(kWarps * 32 + 32), smem, stream, p);
   return sb::check_launch(who);
 }
 
@@ -293,15 +336,15 @@ int launch_scan(const Params& p, int entries, const char* who, cudaStream_t stre
 }
 
 // Steps with as many tokens as entries: a CTA is (entry, head, 32 value columns), a thread kRows elements of one column (what a warp reads of
-// the state is whole 128-byte rows). The state's loads are requested first; `fill(smem, Dp, row)` writes the token's q, k, (g,) v into shared
-// memory meanwhile: q, k, g [Dp] each, zero beyond D, v [32]. The same operations in the same order as scan_kernel: a thread adds its own
-// neighbouring parts, the warps' sums are the upper levels of the tree.
+// the state is whole 128-byte rows). The state's loads are requested first; `fill(smem, Ds, row)` writes the token's q, k, (g,) v into shared
+// memory meanwhile: q, k, g [Ds] each (D in whole warps), zero beyond D, v [32]. The same operations in the same order as scan_kernel: a
+// thread adds its own neighbouring parts, the warps' sums are the upper levels of the tree, in which the parts beyond the last warp's are zeros.
 constexpr int kRows = 16;
 template <int DL, bool GATED, class Fill>
 __device__ __forceinline__ void step_token(const Params& p, float* smem, int slot, int row, int pos, int V, Fill fill) {
-  constexpr int Dp = kLanes * DL, kParts = kRows / DL, warps = Dp / kRows;
-  const int h = blockIdx.y, c0 = blockIdx.z * 32, warp = threadIdx.x >> 5, cl = threadIdx.x & 31;
-  float* sv = smem + (GATED ? 3 : 2) * Dp;
+  constexpr int kParts = kRows / DL, warps = kLanes * DL / kRows;
+  const int h = blockIdx.y, c0 = blockIdx.z * 32, warp = threadIdx.x >> 5, cl = threadIdx.x & 31, Ds = blockDim.x / 32 * kRows;
+  float* sv = smem + (GATED ? 3 : 2) * Ds;
   float* so = sv + 32;         // [warps][32]
   const bool live = c0 + cl < V;
   const int d0 = warp * kRows, dn = min(kRows, p.D - d0);
@@ -310,14 +353,14 @@ __device__ __forceinline__ void step_token(const Params& p, float* smem, int slo
   float2 S[kParts][DL / 2];
 #pragma unroll
   for (int i = 0; i < kRows; ++i) put(S[i / DL], i % DL, pos > 0 && live && i < dn ? st[static_cast<int64_t>(i) * V] : 0.0f);
-  fill(smem, Dp, row);
+  fill(smem, Ds, row);
   __syncthreads();
   float a[kParts];
 #pragma unroll
   for (int j = 0; j < kParts; ++j) {
     const float* sq = smem + d0 + j * DL;
     Part<DL, GATED> x;
-    x.load(sq, sq + Dp, sq + (GATED ? 2 : 0) * Dp);
+    x.template load<4>(sq, sq + Ds, sq + (GATED ? 2 : 0) * Ds);
     a[j] = token<DL, GATED>(S[j], x, j * DL < dn ? sv[cl] : 0.0f, decay);
   }
 #pragma unroll
@@ -334,7 +377,7 @@ __device__ __forceinline__ void step_token(const Params& p, float* smem, int slo
   if (warp == 0 && live) {
     float w[warps];
 #pragma unroll
-    for (int q = 0; q < warps; ++q) w[q] = so[q * 32 + cl];
+    for (int q = 0; q < warps; ++q) w[q] = q * 32 < blockDim.x ? so[q * 32 + cl] : 0.0f;
 #pragma unroll
     for (int m = 1; m < warps; m <<= 1)
 #pragma unroll
@@ -358,7 +401,7 @@ __device__ __forceinline__ void step_core(const Params& p, float* smem, int slot
   }
 }
 
-inline int step_threads(int D) { return kLanes * lane_elements(D) / kRows * 32; }
-inline size_t step_smem(int D, bool gated) { return sizeof(float) * ((gated ? 3 : 2) * kLanes * lane_elements(D) + 32 + step_threads(D)); }
+inline int step_threads(int D) { return (D + kRows - 1) / kRows * 32; }
+inline size_t step_smem(int D, bool gated) { return sizeof(float) * ((gated ? 3 : 2) * (step_threads(D) / 32 * kRows) + 32 + step_threads(D)); }
 
 }  // namespace sbscan

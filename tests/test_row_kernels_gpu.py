@@ -262,3 +262,48 @@ def test_rows_never_meet_keys_they_do_not_see(bad, window, keep):
             clean, got, seen = run(pages, first, count), run(damaged, first, count), sees[first:first + count]
             assert torch.equal(got[~seen], clean[~seen]) and torch.isfinite(clean).all()
             assert not torch.isfinite(got[seen].float()).all() or not seen.any()
+
+
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("D,V", [(64, 128), (10, 40), (128, 40), (126, 30), (200, 128), (130, 30), (256, 16)])
+def test_recurrence_does_not_show_its_columns_a_warp(D, V, gated):
+    """More CTAs of sixteen columns than SMs (four columns a warp) against each entry alone (two) and token by token, in equal bits: key sizes
+    of every number of elements a lane, with and without padding, 16-byte and single-element copies, columns that do not fill a CTA. The
+    outputs of the longest entry lie within 2e-5 of the largest of the recurrence in 64 bits, the bound of the recurrence's other tests."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(D + V)
+    lengths, H, E = [37, 1, 70, 16, 2, 33, 8, 9, 3, 5], 16, 10
+    n, HD, HV = sum(lengths), 16 * D, 16 * V
+    assert E * H * ((V + 15) // 16) > 148 >= H * ((V + 15) // 16)
+    rows = [sum(lengths[:i]) for i in range(E)]
+    x = torch.randn(n, 3 * HD + HV, generator=g) * 0.5
+    x[:, HD:2 * HD] = torch.rand(n, HD, generator=g)
+    x, decay = x.to(DEV), torch.linspace(0.5, 0.999, H, device=DEV)
+
+    def run(first, count, entries, state):
+        meta = torch.tensor([[e[k] for e in entries] for k in range(4)], dtype=torch.int32, device=DEV)
+        part, out = x[first:first + count].contiguous(), torch.zeros(count, HV, device=DEV)
+        if gated:
+            ops.gated_scan(part, 0, HD, 2 * HD, 3 * HD, meta, len(entries), state, out, H, D, V)
+        else:
+            ops.lightning_scan(part, 0, 2 * HD, 3 * HD, meta, len(entries), decay, state, out, H, D, V, torch.empty_like(part))
+        return out
+
+    garbage = torch.randn(E, H, D, V, generator=g).to(DEV)
+    together, alone, single = garbage.clone(), garbage.clone(), garbage.clone()
+    whole = run(0, n, [(E - 1 - i, rows[i], lengths[i], 0) for i in range(E)], together)
+    for i in range(E):
+        assert torch.equal(run(rows[i], lengths[i], [(E - 1 - i, 0, lengths[i], 0)], alone), whole[rows[i]:rows[i] + lengths[i]])
+        for t in range(lengths[i]):
+            assert torch.equal(run(rows[i] + t, 1, [(E - 1 - i, 0, 1, t)], single)[0], whole[rows[i] + t])
+    assert torch.equal(together, alone) and torch.equal(together, single)
+    longest = x[rows[2]:rows[2] + lengths[2]].double()
+    if not gated:
+        longest = torch.nn.functional.silu(longest)
+    q, f, k = (longest[:, i * HD:(i + 1) * HD].view(-1, H, D) for i in range(3))
+    v, S, want = longest[:, 3 * HD:].view(-1, H, V), torch.zeros(H, D, V, dtype=torch.float64, device=DEV), []
+    for t in range(lengths[2]):
+        S = (f[t][:, :, None] if gated else decay.double()[:, None, None]) * S + k[t][:, :, None] * v[t][:, None, :]
+        want.append(torch.einsum("hdv,hd->hv", S, q[t]).reshape(-1))
+    want = torch.stack(want)
+    assert (whole[rows[2]:rows[2] + lengths[2]].double() - want).abs().max() <= 2e-5 * float(want.abs().max())
