@@ -16,7 +16,7 @@ using bf16 = __nv_bfloat16;
 // right first (as the tensor-core kernel adds its K ranges when it does so itself) and then added
 // to h; when partials are given the sum is written back to h. Then
 // r = 1/sqrt(sum(x^2)/H + eps) and out = w * (x * r). VEC = 4 reads float4 (H % 4 == 0);
-// the partials are fetched four at a time so that their loads overlap.
+// FLIGHT partials are fetched together so that their loads overlap.
 template <int VEC>
 struct VecF;
 template <>
@@ -27,10 +27,12 @@ struct VecF<1> { using type = float; };
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 __device__ __forceinline__ float add4(float a, float b) { return a + b; }
 
-// FLIGHT: the partial sums requested together. With few rows 12: every one is a round trip to L2. With more rows than SMs 6: two blocks an SM
-// instead of one (256 rows of 2,048 behind nine buffers 5.4 us, 7.1 with 12). The additions are the same: equal bits.
-template <class TW, class TO, int VEC, int MAXT, int FLIGHT>     // MAXT: the most threads of a block
-__global__ void __launch_bounds__(MAXT, FLIGHT == 6 ? 2 : 1) rmsnorm_kernel(float* __restrict__ h, const float* __restrict__ partials, int n_partials,
+// FLIGHT: the partial sums requested together. 12 while all rows run at once: every one is a round trip to L2. With more rows 6, twice the
+// blocks an SM (256 rows of 2,048 behind nine buffers 5.4 us, 7.1 with 12; 256 rows of 1,024, which run at once with 12, 3.7 and 3.0).
+// The additions are the same: equal bits. BLOCKS: the blocks an SM that the registers are cut for (0: left to the compiler); two in the
+// single-element form (2,048 rows of 2,050 behind one buffer: 30 us, 43 with one).
+template <class TW, class TO, int VEC, int MAXT, int FLIGHT, int BLOCKS>     // MAXT: the most threads of a block
+__global__ void __launch_bounds__(MAXT, BLOCKS) rmsnorm_kernel(float* __restrict__ h, const float* __restrict__ partials, int n_partials,
                                int64_t partial_stride, const TW* __restrict__ weight, TO* __restrict__ out,
                                int H, float eps) {
   using V = typename VecF<VEC>::type;
@@ -62,8 +64,7 @@ __global__ void __launch_bounds__(MAXT, FLIGHT == 6 ? 2 : 1) rmsnorm_kernel(floa
 #pragma unroll
       for (int s = 1; s < kInFlight; ++s)
         if (s < n_partials) sum = add4(sum, part[s]);
-      if constexpr (FLIGHT > 1)
-        for (int s = kInFlight; s < n_partials; ++s) sum = add4(sum, p[s * ps]);
+      for (int s = kInFlight; s < n_partials; ++s) sum = add4(sum, p[s * ps]);
       v = add4(v, sum);
       hr[i] = v;
     }
@@ -224,15 +225,23 @@ __global__ void __launch_bounds__(512) rmsnorm_pairs_kernel(float* __restrict__ 
 // One block per row: x = h + (partial_0 + partial_1 + ...) as in rmsnorm_kernel (written back to h when partials are given);
 // mean = sum(x) / H; var = sum((x - mean)^2) / H; out = (x - mean) / sqrt(var + eps) * w + b. Both sums in the order of sb::block_sum.
 // VEC = 4: four elements an access where the width and every buffer allow it; which form runs depends on the width and the buffers alone,
-// never on the rows, so a row's result does not either. A thread keeps its first kKeep pieces in registers through both sums; wider rows are
-// read again. Bound by memory: 2,048 rows of 2,048 with one partial buffer 10.5 us (22 with the
-// registers for eight partial buffers), single elements in shared memory 24 us.
-template <class TW, class TO, int VEC, int MAXT, bool ONE>     // MAXT: the most threads of a block, ONE: at most one partial buffer, as in rmsnorm_kernel
-__global__ void __launch_bounds__(MAXT) layernorm_kernel(float* __restrict__ h, const float* __restrict__ partials, int n_partials,
+// never on the rows, so a row's result does not either. A thread keeps its first kKeep pieces in registers through both sums, those beyond in
+// shared memory. Bound by memory: 2,048 rows of 2,048 with one partial buffer 10.5 us (22 with the registers for eight partial buffers,
+// hence FLIGHT), single elements in shared memory 24 us.
+// The blocks an SM that its registers are cut for (0: left to the compiler).
+constexpr int layernorm_blocks(int VEC, int MAXT, int FLIGHT, size_t bytes) {
+  if (VEC == 1) return 2048 / MAXT;
+  if (FLIGHT == 1) return bytes == 4 ? 4 : 3;      // (of 512 threads: 32 registers a thread where gain and output are bfloat16, else 40)
+  return FLIGHT == 4 ? 1024 / MAXT : 0;
+}
+template <class TW, class TO, int VEC, int MAXT, int FLIGHT>     // MAXT: the most threads of a block, FLIGHT: the partial sums requested together
+__global__ void __launch_bounds__(MAXT, layernorm_blocks(VEC, MAXT, FLIGHT, sizeof(TW) + sizeof(TO))) layernorm_kernel(float* __restrict__ h, const float* __restrict__ partials, int n_partials,
                                                          int64_t partial_stride, const TW* __restrict__ weight,
                                                          const TW* __restrict__ bias, TO* __restrict__ out, int H, float eps) {
   using V = typename VecF<VEC>::type;
-  constexpr int kKeep = 2;
+  constexpr int kKeep = VEC == 4 ? 2 : 1;
+  constexpr bool kBeyond = VEC == 1 || MAXT > 512 || FLIGHT == 8;      // (512 threads and fewer keep all of a row)
+  extern __shared__ __align__(16) float beyond_raw[];
   __shared__ float red[32];
   sb::grid_launch_dependents();
   sb::grid_dependency_wait();
@@ -242,7 +251,7 @@ __global__ void __launch_bounds__(MAXT) layernorm_kernel(float* __restrict__ h, 
   auto fetch = [&](int i) {
     V v = hr[i];
     if (n_partials > 0) {
-      constexpr int kInFlight = ONE ? 1 : 8;
+      constexpr int kInFlight = FLIGHT;
       const V* p = reinterpret_cast<const V*>(partials + r * H) + i;
       const int64_t ps = partial_stride / VEC;
       V part[kInFlight];
@@ -253,7 +262,7 @@ __global__ void __launch_bounds__(MAXT) layernorm_kernel(float* __restrict__ h, 
 #pragma unroll
       for (int s = 1; s < kInFlight; ++s)
         if (s < n_partials) sum = add4(sum, part[s]);
-      if constexpr (!ONE)
+      if constexpr (FLIGHT > 1)      // (1: there is no more than one)
         for (int s = kInFlight; s < n_partials; ++s) sum = add4(sum, p[s * ps]);
       v = add4(v, sum);
       hr[i] = v;
@@ -272,19 +281,20 @@ __global__ void __launch_bounds__(MAXT) layernorm_kernel(float* __restrict__ h, 
       return fmaf(v - mean, v - mean, sq);
     }
   };
-  const int beyond = kKeep * blockDim.x + threadIdx.x;
+  const int kept = kKeep * blockDim.x, beyond = kept + threadIdx.x;
+  V* rest = reinterpret_cast<V*>(beyond_raw);
   V keep[kKeep];
   float sum = 0.0f;
 #pragma unroll
   for (int j = 0; j < kKeep; ++j)
     if (threadIdx.x + j * blockDim.x < units) sum += total(keep[j] = fetch(threadIdx.x + j * blockDim.x));
-  for (int i = beyond; i < units; i += blockDim.x) sum += total(fetch(i));
+  for (int i = beyond; kBeyond && i < units; i += blockDim.x) sum += total(rest[i - kept] = fetch(i));
   const float mean = sb::block_sum(sum, red) / static_cast<float>(H);
   float sq = 0.0f;
 #pragma unroll
   for (int j = 0; j < kKeep; ++j)
     if (threadIdx.x + j * blockDim.x < units) sq = apart(keep[j], mean, sq);
-  for (int i = beyond; i < units; i += blockDim.x) sq = apart(hr[i], mean, sq);
+  for (int i = beyond; kBeyond && i < units; i += blockDim.x) sq = apart(rest[i - kept], mean, sq);
   const float scale = 1.0f / sqrtf(sb::block_sum(sq, red) / static_cast<float>(H) + eps);
   auto write = [&](int i, V v) {
     if constexpr (VEC == 4) {
@@ -299,7 +309,7 @@ __global__ void __launch_bounds__(MAXT) layernorm_kernel(float* __restrict__ h, 
 #pragma unroll
   for (int j = 0; j < kKeep; ++j)
     if (threadIdx.x + j * blockDim.x < units) write(threadIdx.x + j * blockDim.x, keep[j]);
-  for (int i = beyond; i < units; i += blockDim.x) write(i, hr[i]);
+  for (int i = beyond; kBeyond && i < units; i += blockDim.x) write(i, rest[i - kept]);
 }
 
 }  // namespace
@@ -308,19 +318,29 @@ __global__ void __launch_bounds__(MAXT) layernorm_kernel(float* __restrict__ h, 
 SB_EXPORT int sb_layernorm(float* h, const float* partials, int n_partials, int64_t partial_stride, const void* weight,
                            const void* bias, int weight_dtype, void* out, int out_dtype, int n, int H, float eps, cudaStream_t stream) {
   if (n <= 0) return 0;
-  if (H > 50 * 1024) return sb::fail("sb_layernorm: width %d does not fit the row buffer (max 51200)", H);
+  if (H > 50 * 1024) return sb::fail("sb_layernorm: width %d (at most 51200)", H);
   auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   const bool vec = H % 4 == 0 && aligned(h) && aligned(partials) && aligned(weight) && aligned(bias) && aligned(out) && partial_stride % 4 == 0;
-  const int units = vec ? H / 4 : H, threads = units > 1024 ? 1024 : units > 512 ? 512 : units > 256 ? 256 : 128;
-#define SB_LN_V(TW, TO, VEC, MAXT, ONE)                                                                                       \
-  sb::launch_pdl(layernorm_kernel<TW, TO, VEC, MAXT, ONE>, n, threads, 0, stream, h, partials, n_partials, partial_stride,    \
-                 static_cast<const TW*>(weight), static_cast<const TW*>(bias), static_cast<TO*>(out), H, eps)
+  // single elements: several a thread, so that an SM holds more than one row (2,048 rows of 2,050: 17 us, 44 with 1,024 threads)
+  const int units = vec ? H / 4 : H;
+  const int threads = vec ? (units > 1024 ? 1024 : units > 512 ? 512 : units > 256 ? 256 : 128) : H >= 4096 ? 1024 : H >= 2048 ? 512 : H >= 512 ? 256 : 128;
+  const int kept = (vec ? 2 : 1) * threads;      // (kKeep pieces a thread are in registers)
+  const size_t smem = units > kept ? static_cast<size_t>(units - kept) * (vec ? 16 : 4) : 0;
+  const bool at_once = n <= sb::sm_count() * (512 / threads);      // (with eight partial sums requested together an SM holds 512 threads)
+#define SB_LN_V(TW, TO, VEC, MAXT, FLIGHT)                                                                                       \
+  do {                                                                                                                        \
+    if (smem > 40 * 1024)                                                                                                     \
+      cudaFuncSetAttribute(layernorm_kernel<TW, TO, VEC, MAXT, FLIGHT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    sb::launch_pdl(layernorm_kernel<TW, TO, VEC, MAXT, FLIGHT>, n, threads, smem, stream, h, partials, n_partials, partial_stride, \
+                   static_cast<const TW*>(weight), static_cast<const TW*>(bias), static_cast<TO*>(out), H, eps);              \
+  } while (0)
 #define SB_LN(TW, TO)                                                              \
   do {                                                                             \
-    if (vec && threads <= 512 && n_partials <= 1) SB_LN_V(TW, TO, 4, 512, true);   \
-    else if (vec && threads <= 512) SB_LN_V(TW, TO, 4, 512, false);                \
-    else if (vec) SB_LN_V(TW, TO, 4, 1024, false);                                 \
-    else SB_LN_V(TW, TO, 1, 1024, false);                                          \
+    if (vec && threads <= 512 && n_partials <= 1) SB_LN_V(TW, TO, 4, 512, 1);                    \
+    else if (vec && threads <= 512 && at_once) SB_LN_V(TW, TO, 4, 512, 8);                       \
+    else if (vec && threads <= 512) SB_LN_V(TW, TO, 4, 512, 4);                                  \
+    else if (vec) SB_LN_V(TW, TO, 4, 1024, 4);                                                   \
+    else SB_LN_V(TW, TO, 1, 1024, 8);                                                            \
   } while (0)
   if (weight_dtype == 0 && out_dtype == 0) SB_LN(float, float);
   else if (weight_dtype == 0 && out_dtype == 1) SB_LN(float, bf16);
@@ -341,11 +361,12 @@ SB_EXPORT int sb_rmsnorm(float* h, const float* partials, int n_partials, int64_
   const bool vec = H % 4 == 0 && partial_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(partials)) & 15) == 0;
   const int units = vec ? H / 4 : H;
   const int threads = units >= 1024 ? 1024 : units >= 512 ? 512 : units >= 256 ? 256 : 128;
-#define SB_NORM_V(TW, TO, VEC, MAXT, FLIGHT)                                                                     \
+  const bool at_once = n <= sb::sm_count() * (640 / threads);      // (102 registers a thread: one block of 512 an SM, two of 256, five of 128)
+#define SB_NORM_V(TW, TO, VEC, MAXT, FLIGHT, BLOCKS)                                                                     \
   do {                                                                                                           \
     if (smem > 48 * 1024)                                                                                        \
-      cudaFuncSetAttribute(rmsnorm_kernel<TW, TO, VEC, MAXT, FLIGHT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    sb::launch_pdl(rmsnorm_kernel<TW, TO, VEC, MAXT, FLIGHT>, n, threads, smem, stream, h, partials, n_partials, partial_stride, \
+      cudaFuncSetAttribute(rmsnorm_kernel<TW, TO, VEC, MAXT, FLIGHT, BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    sb::launch_pdl(rmsnorm_kernel<TW, TO, VEC, MAXT, FLIGHT, BLOCKS>, n, threads, smem, stream, h, partials, n_partials, partial_stride, \
                    static_cast<const TW*>(weight), static_cast<TO*>(out), H, eps);                               \
   } while (0)
 #define SB_NORM(TW, TO)                                                                                                         \
@@ -356,11 +377,12 @@ SB_EXPORT int sb_rmsnorm(float* h, const float* partials, int n_partials, int64_
     else if (vec && n <= 64 && threads >= 512 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(weight)) & 15) == 0) \
       sb::launch_pdl_cluster(rmsnorm_cluster_kernel<TW, TO>, dim3(n * kRowBlocks), dim3(threads / kRowBlocks), 0, stream, dim3(kRowBlocks), h, partials, \
                              n_partials, partial_stride, static_cast<const TW*>(weight), static_cast<TO*>(out), H, eps);        \
-    else if (vec && threads > 512) SB_NORM_V(TW, TO, 4, 1024, 8);                                                               \
-    else if (vec && n > sb::sm_count()) SB_NORM_V(TW, TO, 4, 512, 6);                                                           \
-    else if (vec) SB_NORM_V(TW, TO, 4, 512, 12);                                                                                \
-    else if (threads > 512) SB_NORM_V(TW, TO, 1, 1024, 8);                                                                      \
-    else SB_NORM_V(TW, TO, 1, 512, 12);                                                                                         \
+    else if (vec && threads > 512) SB_NORM_V(TW, TO, 4, 1024, 8, 1);                                                            \
+    else if (vec && !at_once) SB_NORM_V(TW, TO, 4, 512, 6, 2);                                                                  \
+    else if (vec) SB_NORM_V(TW, TO, 4, 512, 12, 0);                                                                             \
+    else if (threads > 512 && n > sb::sm_count()) SB_NORM_V(TW, TO, 1, 1024, 8, 0);                                             \
+    else if (threads > 512) SB_NORM_V(TW, TO, 1, 1024, 8, 1);                                                                   \
+    else SB_NORM_V(TW, TO, 1, 512, 12, 0);                                                                                         \
   } while (0)
   if (weight_dtype == 0 && out_dtype == 0) SB_NORM(float, float);
   else if (weight_dtype == 0 && out_dtype == 1) SB_NORM(float, bf16);

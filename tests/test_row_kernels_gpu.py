@@ -307,3 +307,25 @@ def test_recurrence_does_not_show_its_columns_a_warp(D, V, gated):
         want.append(torch.einsum("hdv,hd->hv", S, q[t]).reshape(-1))
     want = torch.stack(want)
     assert (whole[rows[2]:rows[2] + lengths[2]].double() - want).abs().max() <= 2e-5 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("H", [516, 1024, 2048, 2050, 3072, 4100, 9000])
+def test_norms_do_not_show_the_rows(H):
+    """As many rows as run at once, and more: other numbers of partial sums on their way and of blocks an SM, the same bits."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(H)
+    n, w, b = 760, torch.randn(H, generator=g).to(DEV), torch.randn(H, generator=g).to(DEV)
+    h, parts = torch.randn(n, H, generator=g).to(DEV), torch.randn(9, n, H, generator=g).to(DEV)
+
+    def run(m, norm):
+        x, out = h[:m].clone(), torch.empty(m, H, device=DEV)
+        if norm == "rms":
+            ops.rmsnorm(x, w, 1e-5, out, partials=parts[:, :m].contiguous())
+        else:
+            ops.layernorm(x, w, b, 1e-5, out, partials=parts[:, :m].contiguous())
+        return torch.cat([x, out], 1)
+
+    for norm in ("rms", "layer"):
+        whole = run(n, norm)
+        for m in (1, 149, 297, 741):
+            assert torch.equal(run(m, norm), whole[:m]), (norm, m)
