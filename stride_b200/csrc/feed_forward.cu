@@ -54,14 +54,15 @@ __device__ __forceinline__ float4 folded4(const float* p, int n_partials, int64_
 }
 
 // VE = 4: four elements an access where the size and the buffers allow it (never a matter of the rows). A thread keeps its first kKeep pieces
-// in registers between the sums and the stores; what lies beyond is folded again. The three sums share one barrier, each warp adding
+// in registers between the sums and the stores, those beyond in shared memory. The three sums share one barrier, each warp adding
 // up the warps' sums by exchanges: a fixed order. Bound by memory: 1,250 rows of 8,192 17.6 us, 64 us with single elements, a row in shared
 // memory and three block sums one after the other (8 rows: 4.2 us, 13).
 template <class TO, int VE, bool ONE>
-__global__ void __launch_bounds__(1024) polynorm_kernel(const float* __restrict__ up, int n_partials, int64_t partial_stride, TO* __restrict__ out,
+__global__ void __launch_bounds__(1024, VE == 1 ? 2 : 0) polynorm_kernel(const float* __restrict__ up, int n_partials, int64_t partial_stride, TO* __restrict__ out,
                                                          int F, float a, float b, float c, float e, float eps) {
   using V = typename std::conditional<VE == 4, float4, float>::type;
-  constexpr int kKeep = 2;
+  constexpr int kKeep = VE == 4 ? 2 : 1;
+  extern __shared__ __align__(16) float beyond_raw[];
   __shared__ float red[3][32];
   sb::grid_launch_dependents();
   sb::grid_dependency_wait();
@@ -83,6 +84,8 @@ __global__ void __launch_bounds__(1024) polynorm_kernel(const float* __restrict_
     if constexpr (VE == 4) one(v.x), one(v.y), one(v.z), one(v.w);
     else one(v);
   };
+  const int kept = kKeep * blockDim.x;
+  V* rest = reinterpret_cast<V*>(beyond_raw);
   V keep[kKeep];
 #pragma unroll
   for (int j = 0; j < kKeep; ++j)
@@ -90,7 +93,7 @@ __global__ void __launch_bounds__(1024) polynorm_kernel(const float* __restrict_
 #pragma unroll
   for (int j = 0; j < kKeep; ++j)
     if (threadIdx.x + j * blockDim.x < units) sums(keep[j]);
-  for (int i = threadIdx.x + kKeep * blockDim.x; i < units; i += blockDim.x) sums(fetch(i));
+  for (int i = threadIdx.x + kept; i < units; i += blockDim.x) sums(rest[i - kept] = fetch(i));
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
@@ -129,7 +132,7 @@ __global__ void __launch_bounds__(1024) polynorm_kernel(const float* __restrict_
 #pragma unroll
   for (int j = 0; j < kKeep; ++j)
     if (threadIdx.x + j * blockDim.x < units) write(threadIdx.x + j * blockDim.x, keep[j]);
-  for (int i = threadIdx.x + kKeep * blockDim.x; i < units; i += blockDim.x) write(i, fetch(i));
+  for (int i = threadIdx.x + kept; i < units; i += blockDim.x) write(i, rest[i - kept]);
 }
 
 // One warp per token. logits [n][ldz] float32, correction [X] (float32 or bfloat16), weights out [n][X].
@@ -241,11 +244,18 @@ SB_EXPORT int sb_polynorm(const float* up, int n_partials, int64_t partial_strid
                           float c, float e, float eps, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (n_partials < 1 || F <= 0) return sb::fail("sb_polynorm: n_partials %d, size %d", n_partials, F);
-  if (F > 50 * 1024) return sb::fail("sb_polynorm: a row of %d elements does not fit the row buffer", F);
+  if (F > 50 * 1024) return sb::fail("sb_polynorm: a row of %d elements (at most 51200)", F);
   const bool vec = F % 4 == 0 && partial_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-  const int units = vec ? F / 4 : F, threads = units > 1024 ? 1024 : units > 512 ? 512 : units > 256 ? 256 : 128;
-#define SB_POLY(TO, VE, ONE) \
-  sb::launch_pdl(polynorm_kernel<TO, VE, ONE>, dim3(n), dim3(threads), 0, stream, up, n_partials, partial_stride, static_cast<TO*>(out), F, a, b, c, e, eps)
+  const int units = vec ? F / 4 : F;      // (single elements: several a thread, so that an SM holds more than one row)
+  const int threads = vec ? (units > 1024 ? 1024 : units > 512 ? 512 : units > 256 ? 256 : 128) : F >= 4096 ? 1024 : F >= 2048 ? 512 : F >= 512 ? 256 : 128;
+  const int kept = (vec ? 2 : 1) * threads;      // (kKeep pieces a thread are in registers)
+  const size_t smem = units > kept ? static_cast<size_t>(units - kept) * (vec ? 16 : 4) : 0;
+#define SB_POLY(TO, VE, ONE)                                                                                                                  \
+  do {                                                                                                                                        \
+    if (smem > 40 * 1024) cudaFuncSetAttribute(polynorm_kernel<TO, VE, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
+    sb::launch_pdl(polynorm_kernel<TO, VE, ONE>, dim3(n), dim3(threads), smem, stream, up, n_partials, partial_stride, static_cast<TO*>(out), F, \
+                   a, b, c, e, eps);                                                                                                          \
+  } while (0)
   if (out_dtype == 0) {
     if (vec && n_partials == 1) SB_POLY(float, 4, true);
     else if (vec) SB_POLY(float, 4, false);

@@ -50,49 +50,63 @@ __device__ __forceinline__ float4 folded4(const float* p, int n_partials, int64_
 }
 
 // proj [P][n][2 HD + HV]: columns q | f | v. act [n][3 HD + HV]: columns q | g | k | v. grid: (rows, pieces of a row). VE = 4: four elements
-// an access where the sizes and buffers allow it. Bound by memory: 1,250 rows of 16 heads of 128 | 128 15.5 us, 37 us with one element and a
-// 64-bit division a thread and round.
-template <class TW, int VE, bool ONE>
+// an access where the sizes and buffers allow it. PIECES: single elements of a row a thread, requested together (four where the rows are many:
+// blocks of one are then too short-lived). Bound by memory: 1,250 rows of 16 heads of 128 | 128 15.5 us, 37 us with one element and a 64-bit
+// division a thread and round.
+template <class TW, int VE, bool ONE, int PIECES>
 __global__ void __launch_bounds__(128) hgrn2_activate_kernel(const float* __restrict__ proj, int n_partials, int64_t partial_stride,
                                                              const TW* __restrict__ f_bias, const TW* __restrict__ lower, float* __restrict__ act, int HD, int HV) {
   sb::grid_launch_dependents();
-  const int in_w = 2 * HD + HV, j = (blockIdx.y * blockDim.x + threadIdx.x) * VE;
-  if (j >= in_w) return;
-  const bool gate = j >= HD && j < 2 * HD;
-  float l[VE], fb[VE], z[VE], g[VE];
-  if (gate) {
+  const int in_w = 2 * HD + HV, j0 = (blockIdx.y * PIECES * blockDim.x + threadIdx.x) * VE;
+  if (j0 >= in_w) return;
+  float l[PIECES][VE], fb[PIECES][VE], z[PIECES][VE];
 #pragma unroll
-    for (int i = 0; i < VE; ++i) l[i] = sb::widen(lower[j - HD + i]), fb[i] = sb::widen(f_bias[j - HD + i]);
+  for (int k = 0; k < PIECES; ++k) {
+    const int j = j0 + k * blockDim.x * VE;
+    if (j >= HD && j < 2 * HD) {
+#pragma unroll
+      for (int i = 0; i < VE; ++i) l[k][i] = sb::widen(lower[j - HD + i]), fb[k][i] = sb::widen(f_bias[j - HD + i]);
+    }
   }
   sb::grid_dependency_wait();
-  const float* src = proj + static_cast<int64_t>(blockIdx.x) * in_w + j;
-  if constexpr (VE == 4) {
-    const float4 v = folded4<ONE>(src, n_partials, partial_stride);
-    z[0] = v.x, z[1] = v.y, z[2] = v.z, z[3] = v.w;
-  } else {
-    z[0] = folded(src, n_partials, partial_stride);
+  const float* src = proj + static_cast<int64_t>(blockIdx.x) * in_w;
+#pragma unroll
+  for (int k = 0; k < PIECES; ++k) {
+    const int j = j0 + k * blockDim.x * VE;
+    if constexpr (VE == 4) {
+      const float4 v = folded4<ONE>(src + j, n_partials, partial_stride);
+      z[k][0] = v.x, z[k][1] = v.y, z[k][2] = v.z, z[k][3] = v.w;
+    } else if (PIECES == 1 || j < in_w) {
+      z[k][0] = folded(src + j, n_partials, partial_stride);
+    }
   }
   auto store = [&](float* to, const float (&v)[VE]) {
     if constexpr (VE == 4) *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]);
     else to[0] = v[0];
   };
   float* row = act + static_cast<int64_t>(blockIdx.x) * (3 * HD + HV);
-  if (gate) {
 #pragma unroll
-    for (int i = 0; i < VE; ++i) {
-      const float s = 1.0f / (1.0f + expf(-(z[i] + fb[i])));
-      g[i] = fmaf(1.0f - l[i], s, l[i]);
-      z[i] = 1.0f - g[i];
+  for (int k = 0; k < PIECES; ++k) {
+    const int j = j0 + k * blockDim.x * VE;
+    if (PIECES > 1 && j >= in_w) break;
+    if (j >= HD && j < 2 * HD) {
+      float g[VE];
+#pragma unroll
+      for (int i = 0; i < VE; ++i) {
+        const float s = 1.0f / (1.0f + expf(-(z[k][i] + fb[k][i])));
+        g[i] = fmaf(1.0f - l[k][i], s, l[k][i]);
+        z[k][i] = 1.0f - g[i];
+      }
+      store(row + j, g);
+      store(row + HD + j, z[k]);
+      continue;
     }
-    store(row + j, g);
-    store(row + HD + j, z);
-    return;
-  }
-  if (j < HD) {
+    if (j < HD) {
 #pragma unroll
-    for (int i = 0; i < VE; ++i) z[i] = z[i] / (1.0f + expf(-z[i]));
+      for (int i = 0; i < VE; ++i) z[k][i] = z[k][i] / (1.0f + expf(-z[k][i]));
+    }
+    store(row + (j < HD ? j : HD + j), z[k]);
   }
-  store(row + (j < HD ? j : HD + j), z);
 }
 
 // Steps in which every entry brings one token.
@@ -147,21 +161,22 @@ SB_EXPORT int sb_hgrn2_activate(const float* proj, int n_partials, int64_t parti
   if (n <= 0) return 0;
   if (n_partials < 1) return sb::fail("sb_hgrn2_activate: n_partials must be >= 1");
   const bool vec = HD % 4 == 0 && HV % 4 == 0 && partial_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(act)) & 15) == 0;
-  const dim3 grid(n, ((2 * HD + HV) / (vec ? 4 : 1) + 127) / 128);
-#define SB_ACT(TW, VE, ONE) \
-  sb::launch_pdl(hgrn2_activate_kernel<TW, VE, ONE>, grid, dim3(128), 0, stream, proj, n_partials, partial_stride, static_cast<const TW*>(f_bias), \
+  const bool many = !vec && n > 1024;
+  const dim3 grid(n, (2 * HD + HV + (vec || many ? 511 : 127)) / (vec || many ? 512 : 128));
+#define SB_ACT(TW, VE, ONE, PIECES) \
+  sb::launch_pdl(hgrn2_activate_kernel<TW, VE, ONE, PIECES>, grid, dim3(128), 0, stream, proj, n_partials, partial_stride, static_cast<const TW*>(f_bias), \
                  static_cast<const TW*>(lower), act, HD, HV)
-  if (w_dtype == 0) {
-    if (vec && n_partials == 1) SB_ACT(float, 4, true);
-    else if (vec) SB_ACT(float, 4, false);
-    else SB_ACT(float, 1, false);
-  } else if (w_dtype == 1) {
-    if (vec && n_partials == 1) SB_ACT(bf16, 4, true);
-    else if (vec) SB_ACT(bf16, 4, false);
-    else SB_ACT(bf16, 1, false);
-  } else {
-    return sb::fail("sb_hgrn2_activate: unsupported dtype %d", w_dtype);
-  }
+#define SB_ACT_T(TW)                                          \
+  do {                                                        \
+    if (vec && n_partials == 1) SB_ACT(TW, 4, true, 1);       \
+    else if (vec) SB_ACT(TW, 4, false, 1);                    \
+    else if (many) SB_ACT(TW, 1, false, 4);                   \
+    else SB_ACT(TW, 1, false, 1);                             \
+  } while (0)
+  if (w_dtype == 0) SB_ACT_T(float);
+  else if (w_dtype == 1) SB_ACT_T(bf16);
+  else return sb::fail("sb_hgrn2_activate: unsupported dtype %d", w_dtype);
+#undef SB_ACT_T
 #undef SB_ACT
   return sb::check_launch("sb_hgrn2_activate");
 }

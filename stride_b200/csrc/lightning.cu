@@ -55,7 +55,7 @@ __device__ __forceinline__ float4 folded4(const float* p, int n_partials, int64_
   return sum;
 }
 
-// Steps with as many tokens as entries (decoding): the partial sums folded (and activated) inside.
+// Steps in which every entry brings one token (decoding): the partial sums folded (and activated) inside.
 template <int DL>
 __global__ void __launch_bounds__(DL * 64, DL == 2 ? 7 : 1024 / (DL * 64)) lightning_step_kernel(const sbscan::Params p, int n_partials, int64_t partial_stride, int activated) {
   extern __shared__ __align__(16) float smem[];
@@ -108,18 +108,20 @@ __global__ void __launch_bounds__(256) lightning_activate_kernel(const float* __
 // out[r, j] = o[r, j] / sqrt(mean_j(o[r, :]^2) + eps) * gain[j] * sigmoid(gate[r, j]); the gate is a column range of the
 // projection's partial sums. One block per row. VE: 4 where the width and every buffer allow 16-byte accesses, else 1; which one depends on
 // the width and the buffers alone, never on the rows. A thread keeps up to kKeep pieces of o and of the gate in registers, requested before
-// the block's sum; what lies beyond is read again behind it. 2,048 rows of 2,048: 11.6 us, 24 us with single elements and the gate behind the sum.
+// the block's sum; of what lies beyond, o waits in shared memory and the gate is read behind it. 2,048 rows of 2,048: 11.6 us, 24 us with single elements and the gate behind the sum.
 template <class TW, class TO, int VE, bool ONE>
 __global__ void __launch_bounds__(1024) gated_rmsnorm_kernel(const float* __restrict__ o, const float* __restrict__ proj, int n_partials,
                                                               int64_t partial_stride, int width, int g_off,
                                                               const TW* __restrict__ gain, TO* __restrict__ out, int W, float eps) {
   using V = typename std::conditional<VE == 4, float4, float>::type;
   constexpr int kKeep = 2;
+  extern __shared__ __align__(16) float beyond_raw[];
   __shared__ float red[32];
   sb::grid_launch_dependents();
   sb::grid_dependency_wait();
   const int64_t r = blockIdx.x;
-  const int units = W / VE;
+  const int units = W / VE, kept = kKeep * blockDim.x;
+  V* rest = reinterpret_cast<V*>(beyond_raw);
   const V* src = reinterpret_cast<const V*>(o + r * W);
   const float* gate = proj + r * width + g_off;
   auto gate_at = [&](int i) {
@@ -140,7 +142,7 @@ __global__ void __launch_bounds__(1024) gated_rmsnorm_kernel(const float* __rest
 #pragma unroll
   for (int j = 0; j < kKeep; ++j)
     if (threadIdx.x + j * blockDim.x < units) square(v[j]);
-  for (int i = threadIdx.x + kKeep * blockDim.x; i < units; i += blockDim.x) square(src[i]);
+  for (int i = threadIdx.x + kept; i < units; i += blockDim.x) square(rest[i - kept] = src[i]);
   const float scale = 1.0f / sqrtf(sb::block_sum(ss, red) / static_cast<float>(W) + eps);
   auto one = [&](float a, float b, float w) { return a * scale * w * (1.0f / (1.0f + expf(-b))); };
   auto write = [&](int i, V a, V b) {
@@ -166,7 +168,7 @@ __global__ void __launch_bounds__(1024) gated_rmsnorm_kernel(const float* __rest
     const int i = threadIdx.x + j * blockDim.x;
     if (i < units) write(i, v[j], g[j]);
   }
-  for (int i = threadIdx.x + kKeep * blockDim.x; i < units; i += blockDim.x) write(i, src[i], gate_at(i));
+  for (int i = threadIdx.x + kept; i < units; i += blockDim.x) write(i, rest[i - kept], gate_at(i));
 }
 
 }  // namespace
@@ -219,21 +221,23 @@ SB_EXPORT int sb_gated_rmsnorm(const float* o, const float* proj, int n_partials
                                const void* gain, int gain_dtype, void* out, int out_dtype, int n, int W, float eps, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (n_partials < 1) return sb::fail("sb_gated_rmsnorm: n_partials must be >= 1");
-  if (W > 50 * 1024) return sb::fail("sb_gated_rmsnorm: width %d does not fit the row buffer", W);
+  if (W > 50 * 1024) return sb::fail("sb_gated_rmsnorm: width %d (at most 51200)", W);
   auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   const bool vec = W % 4 == 0 && width % 4 == 0 && g_off % 4 == 0 && partial_stride % 4 == 0 && aligned(o) && aligned(proj) && aligned(gain) && aligned(out);
-  const int units = vec ? W / 4 : W, threads = units > 1024 ? 1024 : units > 512 ? 512 : units > 256 ? 256 : 128;
-#define SB_GN(TW, TO)                                                                                                           \
-  do {                                                                                                                          \
-    if (vec && n_partials == 1)                                                                                                 \
-      sb::launch_pdl(gated_rmsnorm_kernel<TW, TO, 4, true>, n, threads, 0, stream, o, proj, n_partials, partial_stride, width, g_off, \
-                     static_cast<const TW*>(gain), static_cast<TO*>(out), W, eps);                                              \
-    else if (vec)                                                                                                               \
-      sb::launch_pdl(gated_rmsnorm_kernel<TW, TO, 4, false>, n, threads, 0, stream, o, proj, n_partials, partial_stride, width, g_off, \
-                     static_cast<const TW*>(gain), static_cast<TO*>(out), W, eps);                                              \
-    else                                                                                                                        \
-      sb::launch_pdl(gated_rmsnorm_kernel<TW, TO, 1, false>, n, threads, 0, stream, o, proj, n_partials, partial_stride, width, g_off, \
-                     static_cast<const TW*>(gain), static_cast<TO*>(out), W, eps);                                              \
+  const int units = vec ? W / 4 : W;      // (single elements: several a thread, so that an SM holds more than one row)
+  const int threads = vec ? (units > 1024 ? 1024 : units > 512 ? 512 : units > 256 ? 256 : 128) : W >= 4096 ? 1024 : W >= 2048 ? 512 : W >= 512 ? 256 : 128;
+  const size_t smem = units > 2 * threads ? static_cast<size_t>(units - 2 * threads) * (vec ? 16 : 4) : 0;      // (kKeep pieces a thread are in registers)
+#define SB_GN_V(TW, TO, VE, ONE)                                                                                                      \
+  do {                                                                                                                                \
+    if (smem > 40 * 1024) cudaFuncSetAttribute(gated_rmsnorm_kernel<TW, TO, VE, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    sb::launch_pdl(gated_rmsnorm_kernel<TW, TO, VE, ONE>, n, threads, smem, stream, o, proj, n_partials, partial_stride, width, g_off, \
+                   static_cast<const TW*>(gain), static_cast<TO*>(out), W, eps);                                                      \
+  } while (0)
+#define SB_GN(TW, TO)                                     \
+  do {                                                    \
+    if (vec && n_partials == 1) SB_GN_V(TW, TO, 4, true); \
+    else if (vec) SB_GN_V(TW, TO, 4, false);              \
+    else SB_GN_V(TW, TO, 1, false);                       \
   } while (0)
   if (gain_dtype == 0 && out_dtype == 0) SB_GN(float, float);
   else if (gain_dtype == 0 && out_dtype == 1) SB_GN(float, bf16);
@@ -241,6 +245,7 @@ SB_EXPORT int sb_gated_rmsnorm(const float* o, const float* proj, int n_partials
   else if (gain_dtype == 1 && out_dtype == 1) SB_GN(bf16, bf16);
   else return sb::fail("sb_gated_rmsnorm: unsupported dtypes gain=%d out=%d", gain_dtype, out_dtype);
 #undef SB_GN
+#undef SB_GN_V
   return sb::check_launch("sb_gated_rmsnorm");
 }
 

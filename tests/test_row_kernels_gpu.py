@@ -329,3 +329,25 @@ def test_norms_do_not_show_the_rows(H):
         whole = run(n, norm)
         for m in (1, 149, 297, 741):
             assert torch.equal(run(m, norm), whole[:m]), (norm, m)
+
+
+@pytest.mark.parametrize("HD,HV", [(6, 10), (250, 130), (128, 64)])
+def test_gates_of_linear_attention_do_not_show_the_rows(HD, HV):
+    """Single elements, one and four a thread, and four neighbouring ones: the bits of a few rows in those of 1,030, and 64 bits within 2e-6."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(HD)
+    n, dev = 1030, lambda *s: torch.randn(*s, generator=g).to(DEV)
+    proj, fb, low = dev(3, n, 2 * HD + HV), dev(HD), torch.rand(HD, generator=g).to(DEV)
+
+    def run(m):
+        act = torch.empty(m, 3 * HD + HV, device=DEV)
+        ops.hgrn2_activate(proj[:, :m].contiguous(), fb, low, act, HD, HV)
+        return act
+
+    whole = run(n)
+    for m in (1, 1024, 1025):
+        assert torch.equal(run(m), whole[:m])
+    z = proj.double().sum(0)
+    gate = low.double() + (1 - low.double()) * torch.sigmoid(z[:, HD:2 * HD] + fb.double())
+    want = torch.cat([torch.nn.functional.silu(z[:, :HD]), gate, 1 - gate, z[:, 2 * HD:]], 1)
+    assert (whole.double() - want).abs().max() <= 2e-6 * float(want.abs().max())      # a few roundings of sums of three
