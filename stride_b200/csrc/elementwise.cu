@@ -161,11 +161,11 @@ __device__ __forceinline__ void store4<bf16>(bf16* dst, float a, float b, float 
 }
 
 // ONE: one partial buffer: without the registers for eight of them more blocks live on an SM (2,048 tokens of 32 + 2 x 8 heads of 64: 16.4 -> 8.0 us).
-template <class TQ, class TKV, bool ONE>
+template <class TQ, class TKV, bool ONE, bool WHOLE>      // WHOLE: all of a head is rotated
 __global__ void rope_append_vec_kernel(RopeAppendParams p) {
   sb::grid_launch_dependents();
   const int row = blockIdx.x;
-  const int D = p.D, rh = p.rotary_dim / 2, quads = D / 8;
+  const int D = p.D, rh = WHOLE ? D / 2 : p.rotary_dim / 2, quads = D / 8;
   const int heads = p.Hq + 2 * p.Hkv;
   const int item = blockIdx.y * blockDim.x + threadIdx.x;
   if (item >= heads * quads) {
@@ -175,8 +175,8 @@ __global__ void rope_append_vec_kernel(RopeAppendParams p) {
   const int pos = p.positions[row];
   const int slot = p.slots[row];
   const int head = item / quads, j = (item % quads) * 4;
-  const bool is_v = head >= p.Hq + p.Hkv, rotate = j < rh && !is_v;
-  const int d0 = j < rh ? j : p.rotary_dim + 2 * (j - rh), d1 = j < rh ? rh + j : d0 + 4;
+  const bool is_v = head >= p.Hq + p.Hkv, rotate = (WHOLE || j < rh) && !is_v;
+  const int d0 = WHOLE || j < rh ? j : p.rotary_dim + 2 * (j - rh), d1 = WHOLE || j < rh ? rh + j : d0 + 4;
   int page = 0;
   if (p.write_kv && head >= p.Hq) page = p.block_table[static_cast<int64_t>(slot) * p.max_pages + pos / p.page_size];
   float4 c01 = make_float4(1.0f, 0.0f, 1.0f, 0.0f), c23 = c01;   // (cos, sin) of pairs j, j+1 and j+2, j+3
@@ -349,13 +349,20 @@ SB_EXPORT int sb_rope_append(const float* qkv, int n_partials, int64_t partial_s
   const int threads = 128;
   const bool aligned = ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(k_base) |
                          reinterpret_cast<uintptr_t>(cos_sin)) & 15) == 0;
-  if (rotary_dim % 8 == 0 && D % 8 == 0 && aligned && partial_stride % 4 == 0 && page_stride % 8 == 0 && v_offset % 8 == 0 &&
+  // A few tokens whose heads are rotated in part: a pair a thread has more of the partial sums on their way.
+  const bool few = rotary_dim != D && (n <= 16 || (n <= 64 && n_partials > 2));
+  if (!few && rotary_dim % 8 == 0 && D % 8 == 0 && aligned && partial_stride % 4 == 0 && page_stride % 8 == 0 && v_offset % 8 == 0 &&
       head_stride % 8 == 0) {
     const dim3 vgrid(n, ((Hq + 2 * Hkv) * (D / 8) + threads - 1) / threads);
-#define SB_ROPE(TQ, TKV)                                                                                                 \
+#define SB_ROPE_W(TQ, TKV, WHOLE)                                                                                        \
   do {                                                                                                                   \
-    if (n_partials == 1) sb::launch_pdl(rope_append_vec_kernel<TQ, TKV, true>, vgrid, threads, 0, stream, p);            \
-    else sb::launch_pdl(rope_append_vec_kernel<TQ, TKV, false>, vgrid, threads, 0, stream, p);                           \
+    if (n_partials == 1) sb::launch_pdl(rope_append_vec_kernel<TQ, TKV, true, WHOLE>, vgrid, threads, 0, stream, p);     \
+    else sb::launch_pdl(rope_append_vec_kernel<TQ, TKV, false, WHOLE>, vgrid, threads, 0, stream, p);                    \
+  } while (0)
+#define SB_ROPE(TQ, TKV)                              \
+  do {                                                \
+    if (rotary_dim == D && n > 64) SB_ROPE_W(TQ, TKV, true);    \
+    else SB_ROPE_W(TQ, TKV, false);                   \
   } while (0)
     if (q_dtype == 0 && kv_dtype == 0) SB_ROPE(float, float);
     else if (q_dtype == 1 && kv_dtype == 1) SB_ROPE(bf16, bf16);
@@ -363,6 +370,7 @@ SB_EXPORT int sb_rope_append(const float* qkv, int n_partials, int64_t partial_s
     else if (q_dtype == 1 && kv_dtype == 0) SB_ROPE(bf16, float);
     else return sb::fail("sb_rope_append: unsupported dtypes q=%d kv=%d", q_dtype, kv_dtype);
 #undef SB_ROPE
+#undef SB_ROPE_W
     return sb::check_launch("sb_rope_append");
   }
   const dim3 grid(n, ((Hq + 2 * Hkv) * (D / 2) + threads - 1) / threads);

@@ -351,3 +351,25 @@ def test_gates_of_linear_attention_do_not_show_the_rows(HD, HV):
     gate = low.double() + (1 - low.double()) * torch.sigmoid(z[:, HD:2 * HD] + fb.double())
     want = torch.cat([torch.nn.functional.silu(z[:, :HD]), gate, 1 - gate, z[:, 2 * HD:]], 1)
     assert (whole.double() - want).abs().max() <= 2e-6 * float(want.abs().max())      # a few roundings of sums of three
+
+
+@pytest.mark.parametrize("D,rot", [(64, 32), (96, 24), (64, 0), (64, 64)])
+@pytest.mark.parametrize("P", [1, 2, 9])
+def test_rotation_does_not_show_the_number_of_tokens(D, rot, P):
+    """A pair a thread for a few tokens of heads rotated in part, four pairs otherwise: the bits of a few tokens in those of 70."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(D + rot)
+    n, Hq, Hkv, page = 70, 5, 2, 16
+    qkv = torch.randn(P, n, (Hq + 2 * Hkv) * D, generator=g).to(DEV)
+    pos, slots = torch.arange(n, dtype=torch.int32, device=DEV), torch.zeros(n, dtype=torch.int32, device=DEV)
+    table, pages = torch.randn(n, max(rot // 2, 1), 2, generator=g).to(DEV), torch.arange(5, dtype=torch.int32, device=DEV)[None]
+
+    def run(m):
+        q, cache = torch.empty(m, Hq * D, device=DEV), torch.zeros(5, 2, Hkv, page, D, device=DEV)
+        ops.rope_append(qkv[:, :m].contiguous(), pos[:m], slots[:m], table, rot, q, cache, pages, Hq, Hkv, D)
+        return q, cache.permute(0, 3, 1, 2, 4).reshape(5 * page, -1)[:m]
+
+    whole = run(n)
+    for m in (1, 16, 17, 64, 65):
+        for x, w in zip(run(m), whole):
+            assert torch.equal(x, w[:m]), m
