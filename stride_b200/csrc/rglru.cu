@@ -164,19 +164,19 @@ __device__ __forceinline__ GateValues gate_values(float sr, float si, float ut, 
 }
 __device__ __forceinline__ float softplus_of(float l) { return l > 20.0f ? l : log1pf(expf(l)); }
 
-// Few tokens: a CTA is (8 tokens, block of channels, 32 of its channels), a thread one gate of one channel over one quarter of the inputs;
-// its weights are requested 32 at a time, the first ones before the kernels in front are waited for. 8 tokens of 16 blocks of 128: 5.5 us
+// Few tokens: a CTA is (TOKENS tokens, block of channels, 32 of its channels), a thread one gate of one channel over one quarter of the inputs;
+// its weights are requested 32 (16) at a time, the first ones before the kernels in front are waited for. 8 tokens of 16 blocks of 128: 5.5 us
 // for what two gates a thread and eight weights at a time behind the wait took 21.
-constexpr int kFewTokens = 8, kFewOutputs = 32;
-template <class TG>
-__global__ void __launch_bounds__(kQuarters * 2 * kFewOutputs) rglru_gates_few_kernel(const TG* __restrict__ gate_w, GateParams p) {
-  extern __shared__ __align__(16) float us[];         // [bw][kFewTokens]
-  __shared__ float red[kQuarters][2][kFewTokens][kFewOutputs];
+constexpr int kFewOutputs = 32;
+template <class TG, int TOKENS>
+__global__ void __launch_bounds__(kQuarters * 2 * kFewOutputs, TOKENS == 16 ? 4 : 0) rglru_gates_few_kernel(const TG* __restrict__ gate_w, GateParams p) {
+  extern __shared__ __align__(16) float us[];         // [bw][TOKENS]
+  __shared__ float red[kQuarters][2][TOKENS][kFewOutputs];
   sb::grid_launch_dependents();
-  const int bw = p.bw, t0 = blockIdx.x * kFewTokens, b = blockIdx.y, nt = min(kFewTokens, p.n - t0);
+  const int bw = p.bw, t0 = blockIdx.x * TOKENS, b = blockIdx.y, nt = min(TOKENS, p.n - t0);
   const int lane = threadIdx.x & 31, gate = (threadIdx.x >> 5) & 1, quarter = threadIdx.x >> 6, j = blockIdx.z * kFewOutputs + lane;
   const int per = (bw + kQuarters - 1) / kQuarters, k_begin = min(bw, quarter * per), k_end = min(bw, k_begin + per);
-  constexpr int kAhead = 32;
+  constexpr int kAhead = TOKENS == 16 ? 16 : 32;
   const TG* w = gate_w + static_cast<int64_t>(b) * bw * 2 * bw + gate * bw + min(j, bw - 1);
   TG ahead[kAhead];
   auto request = [&](int k0) {
@@ -185,26 +185,26 @@ __global__ void __launch_bounds__(kQuarters * 2 * kFewOutputs) rglru_gates_few_k
       if (k0 + i < k_end) ahead[i] = w[static_cast<int64_t>(k0 + i) * 2 * bw];
   };
   request(k_begin);
-  const int ct = threadIdx.x >> 5, c = b * bw + min(j, bw - 1);      // (the epilogue's token and channel)
+  const int c = b * bw + min(j, bw - 1);      // (the epilogue's channel)
   const float rb = p.r_bias[c], ib = p.i_bias[c], softplus = softplus_of(p.lam[c]), yb = p.y_bias[c];
   sb::grid_dependency_wait();
-  for (int i = threadIdx.x; i < kFewTokens * bw; i += blockDim.x) {
+  for (int i = threadIdx.x; i < TOKENS * bw; i += blockDim.x) {
     const int t = i / bw, k = i - t * bw;
-    us[k * kFewTokens + t] = t < nt ? p.u[static_cast<int64_t>(t0 + t) * p.C + b * bw + k] : 0.0f;
+    us[k * TOKENS + t] = t < nt ? p.u[static_cast<int64_t>(t0 + t) * p.C + b * bw + k] : 0.0f;
   }
   __syncthreads();
-  float acc[kFewTokens];
+  float acc[TOKENS];
 #pragma unroll
-  for (int t = 0; t < kFewTokens; ++t) acc[t] = 0.0f;
+  for (int t = 0; t < TOKENS; ++t) acc[t] = 0.0f;
   for (int k0 = k_begin; k0 < k_end; k0 += kAhead) {
     if (k0 != k_begin) request(k0);
 #pragma unroll
     for (int i = 0; i < kAhead; ++i)
       if (k0 + i < k_end) {
         const float wk = sb::widen(ahead[i]);
-        const float4* x4 = reinterpret_cast<const float4*>(us + (k0 + i) * kFewTokens);
+        const float4* x4 = reinterpret_cast<const float4*>(us + (k0 + i) * TOKENS);
 #pragma unroll
-        for (int t = 0; t < kFewTokens / 4; ++t) {
+        for (int t = 0; t < TOKENS / 4; ++t) {
           const float4 x = x4[t];
           acc[4 * t] = fmaf(wk, x.x, acc[4 * t]);
           acc[4 * t + 1] = fmaf(wk, x.y, acc[4 * t + 1]);
@@ -214,79 +214,89 @@ __global__ void __launch_bounds__(kQuarters * 2 * kFewOutputs) rglru_gates_few_k
       }
   }
 #pragma unroll
-  for (int t = 0; t < kFewTokens; ++t) red[quarter][gate][t][lane] = acc[t];
+  for (int t = 0; t < TOKENS; ++t) red[quarter][gate][t][lane] = acc[t];
   __syncthreads();
-  if (j >= bw || ct >= nt) return;
-  float sr = red[0][0][ct][lane], si = red[0][1][ct][lane];
+  if (j >= bw) return;
 #pragma unroll
-  for (int q = 1; q < kQuarters; ++q) sr += red[q][0][ct][lane], si += red[q][1][ct][lane];
-  const float z = folded(p.proj.p + static_cast<int64_t>(t0 + ct) * 2 * p.C + c, p.proj.n_partials, p.proj.stride);
-  const GateValues v = gate_values(sr, si, us[j * kFewTokens + ct], z, rb, ib, softplus, yb);
-  const int64_t i = static_cast<int64_t>(t0 + ct) * p.C + c;
-  p.a[i] = v.a, p.d[i] = v.d, p.y[i] = v.y;
+  for (int ct = threadIdx.x >> 5; ct < TOKENS; ct += 2 * kQuarters) {      // a token a warp
+    if (ct >= nt) break;
+    float sr = red[0][0][ct][lane], si = red[0][1][ct][lane];
+#pragma unroll
+    for (int q = 1; q < kQuarters; ++q) sr += red[q][0][ct][lane], si += red[q][1][ct][lane];
+    const float z = folded(p.proj.p + static_cast<int64_t>(t0 + ct) * 2 * p.C + c, p.proj.n_partials, p.proj.stride);
+    const GateValues v = gate_values(sr, si, us[j * TOKENS + ct], z, rb, ib, softplus, yb);
+    const int64_t i = static_cast<int64_t>(t0 + ct) * p.C + c;
+    p.a[i] = v.a, p.d[i] = v.d, p.y[i] = v.y;
+  }
 }
 
-// Many tokens: a CTA is (32 tokens, block of channels, 64 of its channels), a warp four tokens, a lane two channels with both gates: 16
+// More tokens: a CTA is (TOKENS tokens, block of channels, 64 of its channels), a warp four tokens, a lane two channels with both gates: 16
 // sums a thread for one read of the tokens' inputs and two of the weights a k, both staged in shared memory 32 inputs at a time, the next
 // tile's on their way in registers meanwhile. A thread has whole sums (quarter after quarter) and so makes its outputs without an exchange,
-// its inputs requested together in front of them. VEC: 16-byte requests (blocks of a multiple of 16 channels, aligned buffers).
+// its inputs requested together in front of them. KN: weights a request (16 bytes for blocks of a multiple of 16 channels, four for
+// multiples of four, else one); EVEN: 16-byte requests of the tokens' inputs and 8-byte outputs (blocks of a multiple of 16 channels).
 // 1,250 tokens of 16 blocks of 128: 59 us; 167 us as one channel of 16 tokens a thread with its weights from global memory, 131 us as
 // here but with single-element requests that nothing overlapped.
-constexpr int kManyTokens = 32, kManyOutputs = 64, kManyInputs = 32;
-template <class TG, bool VEC>
-__global__ void __launch_bounds__(256) rglru_gates_kernel(const TG* __restrict__ gate_w, GateParams p) {
+constexpr int kManyOutputs = 64, kManyInputs = 32;
+template <int BYTES>
+struct RawOf;
+template <>
+struct RawOf<16> { using type = uint4; };
+template <>
+struct RawOf<8> { using type = uint2; };
+template <>
+struct RawOf<4> { using type = uint32_t; };
+template <>
+struct RawOf<2> { using type = uint16_t; };
+template <class TG, int KN, bool EVEN, int TOKENS>
+__global__ void __launch_bounds__(TOKENS * 8, TOKENS == 16 && KN == 8 ? 4 : 0) rglru_gates_kernel(const TG* __restrict__ gate_w, GateParams p) {
+  constexpr int kThreads = TOKENS * 8;
   __shared__ __align__(16) float ws[kManyInputs][2][kManyOutputs];
-  __shared__ __align__(16) float us[kManyInputs][kManyTokens + 4];     // (rows of 16-byte pieces that start at different banks)
+  __shared__ __align__(16) float us[kManyInputs][TOKENS + 4];          // (rows of 16-byte pieces that start at different banks)
   sb::grid_launch_dependents();
-  const int bw = p.bw, t0 = blockIdx.x * kManyTokens, b = blockIdx.y, j0 = blockIdx.z * kManyOutputs;
+  const int bw = p.bw, t0 = blockIdx.x * TOKENS, b = blockIdx.y, j0 = blockIdx.z * kManyOutputs;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tg = warp * 4;
   const int per = (bw + kQuarters - 1) / kQuarters;
   const TG* w = gate_w + static_cast<int64_t>(b) * bw * 2 * bw;
   const float* u = p.u + b * bw;
-  constexpr int kN = VEC ? 16 / sizeof(TG) : 1;                        // weights a request
-  constexpr int kW = kManyInputs * 2 * kManyOutputs / kN / 256;        // requests a thread and tile
-  struct __align__(sizeof(TG) * kN) Weights { TG v[kN]; };
-  Weights wr[VEC ? kW : 1];
+  constexpr int kW = kManyInputs * 2 * kManyOutputs / KN / kThreads;   // requests a thread and tile
+  using Raw = typename RawOf<KN * sizeof(TG)>::type;
+  Raw wr[kW];
   float ur[4];
-  auto request = [&](int k0, int nk) {                                 // (VEC)
+  const int st = threadIdx.x / 8, sk = threadIdx.x % 8 * 4;            // the token and the first of the four inputs that a thread stages
+  auto request = [&](int k0, int nk) {
 #pragma unroll
     for (int i = 0; i < kW; ++i) {
-      const int at = (threadIdx.x + 256 * i) * kN, k = at / (2 * kManyOutputs), g = at / kManyOutputs % 2, o = at % kManyOutputs;
-      if (k < nk && j0 + o < bw)
-        *reinterpret_cast<uint4*>(&wr[i]) = *reinterpret_cast<const uint4*>(w + static_cast<int64_t>(k0 + k) * 2 * bw + g * bw + j0 + o);
-      else
-        *reinterpret_cast<uint4*>(&wr[i]) = make_uint4(0, 0, 0, 0);
+      const int at = (threadIdx.x + kThreads * i) * KN, k = at / (2 * kManyOutputs), g = at / kManyOutputs % 2, o = at % kManyOutputs;
+      wr[i] = k < nk && j0 + o < bw ? *reinterpret_cast<const Raw*>(w + static_cast<int64_t>(k0 + k) * 2 * bw + g * bw + j0 + o) : Raw{};
     }
-    const int t = threadIdx.x / 8, k = threadIdx.x % 8 * 4;
-    const float4 x = t0 + t < p.n && k < nk ? *reinterpret_cast<const float4*>(u + static_cast<int64_t>(t0 + t) * p.C + k0 + k) : make_float4(0, 0, 0, 0);
-    ur[0] = x.x, ur[1] = x.y, ur[2] = x.z, ur[3] = x.w;
-  };
-  auto stage = [&](int k0, int nk) {
-    if constexpr (VEC) {
-#pragma unroll
-      for (int i = 0; i < kW; ++i) {
-        const int at = (threadIdx.x + 256 * i) * kN;
-        float* to = &ws[0][0][0] + at;
-#pragma unroll
-        for (int e = 0; e < kN; e += 4)
-          *reinterpret_cast<float4*>(to + e) = make_float4(sb::widen(wr[i].v[e]), sb::widen(wr[i].v[e + 1]), sb::widen(wr[i].v[e + 2]), sb::widen(wr[i].v[e + 3]));
-      }
-      const int t = threadIdx.x / 8, k = threadIdx.x % 8 * 4;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) us[k + e][t] = ur[e];
+    const float* at = u + static_cast<int64_t>(t0 + st) * p.C + k0 + sk;
+    if constexpr (EVEN) {
+      const float4 x = t0 + st < p.n && sk < nk ? *reinterpret_cast<const float4*>(at) : make_float4(0, 0, 0, 0);
+      ur[0] = x.x, ur[1] = x.y, ur[2] = x.z, ur[3] = x.w;
     } else {
-      for (int i = threadIdx.x; i < nk * 2 * kManyOutputs; i += 256) {
-        const int k = i / (2 * kManyOutputs), g = i / kManyOutputs % 2, o = i % kManyOutputs;
-        ws[k][g][o] = j0 + o < bw ? sb::widen(w[static_cast<int64_t>(k0 + k) * 2 * bw + g * bw + j0 + o]) : 0.0f;
-      }
-      for (int i = threadIdx.x; i < kManyInputs * kManyTokens; i += 256) {
-        const int t = i / kManyInputs, k = i % kManyInputs;
-        if (k < nk) us[k][t] = t0 + t < p.n ? u[static_cast<int64_t>(t0 + t) * p.C + k0 + k] : 0.0f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) ur[e] = t0 + st < p.n && sk + e < nk ? at[e] : 0.0f;
+    }
+  };
+  auto stage = [&]() {
+#pragma unroll
+    for (int i = 0; i < kW; ++i) {
+      float* to = &ws[0][0][0] + (threadIdx.x + kThreads * i) * KN;
+      const TG* v = reinterpret_cast<const TG*>(&wr[i]);
+      if constexpr (KN >= 4) {
+#pragma unroll
+        for (int e = 0; e < KN; e += 4)
+          *reinterpret_cast<float4*>(to + e) = make_float4(sb::widen(v[e]), sb::widen(v[e + 1]), sb::widen(v[e + 2]), sb::widen(v[e + 3]));
+      } else {
+        to[0] = sb::widen(v[0]);
       }
     }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) us[sk + e][st] = ur[e];
   };
   sb::grid_dependency_wait();
-  if constexpr (VEC) request(0, min(kManyInputs, min(bw, per)));
+  request(0, min(kManyInputs, min(bw, per)));
   float sum[2][4][2], acc[2][4][2];                    // gate, token, channel
   for (int q = 0; q < kQuarters; ++q) {
     const int k_begin = min(bw, q * per), k_end = min(bw, k_begin + per);
@@ -297,13 +307,11 @@ __global__ void __launch_bounds__(256) rglru_gates_kernel(const TG* __restrict__
     for (int k0 = k_begin; k0 < k_end; k0 += kManyInputs) {
       const int nk = min(kManyInputs, k_end - k0);
       __syncthreads();
-      stage(k0, nk);
+      stage();
       __syncthreads();
-      if constexpr (VEC) {
-        const bool same = k0 + kManyInputs < k_end;    // the next tile, of this quarter or of the next one (blocks of 16 channels and more fill all four)
-        const int next = same ? k0 + kManyInputs : k_end, end = same ? k_end : min(bw, k_end + per);
-        if (next < end) request(next, min(kManyInputs, end - next));
-      }
+      const bool same = k0 + kManyInputs < k_end;      // the next tile, of this quarter or of the next one (only the last ones may be empty)
+      const int next = same ? k0 + kManyInputs : k_end, end = same ? k_end : min(bw, k_end + per);
+      if (next < end) request(next, min(kManyInputs, end - next));
       auto one = [&](int k) {
         const float4 x = *reinterpret_cast<const float4*>(&us[k][tg]);
         const float xs[4] = {x.x, x.y, x.z, x.w};
@@ -340,7 +348,7 @@ __global__ void __launch_bounds__(256) rglru_gates_kernel(const TG* __restrict__
     const int row = t0 + tg + t;
     if (row >= p.n) break;
     const float* zs = p.proj.p + static_cast<int64_t>(row) * 2 * p.C + c;
-    if constexpr (VEC) {
+    if constexpr (EVEN) {
       const float2 x = *reinterpret_cast<const float2*>(p.u + static_cast<int64_t>(row) * p.C + c);
       ut[t][0] = x.x, ut[t][1] = x.y;
       float2 f = *reinterpret_cast<const float2*>(zs);
@@ -364,7 +372,7 @@ __global__ void __launch_bounds__(256) rglru_gates_kernel(const TG* __restrict__
     for (int o = 0; o < 2; ++o)
       if (o == 0 || two) v[o] = gate_values(sum[0][t][o], sum[1][t][o], ut[t][o], z[t][o], rb[o], ib[o], softplus[o], yb[o]);
     const int64_t i = static_cast<int64_t>(row) * p.C + c;
-    if constexpr (VEC) {
+    if constexpr (EVEN) {
       *reinterpret_cast<float2*>(p.a + i) = make_float2(v[0].a, v[1].a);
       *reinterpret_cast<float2*>(p.d + i) = make_float2(v[0].d, v[1].d);
       *reinterpret_cast<float2*>(p.y + i) = make_float2(v[0].y, v[1].y);
@@ -489,24 +497,41 @@ SB_EXPORT int sb_rglru_gates(const void* gate_w, int gate_dtype, const void* r_b
   if (w_dtype != 0) return sb::fail("sb_rglru_gates: biases and lam are float32");
   const GateParams p{static_cast<const float*>(r_bias), static_cast<const float*>(i_bias), static_cast<const float*>(lam), static_cast<const float*>(y_bias),
                      u, Proj{proj, n_partials, partial_stride}, a, d, y, n, C, bw};
-  // up to 128 tokens the weights are read once per 8 tokens by CTAs that are many all the same; beyond, 32 tokens share them
-  const bool few = n <= 128;
-  const dim3 few_grid((n + kFewTokens - 1) / kFewTokens, blocks, (bw + kFewOutputs - 1) / kFewOutputs);
-  const dim3 grid((n + kManyTokens - 1) / kManyTokens, blocks, (bw + kManyOutputs - 1) / kManyOutputs);
-  const size_t smem = sizeof(float) * kFewTokens * bw;
+  // 0, 1: 8 and 16 tokens a CTA with its weights from memory; 2, 3: 16 and 32 tokens that share staged ones. Microseconds with bfloat16 weights,
+  // 16 blocks of 128: 32 tokens 6.0, 9.3, 9.6, 12; 64 tokens 11.6, 13, 13, 12; 128 tokens 22, 14, 17, 18; 200 tokens 33, 23, 17, 21; 400 tokens
+  // 63, 40, 28, 21. Wide blocks leave few CTAs to share the weights' way (one of 2,048, 24 tokens: 76, 88, 67, 103); where every weight is a
+  // request of its own (odd blocks), staging pays later (8 of 33, 700 tokens: 20, 12, 16, 14; 2,048 tokens 54, 33, 28, 26).
+  const int form = bw >= 1024 ? (n < 8 ? 0 : n < 320 ? 2 : 3) : n <= 64 ? 0 : bw % 4 != 0 ? (n <= 128 ? 0 : n <= 1400 ? 1 : 3) : n <= 144 ? 1 : n < 320 ? 2 : 3;
   auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-  const bool vec = bw % 16 == 0 && partial_stride % 4 == 0 && aligned(gate_w) && aligned(u) && aligned(proj) && aligned(a) && aligned(d) && aligned(y);
-#define SB_GATES(TG)                                                                                                                            \
-  do {                                                                                                                                          \
-    if (few && smem > 16 * 1024) cudaFuncSetAttribute(rglru_gates_few_kernel<TG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);      \
-    if (few) sb::launch_pdl(rglru_gates_few_kernel<TG>, few_grid, dim3(kQuarters * 2 * kFewOutputs), smem, stream, static_cast<const TG*>(gate_w), p); \
-    else if (vec) sb::launch_pdl(rglru_gates_kernel<TG, true>, grid, dim3(256), 0, stream, static_cast<const TG*>(gate_w), p);                  \
-    else sb::launch_pdl(rglru_gates_kernel<TG, false>, grid, dim3(256), 0, stream, static_cast<const TG*>(gate_w), p);                          \
+  const bool quads = bw % 4 == 0 && aligned(gate_w);
+  const bool even = bw % 16 == 0 && partial_stride % 4 == 0 && aligned(gate_w) && aligned(u) && aligned(proj) && aligned(a) && aligned(d) && aligned(y);
+#define SB_GATES_FEW(TG, TOKENS)                                                                                                              \
+  do {                                                                                                                                        \
+    const size_t smem = sizeof(float) * TOKENS * bw;                                                                                          \
+    if (smem > 16 * 1024) cudaFuncSetAttribute(rglru_gates_few_kernel<TG, TOKENS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
+    sb::launch_pdl(rglru_gates_few_kernel<TG, TOKENS>, dim3((n + TOKENS - 1) / TOKENS, blocks, (bw + kFewOutputs - 1) / kFewOutputs),         \
+                   dim3(kQuarters * 2 * kFewOutputs), smem, stream, static_cast<const TG*>(gate_w), p);                                       \
+  } while (0)
+#define SB_GATES_MANY(TG, KN, EVEN, TOKENS)                                                                                                   \
+  sb::launch_pdl(rglru_gates_kernel<TG, KN, EVEN, TOKENS>, dim3((n + TOKENS - 1) / TOKENS, blocks, (bw + kManyOutputs - 1) / kManyOutputs),   \
+                 dim3(TOKENS * 8), 0, stream, static_cast<const TG*>(gate_w), p)
+#define SB_GATES(TG)                                                               \
+  do {                                                                             \
+    if (form == 0) SB_GATES_FEW(TG, 8);                                            \
+    else if (form == 1) SB_GATES_FEW(TG, 16);                                      \
+    else if (even && form == 2) SB_GATES_MANY(TG, 16 / (int)sizeof(TG), true, 16); \
+    else if (even) SB_GATES_MANY(TG, 16 / (int)sizeof(TG), true, 32);              \
+    else if (quads && form == 2) SB_GATES_MANY(TG, 4, false, 16);                  \
+    else if (quads) SB_GATES_MANY(TG, 4, false, 32);                               \
+    else if (form == 2) SB_GATES_MANY(TG, 1, false, 16);                           \
+    else SB_GATES_MANY(TG, 1, false, 32);                                          \
   } while (0)
   if (gate_dtype == 0) SB_GATES(float);
   else if (gate_dtype == 1) SB_GATES(bf16);
   else return sb::fail("sb_rglru_gates: unsupported dtype %d", gate_dtype);
 #undef SB_GATES
+#undef SB_GATES_FEW
+#undef SB_GATES_MANY
   return sb::check_launch("sb_rglru_gates");
 }
 

@@ -373,3 +373,26 @@ def test_rotation_does_not_show_the_number_of_tokens(D, rot, P):
     for m in (1, 16, 17, 64, 65):
         for x, w in zip(run(m), whole):
             assert torch.equal(x, w[:m]), m
+
+
+@pytest.mark.parametrize("bw,B,n", [(128, 2, 330), (100, 3, 330), (33, 2, 1410), (16, 3, 330), (272, 1, 330), (1040, 1, 330)])
+def test_gates_do_not_show_their_form(bw, B, n):
+    """8 and 16 tokens a block, 16 and 32 tokens that share staged weights; sixteen bytes, four weights or one a request: the bits of a few
+    tokens in those of n, with float32 weights and with the same numbers stored in bfloat16."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(bw)
+    C = bw * B
+    dev = lambda *s, k=0.3: (torch.randn(*s, generator=g) * k).to(DEV)
+    proj, u, yb, rb, ib, lam = dev(2, n, 2 * C), dev(n, C), dev(C), dev(C), dev(C), dev(C) - 3.0
+    gate_w = dev(B, bw, 2 * bw).bfloat16()
+
+    def run(m, weights):
+        outs = [torch.empty(m, C, device=DEV) for _ in range(3)]
+        ops.rglru_gates(weights, rb, ib, lam, yb, u[:m].contiguous(), proj[:, :m].contiguous(), *outs)
+        return outs
+
+    whole = run(n, gate_w.float())
+    for m in (1, 7, 8, 32, 33, 128, 129, 319, n):
+        for weights in (gate_w, gate_w.float()):
+            for x, w in zip(run(m, weights), whole):
+                assert torch.equal(x, w[:m]), m
