@@ -78,18 +78,19 @@ __device__ __forceinline__ void load_folded(float (&v)[VE], const Proj& proj, in
 }
 
 // u[r, c] = conv_b[c] + sum_j taps[c, j] * x[position - (K - 1 - j)]
-// A thread owns VE neighbouring channels (4 where the sizes and buffers allow 16-byte accesses) and ROWS rows one after the other, so that
-// the taps are read once for them. The order of a sum is the same in every form. 1,250 rows of 2,048 channels and four taps: 24 us, 43 us
-// as one channel of one row a thread.
-template <class TW, int VE, int ROWS>
-__global__ void __launch_bounds__(128) rglru_conv_kernel(Proj proj, const TW* __restrict__ x_bias, const TW* __restrict__ taps, const TW* __restrict__ conv_bias,
+// A thread owns VE neighbouring channels (16-byte accesses with 4) and ROWS rows one after the other, so that the taps are read once for
+// them. The order of a sum is the same in every form. 1,250 rows of 2,048 channels, four taps and one buffer: 22 us, 28 with one row and
+// 44 us with one channel of one row a thread.
+// HELD: taps kept in registers and read before the wait.
+template <class TW, int VE, int ROWS, int HELD>
+__global__ void __launch_bounds__(128, HELD == 0 ? 16 : 0) rglru_conv_kernel(Proj proj, const TW* __restrict__ x_bias, const TW* __restrict__ taps, const TW* __restrict__ conv_bias,
                                   const int32_t* __restrict__ positions, const int32_t* __restrict__ slots, const float* __restrict__ state,
                                   float* __restrict__ u, int n, int C, int K) {
-  constexpr int kHeld = 4;                            // taps kept in registers
+  constexpr int kHeld = HELD;
   sb::grid_launch_dependents();
   const int first = blockIdx.x * ROWS, c = (blockIdx.y * blockDim.x + threadIdx.x) * VE;
   if (c >= C) return;
-  float xb[VE], cb[VE], held[kHeld][VE];
+  float xb[VE], cb[VE], held[kHeld ? kHeld : 1][VE];
 #pragma unroll
   for (int e = 0; e < VE; ++e) {
     xb[e] = sb::widen(x_bias[c + e]), cb[e] = sb::widen(conv_bias[c + e]);
@@ -460,29 +461,30 @@ SB_EXPORT int sb_rglru_conv(const float* proj, int n_partials, int64_t partial_s
   if (K < 1 || K > kMaxTaps) return sb::fail("sb_rglru_conv: %d taps (1 to %d)", K, kMaxTaps);
   if (n_partials < 1) return sb::fail("sb_rglru_conv: n_partials must be >= 1");
   const Proj pr{proj, n_partials, partial_stride};
-  const bool vec = C % 4 == 0 && partial_stride % 4 == 0 &&
-                   ((reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(u)) & 15) == 0;
-  const bool few = n <= 256;        // (a row a block while four would leave SMs idle)
-  const dim3 grid(few ? n : (n + 3) / 4, (C / (vec ? 4 : 1) + 127) / 128);
-#define SB_CONV(TW, VE, ROWS)                                                                                                                    \
-  sb::launch_pdl(rglru_conv_kernel<TW, VE, ROWS>, grid, dim3(128), 0, stream, pr, static_cast<const TW*>(x_bias), static_cast<const TW*>(taps),  \
-                 static_cast<const TW*>(conv_bias), positions, slots, state, u, n, C, K)
-#define SB_CONV_ROWS(TW, VE)       \
-  do {                             \
-    if (few) SB_CONV(TW, VE, 1);   \
-    else SB_CONV(TW, VE, 4);       \
+  // Four channels a thread have four partial sums on their way and the taps' weights in registers up to four: more of either are round trips
+  // one after the other, which only very many elements hide (64 rows of 2,048 behind nine buffers 4.0 us, 5.1 with four channels; with eight
+  // taps and one buffer, 256 rows 19.6 and 19.8, 1,250 rows 84 and 74). Four rows a thread once those threads fill the SMs: 700 rows of 2,048
+  // 14.7 us, 17.3 with one; 256 rows 6.1 and 6.3; 128 rows 5.4 and 3.8.
+  const bool aligned = C % 4 == 0 && partial_stride % 4 == 0 &&
+                       ((reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(u)) & 15) == 0;
+  // Single channels: the taps in registers while the threads are few (8 rows of 2,050 2.1 us, 3.0 without), else more of them an SM without.
+  const int64_t elements = static_cast<int64_t>(n) * C;
+  const bool vec = aligned && n_partials <= 4 && (K <= 4 || elements >= 1 << 21), rows4 = vec && elements >= 1 << 19;
+#define SB_CONV(TW, VE, ROWS, HELD)                                                                                                                    \
+  sb::launch_pdl(rglru_conv_kernel<TW, VE, ROWS, HELD>, dim3((n + ROWS - 1) / ROWS, (C / VE + 127) / 128), dim3(128), 0, stream, pr,                   \
+                 static_cast<const TW*>(x_bias), static_cast<const TW*>(taps), static_cast<const TW*>(conv_bias), positions, slots, state, u, n, C, K)
+#define SB_CONV_T(TW)                              \
+  do {                                             \
+    if (rows4) SB_CONV(TW, 4, 4, 4);               \
+    else if (vec) SB_CONV(TW, 4, 1, 4);            \
+    else if (elements <= 3 << 16) SB_CONV(TW, 1, 1, 4); \
+    else SB_CONV(TW, 1, 1, 0);                     \
   } while (0)
-  if (w_dtype == 0) {
-    if (vec) SB_CONV_ROWS(float, 4);
-    else SB_CONV_ROWS(float, 1);
-  } else if (w_dtype == 1) {
-    if (vec) SB_CONV_ROWS(bf16, 4);
-    else SB_CONV_ROWS(bf16, 1);
-  } else {
-    return sb::fail("sb_rglru_conv: unsupported dtype %d", w_dtype);
-  }
+  if (w_dtype == 0) SB_CONV_T(float);
+  else if (w_dtype == 1) SB_CONV_T(bf16);
+  else return sb::fail("sb_rglru_conv: unsupported dtype %d", w_dtype);
 #undef SB_CONV
-#undef SB_CONV_ROWS
+#undef SB_CONV_T
   return sb::check_launch("sb_rglru_conv");
 }
 

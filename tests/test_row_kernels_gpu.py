@@ -396,3 +396,28 @@ def test_gates_do_not_show_their_form(bw, B, n):
         for weights in (gate_w, gate_w.float()):
             for x, w in zip(run(m, weights), whole):
                 assert torch.equal(x, w[:m]), m
+
+
+@pytest.mark.parametrize("C,K,P,n", [(2048, 4, 2, 300), (2048, 8, 1, 1030), (2048, 4, 9, 80), (2050, 4, 1, 80), (64, 16, 3, 5)])
+def test_convolution_does_not_show_its_form(C, K, P, n):
+    """One and four channels a thread, one and four rows, taps in registers or not: the bits of a few rows in those of n, and the rows within
+    K + P roundings of the sum of the magnitudes in 64 bits."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(C + K)
+    proj, xb, cb, taps = (torch.randn(*s, generator=g).to(DEV) for s in ((P, n, 2 * C), (C,), (C,), (C, K)))
+    pos, slot = torch.arange(n, dtype=torch.int32, device=DEV), torch.zeros(n, dtype=torch.int32, device=DEV)
+
+    def run(m):
+        u = torch.empty(m, C, device=DEV)
+        ops.rglru_conv(proj[:, :m].contiguous(), xb, taps, cb, pos[:m], slot[:m], torch.full((1, K, C), 7.0, device=DEV), u)
+        return u
+
+    whole = run(n)
+    for m in (1, 5, 33, 70, 256):
+        if m < n:
+            assert torch.equal(run(m), whole[:m]), m
+    x = proj[:, :, C:].double().sum(0) + xb.double()
+    x = torch.cat([torch.zeros(K - 1, C, dtype=torch.float64, device=DEV), x])
+    want = sum(taps[:, j].double() * x[j:j + n] for j in range(K)) + cb.double()
+    size = sum(taps[:, j].double().abs() * x[j:j + n].abs() for j in range(K)) + cb.double().abs() + P * 4.0
+    assert ((whole.double() - want).abs() <= (K + P + 2) * 2.0 ** -23 * size * P).all()
