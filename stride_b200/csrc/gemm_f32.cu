@@ -160,14 +160,16 @@ __device__ __forceinline__ void copy16_async(void* dst, const void* src) {
 // In registers a warp kept half as much, drained at every wait, and a second kernel's requests began only when the first had ended. Measured
 // with bfloat16 weights, one token, before -> now: 16384 x 2048 17.0 -> 13.6 us, 128256 x 2048 106 -> 88,
 // 2048 x 8192 13.8 -> 10.2; within a step of the 1B sizes 17.1 -> 14.7 and 13.7 -> 8.6.
-constexpr int kStreamWarps = 16, kPieces = 4;
+constexpr int kStreamWarps = 16;
+template <class TW>
+constexpr int kPiecesOf = 8 / sizeof(TW);      // 2 KB a group and warp
 template <class TX, class TW, int NT, int STAGES>
-__global__ void __launch_bounds__(kStreamWarps * 32) gemv_f32_kernel(const TX* __restrict__ x, int64_t ldx, const TW* __restrict__ w, int64_t ldw,
+__global__ void __launch_bounds__(kStreamWarps * 32, 2) gemv_f32_kernel(const TX* __restrict__ x, int64_t ldx, const TW* __restrict__ w, int64_t ldw,
                                                                       float* __restrict__ out, int64_t ldo, int n, int M, int K, int accumulate) {
   // The tokens, piece by piece: a piece's first four values of all 32 lanes, then its last four (a lane reads its
   // eight with two requests of 16 bytes, each of them consecutive over the lanes). Padded to whole pieces of 256. Behind them the rings.
   extern __shared__ __align__(16) float xs[];
-  constexpr int kLane = 8 * sizeof(TW);                // bytes of a lane's share of a piece
+  constexpr int kLane = 8 * sizeof(TW), kPieces = kPiecesOf<TW>;      // kLane: bytes of a lane's share of a piece
   sb::grid_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = warp * gridDim.x + blockIdx.x, G = gridDim.x * kStreamWarps;      // (the first features spread over all SMs)
@@ -257,7 +259,7 @@ __global__ void __launch_bounds__(kStreamWarps * 32) gemv_f32_kernel(const TX* _
 constexpr size_t kStreamMaxShared = 224 * 1024;
 template <class TW>
 inline size_t stream_shared(int tokens, int K, int stages) {
-  return static_cast<size_t>(tokens) * ((K + 255) / 256) * 256 * sizeof(float) + static_cast<size_t>(kStreamWarps) * stages * kPieces * 32 * 8 * sizeof(TW);
+  return static_cast<size_t>(tokens) * ((K + 255) / 256) * 256 * sizeof(float) + static_cast<size_t>(kStreamWarps) * stages * kPiecesOf<TW> * 32 * 8 * sizeof(TW);
 }
 
 template <class TX, class TW, int NT, int STAGES>
@@ -283,6 +285,7 @@ bool launch_stream(const void* x, int64_t ldx, const void* w, int64_t ldw, float
   if (M <= kStreamWarps * sms && fits(5, 200)) SB_STREAM(5, sms);
   else if (fits(3, 108)) SB_STREAM(3, 2 * sms);
   else if (fits(2, 108)) SB_STREAM(2, 2 * sms);
+  else if (sizeof(TW) == 4 && fits(5, 224)) SB_STREAM(5, sms);
   else if (fits(3, 200)) SB_STREAM(3, sms);
   else if (stream_shared<TW>(NT, K, 2) <= kStreamMaxShared) SB_STREAM(2, sms);
   else return false;
@@ -296,7 +299,13 @@ template <class TX, class TW, bool VEC>
 void dispatch(const void* x, int64_t ldx, const void* w, int64_t ldw, float* out, int64_t ldo, int n, int M, int K, int accumulate,
               cudaStream_t stream) {
   if (!VEC) return launch<TX, TW, false, 1, 4, 1>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream);
-  if (n == 1 && launch_stream<TX, TW, 1>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream)) return;
+  // One token: a stream, with float32 weights only where the features are fewer than its warps and their rows long (1024 x 28672: 36 us, 53
+  // with the tile). Otherwise such weights reach 3.6 TB/s as a stream and 4.6 to 5 in the tile's registers, with two pieces a group where the
+  // warps are many and their rows not so long (16384 x 2048 38 us as a stream, 29 with four pieces, 27 with two; 2048 x 2048 6.9, 6.3, 7.8;
+  // 4096 x 24576 114, 89, 93).
+  const bool narrow = M <= kStreamWarps * sb::sm_count();
+  if (n == 1 && (sizeof(TW) == 2 || (narrow && K >= 8192)) && launch_stream<TX, TW, 1>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream)) return;
+  if (n == 1 && sizeof(TW) == 4 && M >= 4096 && K <= 16384) return launch<TX, TW, true, 1, 1, 2>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream);
   if (n == 1) return launch<TX, TW, true, 1, 1, 4>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream);
   // few outputs (a router's product): as many warps as there are outputs, or a quarter of that, rather than a few that share operands
   // (9 x 2048, 8 and 64 tokens: 30 and 21 us with the shapes below)
@@ -304,7 +313,7 @@ void dispatch(const void* x, int64_t ldx, const void* w, int64_t ldw, float* out
   if (outputs < 16 * sms) return launch<TX, TW, true, 1, 1, 4>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream);
   // (16384 x 2048, four tokens: 26 us as a stream, 45 with the tile below, which reads the tokens again for every piece)
   if (n == 2 && launch_stream<TX, TW, 2>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream)) return;
-  if ((n == 3 || n == 4) && launch_stream<TX, TW, 4>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream)) return;
+  if ((n == 3 || n == 4) && (sizeof(TW) == 2 || K >= 1024) && launch_stream<TX, TW, 4>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream)) return;
   if (n <= 4 || outputs < 64 * sms) return launch<TX, TW, true, 1, 4, 2>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream);
   if (n <= 16) return launch<TX, TW, true, 2, 8, 1>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream);
   return launch<TX, TW, true, 4, 8, 1>(x, ldx, w, ldw, out, ldo, n, M, K, accumulate, stream);
