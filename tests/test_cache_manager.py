@@ -33,6 +33,43 @@ def test_groups_slots_and_views():
     assert [cm.acquire_slot(), cm.acquire_slot(), cm.acquire_slot()] == [1, 2, -1]
 
 
+def test_records_that_start_from_zeros_by_themselves_are_left():
+    needs = [CacheNeed("state", state_shape=(3,)), CacheNeed("state", state_shape=(2,), zeroed=False),
+             [CacheNeed("state", state_shape=(4,), zeroed=False), CacheNeed("state", state_shape=(5,))]]
+    cm = CacheManager(needs, device="cpu", max_slots=2, max_context=8, page_size=4)
+    records = [cm.layer_cache(0).state, cm.layer_cache(1).state, *(part.state for part in cm.layer_cache(2).parts)]
+    slot = cm.acquire_slot()
+    for record in records:
+        record += 7
+    cm.release_slot(slot)
+    assert cm.acquire_slot() == slot
+    assert [float(record[slot].abs().max()) for record in records] == [0, 7, 7, 0]
+    assert all(float(record[1 - slot].min()) == 7 for record in records)        # another slot's record is nobody's business
+
+
+@pytest.mark.parametrize("order", [(0, 1, 2, 3, 4, 5), (0, 2, 5), (4, 5, 1), (3,), (5, 3, 1, 0, 4)])
+def test_changed_rows_reach_the_device_table(order):
+    """Rows of neighbouring slots travel in one copy: every row that changed arrives, in both groups, and no other is touched."""
+    cm = CacheManager(_needs(window=10), device="cpu", max_slots=6, max_context=64, page_size=4, num_pages=90, shuffle_seed=3)
+    for g in cm.groups:
+        g.table_device = g.table_pinned.clone()          # (on the CPU the two may share memory)
+    slots = [cm.acquire_slot() for _ in range(6)]
+    cm.sync()
+    for round_ in (1, 2):
+        for s in order:
+            assert cm.ensure(slots[s], 9 * round_)
+        for g in cm.groups:
+            for s in slots:
+                if s not in order:
+                    g.table_device[s] = -5               # (a copy of an unchanged row would show)
+        cm.sync()
+        for g in cm.groups:
+            for s in slots:
+                want = g.table_pinned[s] if s in order else torch.full_like(g.table_pinned[s], -5)
+                assert torch.equal(g.table_device[s], want)
+            assert torch.equal(g.table_device[cm.pad_slot], g.table_pinned[cm.pad_slot])
+
+
 def test_ensure_is_all_or_nothing_and_pages_are_reused():
     cm = CacheManager(_needs(), device="cpu", max_slots=4, max_context=64, page_size=4, num_pages=6)
     a, b = cm.acquire_slot(), cm.acquire_slot()

@@ -181,6 +181,35 @@ def test_rms_norm_does_not_show_its_form(H):
     assert (out.double() - want[:64]).abs().max() <= 2e-6 * float(want.abs().max())      # sixteen roundings of a 32-bit result
 
 
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("window,keep", [(0, 0), (64, 5)])
+def test_rows_never_meet_keys_they_do_not_see(bad, window, keep):
+    """Two tokens a block share staged keys: the one in front does not see the other's latent, the other has one key less at the window's
+    start. Latents that are no numbers change no row that does not see them, alone in a block or as one of two."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(window)
+    H, D, page, n = 16, 512, 32, 400
+    pages = (torch.randn(13, 1, 1, page, D, generator=g) * 0.5).bfloat16().to(DEV)
+    table = torch.arange(13, dtype=torch.int32, device=DEV)[None]
+    q = torch.randn(n, H * D, generator=g).bfloat16().to(DEV)
+
+    def run(cache, first, count):
+        meta = torch.tensor([[0], [0], [count], [first]], dtype=torch.int32, device=DEV)
+        out = torch.empty(count, H * D, dtype=torch.bfloat16, device=DEV)
+        ops.masked_attention_tiles(q[first:first + count].contiguous(), out, cache, table, meta, 1, None, None, H, 1, D, D, window, keep, 0.05)
+        return out
+
+    i = torch.arange(n, device=DEV)
+    for key in (101, 154, 399):                     # the second and the first token of a block, the last of all
+        damaged = pages.clone()
+        damaged[key // page, 0, 0, key % page] = bad
+        sees = (i >= key) & ((i - key < window) | (key < keep)) if window else i >= key
+        for first, count in ((0, n), (90, 99), (301, 99)):
+            clean, got, seen = run(pages, first, count), run(damaged, first, count), sees[first:first + count]
+            assert torch.equal(got[~seen], clean[~seen]) and torch.isfinite(clean).all()
+            assert not torch.isfinite(got[seen].float()).all() or not seen.any()
+
+
 @pytest.mark.parametrize("gated", [True, False])
 @pytest.mark.parametrize("lengths", [[2, 0], [1, 3, 0, 0], [1, 1, 1]])
 def test_recurrence_with_as_many_tokens_as_entries(gated, lengths):
@@ -235,35 +264,6 @@ def test_recurrence_with_an_infinite_value(D, tokens, gated):
     assert torch.isinf(state[0, 0, :, column]).all() and torch.isinf(state).sum() == D and not torch.isnan(state).any()
 
 
-@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
-@pytest.mark.parametrize("window,keep", [(0, 0), (64, 5)])
-def test_rows_never_meet_keys_they_do_not_see(bad, window, keep):
-    """Two tokens a block share staged keys: the one in front does not see the other's latent, the other has one key less at the window's
-    start. Latents that are no numbers change no row that does not see them, alone in a block or as one of two."""
-    from stride_b200.kernels import ops
-    g = torch.Generator().manual_seed(window)
-    H, D, page, n = 16, 512, 32, 400
-    pages = (torch.randn(13, 1, 1, page, D, generator=g) * 0.5).bfloat16().to(DEV)
-    table = torch.arange(13, dtype=torch.int32, device=DEV)[None]
-    q = torch.randn(n, H * D, generator=g).bfloat16().to(DEV)
-
-    def run(cache, first, count):
-        meta = torch.tensor([[0], [0], [count], [first]], dtype=torch.int32, device=DEV)
-        out = torch.empty(count, H * D, dtype=torch.bfloat16, device=DEV)
-        ops.masked_attention_tiles(q[first:first + count].contiguous(), out, cache, table, meta, 1, None, None, H, 1, D, D, window, keep, 0.05)
-        return out
-
-    i = torch.arange(n, device=DEV)
-    for key in (101, 154, 399):                     # the second and the first token of a block, the last of all
-        damaged = pages.clone()
-        damaged[key // page, 0, 0, key % page] = bad
-        sees = (i >= key) & ((i - key < window) | (key < keep)) if window else i >= key
-        for first, count in ((0, n), (90, 99), (301, 99)):
-            clean, got, seen = run(pages, first, count), run(damaged, first, count), sees[first:first + count]
-            assert torch.equal(got[~seen], clean[~seen]) and torch.isfinite(clean).all()
-            assert not torch.isfinite(got[seen].float()).all() or not seen.any()
-
-
 @pytest.mark.parametrize("gated", [True, False])
 @pytest.mark.parametrize("D,V", [(64, 128), (10, 40), (128, 40), (126, 30), (200, 128), (130, 30), (256, 16)])
 def test_recurrence_does_not_show_its_columns_a_warp(D, V, gated):
@@ -307,72 +307,6 @@ def test_recurrence_does_not_show_its_columns_a_warp(D, V, gated):
         want.append(torch.einsum("hdv,hd->hv", S, q[t]).reshape(-1))
     want = torch.stack(want)
     assert (whole[rows[2]:rows[2] + lengths[2]].double() - want).abs().max() <= 2e-5 * float(want.abs().max())
-
-
-@pytest.mark.parametrize("H", [516, 1024, 2048, 2050, 3072, 4100, 9000])
-def test_norms_do_not_show_the_rows(H):
-    """As many rows as run at once, and more: other numbers of partial sums on their way and of blocks an SM, the same bits."""
-    from stride_b200.kernels import ops
-    g = torch.Generator().manual_seed(H)
-    n, w, b = 760, torch.randn(H, generator=g).to(DEV), torch.randn(H, generator=g).to(DEV)
-    h, parts = torch.randn(n, H, generator=g).to(DEV), torch.randn(9, n, H, generator=g).to(DEV)
-
-    def run(m, norm):
-        x, out = h[:m].clone(), torch.empty(m, H, device=DEV)
-        if norm == "rms":
-            ops.rmsnorm(x, w, 1e-5, out, partials=parts[:, :m].contiguous())
-        else:
-            ops.layernorm(x, w, b, 1e-5, out, partials=parts[:, :m].contiguous())
-        return torch.cat([x, out], 1)
-
-    for norm in ("rms", "layer"):
-        whole = run(n, norm)
-        for m in (1, 149, 297, 741):
-            assert torch.equal(run(m, norm), whole[:m]), (norm, m)
-
-
-@pytest.mark.parametrize("HD,HV", [(6, 10), (250, 130), (128, 64)])
-def test_gates_of_linear_attention_do_not_show_the_rows(HD, HV):
-    """Single elements, one and four a thread, and four neighbouring ones: the bits of a few rows in those of 1,030, and 64 bits within 2e-6."""
-    from stride_b200.kernels import ops
-    g = torch.Generator().manual_seed(HD)
-    n, dev = 1030, lambda *s: torch.randn(*s, generator=g).to(DEV)
-    proj, fb, low = dev(3, n, 2 * HD + HV), dev(HD), torch.rand(HD, generator=g).to(DEV)
-
-    def run(m):
-        act = torch.empty(m, 3 * HD + HV, device=DEV)
-        ops.hgrn2_activate(proj[:, :m].contiguous(), fb, low, act, HD, HV)
-        return act
-
-    whole = run(n)
-    for m in (1, 1024, 1025):
-        assert torch.equal(run(m), whole[:m])
-    z = proj.double().sum(0)
-    gate = low.double() + (1 - low.double()) * torch.sigmoid(z[:, HD:2 * HD] + fb.double())
-    want = torch.cat([torch.nn.functional.silu(z[:, :HD]), gate, 1 - gate, z[:, 2 * HD:]], 1)
-    assert (whole.double() - want).abs().max() <= 2e-6 * float(want.abs().max())      # a few roundings of sums of three
-
-
-@pytest.mark.parametrize("D,rot", [(64, 32), (96, 24), (64, 0), (64, 64)])
-@pytest.mark.parametrize("P", [1, 2, 9])
-def test_rotation_does_not_show_the_number_of_tokens(D, rot, P):
-    """A pair a thread for a few tokens of heads rotated in part, four pairs otherwise: the bits of a few tokens in those of 70."""
-    from stride_b200.kernels import ops
-    g = torch.Generator().manual_seed(D + rot)
-    n, Hq, Hkv, page = 70, 5, 2, 16
-    qkv = torch.randn(P, n, (Hq + 2 * Hkv) * D, generator=g).to(DEV)
-    pos, slots = torch.arange(n, dtype=torch.int32, device=DEV), torch.zeros(n, dtype=torch.int32, device=DEV)
-    table, pages = torch.randn(n, max(rot // 2, 1), 2, generator=g).to(DEV), torch.arange(5, dtype=torch.int32, device=DEV)[None]
-
-    def run(m):
-        q, cache = torch.empty(m, Hq * D, device=DEV), torch.zeros(5, 2, Hkv, page, D, device=DEV)
-        ops.rope_append(qkv[:, :m].contiguous(), pos[:m], slots[:m], table, rot, q, cache, pages, Hq, Hkv, D)
-        return q, cache.permute(0, 3, 1, 2, 4).reshape(5 * page, -1)[:m]
-
-    whole = run(n)
-    for m in (1, 16, 17, 64, 65):
-        for x, w in zip(run(m), whole):
-            assert torch.equal(x, w[:m]), m
 
 
 @pytest.mark.parametrize("bw,B,n", [(128, 2, 330), (100, 3, 330), (33, 2, 1410), (16, 3, 330), (272, 1, 330), (1040, 1, 330)])
@@ -421,3 +355,117 @@ def test_convolution_does_not_show_its_form(C, K, P, n):
     want = sum(taps[:, j].double() * x[j:j + n] for j in range(K)) + cb.double()
     size = sum(taps[:, j].double().abs() * x[j:j + n].abs() for j in range(K)) + cb.double().abs() + P * 4.0
     assert ((whole.double() - want).abs() <= (K + P + 2) * 2.0 ** -23 * size * P).all()
+
+
+@pytest.mark.parametrize("HD,HV", [(6, 10), (250, 130), (128, 64)])
+def test_gates_of_linear_attention_do_not_show_the_rows(HD, HV):
+    """Single elements, one and four a thread, and four neighbouring ones: the bits of a few rows in those of 1,030, and 64 bits within 2e-6."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(HD)
+    n, dev = 1030, lambda *s: torch.randn(*s, generator=g).to(DEV)
+    proj, fb, low = dev(3, n, 2 * HD + HV), dev(HD), torch.rand(HD, generator=g).to(DEV)
+
+    def run(m):
+        act = torch.empty(m, 3 * HD + HV, device=DEV)
+        ops.hgrn2_activate(proj[:, :m].contiguous(), fb, low, act, HD, HV)
+        return act
+
+    whole = run(n)
+    for m in (1, 1024, 1025):
+        assert torch.equal(run(m), whole[:m])
+    z = proj.double().sum(0)
+    gate = low.double() + (1 - low.double()) * torch.sigmoid(z[:, HD:2 * HD] + fb.double())
+    want = torch.cat([torch.nn.functional.silu(z[:, :HD]), gate, 1 - gate, z[:, 2 * HD:]], 1)
+    assert (whole.double() - want).abs().max() <= 2e-6 * float(want.abs().max())      # a few roundings of sums of three
+
+
+@pytest.mark.parametrize("H", [516, 1024, 2048, 2050, 3072, 4100, 9000])
+def test_norms_do_not_show_the_rows(H):
+    """As many rows as run at once, and more: other numbers of partial sums on their way and of blocks an SM, the same bits."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(H)
+    n, w, b = 760, torch.randn(H, generator=g).to(DEV), torch.randn(H, generator=g).to(DEV)
+    h, parts = torch.randn(n, H, generator=g).to(DEV), torch.randn(9, n, H, generator=g).to(DEV)
+
+    def run(m, norm):
+        x, out = h[:m].clone(), torch.empty(m, H, device=DEV)
+        if norm == "rms":
+            ops.rmsnorm(x, w, 1e-5, out, partials=parts[:, :m].contiguous())
+        else:
+            ops.layernorm(x, w, b, 1e-5, out, partials=parts[:, :m].contiguous())
+        return torch.cat([x, out], 1)
+
+    for norm in ("rms", "layer"):
+        whole = run(n, norm)
+        for m in (1, 149, 297, 741):
+            assert torch.equal(run(m, norm), whole[:m]), (norm, m)
+
+
+@pytest.mark.parametrize("D,rot", [(64, 32), (96, 24), (64, 0), (64, 64)])
+@pytest.mark.parametrize("P", [1, 2, 9])
+def test_rotation_does_not_show_the_number_of_tokens(D, rot, P):
+    """A pair a thread for a few tokens of heads rotated in part, four pairs otherwise: the bits of a few tokens in those of 70."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(D + rot)
+    n, Hq, Hkv, page = 70, 5, 2, 16
+    qkv = torch.randn(P, n, (Hq + 2 * Hkv) * D, generator=g).to(DEV)
+    pos, slots = torch.arange(n, dtype=torch.int32, device=DEV), torch.zeros(n, dtype=torch.int32, device=DEV)
+    table, pages = torch.randn(n, max(rot // 2, 1), 2, generator=g).to(DEV), torch.arange(5, dtype=torch.int32, device=DEV)[None]
+
+    def run(m):
+        q, cache = torch.empty(m, Hq * D, device=DEV), torch.zeros(5, 2, Hkv, page, D, device=DEV)
+        ops.rope_append(qkv[:, :m].contiguous(), pos[:m], slots[:m], table, rot, q, cache, pages, Hq, Hkv, D)
+        return q, cache.permute(0, 3, 1, 2, 4).reshape(5 * page, -1)[:m]
+
+    whole = run(n)
+    for m in (1, 16, 17, 64, 65):
+        for x, w in zip(run(m), whole):
+            assert torch.equal(x, w[:m]), m
+
+
+@pytest.mark.parametrize("W", [24, 2048, 4100])
+def test_one_partial_buffer_gives_the_bits_of_several(W):
+    """The forms for a single partial buffer against the same buffer beside a second one of zeros (x + 0 has the bits of x)."""
+    from stride_b200.kernels import ops
+    g = torch.Generator().manual_seed(W)
+    n, dev = 9, lambda *s: torch.randn(*s, generator=g).to(DEV)
+    two = lambda p: torch.cat([p, torch.zeros_like(p)])
+    up, h, w, b, o = dev(1, n, W), dev(n, W), dev(W), dev(W), dev(n, W)
+
+    def polynorm(p):
+        out = torch.empty(n, W, device=DEV)
+        ops.polynorm(p, out, (0.7, -0.3, 0.2, 0.05), 1e-5)
+        return out
+
+    def layernorm(p):
+        x, out = h.clone(), torch.empty(n, W, device=DEV)
+        ops.layernorm(x, w, b, 1e-5, out, partials=p)
+        return torch.cat([x, out])
+
+    def gated_norm(p):
+        out = torch.empty(n, W, device=DEV)
+        ops.gated_rmsnorm(o, p, 0, w, 1e-5, out)
+        return out
+
+    def hgrn2(p):
+        out = torch.empty(n, 3 * (W // 4) + W // 2, device=DEV)
+        ops.hgrn2_activate(p, w[:W // 4], torch.sigmoid(b[:W // 4]), out, W // 4, W // 2)
+        return out
+
+    def lightning(p):
+        H = {24: 1, 2048: 4, 4100: 5}[W]
+        D, V = W // 4 // H, W // 2 // H
+        state, out, meta = torch.zeros(1, H, D, V, device=DEV), torch.empty(n, H * V, device=DEV), torch.tensor([[0], [0], [n], [0]], dtype=torch.int32, device=DEV)
+        ops.lightning_scan(p, 0, H * D, 2 * H * D, meta, 1, torch.full((H,), 0.9, device=DEV), state, out, H, D, V, torch.empty(n * W, device=DEV))
+        return torch.cat([out.flatten(), state.flatten()])
+
+    def rope(p):
+        D, Hq, Hkv = 8, W // 8 - 2, 1
+        turn = torch.stack([torch.linspace(0, 2, 64).cos(), torch.linspace(0, 2, 64).sin()], -1).view(16, 4, 2).to(DEV)
+        q, cache = torch.empty(n, Hq * D, device=DEV), torch.zeros(1, 2, Hkv, 16, D, device=DEV)
+        ops.rope_append(p, torch.arange(n, dtype=torch.int32, device=DEV), torch.zeros(n, dtype=torch.int32, device=DEV), turn, D, q, cache,
+                        torch.zeros(1, 1, dtype=torch.int32, device=DEV), Hq, Hkv, D)
+        return torch.cat([q.flatten(), cache.flatten()])
+
+    for form in (polynorm, layernorm, gated_norm, hgrn2, lightning) + ((rope,) if W % 8 == 0 else ()):
+        assert torch.equal(form(up), form(two(up))), form.__name__
