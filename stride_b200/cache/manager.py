@@ -11,7 +11,8 @@ request and a host block table mirrored on the device. Here:
   free list and its own block table `[slots, pages per sequence]`; one page id
   covers all layers of its group.
 * A request holds one *slot*: a row of every block table and one record of every
-  state arena `[slots, ...]`, zeroed when the slot is taken.
+  state arena `[slots, ...]`, zeroed when the slot is taken unless the mixer's kernels
+  start from zeros by themselves (`CacheNeed.zeroed`).
 * Pages come back when the request releases its slot, and, for a group with a
   window, as soon as every position of the page lies behind the window of all
   tokens still to come (`trim`).

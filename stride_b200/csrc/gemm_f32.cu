@@ -276,7 +276,7 @@ void launch_stream_of(const void* x, int64_t ldx, const void* w, int64_t ldw, fl
 
 // Up to a feature a warp: one block an SM whose warps keep five groups requested (most of a row). More features: two blocks an SM, that is
 // 32 warps and 192 KB on their way, where the tokens leave the room (one block of 16 warps: 23 us for 16384 x 2048 within a step; two blocks
-// with two groups a warp 18.5; with three 13.9). Blocks of more than half an SM are launched once an SM.
+// with two groups a warp 18.5; with three 13.9). Blocks of more than half an SM are launched once an SM, with float32 weights five groups deep.
 template <class TX, class TW, int NT>
 bool launch_stream(const void* x, int64_t ldx, const void* w, int64_t ldw, float* out, int64_t ldo, int n, int M, int K, int accumulate, cudaStream_t stream) {
   const int sms = sb::sm_count();

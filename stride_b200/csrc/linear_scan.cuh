@@ -135,9 +135,11 @@ __device__ __forceinline__ void bar_arrive(int id, int count) { asm volatile("ba
 // parts of 32 / PER tokens' outputs are added up together by exchanges between lanes, so that no part goes through shared memory. One more
 // warp keeps the rows of the next two chunks of tokens on their way into the staging buffers; it announces a chunk before it requests
 // another, since a request waits until its buffer is free. What bounds the kernel is each warp's wait for its own reads and exchanges, with one
-// or two computing warps a scheduler (issue slots 47% busy; without the loads and the exchanges 155 of its 220 us are left).
-// Measured (16 heads of 128 x 128, one entry of 2,048 tokens / eight): eight warps of one column a thread, the outputs' parts through shared
-// memory, 611 / 1,600 us; PER = 4 220 / 721 us, PER = 2 193 / 828 us.
+// or two computing warps a scheduler (PER = 2: issue slots 47% busy; PER = 4: without the loads and the exchanges 155 of 220 us are left).
+// Measured (16 heads of 128 x 128 without gates, one entry of 2,048 tokens / eight, launches one behind another): eight warps of one column a
+// thread, the outputs' parts through shared memory, 611 / 1,600 us; PER = 4 220 / 710 us, PER = 2 187 / 828 us. A launch on its own takes 143 us
+// with PER = 2, whether its rows lie in L2 or not: one behind another its CTAs take their places while the one in front still runs, wherever
+// an SM has room, which probably leaves some SMs with more of them.
 // With eight elements a lane: the row's pieces of four lie the even ones first, then the odd ones, so that the lanes' 16-byte reads take
 // neighbouring places (side by side they would meet in half the banks), and with gates two staging buffers, which leaves two CTAs an SM.
 template <int DL, bool GATED>
@@ -322,7 +324,7 @@ int launch_scan_of(const Params& p, int entries, const char* who, cudaStream_t s
 }
 
 // Launches scan_kernel for the key size (at most 256). Four columns a warp make fewer reads a column; two make twice the CTAs, which is the
-// faster way while they all run at once (193 against 220 us for 128 CTAs of four; 828 against 721 us for 1,024).
+// faster way while they all run at once (187 against 220 us for 128 CTAs of four; 828 against 710 us for 1,024).
 template <bool GATED>
 int launch_scan(const Params& p, int entries, const char* who, cudaStream_t stream) {
   const bool few = static_cast<int64_t>(entries) * p.H * ((p.V + 15) / 16) <= sb::sm_count();

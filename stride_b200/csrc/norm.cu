@@ -116,7 +116,7 @@ __device__ __forceinline__ void store_normed4(TO* o, float4 v, float4 w, float s
 // Few rows behind several partial buffers (decoding): a row's ten reads of 8 KB are more than one SM takes in during a round trip to L2, so a
 // row is a cluster of four blocks, each with a quarter of rmsnorm_kernel's threads and their shares; the warps' sums of squares go to all four
 // blocks' shared memory and are added in rmsnorm_kernel's order: equal bits. One to 64 rows of 2,048 behind nine buffers, within a decode
-// step: 3.5 to 3.8 us, 4.1 to 4.5 as a block a row.
+// step: 3.4 to 4.1 us, 4.1 to 4.5 as a block a row.
 __device__ __forceinline__ void cluster_store(const float* p, uint32_t rank, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(sb::cluster_peer_address(p, rank)), "f"(v) : "memory");
 }
@@ -228,19 +228,21 @@ __global__ void __launch_bounds__(512) rmsnorm_pairs_kernel(float* __restrict__ 
 // never on the rows, so a row's result does not either. A thread keeps its first kKeep pieces in registers through both sums, those beyond in
 // shared memory. Bound by memory: 2,048 rows of 2,048 with one partial buffer 10.5 us (22 with the registers for eight partial buffers,
 // hence FLIGHT), single elements in shared memory 24 us.
-// The blocks an SM that its registers are cut for (0: left to the compiler).
+//
+// layernorm_blocks: the blocks an SM that its registers are cut for (0: left to the compiler).
 constexpr int layernorm_blocks(int VEC, int MAXT, int FLIGHT, size_t bytes) {
   if (VEC == 1) return 2048 / MAXT;
   if (FLIGHT == 1) return bytes == 4 ? 4 : 3;      // (of 512 threads: 32 registers a thread where gain and output are bfloat16, else 40)
   return FLIGHT == 4 ? 1024 / MAXT : 0;
 }
 template <class TW, class TO, int VEC, int MAXT, int FLIGHT>     // MAXT: the most threads of a block, FLIGHT: the partial sums requested together
-__global__ void __launch_bounds__(MAXT, layernorm_blocks(VEC, MAXT, FLIGHT, sizeof(TW) + sizeof(TO))) layernorm_kernel(float* __restrict__ h, const float* __restrict__ partials, int n_partials,
-                                                         int64_t partial_stride, const TW* __restrict__ weight,
-                                                         const TW* __restrict__ bias, TO* __restrict__ out, int H, float eps) {
+__global__ void __launch_bounds__(MAXT, layernorm_blocks(VEC, MAXT, FLIGHT, sizeof(TW) + sizeof(TO))) layernorm_kernel(
+    float* __restrict__ h, const float* __restrict__ partials, int n_partials, int64_t partial_stride, const TW* __restrict__ weight,
+    const TW* __restrict__ bias, TO* __restrict__ out, int H, float eps) {
   using V = typename VecF<VEC>::type;
   constexpr int kKeep = VEC == 4 ? 2 : 1;
-  constexpr bool kBeyond = VEC == 1 || MAXT > 512 || FLIGHT == 8;      // (512 threads and fewer keep all of a row)
+  constexpr bool kBeyond = VEC == 1 || MAXT > 512 || FLIGHT == 8;      // (512 threads and fewer keep all of a
+  // row; with eight partial sums the kernel is the faster one with these loops compiled in: 4.4 us, 5.6 without, 256 rows of 2,048 behind nine)
   extern __shared__ __align__(16) float beyond_raw[];
   __shared__ float red[32];
   sb::grid_launch_dependents();
@@ -321,12 +323,14 @@ SB_EXPORT int sb_layernorm(float* h, const float* partials, int n_partials, int6
   if (H > 50 * 1024) return sb::fail("sb_layernorm: width %d (at most 51200)", H);
   auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   const bool vec = H % 4 == 0 && aligned(h) && aligned(partials) && aligned(weight) && aligned(bias) && aligned(out) && partial_stride % 4 == 0;
-  // single elements: several a thread, so that an SM holds more than one row (2,048 rows of 2,050: 17 us, 44 with 1,024 threads)
+  // Single elements: several a thread, so that an SM holds more than one row (2,048 rows of 2,050: 17 us, 44 with 1,024 threads).
   const int units = vec ? H / 4 : H;
   const int threads = vec ? (units > 1024 ? 1024 : units > 512 ? 512 : units > 256 ? 256 : 128) : H >= 4096 ? 1024 : H >= 2048 ? 512 : H >= 512 ? 256 : 128;
   const int kept = (vec ? 2 : 1) * threads;      // (kKeep pieces a thread are in registers)
   const size_t smem = units > kept ? static_cast<size_t>(units - kept) * (vec ? 16 : 4) : 0;
-  const bool at_once = n <= sb::sm_count() * (512 / threads);      // (with eight partial sums requested together an SM holds 512 threads)
+  const bool at_once = n <= sb::sm_count() * (512 / threads);
+  // (with eight partial sums requested together an SM holds 512 threads; more rows take four together, twice the threads: 2,048 rows of 3,072
+  // behind nine buffers 66 us, 95 with eight)
 #define SB_LN_V(TW, TO, VEC, MAXT, FLIGHT)                                                                                       \
   do {                                                                                                                        \
     if (smem > 40 * 1024)                                                                                                     \
@@ -334,13 +338,13 @@ SB_EXPORT int sb_layernorm(float* h, const float* partials, int n_partials, int6
     sb::launch_pdl(layernorm_kernel<TW, TO, VEC, MAXT, FLIGHT>, n, threads, smem, stream, h, partials, n_partials, partial_stride, \
                    static_cast<const TW*>(weight), static_cast<const TW*>(bias), static_cast<TO*>(out), H, eps);              \
   } while (0)
-#define SB_LN(TW, TO)                                                              \
-  do {                                                                             \
-    if (vec && threads <= 512 && n_partials <= 1) SB_LN_V(TW, TO, 4, 512, 1);                    \
-    else if (vec && threads <= 512 && at_once) SB_LN_V(TW, TO, 4, 512, 8);                       \
-    else if (vec && threads <= 512) SB_LN_V(TW, TO, 4, 512, 4);                                  \
-    else if (vec) SB_LN_V(TW, TO, 4, 1024, 4);                                                   \
-    else SB_LN_V(TW, TO, 1, 1024, 8);                                                            \
+#define SB_LN(TW, TO)                                                                \
+  do {                                                                               \
+    if (vec && threads <= 512 && n_partials <= 1) SB_LN_V(TW, TO, 4, 512, 1);        \
+    else if (vec && threads <= 512 && at_once) SB_LN_V(TW, TO, 4, 512, 8);           \
+    else if (vec && threads <= 512) SB_LN_V(TW, TO, 4, 512, 4);                      \
+    else if (vec) SB_LN_V(TW, TO, 4, 1024, 4);                                       \
+    else SB_LN_V(TW, TO, 1, 1024, 8);                                                \
   } while (0)
   if (weight_dtype == 0 && out_dtype == 0) SB_LN(float, float);
   else if (weight_dtype == 0 && out_dtype == 1) SB_LN(float, bf16);
@@ -357,7 +361,7 @@ SB_EXPORT int sb_rmsnorm(float* h, const float* partials, int n_partials, int64_
                          int weight_dtype, void* out, int out_dtype, int n, int H, float eps, cudaStream_t stream) {
   if (n <= 0) return 0;
   const size_t smem = static_cast<size_t>(H) * sizeof(float);
-  if (smem > 200 * 1024) return sb::fail("sb_rmsnorm: width %d does not fit the row buffer (max 51200)", H);
+  if (smem > 200 * 1024) return sb::fail("sb_rmsnorm: width %d (at most 51200)", H);      // (rmsnorm_kernel's row; one limit for every form)
   const bool vec = H % 4 == 0 && partial_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(partials)) & 15) == 0;
   const int units = vec ? H / 4 : H;
   const int threads = units >= 1024 ? 1024 : units >= 512 ? 512 : units >= 256 ? 256 : 128;
@@ -369,6 +373,8 @@ SB_EXPORT int sb_rmsnorm(float* h, const float* partials, int n_partials, int64_
     sb::launch_pdl(rmsnorm_kernel<TW, TO, VEC, MAXT, FLIGHT, BLOCKS>, n, threads, smem, stream, h, partials, n_partials, partial_stride, \
                    static_cast<const TW*>(weight), static_cast<TO*>(out), H, eps);                               \
   } while (0)
+  // Clusters: 32 rows behind nine buffers, width 2,048 3.0 us, 3.1 as a block a row (one row 2.3 and 2.8), 8,192 4.5 and 6.5; 64 rows 3.2 and 3.1,
+  // 4.7 and 6.6. Narrower rows are one round trip of a block either way (1,024: one row 2.2, 64 rows 2.9).
 #define SB_NORM(TW, TO)                                                                                                         \
   do {                                                                                                                          \
     if (vec && n_partials <= 1 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(weight)) & 15) == 0)         \
@@ -382,7 +388,7 @@ SB_EXPORT int sb_rmsnorm(float* h, const float* partials, int n_partials, int64_
     else if (vec) SB_NORM_V(TW, TO, 4, 512, 12, 0);                                                                             \
     else if (threads > 512 && n > sb::sm_count()) SB_NORM_V(TW, TO, 1, 1024, 8, 0);                                             \
     else if (threads > 512) SB_NORM_V(TW, TO, 1, 1024, 8, 1);                                                                   \
-    else SB_NORM_V(TW, TO, 1, 512, 12, 0);                                                                                         \
+    else SB_NORM_V(TW, TO, 1, 512, 12, 0);                                                                                      \
   } while (0)
   if (weight_dtype == 0 && out_dtype == 0) SB_NORM(float, float);
   else if (weight_dtype == 0 && out_dtype == 1) SB_NORM(float, bf16);
