@@ -17,6 +17,7 @@
 // head) and `head_linear_kernel` (a matrix per head: the key projection taken into the queries in front of the attention, the value
 // projection behind it, there with a sigmoid gate per element on the way out where a design has one).
 #include "common.cuh"
+#include "latent_attention_tc5.cuh"
 #include "step_ops.h"
 
 SB_DEFINE_LAST_ERROR()
@@ -916,6 +917,52 @@ int launch_tiles(const TileParams& p, int n, cudaStream_t stream) {
   return sb::check_launch("sb_masked_attention_tiles");
 }
 
+// Whether latent_attention_tc5_kernel takes a call: latents of 512 that are key and value, no score terms but a window and sinks, pages that
+// TMA can address, `pages` of them (0: not known). Which calls are worth it is launch_latent's rule.
+bool latent_shape(const TileParams& p, int pages) {
+  const int Hg = p.H / p.G;
+  return pages > 0 && p.D == sb::latent5::kDim && p.Dv == p.D && p.Dc == p.D && p.v_offset == 0 && Hg <= 128 && 128 % Hg == 0 && p.G <= 65535 &&
+         p.slopes == nullptr && p.keep_first == 0 && p.chunk == 0 && p.cap <= 0.0f && !p.out_f32 && p.page_size >= 8 &&
+         (p.page_size & (p.page_size - 1)) == 0 && p.page_stride % p.D == 0 && p.head_stride % p.D == 0 &&
+         ((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.pages)) & 15) == 0;
+}
+
+// From two tiles of 128 rows an entry on. (us, tile kernel / here, 16 heads, 700 cached tokens, window 1,024: one entry of 16 tokens 70 / 45,
+// 16 entries of 16 tokens 140 / 47, of 64 tokens 284 / 94, of 128 tokens 530 / 191; four of 512 tokens 625 / 213.)
+int launch_latent(const TileParams& p, int pages, int n, cudaStream_t stream, bool* done) {
+  using namespace sb::latent5;
+  const int Hg = p.H / p.G, ppt = kRows / Hg;
+  const int64_t tiles = (n + ppt - 1) / ppt + p.entries;
+  *done = n >= 2 * static_cast<int64_t>(ppt) * p.entries;
+  if (!*done) return 0;
+  int* status = sb::tc5::status_word();
+  if (!status) return sb::fail("sb_masked_attention_tiles: cannot allocate the status word");
+  Params q{};
+  q.out = p.out, q.block_table = p.block_table, q.max_pages = p.max_pages, q.page_size = p.page_size;
+  while ((1 << q.page_shift) < p.page_size) ++q.page_shift;
+  q.rows_per_page = static_cast<int>(p.page_stride / kDim), q.rows_head = static_cast<int>(p.head_stride / kDim);
+  q.box_rows = p.page_size < kKeys ? p.page_size : kKeys;
+  q.meta = p.meta, q.meta_stride = p.meta_stride, q.entries = p.entries, q.sinks = p.sinks;
+  q.H = p.H, q.G = p.G, q.window = p.window, q.scale = p.scale, q.status = status;
+  CUtensorMap map_q, map_k;
+  const int64_t qdims[3] = {kDim, p.H, n}, qstrides[3] = {1, kDim, static_cast<int64_t>(p.H) * kDim};
+  const int qbox[3] = {64, Hg, ppt};
+  const int64_t rows = static_cast<int64_t>(pages - 1) * q.rows_per_page + static_cast<int64_t>(p.G - 1) * q.rows_head + p.page_size;
+  const int64_t kdims[2] = {kDim, rows}, kstrides[2] = {1, kDim};
+  const int kbox[2] = {64, q.box_rows};
+  if (!sb::tc5::tensor_map_bf16(p.q, 3, qdims, qstrides, qbox, &map_q) || !sb::tc5::tensor_map_bf16(p.pages, 2, kdims, kstrides, kbox, &map_k))
+    return sb::fail("sb_masked_attention_tiles: cuTensorMapEncodeTiled failed");
+  static sb::DeviceOnce once;
+  if (once.needed()) {
+    if (cudaFuncSetAttribute(latent_attention_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes + 1024) != cudaSuccess)
+      return sb::fail("sb_masked_attention_tiles: cannot raise the shared memory limit");
+    once.done();
+  }
+  sb::launch_pdl(latent_attention_tc5_kernel, dim3(static_cast<unsigned>(2 * tiles), p.G), dim3(kThreads), static_cast<size_t>(kSmemBytes + 1024), stream,
+                 map_q, map_k, q);
+  return sb::check_launch("sb_masked_attention_tiles");
+}
+
 PageRef page_ref(void* pages, const int32_t* block_table, int max_pages, int page_size, int64_t page_stride, int64_t v_offset, int64_t head_stride,
                  int Dc) {
   return PageRef{pages, block_table, max_pages, page_size, page_stride, v_offset, head_stride, Dc};
@@ -1063,8 +1110,9 @@ SB_EXPORT int sb_masked_attention_tiles_supported(int H, int G, int D, int Dv, i
   return heads && D % 16 == 0 && D >= 16 && Dv % 16 == 0 && Dv >= 16 && Dv <= 512 && Dv <= Dc && Dc % 8 == 0 && v_offset % 8 == 0 && stage <= 200 * 1024;
 }
 
-SB_EXPORT int sb_masked_attention_tiles_ex(const void* q, void* out, const void* pages, const int32_t* block_table, int max_pages, int page_size,
-                                           int64_t page_stride, int64_t v_offset, int64_t head_stride, const int32_t* meta, int meta_stride,
+// `arena_pages`: pages of the arena behind `pages` (0: not known; the form that addresses pages by TMA is then left out).
+SB_EXPORT int sb_masked_attention_tiles_in(const void* q, void* out, const void* pages, int arena_pages, const int32_t* block_table, int max_pages,
+                                           int page_size, int64_t page_stride, int64_t v_offset, int64_t head_stride, const int32_t* meta, int meta_stride,
                                            int entries, const float* slopes, const float* sinks, int n, int H, int G, int D, int Dv, int Dc,
                                            int window, int keep_first, float scale, int chunk, int out_f32, float cap, cudaStream_t stream) {
   if (n <= 0 || entries <= 0) return 0;
@@ -1074,6 +1122,11 @@ SB_EXPORT int sb_masked_attention_tiles_ex(const void* q, void* out, const void*
   if (window < 0 || keep_first < 0) return sb::fail("sb_masked_attention_tiles: window %d, kept first tokens %d", window, keep_first);
   TileParams p{static_cast<const bf16*>(q), static_cast<bf16*>(out), static_cast<const bf16*>(pages), block_table, max_pages, page_size, page_stride,
                v_offset, head_stride, meta, meta_stride, entries, slopes, sinks, H, G, D, Dv, Dc, window, keep_first, scale, 2, chunk, out_f32, cap};
+  if (latent_shape(p, arena_pages)) {
+    bool done = false;
+    const int rc = launch_latent(p, arena_pages, n, stream, &done);
+    if (done) return rc;
+  }
   const int groups = (Dv / 16 + 3) / 4;
   switch (groups) {
     case 1: return launch_tiles<1>(p, n, stream);
@@ -1082,6 +1135,17 @@ SB_EXPORT int sb_masked_attention_tiles_ex(const void* q, void* out, const void*
     default: return launch_tiles<8>(p, n, stream);
   }
 }
+
+SB_EXPORT int sb_masked_attention_tiles_ex(const void* q, void* out, const void* pages, const int32_t* block_table, int max_pages, int page_size,
+                                           int64_t page_stride, int64_t v_offset, int64_t head_stride, const int32_t* meta, int meta_stride,
+                                           int entries, const float* slopes, const float* sinks, int n, int H, int G, int D, int Dv, int Dc,
+                                           int window, int keep_first, float scale, int chunk, int out_f32, float cap, cudaStream_t stream) {
+  return sb_masked_attention_tiles_in(q, out, pages, 0, block_table, max_pages, page_size, page_stride, v_offset, head_stride, meta, meta_stride, entries,
+                                      slopes, sinks, n, H, G, D, Dv, Dc, window, keep_first, scale, chunk, out_f32, cap, stream);
+}
+
+// From now on the kernels of this library that wait on barriers report into `device_word` (see sb_gemm_tc_use_status_word).
+SB_EXPORT void sb_masked_attention_use_status_word(int* device_word) { sb::tc5::status_word_given() = device_word; }
 
 SB_EXPORT int sb_masked_attention_tiles(const void* q, void* out, const void* pages, const int32_t* block_table, int max_pages, int page_size,
                                         int64_t page_stride, int64_t v_offset, int64_t head_stride, const int32_t* meta, int meta_stride, int entries,
@@ -1178,12 +1242,13 @@ SB_EXPORT int sb_op_masked_attention(const SbOp* op, const SbStep* s, void* stre
 }
 
 // i: 0 q, 1 out, 2 pages, 3 block table, 4 max_pages, 5 page_size, 6 page_stride, 7 v_offset, 8 head_stride, 9 slopes, 10 sinks, 11 H, 12 G, 13 D,
-//    14 Dv, 15 Dc, 16 window, 17 keep_first, 18 chunk, 19 the result as float32      f: 0 scale, 1 soft cap of the scores (0: none)
+//    14 Dv, 15 Dc, 16 window, 17 keep_first, 18 chunk, 19 the result as float32, 20 pages of the arena (0: not known)
+// f: 0 scale, 1 soft cap of the scores (0: none)
 SB_EXPORT int sb_op_masked_attention_tiles(const SbOp* op, const SbStep* s, void* stream) {
   using namespace sbstep;
   if (s->n <= 0) return SB_OP_SKIPPED;
-  return sb_masked_attention_tiles_ex(ptr<const void>(op->i[0]), ptr<void>(op->i[1]), ptr<const void>(op->i[2]), ptr<const int32_t>(op->i[3]), (int)op->i[4],
-                                   (int)op->i[5], op->i[6], op->i[7], op->i[8], entry_meta(s), s->max_rows, s->entries, ptr<const float>(op->i[9]),
+  return sb_masked_attention_tiles_in(ptr<const void>(op->i[0]), ptr<void>(op->i[1]), ptr<const void>(op->i[2]), (int)op->i[20], ptr<const int32_t>(op->i[3]),
+                                   (int)op->i[4], (int)op->i[5], op->i[6], op->i[7], op->i[8], entry_meta(s), s->max_rows, s->entries, ptr<const float>(op->i[9]),
                                    ptr<const float>(op->i[10]), s->n, (int)op->i[11], (int)op->i[12], (int)op->i[13], (int)op->i[14], (int)op->i[15],
                                    (int)op->i[16], (int)op->i[17], (float)op->f[0], (int)op->i[18], (int)op->i[19], (float)op->f[1],
                                    static_cast<cudaStream_t>(stream));

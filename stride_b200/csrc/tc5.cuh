@@ -158,6 +158,15 @@ __device__ __forceinline__ void umma_ts_bf16(uint32_t tmem_d, uint32_t tmem_a, u
       "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// Sixteen consecutive columns of this thread's TMEM lane, as raw bits and without waiting (tmem_load_wait()).
+__device__ __forceinline__ void tmem_load16_nowait(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
 // 32 consecutive columns of this thread's TMEM lane (the warp reads lanes 32 * (warp % 4) ..), as raw bits and without
 // waiting: several loads can be in flight; tmem_load_wait() before the first use of any of them.
 __device__ __forceinline__ void tmem_load32_nowait(uint32_t taddr, uint32_t* r) {

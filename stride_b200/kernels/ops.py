@@ -306,6 +306,7 @@ def gemm_tc_status() -> int:
 _status_word = None
 _status_users = {"gemm_tc": "sb_gemm_tc_use_status_word", "attention_tc5": "sb_attention_tc5_use_status_word",
                  "decode_chain": "sb_decode_chain_use_status_word", "grouped_gemm": "sb_grouped_gemm_use_status_word",
+                 "masked_attention": "sb_masked_attention_use_status_word",
                  "sampling": "sb_sampling_use_status_word"}   # the sampling kernels only read it
 _status_registered: set = set()
 
@@ -696,11 +697,13 @@ def masked_attention_tiles(q, out, cache_layer, block_table, entry_meta, entries
     _cuda(q, out, cache_layer, block_table, entry_meta, slopes, sinks)
     if not (q.dtype == out.dtype == cache_layer.dtype == torch.bfloat16):
         raise TypeError("masked_attention_tiles takes bfloat16 q, out and cache")
-    lib, fn = _fn("masked_attention", "sb_masked_attention_tiles",
-                  [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int64, c_int64, c_int64, c_void_p, c_int, c_int, c_void_p, c_void_p,
-                   c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p])
-    _check(lib, fn(_ptr(q), _ptr(out), *_page_args(cache_layer, block_table), _ptr(entry_meta), entry_meta.stride(0), entries, _ptr(slopes),
-                   _ptr(sinks), q.shape[0], num_heads, num_kv_heads, key_dim, value_dim, cache_layer.shape[4], window, keep_first, scale, _stream()))
+    lib, fn = _fn("masked_attention", "sb_masked_attention_tiles_in",
+                  [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int64, c_int64, c_int64, c_void_p, c_int, c_int, c_void_p, c_void_p,
+                   c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_float, c_void_p])
+    pages, *where = _page_args(cache_layer, block_table)
+    _check(lib, fn(_ptr(q), _ptr(out), pages, cache_layer.shape[0], *where, _ptr(entry_meta), entry_meta.stride(0), entries, _ptr(slopes),
+                   _ptr(sinks), q.shape[0], num_heads, num_kv_heads, key_dim, value_dim, cache_layer.shape[4], window, keep_first, scale, 0, 0, 0.0,
+                   _stream()))
 
 
 def head_linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, tail: int = 0) -> None:

@@ -53,7 +53,8 @@ def _emit_attend(program, q, out, cache, slopes, sinks, H, G, D, Dv, window, kee
     pages, table = cache.pages, cache.block_table
     if tiles:
         program.add("masked_attention", "sb_op_masked_attention_tiles",
-                    [q, out, pages, table, *_page_where(pages, table), slopes, sinks, H, G, D, Dv, pages.shape[4], window, keep_first], [scale, cap])
+                    [q, out, pages, table, *_page_where(pages, table), slopes, sinks, H, G, D, Dv, pages.shape[4], window, keep_first, 0, 0, pages.shape[0]],
+                    [scale, cap])
     else:
         program.add("masked_attention", "sb_op_masked_attention",
                     [q, out, q.dtype, pages, table, *_page_where(pages, table), slopes, sinks, H, G, D, Dv, pages.shape[4], window, keep_first],

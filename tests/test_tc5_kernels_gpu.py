@@ -1,0 +1,88 @@
+"""The tcgen05 kernels that stand beside mma.sync kernels of the same arithmetic: equal bits, and a plain computation in 64 bits."""
+from ctypes import c_float, c_int, c_int64, c_void_p
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEVICE = "cuda:0"
+INF, NAN = float("inf"), float("nan")
+
+
+def _call(name, argtypes, args):
+    from stride_b200.kernels import ops
+    lib, fn = ops._fn("masked_attention", name, argtypes)
+    ops._check(lib, fn(*args))
+
+
+def _latent_case(entries, H, G, page, odd=(), seed=0):
+    """q, cache layer, block table, entry meta and sinks; entries are (tokens, tokens in front), memory that no token filled is NaN, `odd` are
+    (entry, position, element, value) of latents."""
+    gen = torch.Generator(device=DEVICE).manual_seed(seed)
+    D, n = 512, sum(l for l, _ in entries)
+    need = [-(-(l + f) // page) for l, f in entries]
+    cache = torch.full((sum(need) + 2, 1, G, page, D), NAN, device=DEVICE, dtype=torch.bfloat16)
+    order = torch.randperm(sum(need) + 2, generator=torch.Generator().manual_seed(seed)).tolist()
+    table, meta, at, row = torch.zeros((len(entries), max(need)), dtype=torch.int32), [], 0, 0
+    for e, (l, f) in enumerate(entries):
+        table[e, :need[e]] = torch.tensor(order[at:at + need[e]], dtype=torch.int32)
+        meta.append([e, row, l, f])
+        at, row = at + need[e], row + l
+    table = table.to(DEVICE)
+    for e, (l, f) in enumerate(entries):
+        j = torch.arange(l + f, device=DEVICE)
+        for g in range(G):
+            cache[table[e, j // page].long(), 0, g, j % page] = torch.randn((l + f, D), device=DEVICE, generator=gen).bfloat16()
+    for e, j, c, v in odd:
+        cache[table[e, j // page].long(), 0, 0, j % page, c] = v
+    q = (torch.randn((n, H * D), device=DEVICE, generator=gen) * 0.5).bfloat16()
+    return q, cache, table, torch.tensor(meta, dtype=torch.int32).T.contiguous().to(DEVICE), torch.randn(H, device=DEVICE, generator=gen)
+
+
+def _latent(case, window, pages):
+    """pages: of the arena, or 0: the form that addresses pages by TMA is left out."""
+    q, cache, table, meta, sinks = case
+    H, G = sinks.numel(), cache.shape[2]
+    out = torch.zeros_like(q)
+    _call("sb_masked_attention_tiles_in",
+          [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int64, c_int64, c_int64, c_void_p, c_int, c_int, c_void_p, c_void_p] +
+          [c_int] * 8 + [c_float, c_int, c_int, c_float, c_void_p],
+          [q.data_ptr(), out.data_ptr(), cache.data_ptr(), pages, table.data_ptr(), table.shape[1], cache.shape[3], cache.stride(0), 0, cache.stride(2),
+           meta.data_ptr(), meta.stride(0), meta.shape[1], None, sinks.data_ptr(), q.shape[0], H, G, 512, 512, 512, window, 0, 0.03, 0, 0, 0.0,
+           torch.cuda.current_stream().cuda_stream])
+    torch.cuda.synchronize()
+    return out
+
+
+LATENT = [  # entries, H, G, window, page size, odd latents
+    ([(16, 0)], 16, 1, 0, 64, ()), ([(17, 47)], 16, 1, 0, 64, ()), ([(64, 0)], 16, 1, 0, 64, ()),
+    ([(200, 0), (33, 100), (65, 7)], 16, 1, 1024, 64, ()), ([(150, 100), (90, 7)], 16, 1, 70, 16, ()), ([(70, 300)], 16, 1, 3, 8, ()),
+    ([(100, 500), (41, 7)], 32, 2, 64, 128, ()), ([(100, 30)], 4, 1, 65, 32, ()), ([(20, 50)], 128, 1, 0, 64, ()), ([(300, 0)], 1, 1, 0, 64, ()),
+    # infinities and NaN at keys that some rows of a tile see and others do not: at the causal edge and at the window's
+    ([(100, 0), (64, 3)], 16, 1, 0, 64, ((0, 50, 3, INF), (0, 51, 300, NAN), (1, 66, 511, -INF))),
+    ([(100, 30), (64, 3)], 16, 1, 20, 64, ((0, 50, 3, INF), (0, 129, 300, NAN), (1, 3, 511, -INF), (1, 4, 0, INF))),
+]
+
+
+@pytest.mark.parametrize("entries, H, G, window, page, odd", LATENT)
+def test_latent_attention_on_tcgen05_has_the_bits_of_the_tile_kernel(entries, H, G, window, page, odd):
+    from stride_b200.kernels import ops
+    word = ops.shared_status_word({"masked_attention"})
+    case = _latent_case(entries, H, G, page, odd)
+    many = _latent(case, window, case[1].shape[0])
+    assert torch.equal(many.view(torch.int16), _latent(case, window, 0).view(torch.int16))
+    assert word.item() == 0
+    if odd:
+        return
+    # a plain computation in 64 bits. bfloat16 results: half a unit in the last place, 2^-9 of the largest element; scores and sums in 32 bits
+    q, cache, table, meta, sinks = case
+    for e, row, l, f in meta.T.tolist():
+        j = torch.arange(l + f, device=DEVICE)
+        keys = torch.stack([cache[table[e, j // page].long(), 0, g, j % page] for g in range(G)]).double()
+        s = torch.einsum("tgrd,gsd->grts", q[row:row + l].view(l, G, H // G, 512).double(), keys) * 0.03
+        pos = torch.arange(f, f + l, device=DEVICE)[:, None]
+        seen = (j[None, :] <= pos) & ((pos - j[None, :] < window) if window else True)
+        s = torch.cat([s.masked_fill(~seen, -INF), sinks.double().view(G, H // G, 1, 1).expand(-1, -1, l, 1)], dim=-1)
+        want = torch.einsum("grts,gsd->tgrd", torch.softmax(s, -1)[..., :-1], keys).reshape(l, -1)
+        got = many[row:row + l].double()
+        assert ((got - want).abs().max() / want.abs().max()).item() < 2.0 ** -9 + 1e-4
