@@ -74,7 +74,8 @@ def test_latent_attention_on_tcgen05_has_the_bits_of_the_tile_kernel(entries, H,
     assert word.item() == 0
     if odd:
         return
-    # a plain computation in 64 bits. bfloat16 results: half a unit in the last place, 2^-9 of the largest element; scores and sums in 32 bits
+    # a plain computation in 64 bits. bfloat16 results have eight significant bits: half a unit in the last place is up to 2^-8 of the largest
+    # element (2^-8 2^e beside a value of at least 2^e); scores and sums are of 32 bits
     q, cache, table, meta, sinks = case
     for e, row, l, f in meta.T.tolist():
         j = torch.arange(l + f, device=DEVICE)
@@ -85,4 +86,4 @@ def test_latent_attention_on_tcgen05_has_the_bits_of_the_tile_kernel(entries, H,
         s = torch.cat([s.masked_fill(~seen, -INF), sinks.double().view(G, H // G, 1, 1).expand(-1, -1, l, 1)], dim=-1)
         want = torch.einsum("grts,gsd->tgrd", torch.softmax(s, -1)[..., :-1], keys).reshape(l, -1)
         got = many[row:row + l].double()
-        assert ((got - want).abs().max() / want.abs().max()).item() < 2.0 ** -9 + 1e-4
+        assert ((got - want).abs().max() / want.abs().max()).item() < 2.0 ** -8 + 1e-4
