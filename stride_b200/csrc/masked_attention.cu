@@ -16,7 +16,10 @@
 // latent normed and appended, or left out by layers that read another layer's), `rotate_heads_kernel` (rotation of a slice of every query
 // head) and `head_linear_kernel` (a matrix per head: the key projection taken into the queries in front of the attention, the value
 // projection behind it, there with a sigmoid gate per element on the way out where a design has one).
+#include <algorithm>
+
 #include "common.cuh"
+#include "head_linear_tc5.cuh"
 #include "latent_attention_tc5.cuh"
 #include "step_ops.h"
 
@@ -963,6 +966,47 @@ int launch_latent(const TileParams& p, int pages, int n, cudaStream_t stream, bo
   return sb::check_launch("sb_masked_attention_tiles");
 }
 
+// The matrix per head for many tokens: sizes that its pieces divide, and the gate in one piece that takes 16-byte accesses (a thread reads its
+// row's gates line by line, which the partial sums of nine K ranges make slower than what the tensor cores save). Microseconds, mma.sync / here,
+// 16 heads: 128 -> 512 for 64 tokens 3.8 / 3.9, 128 tokens 5.6 / 4.5, 512 9.1 / 6.1, 2,048 29.6 / 11.7; 512 -> 128 with a gate in one piece for
+// 1,024 tokens 20.7 / 17.4, 2,048 30.4 / 19.2; in nine for 256 18 / 38.
+bool takes_heads5(const HeadLinearParams& p) {
+  if (p.K % 64 != 0 || p.N % 64 != 0 || p.tail != 0 || p.H > 65535) return false;
+  if (p.gate == nullptr) return p.n >= 128;
+  return p.n >= 512 && p.gate_partials == 1 && p.gate_width % 4 == 0 && (reinterpret_cast<uintptr_t>(p.gate) & 15) == 0;
+}
+
+int launch_heads5(const HeadLinearParams& p, cudaStream_t stream) {
+  using namespace sb::heads5;
+  Params q{};
+  q.n = p.n, q.K = p.K, q.N = p.N;
+  for (q.cols = 256; p.N % q.cols != 0;) q.cols -= 64;
+  const int stage_bytes = kABytes + q.cols * 128;
+  q.stages = std::max(2, std::min({kMaxStages, kSmemBudget / stage_bytes, p.K / 64}));
+  q.gate = p.gate, q.gate_width = p.gate_width;
+  q.status = sb::tc5::status_word();
+  if (!q.status) return sb::fail("sb_head_linear: cannot allocate the status word");
+  CUtensorMap map_in, map_w, map_out;
+  const int64_t idims[3] = {p.K, p.H, p.n}, istrides[3] = {1, p.in_head, p.in_row}, odims[3] = {p.N, p.H, p.n}, ostrides[3] = {1, p.out_head, p.out_row};
+  const int64_t wdims[2] = {p.N, static_cast<int64_t>(p.H) * p.K}, wstrides[2] = {1, p.N};
+  const int ibox[3] = {64, 1, kRows}, wbox[2] = {64, 64};
+  if (!sb::tc5::tensor_map_bf16(p.in, 3, idims, istrides, ibox, &map_in) || !sb::tc5::tensor_map_bf16(p.w, 2, wdims, wstrides, wbox, &map_w) ||
+      !sb::tc5::tensor_map_bf16(p.out, 3, odims, ostrides, ibox, &map_out))
+    return sb::fail("sb_head_linear: cuTensorMapEncodeTiled failed");
+  const dim3 grid((p.n + kRows - 1) / kRows, p.H, p.N / q.cols);
+  const size_t smem = static_cast<size_t>(q.stages) * stage_bytes + 1024;
+  static sb::DeviceOnce once;
+  if (once.needed()) {
+    if (cudaFuncSetAttribute(head_linear_tc5_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget + 1024) != cudaSuccess ||
+        cudaFuncSetAttribute(head_linear_tc5_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget + 1024) != cudaSuccess)
+      return sb::fail("sb_head_linear: cannot raise the shared memory limit");
+    once.done();
+  }
+  if (p.gate != nullptr) sb::launch_pdl(head_linear_tc5_kernel<true>, grid, dim3(kThreads), smem, stream, map_in, map_w, map_out, q);
+  else sb::launch_pdl(head_linear_tc5_kernel<false>, grid, dim3(kThreads), smem, stream, map_in, map_w, map_out, q);
+  return sb::check_launch("sb_head_linear");
+}
+
 PageRef page_ref(void* pages, const int32_t* block_table, int max_pages, int page_size, int64_t page_stride, int64_t v_offset, int64_t head_stride,
                  int Dc) {
   return PageRef{pages, block_table, max_pages, page_size, page_stride, v_offset, head_stride, Dc};
@@ -1045,7 +1089,9 @@ SB_EXPORT int sb_head_linear_gated(const void* in, int64_t in_row, int64_t in_he
   HeadLinearParams p{in, in_row, in_head, w, out, out_row, out_head, n, H, K, N, tail, gate, gate_partials, gate_width, gate_stride};
   const bool aligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   if (dtype == 1 && aligned && K % 16 == 0 && N % 8 == 0 && in_row % 8 == 0 && in_head % 8 == 0 && out_row % 8 == 0 && out_head % 8 == 0) {
-    // (what decides for the tensor cores is the shape alone, never the number of rows: a token has one form whatever step it is in)
+    // (what decides for the tensor cores is the shape alone, never the number of rows: a token has one form whatever step it is in; the two
+    // kernels have the same bits)
+    if (takes_heads5(p)) return launch_heads5(p, stream);
     sb::launch_pdl(head_linear_tc_kernel, dim3((n + kHlTile - 1) / kHlTile, H, (N + kHlTile - 1) / kHlTile), dim3(128), 0, stream, p);
     return sb::check_launch("sb_head_linear");
   }

@@ -87,3 +87,32 @@ def test_latent_attention_on_tcgen05_has_the_bits_of_the_tile_kernel(entries, H,
         want = torch.einsum("grts,gsd->tgrd", torch.softmax(s, -1)[..., :-1], keys).reshape(l, -1)
         got = many[row:row + l].double()
         assert ((got - want).abs().max() / want.abs().max()).item() < 2.0 ** -8 + 1e-4
+
+
+@pytest.mark.parametrize("n, H, K, N, partials, pad", [(130, 2, 128, 512, 0, 0), (256, 1, 64, 64, 0, 0), (383, 3, 64, 192, 1, 0), (513, 2, 512, 128, 3, 0),
+                                                       (300, 5, 192, 320, 2, 0), (257, 16, 512, 128, 9, 0), (700, 4, 128, 64, 0, 8)])
+def test_matrix_per_head_has_one_result_for_any_number_of_rows(n, H, K, N, partials, pad):
+    """Many rows take the tcgen05 kernel, a few the mma.sync kernel: the same bits, and nothing written beyond the rows or the columns."""
+    gen = torch.Generator(device=DEVICE).manual_seed(n)
+    x = torch.randn((n, H, K + pad), device=DEVICE, generator=gen).bfloat16()
+    w = (torch.randn((H, K, N), device=DEVICE, generator=gen) * 0.05).bfloat16()
+    width = H * N + 64
+    gate = torch.randn((partials, n, width), device=DEVICE, generator=gen) if partials else None
+
+    def run(first, rows):
+        out = torch.full((rows + 1, H, N + pad), 7.0, device=DEVICE, dtype=torch.bfloat16)
+        at = gate.data_ptr() + 4 * first * width if partials else None
+        _call("sb_head_linear_gated",
+              [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int64, c_int64] + [c_int] * 6 + [c_void_p, c_int, c_int64, c_int, c_void_p],
+              [x[first:].data_ptr(), x.stride(0), x.stride(1), w.data_ptr(), out.data_ptr(), out.stride(0), out.stride(1), 1, rows, H, K, N, 0, at, partials,
+               n * width, width, torch.cuda.current_stream().cuda_stream])
+        torch.cuda.synchronize()
+        assert (out[rows] == 7).all() and (out[:, :, N:] == 7).all()
+        return out[:rows, :, :N]
+    whole = run(0, n)
+    assert torch.equal(whole, torch.cat([run(a, min(60, n - a)) for a in range(0, n, 60)]))
+    want = torch.einsum("nhk,hkm->nhm", x[..., :K].double(), w.double())
+    if partials:
+        want = want * torch.sigmoid(gate[..., :H * N].double().sum(0)).view(n, H, N)
+    # half a unit in the last place of a bfloat16 (up to 2^-8 of the largest element) and sums of 32 bits whose terms the tensor cores truncate
+    assert ((whole.double() - want).abs().max() / want.abs().max()).item() < 2.0 ** -8 + 1e-4
