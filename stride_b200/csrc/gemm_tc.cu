@@ -68,6 +68,7 @@ struct GemmParams {
   int stages;
   int kblocks_per_split;
   int tiles_m, tiles_n, splits;
+  int vec_out;           // kSwiglu of pairs: the output takes 16-byte stores
   int half_rows;         // kSwiglu: rows of the gate half (intermediate size); W is [2 * half_rows, K]
   Gate gate;             // kSwiglu: the gate's activation and its constants (sb::gemm_tile::Gate)
   int* status;
@@ -547,7 +548,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   __shared__ __align__(8) uint64_t accum_full[2];           // in each CTA: an accumulator is complete
   __shared__ __align__(8) uint64_t accum_empty[2];          // used in the leader: both CTAs have drained an accumulator
   __shared__ uint32_t tmem_base_s;
-  __shared__ float xch2[EPI == kSwiglu ? 2 : 1][EPI == kSwiglu ? 16 * 64 : 1];   // gate/up exchange of the SwiGLU epilogue, per warp set
+  __shared__ float xch2[2][EPI == kSwiglu ? 2 * 16 * 64 : 1];               // swiglu_set's buffers, per warp set
+  __shared__ __align__(16) bf16 done2[2][EPI == kSwiglu ? 2 * 16 * 64 : 8];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = static_cast<int>(sb::cluster_rank());
@@ -646,40 +648,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16);
         const int n0 = tile_n * BN;
-        // lanes 0..63 hold gate rows, lanes 64..127 the matching up rows; the two sets of four warps take
-        // alternate groups of sixteen tokens, each set with its own exchange buffer and barrier
-        const int j = tile_m * 128 + rank * 64 + (quarter & 1) * 32 + lane;  // output feature
         const int set = (warp - 2) >> 2;
-        float* xch = xch2[set];
-        bf16* out = reinterpret_cast<bf16*>(p.out);
-        for (int c0 = 16 * set; c0 < BN; c0 += 32) {
-          float v[16];
-          tmem_load16(tmem_d + c0, v);
-          // gate warps hand over columns 8..15, up warps columns 0..7: every warp then finishes eight columns
-          if (quarter >= 2) {
-#pragma unroll
-            for (int c = 0; c < 8; ++c) xch[c * 64 + (quarter - 2) * 32 + lane] = v[c];
-          } else {
-#pragma unroll
-            for (int c = 0; c < 8; ++c) xch[(8 + c) * 64 + quarter * 32 + lane] = v[8 + c];
-          }
-          if (set == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
-          else asm volatile("bar.sync 2, 128;" ::: "memory");
-          if (ok && j < p.half_rows) {
-            const int cb = quarter >= 2 ? 8 : 0;
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-              const int n = n0 + c0 + cb + c;
-              if (n < p.N) {
-                const float other = xch[(cb + c) * 64 + (quarter & 1) * 32 + lane];
-                const float g = quarter >= 2 ? other : v[c], u = quarter >= 2 ? v[8 + c] : other;
-                out[static_cast<int64_t>(n) * p.ldo + j] = __float2bfloat16_rn(gated_product(g, u, p.gate));
-              }
-            }
-          }
-          if (set == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
-          else asm volatile("bar.sync 2, 128;" ::: "memory");
-        }
+        swiglu_set(tmem_d, xch2[set], done2[set], reinterpret_cast<bf16*>(p.out), p.ldo, tile_m * 128 + rank * 64, p.half_rows, n0, p.N, BN, set, quarter, lane,
+                   ok, p.vec_out != 0, p.gate);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_leader(smem_u32(&accum_empty[acc]));
@@ -1035,6 +1006,7 @@ SB_EXPORT int sb_gemm_tc_gated(const void* x, int64_t ldx, const void* w, int64_
       return sb::fail("sb_gemm_tc: %d splits leave an empty K range (use sb_gemm_tc_splits)", splits);
     p.half_rows = half_rows;
     p.status = status;
+    p.vec_out = half_rows % 8 == 0 && ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
     p.tiles_m = static_cast<int>(tm);
     p.tiles_n = (n + p.block_n - 1) / p.block_n;
     p.splits = splits;
