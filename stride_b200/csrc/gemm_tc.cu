@@ -69,16 +69,47 @@ struct GemmParams {
   int kblocks_per_split;
   int tiles_m, tiles_n, splits;
   int vec_out;           // kSwiglu of pairs: the output takes 16-byte stores
+  int tma_out;           // kStore: a finished tile goes to memory through shared memory by TMA (map_out)
   int half_rows;         // kSwiglu: rows of the gate half (intermediate size); W is [2 * half_rows, K]
   Gate gate;             // kSwiglu: the gate's activation and its constants (sb::gemm_tile::Gate)
   int* status;
 };
 
+// Sixteen tokens of a warp's 32 features from shared memory [16][32] to `out` by TMA; the warp's lanes have written them.
+__device__ __forceinline__ void store_strip(const CUtensorMap& map_out, uint32_t strip, int m, int n, int range, int lane) {
+  fence_async_smem();
+  __syncwarp();
+  if (lane == 0) tma_store_3d(&map_out, strip, m, n, range);
+}
+// Rows of one accumulator tile to global memory: a warp's 32 features (lane = feature) in strips of sixteen tokens, staged in shared memory
+// (BN * 128 bytes of the warp's own, over the used-up ring) and stored by TMA. A store a token and warp, 128 bytes each, took 6 of the 24.8 us of
+// [2048, 2048] at 2,048 tokens (128 KB a CTA). Products with K ranges, microseconds, stored a token at a time / so: 256 tokens 7.5 / 6.5,
+// 8.3 / 7.3 and 12.0 / 11.0 ([2048, 2048], [3072, 2048], [2048, 8192]).
+__device__ __forceinline__ void store_tile_tma(uint32_t tmem_row, uint32_t staged, uint8_t* staged_p, const CUtensorMap& map_out, int m0, int M, int n0, int N,
+                                               int BN, int range, int lane) {
+  if (m0 >= M) return;
+  const int cols = min(BN, (N - n0 + 15) & ~15);
+  uint32_t v[2][16];
+  float* to = reinterpret_cast<float*>(staged_p) + lane;
+  tmem_load16_nowait(tmem_row, v[0]);
+#pragma unroll 2
+  for (int c0 = 0, i = 0; c0 < cols; c0 += 16, i ^= 1, to += 16 * 32) {
+    tmem_load_wait();
+    uint32_t* at = v[i];
+    if (c0 + 16 < cols) tmem_load16_nowait(tmem_row + c0 + 16, v[i ^ 1]);
+#pragma unroll
+    for (int c = 0; c < 16; ++c) to[c * 32] = __uint_as_float(at[c]);
+    store_strip(map_out, staged + c0 * 128, m0, n0 + c0, range, lane);
+  }
+  if (lane == 0) tma_store_wait();
+}
+
 // One tile per CTA: the lean form used when every tile has a CTA of its own (every decode-sized launch).
 // blockIdx = (weight tile, token tile, K range).
 template <int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_tc_single_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GemmParams p) {
+gemm_tc_single_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_out,
+                      const GemmParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kMaxStages];
   __shared__ __align__(8) uint64_t empty_bar[kMaxStages];
@@ -192,6 +223,10 @@ gemm_tc_single_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     if (EPI == kSwiglu) {
       float* xch = reinterpret_cast<float*>(smem_raw + ((smem0 - smem_u32(smem_raw))));  // stage 0 is free by now
       swiglu_tile(tmem_base, xch, reinterpret_cast<bf16*>(p.out), p.ldo, tile_m, p.half_rows, n0, p.N, BN, quarter, lane, ok, p.gate);
+    } else if (EPI == kStore && p.tma_out) {
+      if (ok)
+        store_tile_tma(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16), smem0 + quarter * BN * 128,
+                       smem_raw + (smem0 - smem_u32(smem_raw)) + quarter * BN * 128, map_out, tile_m * kTileM + quarter * 32, p.M, n0, p.N, BN, split, lane);
     } else {
       store_tile<EPI>(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16), p.out + static_cast<int64_t>(split) * p.split_stride,
                       tile_m * kTileM + quarter * 32 + lane, p.M, n0, p.N, p.ldo, BN, ok);
@@ -540,7 +575,8 @@ gemm_tc_fold_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 // the bits of the single-CTA kernels: the same accumulation chain per element and the same order of the ranges.
 template <int EPI>
 __global__ void __launch_bounds__(kFoldThreads, 1)
-gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GemmParams p) {
+gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_out,
+                    const GemmParams p) {
   constexpr int kEpiWarps = 8;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kMaxStages];    // used in the leader: both CTAs' tiles have landed
@@ -687,7 +723,21 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
           __syncwarp();
           if (lane == 0) mbar_arrive_leader(smem_u32(&accum_empty[acc]));
         }
-        if (live) {
+        if (p.tma_out && tile + pairs >= total_tiles) {      // (behind the last tile the ring is free; behind the others the next tile hides the stores)
+          const int m0 = tile_m * 256 + rank * kTileM + quarter * 32, at = (half * 4 + quarter) * cols * 128;
+          float* to = reinterpret_cast<float*>(smem_raw + (smem0 - smem_u32(smem_raw)) + at) + lane;
+          if (m0 < p.M) {
+#pragma unroll
+            for (int c0 = 0; c0 < kFoldCols; c0 += 16) {
+              if (c0 < cols && n0 + c0 < p.N) {
+#pragma unroll
+                for (int c = 0; c < 16; ++c) to[(c0 + c) * 32] = run[c0 + c];
+                store_strip(map_out, smem0 + at + c0 * 128, m0, n0 + c0, 0, lane);
+              }
+            }
+            if (lane == 0) tma_store_wait();
+          }
+        } else if (live) {
 #pragma unroll
           for (int c = 0; c < kFoldCols; ++c)
             if (c < cols && n0 + c < p.N) o[static_cast<int64_t>(c) * p.ldo] = run[c];
@@ -943,6 +993,14 @@ SB_EXPORT int sb_gemm_tc_gated(const void* x, int64_t ldx, const void* w, int64_
   p.gate = gate;
   p.status = status;
 
+  // The map by which finished tiles go to memory: [range][token][feature], boxes of 32 features of sixteen tokens.
+  auto map_rows_out = [&](int ranges, CUtensorMap* to) {
+    if (M % 4 != 0 || ldo % 4 != 0 || split_stride % 4 != 0 || (reinterpret_cast<uintptr_t>(out) & 15) != 0) return false;
+    const int64_t dims[3] = {M, n, ranges}, strides[3] = {1, ldo, ranges > 1 ? split_stride : ldo * n};
+    const int box[3] = {32, 16, 1};
+    return tensor_map_of(true, out, 3, dims, strides, box, to);
+  };
+
   // The SwiGLU product of many tokens runs on pairs of CTAs or with two weight tiles a CTA; both bring the same bytes
   // from L2 (what bounds these products), the pairs in units half as large. Whichever needs fewer rounds of units of
   // 128 features x 256 tokens a CTA takes it (two weight tiles on a tie: no traffic between the SMs of a pair).
@@ -1013,6 +1071,8 @@ SB_EXPORT int sb_gemm_tc_gated(const void* x, int64_t ldx, const void* w, int64_
     CUtensorMap pw, px;
     if (!tensor_map(w, M, K, ldw, epilogue == kSwiglu ? 64 : kTileM, &pw) || !tensor_map(x, n, K, ldx, p.block_n / 2, &px))
       return sb::fail("sb_gemm_tc: cuTensorMapEncodeTiled failed (M %d N %d K %d)", M, n, K);
+    CUtensorMap po = px;
+    p.tma_out = epilogue == kStore && p.stages * pair_stage >= 512 * p.block_n && map_rows_out(1, &po);
     const long long tiles = static_cast<long long>(p.tiles_m) * p.tiles_n;
     if (tiles > (1ll << 30)) return sb::fail("sb_gemm_tc: too many tiles");
     const dim3 grid(static_cast<unsigned>(2 * min(tiles, pairs)));
@@ -1025,9 +1085,9 @@ SB_EXPORT int sb_gemm_tc_gated(const void* x, int64_t ldx, const void* w, int64_
       once.done();
     }
     if (epilogue == kStore)
-      sb::launch_pdl_cluster(gemm_tc_pair_kernel<kStore>, grid, dim3(kFoldThreads), psmem, stream, dim3(2, 1, 1), pw, px, p);
+      sb::launch_pdl_cluster(gemm_tc_pair_kernel<kStore>, grid, dim3(kFoldThreads), psmem, stream, dim3(2, 1, 1), pw, px, po, p);
     else
-      sb::launch_pdl_cluster(gemm_tc_pair_kernel<kSwiglu>, grid, dim3(kFoldThreads), psmem, stream, dim3(2, 1, 1), pw, px, p);
+      sb::launch_pdl_cluster(gemm_tc_pair_kernel<kSwiglu>, grid, dim3(kFoldThreads), psmem, stream, dim3(2, 1, 1), pw, px, po, p);
     return sb::check_launch("sb_gemm_tc");
   }
 
@@ -1060,6 +1120,9 @@ SB_EXPORT int sb_gemm_tc_gated(const void* x, int64_t ldx, const void* w, int64_
   const bool multi = total_tiles > resident;
   if (!multi && (p.tiles_n > 65535 || splits > 65535)) return sb::fail("sb_gemm_tc: grid too large");
   const dim3 grid(static_cast<unsigned>(multi ? resident : total_tiles));
+  CUtensorMap map_out = map_x;
+  // (Few tokens leave a tile so few strips that the detour through shared memory costs what it saves.)
+  p.tma_out = !multi && epilogue == kStore && n > 128 && p.block_n >= 32 && p.stages * stage_bytes >= 512 * p.block_n && map_rows_out(splits, &map_out);
 #define SB_LAUNCH_M(EPI, MULTI)                                                                         \
   do {                                                                                                  \
     static sb::DeviceOnce once;                                                                       \
@@ -1080,7 +1143,7 @@ SB_EXPORT int sb_gemm_tc_gated(const void* x, int64_t ldx, const void* w, int64_
         return sb::fail("sb_gemm_tc: cannot raise the shared memory limit");                            \
       once.done();                                                                                  \
     }                                                                                                   \
-    sb::launch_pdl(gemm_tc_single_kernel<EPI>, dim3(p.tiles_m, p.tiles_n, splits), dim3(kThreads), smem, stream, map_w, map_x, p); \
+    sb::launch_pdl(gemm_tc_single_kernel<EPI>, dim3(p.tiles_m, p.tiles_n, splits), dim3(kThreads), smem, stream, map_w, map_x, map_out, p); \
   } while (0)
 #define SB_LAUNCH(EPI)                  \
   do {                                  \

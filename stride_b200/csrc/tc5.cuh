@@ -242,12 +242,12 @@ inline EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// Tensor map of a bfloat16 tensor of `rank` dimensions (dims[0] contiguous; strides in elements for dims 1..),
-// with the given box and the 128-byte swizzle (box[0] * 2 bytes must be 128). Cached by all its arguments.
-inline bool tensor_map_bf16(const void* base, int rank, const int64_t* dims, const int64_t* strides, const int* box, CUtensorMap* out) {
+// Tensor map of a tensor of `rank` dimensions (dims[0] contiguous; strides in elements for dims 1..) with the given box: bfloat16 in the
+// 128-byte swizzle (box[0] * 2 bytes must be 128), or float32 as it lies in memory. Cached by all its arguments.
+inline bool tensor_map_of(bool f32, const void* base, int rank, const int64_t* dims, const int64_t* strides, const int* box, CUtensorMap* out) {
   static std::map<std::vector<int64_t>, CUtensorMap> cache;
   static std::mutex mu;
-  std::vector<int64_t> key{reinterpret_cast<int64_t>(base), rank};
+  std::vector<int64_t> key{reinterpret_cast<int64_t>(base), rank, f32};
   for (int i = 0; i < rank; ++i) {
     key.push_back(dims[i]);
     key.push_back(i ? strides[i] : 1);
@@ -267,17 +267,20 @@ inline bool tensor_map_bf16(const void* base, int rank, const int64_t* dims, con
     gdims[i] = static_cast<cuuint64_t>(dims[i]);
     gbox[i] = static_cast<cuuint32_t>(box[i]);
     gelem[i] = 1;
-    if (i) gstrides[i - 1] = static_cast<cuuint64_t>(strides[i]) * 2;
+    if (i) gstrides[i - 1] = static_cast<cuuint64_t>(strides[i]) * (f32 ? 4 : 2);
   }
   CUtensorMap m;
-  if (fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), gdims, gstrides, gbox, gelem,
-         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+  if (fn(&m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), gdims, gstrides, gbox, gelem,
+         CU_TENSOR_MAP_INTERLEAVE_NONE, f32 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return false;
   if (cache.size() > 4096) cache.clear();
   cache[key] = m;
   *out = m;
   return true;
+}
+inline bool tensor_map_bf16(const void* base, int rank, const int64_t* dims, const int64_t* strides, const int* box, CUtensorMap* out) {
+  return tensor_map_of(false, base, rank, dims, strides, box, out);
 }
 
 // One int of device memory for the bounded waits' error codes: the library's own, or the one its user handed it
