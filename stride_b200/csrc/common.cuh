@@ -106,6 +106,19 @@ inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
   cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);   // errors surface through check_launch()
 }
 
+// The same without the early start: the grid begins when the kernel in front has ended, on SMs that are all free. For few long CTAs: let in
+// early they take a place wherever one is free beside the kernel in front, and stay where they are, however uneven that is.
+template <class... KArgs, class... Args>
+inline void launch_behind(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  prefer_max_shared(reinterpret_cast<const void*>(kernel));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);   // errors surface through check_launch()
+}
+
 // The same with the grid cut into thread-block clusters of `cluster` CTAs.
 template <class... KArgs, class... Args>
 inline void launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, dim3 cluster,

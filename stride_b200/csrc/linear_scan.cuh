@@ -137,9 +137,9 @@ __device__ __forceinline__ void bar_arrive(int id, int count) { asm volatile("ba
 // another, since a request waits until its buffer is free. What bounds the kernel is each warp's wait for its own reads and exchanges, with one
 // or two computing warps a scheduler (PER = 2: issue slots 47% busy; PER = 4: without the loads and the exchanges 155 of 220 us are left).
 // Measured (16 heads of 128 x 128 without gates, one entry of 2,048 tokens / eight, launches one behind another): eight warps of one column a
-// thread, the outputs' parts through shared memory, 611 / 1,600 us; PER = 4 220 / 710 us, PER = 2 187 / 828 us. A launch on its own takes 143 us
-// with PER = 2, whether its rows lie in L2 or not: one behind another its CTAs take their places while the one in front still runs, wherever
-// an SM has room, which probably leaves some SMs with more of them.
+// thread, the outputs' parts through shared memory, 611 / 1,600 us; PER = 4 220 / 710 us, PER = 2 187 / 828 us, and 143 us on its own, which it
+// takes in a row too (151) now that it starts behind the kernel in front (launch_scan_of): let in early, its CTAs took their places while that
+// one still ran, wherever an SM had room, and some SMs got more of them.
 // With eight elements a lane: the row's pieces of four lie the even ones first, then the odd ones, so that the lanes' 16-byte reads take
 // neighbouring places (side by side they would meet in half the banks), and with gates two staging buffers, which leaves two CTAs an SM.
 template <int DL, bool GATED>
@@ -319,12 +319,17 @@ int launch_scan_of(const Params& p, int entries, const char* who, cudaStream_t s
       cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     once.done();
   }
-  sb::launch_pdl(kernel, dim3(entries, p.H, (p.V + kCols - 1) / kCols), dim3(kWarps * 32 + 32), smem, stream, p);
+  const dim3 grid(entries, p.H, (p.V + kCols - 1) / kCols), block(kWarps * 32 + 32);
+  // Two columns a warp: one or two long CTAs an SM, which have to be dealt out evenly (one entry of 2,048 tokens, 16 heads of 128 x 128: 204 us let
+  // in early, 153 behind the kernel in front, with gates 236 and 164; 512 tokens 40 and 41, 61 and 43; 64 tokens 10.1 and 9.4, 10.4 and 8.2). More
+  // entries fill the SMs either way, and start early (16 entries of 64 tokens 59 us, 61 behind).
+  if constexpr (PER == 2) sb::launch_behind(kernel, grid, block, smem, stream, p);
+  else sb::launch_pdl(kernel, grid, block, smem, stream, p);
   return sb::check_launch(who);
 }
 
 // Launches scan_kernel for the key size (at most 256). Four columns a warp make fewer reads a column; two make twice the CTAs, which is the
-// faster way while they all run at once (187 against 220 us for 128 CTAs of four; 828 against 710 us for 1,024).
+// faster way while they all run at once (153 against 220 us for 128 CTAs of four; 828 against 710 us for 1,024).
 template <bool GATED>
 int launch_scan(const Params& p, int entries, const char* who, cudaStream_t stream) {
   const bool few = static_cast<int64_t>(entries) * p.H * ((p.V + 15) / 16) <= sb::sm_count();
