@@ -116,3 +116,40 @@ def test_matrix_per_head_has_one_result_for_any_number_of_rows(n, H, K, N, parti
         want = want * torch.sigmoid(gate[..., :H * N].double().sum(0)).view(n, H, N)
     # half a unit in the last place of a bfloat16 (up to 2^-8 of the largest element) and sums of 32 bits whose terms the tensor cores truncate
     assert ((whole.double() - want).abs().max() / want.abs().max()).item() < 2.0 ** -8 + 1e-4
+
+
+@pytest.mark.parametrize("n", [129, 145, 256, 300, 513, 700])
+@pytest.mark.parametrize("M, K, gated", [(1040, 520, False), (1042, 520, False), (300, 2048, False), (1040, 264, True), (1032, 264, True), (1034, 264, True)])
+def test_products_of_many_tokens_store_what_products_of_a_few_store(n, M, K, gated):
+    """More than 128 tokens: tiles that go to memory by TMA (rows of a multiple of four elements) or element by element, and the SwiGLU epilogue
+    of pairs with 16-byte stores (a multiple of eight features) or without; portions of at most 100 tokens take neither. The same bits."""
+    from stride_b200.kernels import ops
+    gen = torch.Generator(device=DEVICE).manual_seed(n)
+    x = torch.randn((n, K), device=DEVICE, generator=gen).bfloat16()
+    w = (torch.randn((M, K), device=DEVICE, generator=gen) * 0.05).bfloat16()
+    S = 1 if gated else ops.gemm_tc_splits(M, K)
+
+    def run(part):
+        rows = part.shape[0]
+        if gated:
+            out = torch.full((rows + 1, M // 2), 7.0, device=DEVICE, dtype=torch.bfloat16)
+            ops.gemm_tc(part, w, out[:rows], ops.SWIGLU, half_rows=M // 2)
+            assert (out[rows] == 7).all()
+            return out[:rows]
+        ranges = S if rows <= ops.gemm_tc_partial_tokens() else 1
+        out = torch.full((ranges * rows + 1, M), 7.0, device=DEVICE)
+        ops.gemm_tc(part, w, out[:-1].view(ranges, rows, M) if ranges > 1 else out[:-1], ops.STORE, splits=S)
+        assert (out[-1] == 7).all()
+        total = out[:rows].clone()
+        for s in range(1, ranges):
+            total += out[s * rows:(s + 1) * rows]
+        return total
+    whole = run(x)
+    assert torch.equal(whole, torch.cat([run(x[a:a + 100]) for a in range(0, n, 100)]))
+    y = x.double() @ w.double().T
+    if gated:
+        y = torch.nn.functional.silu(y[:, :M // 2]) * y[:, M // 2:]
+    # bfloat16 results: half a unit in the last place, 2^-8 of the largest; sums of 32 bits whose terms the tensor cores truncate (2e-6 on average
+    # over 2,048 of them)
+    assert ((whole.double() - y).abs().max() / y.abs().max()).item() < (2.0 ** -8 + 1e-4 if gated else 1e-4)
+    assert ops.gemm_tc_status() == 0
