@@ -69,7 +69,7 @@ struct GemmParams {
   int kblocks_per_split;
   int tiles_m, tiles_n, splits;
   int vec_out;           // kSwiglu of pairs: the output takes 16-byte stores
-  int tma_out;           // kStore: a finished tile goes to memory through shared memory by TMA (map_out)
+  int tma_out;           // kStore of pairs: a CTA's last tile goes to memory through shared memory by TMA (map_out)
   int half_rows;         // kSwiglu: rows of the gate half (intermediate size); W is [2 * half_rows, K]
   Gate gate;             // kSwiglu: the gate's activation and its constants (sb::gemm_tile::Gate)
   int* status;
@@ -106,10 +106,9 @@ __device__ __forceinline__ void store_tile_tma(uint32_t tmem_row, uint32_t stage
 
 // One tile per CTA: the lean form used when every tile has a CTA of its own (every decode-sized launch).
 // blockIdx = (weight tile, token tile, K range).
-template <int EPI>
-__global__ void __launch_bounds__(kThreads, 1)
-gemm_tc_single_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_out,
-                      const GemmParams p) {
+// TMA: a finished kStore tile goes to memory through shared memory by map_out.
+template <int EPI, bool TMA>
+__device__ __forceinline__ void single_tile(const CUtensorMap& map_w, const CUtensorMap& map_x, const CUtensorMap& map_out, const GemmParams& p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kMaxStages];
   __shared__ __align__(8) uint64_t empty_bar[kMaxStages];
@@ -223,7 +222,7 @@ gemm_tc_single_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     if (EPI == kSwiglu) {
       float* xch = reinterpret_cast<float*>(smem_raw + ((smem0 - smem_u32(smem_raw))));  // stage 0 is free by now
       swiglu_tile(tmem_base, xch, reinterpret_cast<bf16*>(p.out), p.ldo, tile_m, p.half_rows, n0, p.N, BN, quarter, lane, ok, p.gate);
-    } else if (EPI == kStore && p.tma_out) {
+    } else if (TMA) {
       if (ok)
         store_tile_tma(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16), smem0 + quarter * BN * 128,
                        smem_raw + (smem0 - smem_u32(smem_raw)) + quarter * BN * 128, map_out, tile_m * kTileM + quarter * 32, p.M, n0, p.N, BN, split, lane);
@@ -238,6 +237,18 @@ gemm_tc_single_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     tc_fence_after();
     tmem_dealloc(tmem_base, tmem_cols);
   }
+}
+
+template <int EPI>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_tc_single_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GemmParams p) {
+  single_tile<EPI, false>(map_w, map_x, map_x, p);
+}
+// (A kernel of its own: a third tensor map among the parameters of every decode-sized launch cost a step of one to 64 tokens 0.7%.)
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_tc_single_store_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                            const __grid_constant__ CUtensorMap map_out, const GemmParams p) {
+  single_tile<kStore, true>(map_w, map_x, map_out, p);
 }
 
 template <int EPI, bool MULTI>   // MULTI: a CTA may walk several tiles (two accumulators); else exactly one
@@ -1120,9 +1131,18 @@ SB_EXPORT int sb_gemm_tc_gated(const void* x, int64_t ldx, const void* w, int64_
   const bool multi = total_tiles > resident;
   if (!multi && (p.tiles_n > 65535 || splits > 65535)) return sb::fail("sb_gemm_tc: grid too large");
   const dim3 grid(static_cast<unsigned>(multi ? resident : total_tiles));
-  CUtensorMap map_out = map_x;
+  CUtensorMap map_out;
   // (Few tokens leave a tile so few strips that the detour through shared memory costs what it saves.)
-  p.tma_out = !multi && epilogue == kStore && n > 128 && p.block_n >= 32 && p.stages * stage_bytes >= 512 * p.block_n && map_rows_out(splits, &map_out);
+  if (!multi && epilogue == kStore && n > 128 && p.block_n >= 32 && p.stages * stage_bytes >= 512 * p.block_n && map_rows_out(splits, &map_out)) {
+    static sb::DeviceOnce once;
+    if (once.needed()) {
+      if (cudaFuncSetAttribute(gemm_tc_single_store_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget + 2048) != cudaSuccess)
+        return sb::fail("sb_gemm_tc: cannot raise the shared memory limit");
+      once.done();
+    }
+    sb::launch_pdl(gemm_tc_single_store_kernel, dim3(p.tiles_m, p.tiles_n, splits), dim3(kThreads), smem, stream, map_w, map_x, map_out, p);
+    return sb::check_launch("sb_gemm_tc");
+  }
 #define SB_LAUNCH_M(EPI, MULTI)                                                                         \
   do {                                                                                                  \
     static sb::DeviceOnce once;                                                                       \
@@ -1143,7 +1163,7 @@ SB_EXPORT int sb_gemm_tc_gated(const void* x, int64_t ldx, const void* w, int64_
         return sb::fail("sb_gemm_tc: cannot raise the shared memory limit");                            \
       once.done();                                                                                  \
     }                                                                                                   \
-    sb::launch_pdl(gemm_tc_single_kernel<EPI>, dim3(p.tiles_m, p.tiles_n, splits), dim3(kThreads), smem, stream, map_w, map_x, map_out, p); \
+    sb::launch_pdl(gemm_tc_single_kernel<EPI>, dim3(p.tiles_m, p.tiles_n, splits), dim3(kThreads), smem, stream, map_w, map_x, p); \
   } while (0)
 #define SB_LAUNCH(EPI)                  \
   do {                                  \
