@@ -55,7 +55,7 @@ def _latent(case, window, pages):
 
 
 LATENT = [  # entries, H, G, window, page size, odd latents
-    ([(16, 0)], 16, 1, 0, 64, ()), ([(17, 47)], 16, 1, 0, 64, ()), ([(64, 0)], 16, 1, 0, 64, ()),
+    ([(16, 0)], 16, 1, 0, 64, ()), ([(17, 47)], 16, 1, 0, 64, ()), ([(1, 700), (1, 63), (1, 64), (3, 0)], 16, 1, 100, 64, ()), ([(1, 200)], 64, 1, 0, 16, ()), ([(64, 0)], 16, 1, 0, 64, ()),
     ([(200, 0), (33, 100), (65, 7)], 16, 1, 1024, 64, ()), ([(150, 100), (90, 7)], 16, 1, 70, 16, ()), ([(70, 300)], 16, 1, 3, 8, ()),
     ([(100, 500), (41, 7)], 32, 2, 64, 128, ()), ([(100, 30)], 4, 1, 65, 32, ()), ([(20, 50)], 128, 1, 0, 64, ()), ([(300, 0)], 1, 1, 0, 64, ()),
     # infinities and NaN at keys that some rows of a tile see and others do not: at the causal edge and at the window's
