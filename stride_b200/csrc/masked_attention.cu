@@ -930,15 +930,17 @@ bool latent_shape(const TileParams& p, int pages) {
          ((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.pages)) & 15) == 0;
 }
 
-// From two tiles of 128 rows an entry on, and for any entries, single tokens too, whose blocks take three quarters of the SMs at most. (us, tile kernel / here, 16 heads, 700 cached tokens, window 1,024: one entry of 16 tokens 70 / 45,
-// 16 entries of 16 tokens 140 / 47, of 64 tokens 284 / 94, of 128 tokens 530 / 191; four of 512 tokens 625 / 213.
-// Eight entries of one token behind 20 tokens 10.3 / 9.0, 150 tokens 20.8 / 16.2, 700 tokens 65 / 47, 3,000 tokens 98 / 68; 64 entries, nearly all of the
-// SMs, behind 60 tokens 11.2 / 13.3; 300 entries behind 700 tokens 130 against about 300 in several rounds. Four entries of 16 tokens at their start 10.7 / 11.4.)
+// From two tiles of 128 rows an entry on, and for any entries, single tokens too, whose blocks take three quarters of the SMs at most.
+// Microseconds, tile kernel / here, window 1,024: 16 heads, 700 cached tokens: one entry of 16 tokens 70 / 45, 16 entries of 16 tokens 140 / 47, of 64 tokens 284 / 94, of 128 tokens 530 / 191; four of
+// 512 tokens 625 / 213; eight of one token 65 / 47, and behind 20 tokens 10.3 / 9.0, 150 tokens 20.8 / 16.2, 3,000 tokens 98 / 68.
+// The line: 64 entries of one token are 144 blocks of 148, and behind 20 or 60 tokens took 11.2 / 13.3 (behind 150 tokens 21.6 / 20.0, 700 tokens
+// 66 / 49, which the line gives up); 32 entries, 72 blocks, behind 20 tokens 10.9 / 9.3; between the two nothing was measured. Slower within it: four
+// entries of 8 or 16 tokens behind 20 tokens 10.7 / 11.4, one of one token with 128 heads behind 20 tokens 10.5 / 11.1.
 int launch_latent(const TileParams& p, int pages, int n, cudaStream_t stream, bool* done) {
   using namespace sb::latent5;
   const int Hg = p.H / p.G, ppt = kRows / Hg;
   const int64_t tiles = (n + ppt - 1) / ppt + p.entries;
-  *done = n >= 2 * static_cast<int64_t>(ppt) * p.entries || 2 * tiles * p.G * 4 <= 3 * static_cast<int64_t>(sb::sm_count());
+  *done = n >= 2 * static_cast<int64_t>(ppt) * p.entries || 4 * 2 * tiles * p.G <= 3 * static_cast<int64_t>(sb::sm_count());
   if (!*done) return 0;
   int* status = sb::tc5::status_word();
   if (!status) return sb::fail("sb_masked_attention_tiles: cannot allocate the status word");
