@@ -152,6 +152,12 @@ def test_experts_by_table(W, E, top, ff, shared, n, dtype):
     assert torch.equal(run(list(range(n))), got)
 
 
+@pytest.mark.parametrize("E,top,n", [(40, 3, 43), (40, 5, 205), (40, 16, 256), (40, 17, 241), (31, 20, 251)])     # 129, 1,025, 4,096, 4,097 and 5,020 pairs
+def test_experts_by_table_in_portions_of_the_sort(E, top, n):
+    """One pair more than a thread's first, exactly four a thread, and beyond them: the same as the plain experts, rows alone in the same bits."""
+    test_experts_by_table(64, E, top, 16, 0, n, BF)
+
+
 def _latent_case(H, D, V, R, W, g, own=True, scale=0.4):
     t = {"p.q": torch.randn(H * D, W, generator=g), "p.g": torch.randn(H * V, W, generator=g), "p.uk": torch.randn(H * D, R, generator=g),
          "p.uv": torch.randn(H * V, R, generator=g), "p.o": torch.randn(W, H * V, generator=g), "p.sink": torch.randn(H, generator=g) + 1.0}
