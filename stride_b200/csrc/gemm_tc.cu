@@ -1014,13 +1014,16 @@ SB_EXPORT int sb_gemm_tc_gated(const void* x, int64_t ldx, const void* w, int64_
 
   // The SwiGLU product of many tokens runs on pairs of CTAs or with two weight tiles a CTA; both bring the same bytes
   // from L2 (what bounds these products), the pairs in units half as large. Whichever needs fewer rounds of units of
-  // 128 features x 256 tokens a CTA takes it (two weight tiles on a tie: no traffic between the SMs of a pair).
+  // 128 features x 256 tokens a CTA takes it; on a tie the pairs up to K 3,072, whose epilogue runs beside the next tile's products, and two weight
+  // tiles beyond. (Ties, us, two weight tiles / pairs; K 1,024, 2,056, 3,072, 3,584, 8,192: 8,192 gate and up rows of 2,048 tokens 42 / 33, 78 / 63,
+  // 84 / 82, 96 / 96, 199 / 218; 16,384 rows of 1,024 tokens 44 / 33, 82 / 66, 92 / 93, 104 / 108, at 4,096 112 / 117; 16,384 of 300 tokens 23 / 18,
+  // 44 / 33, 44 / 42, 49 / 48; 4,096 of 1,500 tokens 22 / 18, 38 / 32, 42 / 42, 48 / 51, 88 / 94. Between 3,072 and 3,584 nothing was measured.)
   bool wide = false;
   if (n > 256 && epilogue == kSwiglu) {
     const long long tn = (n + 255) / 256;
     const long long pair_rounds = (((half_rows + 127) / 128) * tn + pairs - 1) / pairs;
     const long long wide_rounds = 2 * ((((half_rows + kTileM - 1) / kTileM) * tn + sms - 1) / sms);
-    wide = wide_rounds <= pair_rounds;
+    wide = wide_rounds < pair_rounds || (wide_rounds == pair_rounds && K > 3072);
   }
   if (wide) {
     const long long tm = (half_rows + kTileM - 1) / kTileM;
