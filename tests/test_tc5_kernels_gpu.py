@@ -153,3 +153,10 @@ def test_products_of_many_tokens_store_what_products_of_a_few_store(n, M, K, gat
     # over 2,048 of them)
     assert ((whole.double() - y).abs().max() / y.abs().max()).item() < (2.0 ** -8 + 1e-4 if gated else 1e-4)
     assert ops.gemm_tc_status() == 0
+
+
+@pytest.mark.parametrize("K", [3064, 3072, 3080])
+@pytest.mark.parametrize("M, n", [(8192, 700), (8204, 513), (16384, 300)])
+def test_gated_products_that_take_as_many_rounds_on_pairs(M, n, K):
+    """As many rounds on pairs of CTAs as with two weight tiles a CTA: K at the line between the two, features that no tile and no 16-byte store divides."""
+    test_products_of_many_tokens_store_what_products_of_a_few_store(n, M, K, True)
