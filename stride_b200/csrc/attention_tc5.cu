@@ -485,7 +485,7 @@ SB_EXPORT int sb_attention_tc5_extra(const void* q, void* out, const void* k_bas
     return sb::fail("sb_attention_tc5: the cache strides must be multiples of the head size and the pointers 16-byte aligned");
   if (Hkv > 65535) return sb::fail("sb_attention_tc5: too many key/value heads");
   int* status = status_word();
-  if (!status) return sb::fail("sb_attention_tc5: cannot allocate the status word");
+  if (!status) return sb::fail("sb_attention_tc5: no status word");
   const int G = Hq / Hkv, ppt = kRows / G;
   Fa5Params p{};
   p.out = static_cast<bf16*>(out);

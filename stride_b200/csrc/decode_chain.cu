@@ -725,7 +725,7 @@ SB_EXPORT int sb_op_decode_chain(const SbOp* op, const SbStep* s, void* stream) 
   p.sync = c->d_sync;
   p.trace = c->trace;
   p.status = status_word();
-  if (!p.status) return sb::fail("sb_op_decode_chain: cannot allocate the status word");
+  if (!p.status) return sb::fail("sb_op_decode_chain: no status word");
   const int BN = 16 << p.bn_log;
   const int D = c->D ? c->D : 64;
   const size_t fixed = D == 128 ? chain_smem<128>(0, BN, max_H) : chain_smem<64>(0, BN, max_H);

@@ -946,7 +946,7 @@ SB_EXPORT int sb_gemm_tc_gated(const void* x, int64_t ldx, const void* w, int64_
   const int kblocks = (K + kTileK - 1) / kTileK;
   if (splits < 1 || splits > kblocks) return sb::fail("sb_gemm_tc: %d splits for %d blocks of K", splits, kblocks);
   int* status = status_word();
-  if (!status) return sb::fail("sb_gemm_tc: cannot allocate the status word");
+  if (!status) return sb::fail("sb_gemm_tc: no status word");
 
   const long long sms = sb::sm_count(), pairs = sms / 2;
   GemmParams p{};
@@ -1208,7 +1208,7 @@ __global__ void lost_signal_kernel(int* status, int code) {
 // reads `code` until somebody clears it.
 SB_EXPORT int sb_gemm_tc_lost_signal_selftest(int code, cudaStream_t stream) {
   int* status = status_word();
-  if (!status) return sb::fail("sb_gemm_tc: cannot allocate the status word");
+  if (!status) return sb::fail("sb_gemm_tc: no status word");
   lost_signal_kernel<<<1, 1, 0, stream>>>(status, code);
   return sb::check_launch("sb_gemm_tc_lost_signal_selftest");
 }

@@ -495,7 +495,7 @@ SB_EXPORT int sb_op_expert_linear(const SbOp* op, const SbStep* s, void* stream)
   TcParams p{};
   p.out = out, p.M = M, p.K = K, p.half_rows = M / 2, p.tiles = tiles, p.order = order, p.block_n = tile, p.pair_weight = pair_weight;
   p.status = status_word();
-  if (!p.status) return sb::fail("sb_op_expert_linear: cannot allocate the status word"), SB_OP_FAILED;
+  if (!p.status) return sb::fail("sb_op_expert_linear: no status word"), SB_OP_FAILED;
   const int stage_bytes = kStageA + tile * 128;
   // two CTAs an SM: one's prologue and epilogue run beside the other's products
   p.stages = std::max(2, std::min({kMaxStages, (kSmemBudget / 2) / stage_bytes, (K + kTileK - 1) / kTileK}));

@@ -943,7 +943,7 @@ int launch_latent(const TileParams& p, int pages, int n, cudaStream_t stream, bo
   *done = n >= 2 * static_cast<int64_t>(ppt) * p.entries || 4 * 2 * tiles * p.G <= 3 * static_cast<int64_t>(sb::sm_count());
   if (!*done) return 0;
   int* status = sb::tc5::status_word();
-  if (!status) return sb::fail("sb_masked_attention_tiles: cannot allocate the status word");
+  if (!status) return sb::fail("sb_masked_attention_tiles: no status word");
   Params q{};
   q.out = p.out, q.block_table = p.block_table, q.max_pages = p.max_pages, q.page_size = p.page_size;
   while ((1 << q.page_shift) < p.page_size) ++q.page_shift;
@@ -989,7 +989,7 @@ int launch_heads5(const HeadLinearParams& p, cudaStream_t stream) {
   q.stages = std::max(2, std::min({kMaxStages, kSmemBudget / stage_bytes, p.K / 64}));
   q.gate = p.gate, q.gate_width = p.gate_width;
   q.status = sb::tc5::status_word();
-  if (!q.status) return sb::fail("sb_head_linear: cannot allocate the status word");
+  if (!q.status) return sb::fail("sb_head_linear: no status word");
   CUtensorMap map_in, map_w, map_out;
   const int64_t idims[3] = {p.K, p.H, p.n}, istrides[3] = {1, p.in_head, p.in_row}, odims[3] = {p.N, p.H, p.n}, ostrides[3] = {1, p.out_head, p.out_row};
   const int64_t wdims[2] = {p.N, static_cast<int64_t>(p.H) * p.K}, wstrides[2] = {1, p.N};

@@ -5,6 +5,7 @@
 
 #include <cuda.h>
 
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <vector>
@@ -283,19 +284,25 @@ inline bool tensor_map_bf16(const void* base, int rank, const int64_t* dims, con
   return tensor_map_of(false, base, rank, dims, strides, box, out);
 }
 
-// One int of device memory for the bounded waits' error codes: the library's own, or the one its user handed it
-// (so that all libraries of a process report into one word, which an engine can read back with every step).
+// One int of device memory for the bounded waits' error codes: the library's own on the current device (a variable of its module, so that
+// nothing is allocated: a first call may be part of a stream capture), or the one its user handed it (so that all libraries of a process
+// report into one word, which an engine can read back with every step).
+static __device__ int own_status_word;
 inline int*& status_word_given() {
   static int* word = nullptr;
   return word;
 }
 inline int* status_word() {
   if (status_word_given()) return status_word_given();
-  static int* word = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    if (cudaMalloc(&word, sizeof(int)) == cudaSuccess) cudaMemset(word, 0, sizeof(int));
-  });
+  static std::atomic<int*> words[64];
+  int d = 0;
+  cudaGetDevice(&d);
+  int* word = words[d & 63].load(std::memory_order_acquire);
+  if (word == nullptr) {
+    void* at = nullptr;
+    if (cudaGetSymbolAddress(&at, own_status_word) != cudaSuccess) return nullptr;
+    words[d & 63].store(word = static_cast<int*>(at), std::memory_order_release);
+  }
   return word;
 }
 

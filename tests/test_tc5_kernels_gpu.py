@@ -1,5 +1,8 @@
 """The tcgen05 kernels that stand beside mma.sync kernels of the same arithmetic: equal bits, and a plain computation in 64 bits."""
+import subprocess
+import sys
 from ctypes import c_float, c_int, c_int64, c_void_p
+from pathlib import Path
 
 import pytest
 import torch
@@ -160,3 +163,26 @@ def test_products_of_many_tokens_store_what_products_of_a_few_store(n, M, K, gat
 def test_gated_products_that_take_as_many_rounds_on_pairs(M, n, K):
     """As many rounds on pairs of CTAs as with two weight tiles a CTA: K at the line between the two, features that no tile and no 16-byte store divides."""
     test_products_of_many_tokens_store_what_products_of_a_few_store(n, M, K, True)
+
+
+FIRST_CALL = """
+import torch
+from stride_b200.kernels import ops
+x = torch.randn((300, 16, 128), device="cuda").bfloat16()
+w = torch.randn((16, 128, 512), device="cuda").bfloat16()
+few, many = (torch.zeros((n, 16, 512), device="cuda", dtype=torch.bfloat16) for n in (60, 300))
+ops.head_linear(x[:60], w, few)
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    ops.head_linear(x, w, many)
+graph.replay()
+torch.cuda.synchronize()
+assert torch.equal(few, many[:60])
+"""
+
+
+def test_a_first_call_on_many_rows_can_be_captured():
+    """A program that has only run a few rows may record many: the kernel's status word is there without an allocation."""
+    run = subprocess.run([sys.executable, "-c", FIRST_CALL], cwd=Path(__file__).resolve().parent.parent, capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr[-2000:]
