@@ -1017,7 +1017,8 @@ SB_EXPORT int sb_gemm_tc_gated(const void* x, int64_t ldx, const void* w, int64_
   // 128 features x 256 tokens a CTA takes it; on a tie the pairs up to K 3,072, whose epilogue runs beside the next tile's products, and two weight
   // tiles beyond. (Ties, us, two weight tiles / pairs; K 1,024, 2,056, 3,072, 3,584, 8,192: 8,192 gate and up rows of 2,048 tokens 42 / 33, 78 / 63,
   // 84 / 82, 96 / 96, 199 / 218; 16,384 rows of 1,024 tokens 44 / 33, 82 / 66, 92 / 93, 104 / 108, at 4,096 112 / 117; 16,384 of 300 tokens 23 / 18,
-  // 44 / 33, 44 / 42, 49 / 48; 4,096 of 1,500 tokens 22 / 18, 38 / 32, 42 / 42, 48 / 51, 88 / 94. Between 3,072 and 3,584 nothing was measured.)
+  // 44 / 33, 44 / 42, 49 / 48; 4,096 of 1,500 tokens 22 / 18, 38 / 32, 42 / 42, 48 / 51, 88 / 94. Between 3,072 and 3,584 nothing was measured. Without
+  // 16-byte stores, 4,100 rows at K 1,024: 1,100 tokens 22.4 / 19.3, 2,048 tokens 22.2 / 23.1.)
   bool wide = false;
   if (n > 256 && epilogue == kSwiglu) {
     const long long tn = (n + 255) / 256;

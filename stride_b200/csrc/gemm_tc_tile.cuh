@@ -142,8 +142,11 @@ __device__ __forceinline__ void swiglu_tile(uint32_t tmem_base, float* xch, bf16
 
 // The same for two sets of four warps, each of which takes alternate groups of sixteen tokens with buffers and a named barrier (1 + set) of its
 // own. One barrier a group: a group's values are exchanged while the results of the group before travel through shared memory to rows of 64
-// features, of which a thread stores eight of a token at once; the buffers (xch2 2 x 16 x 64 floats, done2 as many bfloat16) alternate.
-// (8,192 features of 256 tokens, the whole product: 21.5 us with a group at a time, two barriers and two-byte stores, 19.4 so.)
+// features, of which a thread stores eight of a token at once or, without 16-byte stores, one of eight tokens beside its neighbours'; the buffers
+// (xch2 2 x 16 x 64 floats, done2 as many bfloat16) alternate.
+// (8,192 features of 256 tokens, the whole product: 21.5 us with a group at a time, two barriers and two-byte stores, 19.4 so. Features that eight
+// does not divide, a group at a time / so / so with eight neighbours a thread: 4,100 rows, K 1,024, 256 tokens 11.6 / 11.6 / 13.4, 8,204 rows, K 2,048
+// 19.9 / 18.3 / 21.4.)
 // tmem_d: the accumulator, this warp's lanes; j0: the first output feature; `vec`: the output takes 16-byte stores.
 __device__ __forceinline__ void swiglu_set(uint32_t tmem_d, float* xch2, bf16* done2, bf16* out, int64_t ldo, int j0, int half_rows, int n0, int N, int BN,
                                            int set, int quarter, int lane, bool ok, bool vec, const Gate& gate, const float* column_weight = nullptr) {
@@ -168,17 +171,16 @@ __device__ __forceinline__ void swiglu_set(uint32_t tmem_d, float* xch2, bf16* d
     if (set == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
     else asm volatile("bar.sync 2, 128;" ::: "memory");
     if (i > 0) {
-      const int n = n0 + c0 - 32 + (t >> 3), j = j0 + (t & 7) * 8;
-      const bf16* from = done2 + ((i - 1) & 1) * (16 * 64) + t * 8;
-      bf16* to = out + static_cast<int64_t>(n) * ldo + j;
-      if (ok && n < N) {
-        if (vec) {
-          if (j < half_rows) *reinterpret_cast<uint4*>(to) = *reinterpret_cast<const uint4*>(from);
-        } else {
+      const bf16* from = done2 + ((i - 1) & 1) * (16 * 64);
+      if (vec) {
+        const int n = n0 + c0 - 32 + (t >> 3), j = j0 + (t & 7) * 8;
+        if (ok && n < N && j < half_rows) *reinterpret_cast<uint4*>(out + static_cast<int64_t>(n) * ldo + j) = *reinterpret_cast<const uint4*>(from + t * 8);
+      } else if (ok && j0 + (t & 63) < half_rows) {
+        const int n = n0 + c0 - 32 + (t >> 6);
+        bf16* to = out + static_cast<int64_t>(n) * ldo + j0 + (t & 63);
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            if (j + k < half_rows) to[k] = from[k];
-        }
+        for (int k = 0; k < 16; k += 2)
+          if (n + k < N) to[k * ldo] = from[k * 64 + t];
       }
     }
     if (!more) break;
