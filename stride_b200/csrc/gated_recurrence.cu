@@ -192,7 +192,7 @@ SB_EXPORT int sb_gated_scan(const float* act, int width, int q_off, int g_off, i
     sb::launch_pdl(kernel, dim3(entries, H, (V + 31) / 32), dim3(sbscan::step_threads(D)), sbscan::step_smem(D, true), stream, p);
     return sb::check_launch("sb_gated_scan");
   }
-  return sbscan::launch_scan<true>(p, entries, "sb_gated_scan", stream);
+  return sbscan::launch_scan<true>(p, entries, n, "sb_gated_scan", stream);
 }
 
 SB_EXPORT int sb_group_rmsnorm(const float* o, const void* gain, int gain_dtype, void* out, int out_dtype, int n, int H, int V, float eps,

@@ -195,7 +195,7 @@ SB_EXPORT int sb_lightning_scan_ex(const float* proj, int n_partials, int64_t pa
   // steps with longer entries: the activation once for all tokens, then the recurrence
   if (ready) {
     if (n_partials != 1) return sb::fail("sb_lightning_scan: ready-made q, k, v come as one buffer");
-    return sbscan::launch_scan<false>(p, entries, "sb_lightning_scan", stream);
+    return sbscan::launch_scan<false>(p, entries, n, "sb_lightning_scan", stream);
   }
   if (act == nullptr) return sb::fail("sb_lightning_scan: a step with an entry of several tokens needs the scratch for the activated sums");
   const int cols = max(max(q_off + H * D, k_off + H * D), v_off + H * V);
@@ -206,7 +206,7 @@ SB_EXPORT int sb_lightning_scan_ex(const float* proj, int n_partials, int64_t pa
   else sb::launch_pdl(lightning_activate_kernel<1, false>, dim3(n, (cols + 1023) / 1024), dim3(256), 0, stream, proj, n_partials, partial_stride, width, act, cols);
   p.rows = act;
   p.width = cols;
-  return sbscan::launch_scan<false>(p, entries, "sb_lightning_scan", stream);
+  return sbscan::launch_scan<false>(p, entries, n, "sb_lightning_scan", stream);
 }
 
 SB_EXPORT int sb_lightning_scan(const float* proj, int n_partials, int64_t partial_stride, int width, int q_off, int k_off, int v_off,

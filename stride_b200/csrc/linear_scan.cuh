@@ -301,8 +301,26 @@ __global__ void __launch_bounds__(kWarps * 32 + 32, DL == 8 ? 2 : DL == 4 && PER
   }
 }
 
+// Whether a launch with two columns a warp begins behind the kernel in front instead of early: one or two long CTAs an SM have to be dealt out
+// evenly, which CTAs that are let in beside a running kernel are not, and a CTA that begins late lacks 0.4 to 0.9 us. `tokens`: an entry's, on
+// average. In a row with the kernels in front and behind, us, early / behind (906 points of 26 shapes of heads). More CTAs than half the SMs, keys
+// of 65 to 128: 16 heads of 128 x 128 (256 CTAs) 2 tokens 8.5 / 8.2, 64 tokens 14.3 / 12.6, 2,048 tokens 204 / 153, with gates 8.7 / 7.7, 14.8 /
+// 12.6, 236 / 164; 80 CTAs 4 tokens 6.3 / 6.7, 16 tokens 6.6 / 6.6, 256 tokens 28 / 19, with gates 6.4 / 6.1, 6.9 / 6.1, 33 / 19. Keys up to 64: 32
+// heads of 64 x 64 4 tokens 6.7 / 7.0, 16 tokens 7.0 / 7.0, 64 tokens 12.2 / 9.9; 256 CTAs of 32 x 32 32 tokens 8.1 / 8.5, 64 tokens 11.8 / 10.7. Keys beyond
+// 128, which leave an SM one CTA: 128 CTAs 2 tokens 9.4 / 7.9, 128 tokens 28.6 / 19.5 (with gates 8 tokens 8.6 / 8.9), more CTAs than SMs 2 tokens
+// 8.8 / 9.6, 128 tokens 29.0 / 30.5. Up to half the SMs: 64 CTAs of 128 x 128 64 tokens 8.8 / 9.2, 128 tokens 13.9 / 12.2, with gates 16 tokens 6.3 / 6.2, 64
+// tokens 9.4 / 8.8; 32 CTAs 128 tokens 10.6 / 12.0, 256 tokens 22 / 18; 16 CTAs 256 tokens 16.5 / 17.3, 512 tokens 34 / 28.
+template <int DL, bool GATED>
+bool starts_behind(int64_t ctas, int D, int64_t tokens) {
+  const int64_t sms = sb::sm_count();
+  if (DL == 8) return ctas <= sms;
+  if (2 * ctas <= sms) return tokens >= (8 * ctas <= sms ? 512 : 4 * ctas <= sms ? 256 : DL == 4 && GATED ? 32 : 128);
+  if (DL == 4) return GATED || 4 * ctas > 3 * sms || tokens >= 16;
+  return tokens >= (D > 32 ? 16 : 64);
+}
+
 template <int DL, int PER, bool GATED>
-int launch_scan_of(const Params& p, int entries, const char* who, cudaStream_t stream) {
+int launch_scan_of(const Params& p, int entries, int n, const char* who, cudaStream_t stream) {
   constexpr int kCols = kWarps * PER;
   constexpr size_t smem = sizeof(float) * stages_of<DL, GATED>() * kChunk * ((GATED ? 3 : 2) * kLanes * DL + kCols);
   static_assert(smem <= 200 * 1024, "staging buffers");
@@ -320,20 +338,19 @@ int launch_scan_of(const Params& p, int entries, const char* who, cudaStream_t s
     once.done();
   }
   const dim3 grid(entries, p.H, (p.V + kCols - 1) / kCols), block(kWarps * 32 + 32);
-  // Two columns a warp: one or two long CTAs an SM, which have to be dealt out evenly (one entry of 2,048 tokens, 16 heads of 128 x 128: 204 us let
-  // in early, 153 behind the kernel in front, with gates 236 and 164; 512 tokens 40 and 41, 61 and 43; 64 tokens 10.1 and 9.4, 10.4 and 8.2). More
-  // entries fill the SMs either way, and start early (16 entries of 64 tokens 59 us, 61 behind).
-  if constexpr (PER == 2) sb::launch_behind(kernel, grid, block, smem, stream, p);
+  // (four columns a warp: entries enough to fill the SMs either way; 16 entries of 64 tokens 59 us early, 61 behind)
+  if (PER == 2 && starts_behind<DL, GATED>(static_cast<int64_t>(grid.x) * grid.y * grid.z, p.D, n / entries)) sb::launch_behind(kernel, grid, block, smem, stream, p);
   else sb::launch_pdl(kernel, grid, block, smem, stream, p);
   return sb::check_launch(who);
 }
 
 // Launches scan_kernel for the key size (at most 256). Four columns a warp make fewer reads a column; two make twice the CTAs, which is the
-// faster way while they all run at once (153 against 220 us for 128 CTAs of four; 828 against 710 us for 1,024).
+// faster way for long entries while they all run at once (16 heads of 128 x 128 in a row with the kernels around them, 1,024 tokens: 85 against
+// 131 us for 128 CTAs of four, 16 tokens 8.8 against 8.5; alone, eight entries of 2,048 tokens, 828 against 710 us for 1,024).
 template <bool GATED>
-int launch_scan(const Params& p, int entries, const char* who, cudaStream_t stream) {
+int launch_scan(const Params& p, int entries, int n, const char* who, cudaStream_t stream) {
   const bool few = static_cast<int64_t>(entries) * p.H * ((p.V + 15) / 16) <= sb::sm_count();
-#define SB_SCAN_OF(DL) (few ? launch_scan_of<DL, 2, GATED>(p, entries, who, stream) : launch_scan_of<DL, 4, GATED>(p, entries, who, stream))
+#define SB_SCAN_OF(DL) (few ? launch_scan_of<DL, 2, GATED>(p, entries, n, who, stream) : launch_scan_of<DL, 4, GATED>(p, entries, n, who, stream))
   switch (lane_elements(p.D)) {
     case 2: return SB_SCAN_OF(2);
     case 4: return SB_SCAN_OF(4);

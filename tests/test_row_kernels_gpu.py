@@ -241,6 +241,38 @@ def test_recurrence_with_as_many_tokens_as_entries(gated, lengths):
 
 
 @pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("H,D,tokens", [(1, 64, 511), (1, 64, 512), (4, 96, 255), (4, 96, 256), (8, 40, 127), (8, 40, 128), (8, 128, 31), (8, 128, 32), (12, 100, 15),
+                                        (12, 100, 16), (12, 64, 15), (12, 64, 16), (12, 32, 63), (12, 32, 64), (18, 200, 20), (19, 200, 20)])
+def test_recurrence_that_starts_early_or_behind_the_kernel_in_front(H, D, tokens, gated):
+    """Launches on both sides of the lines between the two starts, their rows written by the kernel in front over NaN: the bits of portions of
+    at most ten tokens."""
+    from stride_b200.kernels import ops
+    g = torch.Generator(device=DEV).manual_seed(H * D + tokens)
+    V, HD, HV = 64, H * D, H * 64
+    proj = torch.randn((1, tokens, 2 * HD + HV), device=DEV, generator=g) * 0.3
+    lower, zero = torch.rand(HD, device=DEV, generator=g) * 0.5, torch.zeros(HD, device=DEV)
+    decay = torch.rand(H, device=DEV, generator=g) * 0.5 + 0.4
+
+    def run(first, count, state):
+        act = torch.full((count, (3 if gated else 2) * HD + HV), float("nan"), device=DEV)
+        meta = torch.tensor([[0], [0], [count], [first]], dtype=torch.int32, device=DEV)
+        out = torch.zeros((count, HV), device=DEV)
+        part = proj[:, first:first + count].contiguous()
+        torch.cuda.synchronize()
+        if gated:
+            ops.hgrn2_activate(part, zero, lower, act, HD, HV)
+            ops.gated_scan(act, 0, HD, 2 * HD, 3 * HD, meta, 1, state, out, H, D, V)
+        else:
+            ops.lightning_scan(part, 0, HD, 2 * HD, meta, 1, decay, state, out, H, D, V, act)
+        return out
+
+    whole, cut = (torch.full((1, H, D, V), float("nan"), device=DEV) for _ in range(2))
+    out = run(0, tokens, whole)
+    assert torch.isfinite(out).all()
+    assert torch.equal(out, torch.cat([run(a, min(10, tokens - a), cut) for a in range(0, tokens, 10)])) and torch.equal(whole, cut)
+
+
+@pytest.mark.parametrize("gated", [True, False])
 @pytest.mark.parametrize("D,tokens", [(144, 40), (144, 1), (40, 40), (40, 1), (16, 20)])
 def test_recurrence_with_an_infinite_value(D, tokens, gated):
     """Key sizes that do not fill the lanes: an infinite value makes its own column infinite from its token on (all keys, queries and states
