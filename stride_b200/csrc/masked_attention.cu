@@ -970,21 +970,51 @@ int launch_latent(const TileParams& p, int pages, int n, cudaStream_t stream, bo
   return sb::check_launch("sb_masked_attention_tiles");
 }
 
+// CTAs of the matrix per head on tcgen05 with `cols` columns each.
+int64_t heads5_ctas(const HeadLinearParams& p, int cols) {
+  return static_cast<int64_t>((p.n + sb::heads5::kRows - 1) / sb::heads5::kRows) * p.H * (p.N / cols);
+}
+
+// Columns of a CTA: as many as divide the matrix, up to 256, so that the rows brought in serve as many as they can; 64 where CTAs of 64 still have an
+// SM each, since what counts there is one CTA's time, and that is mostly its epilogue (us on mma.sync / here with 256 columns / with 64: 256 -> 512, two
+// heads, 1,024 tokens 7.5 / 5.7 / 4.1, one head, 512 tokens 4.0 / 5.5 / 3.7). With gates always the first.
+int heads5_cols(const HeadLinearParams& p) {
+  if (p.gate == nullptr && heads5_ctas(p, 64) <= sb::sm_count()) return 64;
+  int cols = 256;
+  while (p.N % cols != 0) cols -= 64;
+  return cols;
+}
+
 // The matrix per head for many tokens: sizes that its pieces divide, and the gate in one piece that takes 16-byte accesses (a thread reads its
-// row's gates line by line, which the partial sums of nine K ranges make slower than what the tensor cores save). Microseconds, mma.sync / here,
-// 16 heads: 128 -> 512 for 64 tokens 3.8 / 3.9, 128 tokens 5.6 / 4.5, 512 9.1 / 6.1, 2,048 29.6 / 11.7; 512 -> 128 with a gate in one piece for
-// 1,024 tokens 20.7 / 17.4, 2,048 30.4 / 19.2; in nine for 256 18 / 38.
+// row's gates line by line, which the partial sums of nine K ranges make slower than what the tensor cores save). 3,024 points of 1 to 32 heads, K 64 to
+// 1,024, N 64 to 1,024, 128 to 2,048 tokens, mma.sync / here, us. Without a gate from K 192 on always, below where the other kernel's blocks of
+// 64 x 64 take more than three quarters of the SMs: 64 -> 64 64 blocks 2.5 / 2.7, 128 blocks 2.9 / 2.75, 256 blocks 3.9 / 3.1; 128 -> 512, four heads,
+// 512 tokens 5.1 / 3.5, 16 heads, 2,048 tokens 29.4 / 11.2. (Fewer than 128 tokens were measured at one shape: 64 tokens of that 3.8 / 3.9.)
+// With a gate the row's sigmoids are the larger part of a CTA's time, two CTAs an SM share it, and the other kernel spreads them over four times
+// as many warps. More CTAs than SMs, all at once: K 192, 256 CTAs 0.88 to 0.98 of the other's time, K 128 1.0 to 1.15. Up to one an SM, CTAs by
+// columns and K: at K 512 and 128 columns 64 CTAs 1.05, 80 CTAs 0.89; 192 columns 64 CTAs 1.14, 128 0.93; 256 columns 128 CTAs 1.03, 256 0.70; at
+// K 1,024 and 128 columns 32 CTAs 1.05, 64 0.75; at K 384 64 columns 128 CTAs 0.86, 192 columns 1.05. In rounds: at K 512 always (0.73 to 1.02),
+// from K 320 where the rounds are nearly full (512 CTAs 0.85 to 0.97, 320 and 640 1.04 to 1.24; with five CTAs a row 1,280 of them 1.04 to 1.10),
+// below never (K 256, 320 CTAs 1.35). 512 -> 128, 16 heads: 1,024 tokens 20.5 / 17.3, 2,048 tokens 29.7 / 19.2.
 bool takes_heads5(const HeadLinearParams& p) {
   if (p.K % 64 != 0 || p.N % 64 != 0 || p.tail != 0 || p.H > 65535) return false;
-  if (p.gate == nullptr) return p.n >= 128;
-  return p.n >= 512 && p.gate_partials == 1 && p.gate_width % 4 == 0 && (reinterpret_cast<uintptr_t>(p.gate) & 15) == 0;
+  const int64_t sms = sb::sm_count();
+  if (p.gate == nullptr) {
+    if (p.n < 128) return false;
+    return p.K >= 192 || 4 * static_cast<int64_t>((p.n + kHlTile - 1) / kHlTile) * p.H * (p.N / kHlTile) > 3 * sms;
+  }
+  if (p.n < 512 || p.gate_partials != 1 || p.gate_width % 4 != 0 || (reinterpret_cast<uintptr_t>(p.gate) & 15) != 0) return false;
+  const int cols = heads5_cols(p);
+  const int64_t ctas = heads5_ctas(p, cols), rounds = (ctas + 2 * sms - 1) / (2 * sms);
+  if (rounds > 1) return p.K >= 512 || (p.K >= 320 && p.N <= 4 * cols && 5 * ctas >= 4 * 2 * sms * rounds);
+  return p.K >= 384 ? ctas * p.K > 2 * sms * std::max(cols, 128) : p.K >= 192 && ctas > sms;
 }
 
 int launch_heads5(const HeadLinearParams& p, cudaStream_t stream) {
   using namespace sb::heads5;
   Params q{};
   q.n = p.n, q.K = p.K, q.N = p.N;
-  for (q.cols = 256; p.N % q.cols != 0;) q.cols -= 64;
+  q.cols = heads5_cols(p);
   const int stage_bytes = kABytes + q.cols * 128;
   q.stages = std::max(2, std::min({kMaxStages, kSmemBudget / stage_bytes, p.K / 64}));
   q.gate = p.gate, q.gate_width = p.gate_width;

@@ -92,14 +92,38 @@ def test_latent_attention_on_tcgen05_has_the_bits_of_the_tile_kernel(entries, H,
         assert ((got - want).abs().max() / want.abs().max()).item() < 2.0 ** -8 + 1e-4
 
 
-@pytest.mark.parametrize("n, H, K, N, partials, pad", [(130, 2, 128, 512, 0, 0), (256, 1, 64, 64, 0, 0), (383, 3, 64, 192, 1, 0), (513, 2, 512, 128, 3, 0),
-                                                       (300, 5, 192, 320, 2, 0), (257, 16, 512, 128, 9, 0), (700, 4, 128, 64, 0, 8)])
-def test_matrix_per_head_has_one_result_for_any_number_of_rows(n, H, K, N, partials, pad):
-    """Many rows take the tcgen05 kernel, a few the mma.sync kernel: the same bits, and nothing written beyond the rows or the columns."""
+def _kernels(call):
+    """What call() returns and the names of the kernels that it launches."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        result = call()
+        torch.cuda.synchronize()
+    return result, " ".join(e.name for e in p.events())
+
+
+HEADS = [  # n, H, K, N, partial sums of the gate, elements behind a row, elements behind a gate's row, whether the tcgen05 form is taken
+    (130, 2, 128, 512, 0, 0, 64, False), (256, 1, 64, 64, 0, 0, 64, False), (127, 16, 192, 320, 0, 0, 64, False), (128, 1, 192, 64, 0, 0, 64, True),
+    (300, 5, 192, 320, 0, 0, 64, True), (700, 4, 256, 64, 0, 8, 64, True), (383, 3, 512, 192, 0, 8, 64, True),
+    # at the line of three quarters of the SMs (blocks of 64 x 64), and at one CTA of 64 columns an SM, where the columns become more
+    (256, 27, 64, 64, 0, 0, 64, False), (256, 28, 64, 64, 0, 0, 64, True), (256, 37, 64, 128, 0, 0, 64, True), (256, 38, 64, 128, 0, 0, 64, True),
+    (513, 15, 128, 256, 0, 0, 64, True), (2000, 5, 1024, 192, 0, 0, 64, True),
+    # gates: several partial sums, few CTAs, too few tokens, widths and places without 16-byte accesses; then the form itself, in one round and in several
+    (513, 2, 512, 128, 3, 0, 64, False), (257, 16, 512, 128, 9, 0, 64, False), (513, 2, 512, 128, 1, 0, 64, False), (511, 32, 512, 128, 1, 0, 64, False),
+    (640, 16, 512, 128, 1, 0, 62, False), (640, 16, 512, 128, 1, 0, 65, False),
+    (640, 16, 512, 128, 1, 0, 64, True), (512, 32, 512, 128, 1, 8, 4, True), (515, 16, 1024, 64, 1, 0, 64, True), (700, 30, 192, 128, 1, 0, 64, True),
+    (700, 32, 512, 192, 1, 0, 64, True), (515, 16, 512, 320, 1, 0, 64, True), (1030, 18, 384, 256, 1, 0, 64, False), (1030, 24, 384, 256, 1, 0, 64, True), (2047, 32, 320, 64, 1, 0, 64, True),
+    (2047, 32, 256, 64, 1, 0, 64, False),
+]
+
+
+@pytest.mark.parametrize("n, H, K, N, partials, pad, gate_pad, many", HEADS)
+def test_matrix_per_head_has_one_result_for_any_number_of_rows(n, H, K, N, partials, pad, gate_pad, many):
+    """The tcgen05 kernel where the rule says so, the mma.sync kernel for a few rows: the same bits, and nothing written beyond the rows or the
+    columns."""
     gen = torch.Generator(device=DEVICE).manual_seed(n)
     x = torch.randn((n, H, K + pad), device=DEVICE, generator=gen).bfloat16()
     w = (torch.randn((H, K, N), device=DEVICE, generator=gen) * 0.05).bfloat16()
-    width = H * N + 64
+    width = H * N + gate_pad
     gate = torch.randn((partials, n, width), device=DEVICE, generator=gen) if partials else None
 
     def run(first, rows):
@@ -112,7 +136,8 @@ def test_matrix_per_head_has_one_result_for_any_number_of_rows(n, H, K, N, parti
         torch.cuda.synchronize()
         assert (out[rows] == 7).all() and (out[:, :, N:] == 7).all()
         return out[:rows, :, :N]
-    whole = run(0, n)
+    whole, names = _kernels(lambda: run(0, n))
+    assert ("head_linear_tc5_kernel" in names) == many and ("head_linear_tc_kernel" in names) != many
     assert torch.equal(whole, torch.cat([run(a, min(60, n - a)) for a in range(0, n, 60)]))
     want = torch.einsum("nhk,hkm->nhm", x[..., :K].double(), w.double())
     if partials:
