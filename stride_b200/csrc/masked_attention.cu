@@ -930,17 +930,23 @@ bool latent_shape(const TileParams& p, int pages) {
          ((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.pages)) & 15) == 0;
 }
 
-// From two tiles of 128 rows an entry on, and for any entries, single tokens too, whose blocks take three quarters of the SMs at most.
-// Microseconds, tile kernel / here, window 1,024: 16 heads, 700 cached tokens: one entry of 16 tokens 70 / 45, 16 entries of 16 tokens 140 / 47, of 64 tokens 284 / 94, of 128 tokens 530 / 191; four of
-// 512 tokens 625 / 213; eight of one token 65 / 47, and behind 20 tokens 10.3 / 9.0, 150 tokens 20.8 / 16.2, 3,000 tokens 98 / 68.
-// The line: 64 entries of one token are 144 blocks of 148, and behind 20 or 60 tokens took 11.2 / 13.3 (behind 150 tokens 21.6 / 20.0, 700 tokens
-// 66 / 49, which the line gives up); 32 entries, 72 blocks, behind 20 tokens 10.9 / 9.3; between the two nothing was measured. Slower within it: four
-// entries of 8 or 16 tokens behind 20 tokens 10.7 / 11.4, one of one token with 128 heads behind 20 tokens 10.5 / 11.1.
-int launch_latent(const TileParams& p, int pages, int n, cudaStream_t stream, bool* done) {
+// From two tiles of 128 rows an entry on; and any entries, single tokens too, whose blocks are few. Microseconds, tile kernel / here, window
+// 1,024, 1,743 points of 1 to 128 heads a latent, 1 to 100 entries, 0 to 3,000 tokens in front: 16 heads, 700 tokens in front: 16 entries of 16
+// tokens 140 / 46, four of 64 tokens 140 / 45, eight of 256 tokens 566 / 193; eight of one token 65 / 47, behind 3,000 tokens 98 / 68.
+// Few blocks: where some request has 128 keys or more in its window, three quarters of the SMs (150 tokens in front: 64 blocks 0.64 to 0.90 of
+// the other's time, 110 blocks 0.69 to 0.98, 128 blocks 0.63 to 1.05; from 160 blocks on with few heads 1.4 and more). Where all have fewer, or
+// the host does not know, a CTA's time is mostly its beginning and its end: with 32 heads and more the same line (110 blocks 0.67 to 0.76), with
+// 8 and 16 heads half the SMs (up to 60 tokens in front: 64 blocks 0.88 to 1.02, 80 blocks 0.92 to 1.04, 110 blocks 1.05 to 1.19), with fewer
+// none (1.00 to 1.12 at 2 to 64 blocks).
+// Slower all the same: what a recorded step takes as known, half of the keys that it is planned for, is 128 in the shortest of them: a step of
+// requests with up to 64 keys and four heads or fewer a latent then takes up to 1 us longer (8.6 / 9.6), one with more takes 2 to 7 us less.
+int launch_latent(const TileParams& p, int pages, int n, int longest, cudaStream_t stream, bool* done) {
   using namespace sb::latent5;
   const int Hg = p.H / p.G, ppt = kRows / Hg;
-  const int64_t tiles = (n + ppt - 1) / ppt + p.entries;
-  *done = n >= 2 * static_cast<int64_t>(ppt) * p.entries || 4 * 2 * tiles * p.G <= 3 * static_cast<int64_t>(sb::sm_count());
+  const int64_t sms = sb::sm_count();
+  const int64_t tiles = static_cast<int64_t>(n - p.entries) / ppt + p.entries, blocks = 2 * tiles * p.G;      // (the most: an entry has ceil(its tokens / ppt))
+  const bool far = (p.window > 0 ? std::min(p.window, longest) : longest) >= 128;
+  *done = n >= 2 * static_cast<int64_t>(ppt) * p.entries || (far || Hg >= 32 ? 4 * blocks <= 3 * sms : Hg >= 8 && 2 * blocks <= sms);
   if (!*done) return 0;
   int* status = sb::tc5::status_word();
   if (!status) return sb::fail("sb_masked_attention_tiles: no status word");
@@ -1190,9 +1196,10 @@ SB_EXPORT int sb_masked_attention_tiles_supported(int H, int G, int D, int Dv, i
   return heads && D % 16 == 0 && D >= 16 && Dv % 16 == 0 && Dv >= 16 && Dv <= 512 && Dv <= Dc && Dc % 8 == 0 && v_offset % 8 == 0 && stage <= 200 * 1024;
 }
 
-// `arena_pages`: pages of the arena behind `pages` (0: not known; the form that addresses pages by TMA is then left out).
-SB_EXPORT int sb_masked_attention_tiles_in(const void* q, void* out, const void* pages, int arena_pages, const int32_t* block_table, int max_pages,
-                                           int page_size, int64_t page_stride, int64_t v_offset, int64_t head_stride, const int32_t* meta, int meta_stride,
+// `arena_pages`: pages of the arena behind `pages` (0: not known; the form that addresses pages by TMA is then left out). `longest`: tokens of the
+// longest request with this step's, as far as known (0: not).
+SB_EXPORT int sb_masked_attention_tiles_in(const void* q, void* out, const void* pages, int arena_pages, int longest, const int32_t* block_table,
+                                           int max_pages, int page_size, int64_t page_stride, int64_t v_offset, int64_t head_stride, const int32_t* meta, int meta_stride,
                                            int entries, const float* slopes, const float* sinks, int n, int H, int G, int D, int Dv, int Dc,
                                            int window, int keep_first, float scale, int chunk, int out_f32, float cap, cudaStream_t stream) {
   if (n <= 0 || entries <= 0) return 0;
@@ -1204,7 +1211,7 @@ SB_EXPORT int sb_masked_attention_tiles_in(const void* q, void* out, const void*
                v_offset, head_stride, meta, meta_stride, entries, slopes, sinks, H, G, D, Dv, Dc, window, keep_first, scale, 2, chunk, out_f32, cap};
   if (latent_shape(p, arena_pages)) {
     bool done = false;
-    const int rc = launch_latent(p, arena_pages, n, stream, &done);
+    const int rc = launch_latent(p, arena_pages, n, longest, stream, &done);
     if (done) return rc;
   }
   const int groups = (Dv / 16 + 3) / 4;
@@ -1220,7 +1227,7 @@ SB_EXPORT int sb_masked_attention_tiles_ex(const void* q, void* out, const void*
                                            int64_t page_stride, int64_t v_offset, int64_t head_stride, const int32_t* meta, int meta_stride,
                                            int entries, const float* slopes, const float* sinks, int n, int H, int G, int D, int Dv, int Dc,
                                            int window, int keep_first, float scale, int chunk, int out_f32, float cap, cudaStream_t stream) {
-  return sb_masked_attention_tiles_in(q, out, pages, 0, block_table, max_pages, page_size, page_stride, v_offset, head_stride, meta, meta_stride, entries,
+  return sb_masked_attention_tiles_in(q, out, pages, 0, 0, block_table, max_pages, page_size, page_stride, v_offset, head_stride, meta, meta_stride, entries,
                                       slopes, sinks, n, H, G, D, Dv, Dc, window, keep_first, scale, chunk, out_f32, cap, stream);
 }
 
@@ -1327,9 +1334,9 @@ SB_EXPORT int sb_op_masked_attention(const SbOp* op, const SbStep* s, void* stre
 SB_EXPORT int sb_op_masked_attention_tiles(const SbOp* op, const SbStep* s, void* stream) {
   using namespace sbstep;
   if (s->n <= 0) return SB_OP_SKIPPED;
-  return sb_masked_attention_tiles_in(ptr<const void>(op->i[0]), ptr<void>(op->i[1]), ptr<const void>(op->i[2]), (int)op->i[20], ptr<const int32_t>(op->i[3]),
-                                   (int)op->i[4], (int)op->i[5], op->i[6], op->i[7], op->i[8], entry_meta(s), s->max_rows, s->entries, ptr<const float>(op->i[9]),
-                                   ptr<const float>(op->i[10]), s->n, (int)op->i[11], (int)op->i[12], (int)op->i[13], (int)op->i[14], (int)op->i[15],
+  return sb_masked_attention_tiles_in(ptr<const void>(op->i[0]), ptr<void>(op->i[1]), ptr<const void>(op->i[2]), (int)op->i[20], s->longest,
+                                   ptr<const int32_t>(op->i[3]), (int)op->i[4], (int)op->i[5], op->i[6], op->i[7], op->i[8], entry_meta(s), s->max_rows,
+                                   s->entries, ptr<const float>(op->i[9]), ptr<const float>(op->i[10]), s->n, (int)op->i[11], (int)op->i[12], (int)op->i[13], (int)op->i[14], (int)op->i[15],
                                    (int)op->i[16], (int)op->i[17], (float)op->f[0], (int)op->i[18], (int)op->i[19], (float)op->f[1],
                                    static_cast<cudaStream_t>(stream));
 }

@@ -976,6 +976,9 @@ SB_API int sb_program_prepare(void* program, int E, const int32_t* count, const 
   step->n = n, step->entries = E, step->wanted = wanted, step->static_keys = static_keys, step->max_rows = p->R;
   step->n_plans = (int)p->plans.size();
   step->ints = device_ints;
+  step->longest = static_keys / 2;
+  if (static_keys == 0)
+    for (int e = 0; e < E; ++e) step->longest = std::max(step->longest, first[e] + count[e]);
   int32_t* work = staging + 9 * (int64_t)p->R;
   int at = 0;
   for (size_t k = 0; k < p->plans.size(); ++k) {

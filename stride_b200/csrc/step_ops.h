@@ -45,6 +45,8 @@ typedef struct SbStep {
   int32_t static_keys;   // > 0: a decode step recorded into a CUDA graph; no key lies at or beyond this position
   int32_t max_rows;      // R: the regions of `ints` are R apart
   int32_t n_plans;
+  int32_t longest;       // tokens that the step's longest request has with this step, as far as the host knows: of a recorded step half of static_keys
+  int32_t reserved;
   // The step's integer inputs on the device: tokens [0, R), positions [R, 2R), slots [2R, 3R), wanted rows [3R, 4R),
   // entry records [4R, 8R) (slot, first row, length, first position: four rows of R), the slot of every wanted
   // row [8R, 9R), work lists from 9R on.

@@ -34,7 +34,7 @@ class SbTilePlan(ctypes.Structure):
 
 class SbStep(ctypes.Structure):
     _fields_ = [("n", c_int32), ("entries", c_int32), ("wanted", c_int32), ("static_keys", c_int32), ("max_rows", c_int32),
-                ("n_plans", c_int32), ("ints", c_void_p), ("plan", SbTilePlan * MAX_PLANS)]
+                ("n_plans", c_int32), ("longest", c_int32), ("reserved", c_int32), ("ints", c_void_p), ("plan", SbTilePlan * MAX_PLANS)]
 
 
 class SbOp(ctypes.Structure):
@@ -320,6 +320,7 @@ class ImmediateProgram(_StreamHolder):
         self.step = SbStep()
         self.step.n, self.step.entries, self.step.wanted = ctx.n, len(ctx.entry_length), 0
         self.step.static_keys, self.step.max_rows, self.step.n_plans, self.step.ints = ctx.static_keys, R, 0, base
+        self.step.longest = ctx.static_keys // 2 or max((p + n for p, n in zip(ctx.entry_first_pos, ctx.entry_length)), default=0)
         self.sampled = ctx.sampled if sampled is None else sampled
         self.embedding_output = ctx.embedding_output
         self.pending = None

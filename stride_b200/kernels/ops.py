@@ -698,10 +698,10 @@ def masked_attention_tiles(q, out, cache_layer, block_table, entry_meta, entries
     if not (q.dtype == out.dtype == cache_layer.dtype == torch.bfloat16):
         raise TypeError("masked_attention_tiles takes bfloat16 q, out and cache")
     lib, fn = _fn("masked_attention", "sb_masked_attention_tiles_in",
-                  [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int64, c_int64, c_int64, c_void_p, c_int, c_int, c_void_p, c_void_p,
+                  [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int64, c_int64, c_int64, c_void_p, c_int, c_int, c_void_p, c_void_p,
                    c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_float, c_void_p])
     pages, *where = _page_args(cache_layer, block_table)
-    _check(lib, fn(_ptr(q), _ptr(out), pages, cache_layer.shape[0], *where, _ptr(entry_meta), entry_meta.stride(0), entries, _ptr(slopes),
+    _check(lib, fn(_ptr(q), _ptr(out), pages, cache_layer.shape[0], 0, *where, _ptr(entry_meta), entry_meta.stride(0), entries, _ptr(slopes),
                    _ptr(sinks), q.shape[0], num_heads, num_kv_heads, key_dim, value_dim, cache_layer.shape[4], window, keep_first, scale, 0, 0, 0.0,
                    _stream()))
 

@@ -18,6 +18,15 @@ def _call(name, argtypes, args):
     ops._check(lib, fn(*args))
 
 
+def _kernels(call):
+    """What call() returns and the names of the kernels that it launches."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        result = call()
+        torch.cuda.synchronize()
+    return result, " ".join(e.name for e in p.events())
+
+
 def _latent_case(entries, H, G, page, odd=(), seed=0):
     """q, cache layer, block table, entry meta and sinks; entries are (tokens, tokens in front), memory that no token filled is NaN, `odd` are
     (entry, position, element, value) of latents."""
@@ -42,15 +51,15 @@ def _latent_case(entries, H, G, page, odd=(), seed=0):
     return q, cache, table, torch.tensor(meta, dtype=torch.int32).T.contiguous().to(DEVICE), torch.randn(H, device=DEVICE, generator=gen)
 
 
-def _latent(case, window, pages):
+def _latent(case, window, pages, longest=0):
     """pages: of the arena, or 0: the form that addresses pages by TMA is left out."""
     q, cache, table, meta, sinks = case
     H, G = sinks.numel(), cache.shape[2]
     out = torch.zeros_like(q)
     _call("sb_masked_attention_tiles_in",
-          [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int64, c_int64, c_int64, c_void_p, c_int, c_int, c_void_p, c_void_p] +
+          [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int64, c_int64, c_int64, c_void_p, c_int, c_int, c_void_p, c_void_p] +
           [c_int] * 8 + [c_float, c_int, c_int, c_float, c_void_p],
-          [q.data_ptr(), out.data_ptr(), cache.data_ptr(), pages, table.data_ptr(), table.shape[1], cache.shape[3], cache.stride(0), 0, cache.stride(2),
+          [q.data_ptr(), out.data_ptr(), cache.data_ptr(), pages, longest, table.data_ptr(), table.shape[1], cache.shape[3], cache.stride(0), 0, cache.stride(2),
            meta.data_ptr(), meta.stride(0), meta.shape[1], None, sinks.data_ptr(), q.shape[0], H, G, 512, 512, 512, window, 0, 0.03, 0, 0, 0.0,
            torch.cuda.current_stream().cuda_stream])
     torch.cuda.synchronize()
@@ -61,6 +70,9 @@ LATENT = [  # entries, H, G, window, page size, odd latents
     ([(16, 0)], 16, 1, 0, 64, ()), ([(17, 47)], 16, 1, 0, 64, ()), ([(1, 700), (1, 63), (1, 64), (3, 0)], 16, 1, 100, 64, ()), ([(1, 200)], 64, 1, 0, 16, ()), ([(64, 0)], 16, 1, 0, 64, ()),
     ([(200, 0), (33, 100), (65, 7)], 16, 1, 1024, 64, ()), ([(150, 100), (90, 7)], 16, 1, 70, 16, ()), ([(70, 300)], 16, 1, 3, 8, ()),
     ([(100, 500), (41, 7)], 32, 2, 64, 128, ()), ([(100, 30)], 4, 1, 65, 32, ()), ([(20, 50)], 128, 1, 0, 64, ()), ([(300, 0)], 1, 1, 0, 64, ()),
+    # as many tiles as entries of that many tokens can have: a token beyond every entry's last full tile
+    ([(9, 130), (17, 0), (1, 5), (25, 40)], 16, 1, 0, 64, ()), ([(3, 200)] * 5, 64, 1, 0, 64, ()), ([(1, 127)] * 55, 128, 1, 0, 64, ()),
+    ([(17, 150), (17, 20)], 16, 2, 0, 64, ()),
     # infinities and NaN at keys that some rows of a tile see and others do not: at the causal edge and at the window's
     ([(100, 0), (64, 3)], 16, 1, 0, 64, ((0, 50, 3, INF), (0, 51, 300, NAN), (1, 66, 511, -INF))),
     ([(100, 30), (64, 3)], 16, 1, 20, 64, ((0, 50, 3, INF), (0, 129, 300, NAN), (1, 3, 511, -INF), (1, 4, 0, INF))),
@@ -72,7 +84,8 @@ def test_latent_attention_on_tcgen05_has_the_bits_of_the_tile_kernel(entries, H,
     from stride_b200.kernels import ops
     word = ops.shared_status_word({"masked_attention"})
     case = _latent_case(entries, H, G, page, odd)
-    many = _latent(case, window, case[1].shape[0])
+    many, names = _kernels(lambda: _latent(case, window, case[1].shape[0], max(l + f for l, f in entries)))
+    assert "latent_attention_tc5_kernel" in names
     assert torch.equal(many.view(torch.int16), _latent(case, window, 0).view(torch.int16))
     assert word.item() == 0
     if odd:
@@ -92,13 +105,16 @@ def test_latent_attention_on_tcgen05_has_the_bits_of_the_tile_kernel(entries, H,
         assert ((got - want).abs().max() / want.abs().max()).item() < 2.0 ** -8 + 1e-4
 
 
-def _kernels(call):
-    """What call() returns and the names of the kernels that it launches."""
-    from torch.profiler import ProfilerActivity, profile
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
-        result = call()
-        torch.cuda.synchronize()
-    return result, " ".join(e.name for e in p.events())
+@pytest.mark.parametrize("count, H, G, window, longest, taken", [
+    (55, 16, 1, 0, 150, True), (56, 16, 1, 0, 150, False), (37, 16, 1, 0, 0, True), (38, 16, 1, 0, 127, False), (38, 16, 1, 0, 128, True), (38, 16, 1, 100, 700, False),
+    (55, 32, 1, 0, 0, True), (56, 32, 1, 0, 0, False), (8, 4, 1, 0, 60, False), (8, 4, 1, 0, 128, True), (1, 1, 1, 0, 0, False), (27, 32, 2, 0, 128, True),
+    (28, 32, 2, 0, 128, False)])
+def test_which_latent_attention_single_tokens_take(count, H, G, window, longest, taken):
+    """Both sides of the lines between the two forms, which have the same bits."""
+    case = _latent_case([(1, 20)] * count, H, G, 64)
+    got, names = _kernels(lambda: _latent(case, window, case[1].shape[0], longest))
+    assert ("latent_attention_tc5_kernel" in names) == taken
+    assert torch.equal(got.view(torch.int16), _latent(case, window, 0).view(torch.int16))
 
 
 HEADS = [  # n, H, K, N, partial sums of the gate, elements behind a row, elements behind a gate's row, whether the tcgen05 form is taken
