@@ -52,6 +52,7 @@ def test_tile_plans_match_their_restatement(seed):
     assert rc == 0, lib.sb_last_error().decode()
     assert (step.n, step.entries, step.wanted, step.max_rows, step.n_plans, step.ints) == (int(count.sum()), E, 3, R, 3, 4096)
     assert (staging[:9 * R] == -7).all()                                           # only the work lists are written
+    assert step.longest == max(c + f for c, f in zip(counts, firsts))
     for k, (group, tile_rows, kv_heads, limit) in enumerate(keys):
         work, tiles, items, chunks = _plain_plan(counts, firsts, group, tile_rows)
         p = step.plan[k]
@@ -62,6 +63,7 @@ def test_tile_plans_match_their_restatement(seed):
     # a recorded decode step: every entry one item, chunks from the key range it was recorded for
     rc = lib.sb_program_prepare(program, 5, None, None, 5, 5, 1024, staging.ctypes.data_as(_I32P), 4096, ctypes.byref(step))
     assert rc == 0
+    assert step.longest == 512
     p = step.plan[0]
     assert (p.tiles, p.items, p.chunks, step.static_keys) == (0, 5, 4, 1024)
     assert staging[9 * R + p.work_offset:9 * R + p.work_offset + 5].tolist() == [0, 1, 2, 3, 4]

@@ -199,6 +199,14 @@ def test_products_of_many_tokens_store_what_products_of_a_few_store(n, M, K, gat
     assert ops.gemm_tc_status() == 0
 
 
+@pytest.mark.parametrize("n", [2048, 2061])
+@pytest.mark.parametrize("M, K", [(3072, 136), (5124, 136), (3072, 2048), (5124, 2048), (5122, 136)])
+def test_pairs_that_walk_several_tiles_store_what_products_of_a_few_store(M, K, n):
+    """96 to 189 tiles on 74 pairs of CTAs: a pair's last tile goes to memory by TMA over the ring, the ones in front of it element by element;
+    one and several ranges of K, rows that the tiles do not divide, and rows that TMA does not take."""
+    test_products_of_many_tokens_store_what_products_of_a_few_store(n, M, K, False)
+
+
 @pytest.mark.parametrize("K", [3064, 3072, 3080])
 @pytest.mark.parametrize("M, n", [(8192, 700), (8204, 513), (16384, 300)])
 def test_gated_products_that_take_as_many_rounds_on_pairs(M, n, K):

@@ -593,6 +593,60 @@ def test_steps_of_many_tokens_give_the_bits_of_small_ones(tmp_path):
         assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2]), dtype
 
 
+# Latents of 512 and values of 64: prompts and single tokens in the tcgen05 forms of the latent attention and of the matrices per head.
+RANK_512 = {"architecture": "Viperax", "vocab": 200, "width": 128, "streams": 2, "norm": {"eps": 1e-5}, "embedding": {"scale": 1.0},
+            "layers": [{"type": "latent_attention", "mixer": {"heads": 16, "dim": 64, "vdim": 64, "kv_rank": 512, "scale": 0.125, **more},
+                        "mlp": {"kind": "dense", "ff": 64}} for more in ({"mask": {"size": 300}}, {"kv_from": 0})]}
+
+
+def test_latents_of_512_in_prompts_and_in_recorded_decode_steps(tmp_path):
+    """A prompt of 700 tokens in one step against portions of 64; then three requests of 700, 40 and 130 tokens decoded from recorded graphs,
+    through two of them, against the same steps without graphs and against the requests' tokens in one step each: the same bits."""
+    from torch.profiler import ProfilerActivity, profile
+    from stride_b200.engine.engine import StepEntry
+    folder = write_model(tmp_path / "m", "", config=RANK_512, seed=77)
+    start, more = [700, 40, 130], 130
+    reqs = [random_tokens(200, n + more, 900 + n) for n in start]
+
+    def feed(eng, slot, toks, first, sizes):
+        at, got = first, []
+        for n in sizes:
+            eng.cache.ensure(slot, at + n)
+            got.append(eng.step([StepEntry(slot, at, toks[at:at + n], list(range(n)))]).cpu().clone())
+            at += n
+        return torch.cat(got)
+
+    whole, decoded = [], []
+    for graphs in (True, False):
+        eng = _engine(folder, "bfloat16", 64, 40, rows=1024, cuda_graphs=graphs)
+        slots = [eng.cache.acquire_slot() for _ in reqs]
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            prompts = [feed(eng, slots[i], reqs[i], 0, [start[i]] if graphs else [64] * (start[i] // 64) + [start[i] % 64]) for i in range(3)]
+            torch.cuda.synchronize()
+        names = " ".join(e.name for e in p.events())
+        assert "latent_attention_tc5_kernel" in names
+        if graphs:
+            assert "head_linear_tc5_kernel<true>" in names and "head_linear_tc5_kernel<false>" in names
+        steps = []
+        for t in range(more):
+            for i in range(3):
+                eng.cache.ensure(slots[i], start[i] + t + 1)
+            steps.append(eng.step([StepEntry(slots[i], start[i] + t, [reqs[i][start[i] + t]], [0]) for i in range(3)]).cpu().clone())
+        assert (eng.graph_replays >= more - 2) == graphs
+        eng.check_kernels()
+        whole.append(prompts)
+        decoded.append(torch.stack(steps, 1))
+    for i in range(3):
+        assert torch.equal(whole[0][i], whole[1][i]), f"prompt {i}"
+    assert torch.equal(decoded[0], decoded[1])
+    eng = _engine(folder, "bfloat16", 64, 40, rows=1024)
+    for i in range(3):
+        slot = eng.cache.acquire_slot()
+        out = feed(eng, slot, reqs[i], 0, [len(reqs[i])])
+        eng.cache.release_slot(slot)
+        assert torch.equal(out[start[i]:], decoded[0][i]), f"request {i} in one step"
+
+
 def test_greedy_generation_through_the_entry_point(viperax_dirs):
     """LLM.generate with its scheduler (three requests on two slots, prompts cut into portions, decode steps replayed from CUDA
     graphs, the experts' table read for tokens that are still being chosen): the tokens of greedy decoding with the plain implementation."""
