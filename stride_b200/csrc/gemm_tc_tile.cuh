@@ -149,7 +149,7 @@ __device__ __forceinline__ void swiglu_tile(uint32_t tmem_base, float* xch, bf16
 // 19.9 / 18.3 / 21.4.)
 // tmem_d: the accumulator, this warp's lanes; j0: the first output feature; `vec`: the output takes 16-byte stores.
 __device__ __forceinline__ void swiglu_set(uint32_t tmem_d, float* xch2, bf16* done2, bf16* out, int64_t ldo, int j0, int half_rows, int n0, int N, int BN,
-                                           int set, int quarter, int lane, bool ok, bool vec, const Gate& gate, const float* column_weight = nullptr) {
+                                           int set, int quarter, int lane, bool ok, bool vec, const Gate& gate) {
   const int t = quarter * 32 + lane, jl = (quarter & 1) * 32 + lane;      // a thread's number in its set; its feature within the 64
   const int cb = quarter >= 2 ? 8 : 0;            // gate warps hand over columns 8..15, up warps 0..7: every warp finishes eight columns
   uint32_t v[16];
@@ -189,8 +189,7 @@ __device__ __forceinline__ void swiglu_set(uint32_t tmem_d, float* xch2, bf16* d
     for (int c = 0; c < 8; ++c) other[c] = xch[(cb + c) * 64 + jl];
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-      float g = quarter >= 2 ? other[c] : own[c], u = quarter >= 2 ? own[c] : other[c];
-      if (column_weight != nullptr) g *= column_weight[c0 + cb + c], u *= column_weight[c0 + cb + c];
+      const float g = quarter >= 2 ? other[c] : own[c], u = quarter >= 2 ? own[c] : other[c];
       done[(cb + c) * 64 + jl] = __float2bfloat16_rn(gated_product(g, u, gate));
     }
   }

@@ -1198,10 +1198,10 @@ SB_EXPORT int sb_masked_attention_tiles_supported(int H, int G, int D, int Dv, i
 
 // `arena_pages`: pages of the arena behind `pages` (0: not known; the form that addresses pages by TMA is then left out). `longest`: tokens of the
 // longest request with this step's, as far as known (0: not).
-SB_EXPORT int sb_masked_attention_tiles_in(const void* q, void* out, const void* pages, int arena_pages, int longest, const int32_t* block_table,
-                                           int max_pages, int page_size, int64_t page_stride, int64_t v_offset, int64_t head_stride, const int32_t* meta, int meta_stride,
-                                           int entries, const float* slopes, const float* sinks, int n, int H, int G, int D, int Dv, int Dc,
-                                           int window, int keep_first, float scale, int chunk, int out_f32, float cap, cudaStream_t stream) {
+SB_EXPORT int sb_masked_attention_tiles(const void* q, void* out, const void* pages, int arena_pages, int longest, const int32_t* block_table,
+                                        int max_pages, int page_size, int64_t page_stride, int64_t v_offset, int64_t head_stride, const int32_t* meta,
+                                        int meta_stride, int entries, const float* slopes, const float* sinks, int n, int H, int G, int D, int Dv,
+                                        int Dc, int window, int keep_first, float scale, int chunk, int out_f32, float cap, cudaStream_t stream) {
   if (n <= 0 || entries <= 0) return 0;
   if (chunk < 0) return sb::fail("sb_masked_attention_tiles: chunk %d", chunk);
   if (!sb_masked_attention_tiles_supported(H, G, D, Dv, Dc, v_offset))
@@ -1223,24 +1223,8 @@ SB_EXPORT int sb_masked_attention_tiles_in(const void* q, void* out, const void*
   }
 }
 
-SB_EXPORT int sb_masked_attention_tiles_ex(const void* q, void* out, const void* pages, const int32_t* block_table, int max_pages, int page_size,
-                                           int64_t page_stride, int64_t v_offset, int64_t head_stride, const int32_t* meta, int meta_stride,
-                                           int entries, const float* slopes, const float* sinks, int n, int H, int G, int D, int Dv, int Dc,
-                                           int window, int keep_first, float scale, int chunk, int out_f32, float cap, cudaStream_t stream) {
-  return sb_masked_attention_tiles_in(q, out, pages, 0, 0, block_table, max_pages, page_size, page_stride, v_offset, head_stride, meta, meta_stride, entries,
-                                      slopes, sinks, n, H, G, D, Dv, Dc, window, keep_first, scale, chunk, out_f32, cap, stream);
-}
-
 // From now on the kernels of this library that wait on barriers report into `device_word` (see sb_gemm_tc_use_status_word).
 SB_EXPORT void sb_masked_attention_use_status_word(int* device_word) { sb::tc5::status_word_given() = device_word; }
-
-SB_EXPORT int sb_masked_attention_tiles(const void* q, void* out, const void* pages, const int32_t* block_table, int max_pages, int page_size,
-                                        int64_t page_stride, int64_t v_offset, int64_t head_stride, const int32_t* meta, int meta_stride, int entries,
-                                        const float* slopes, const float* sinks, int n, int H, int G, int D, int Dv, int Dc, int window, int keep_first,
-                                        float scale, cudaStream_t stream) {
-  return sb_masked_attention_tiles_ex(q, out, pages, block_table, max_pages, page_size, page_stride, v_offset, head_stride, meta, meta_stride, entries,
-                                      slopes, sinks, n, H, G, D, Dv, Dc, window, keep_first, scale, 0, 0, 0.0f, stream);
-}
 
 // ------------------------------------------------------------------ operations of the native step program (step_ops.h)
 // i: 0 qkv partial sums (flat), 1 K ranges S, 2 most tokens with a buffer per range, 3 bias, 4 q gain, 5 k gain, 6 q out, 7 dtype, 8 pages,
@@ -1334,7 +1318,7 @@ SB_EXPORT int sb_op_masked_attention(const SbOp* op, const SbStep* s, void* stre
 SB_EXPORT int sb_op_masked_attention_tiles(const SbOp* op, const SbStep* s, void* stream) {
   using namespace sbstep;
   if (s->n <= 0) return SB_OP_SKIPPED;
-  return sb_masked_attention_tiles_in(ptr<const void>(op->i[0]), ptr<void>(op->i[1]), ptr<const void>(op->i[2]), (int)op->i[20], s->longest,
+  return sb_masked_attention_tiles(ptr<const void>(op->i[0]), ptr<void>(op->i[1]), ptr<const void>(op->i[2]), (int)op->i[20], s->longest,
                                    ptr<const int32_t>(op->i[3]), (int)op->i[4], (int)op->i[5], op->i[6], op->i[7], op->i[8], entry_meta(s), s->max_rows,
                                    s->entries, ptr<const float>(op->i[9]), ptr<const float>(op->i[10]), s->n, (int)op->i[11], (int)op->i[12], (int)op->i[13], (int)op->i[14], (int)op->i[15],
                                    (int)op->i[16], (int)op->i[17], (float)op->f[0], (int)op->i[18], (int)op->i[19], (float)op->f[1],

@@ -697,7 +697,7 @@ def masked_attention_tiles(q, out, cache_layer, block_table, entry_meta, entries
     _cuda(q, out, cache_layer, block_table, entry_meta, slopes, sinks)
     if not (q.dtype == out.dtype == cache_layer.dtype == torch.bfloat16):
         raise TypeError("masked_attention_tiles takes bfloat16 q, out and cache")
-    lib, fn = _fn("masked_attention", "sb_masked_attention_tiles_in",
+    lib, fn = _fn("masked_attention", "sb_masked_attention_tiles",
                   [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int64, c_int64, c_int64, c_void_p, c_int, c_int, c_void_p, c_void_p,
                    c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_float, c_void_p])
     pages, *where = _page_args(cache_layer, block_table)

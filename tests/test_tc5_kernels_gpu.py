@@ -56,7 +56,7 @@ def _latent(case, window, pages, longest=0):
     q, cache, table, meta, sinks = case
     H, G = sinks.numel(), cache.shape[2]
     out = torch.zeros_like(q)
-    _call("sb_masked_attention_tiles_in",
+    _call("sb_masked_attention_tiles",
           [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int64, c_int64, c_int64, c_void_p, c_int, c_int, c_void_p, c_void_p] +
           [c_int] * 8 + [c_float, c_int, c_int, c_float, c_void_p],
           [q.data_ptr(), out.data_ptr(), cache.data_ptr(), pages, longest, table.data_ptr(), table.shape[1], cache.shape[3], cache.stride(0), 0, cache.stride(2),
