@@ -982,7 +982,7 @@ def _viperax_kernels(timed, pk: dict, width: int, ff: int) -> dict:
         seen = lambda i: min(window, i + 1)
         keys = sum(seen(past + t) for t in range(length)) * entries
         moved = (entries * seen(past) * R * 2.0 + n * H * 2 * R * 2.0) if length == 1 else None
-        ms = timed(op("sb_op_masked_attention_tiles", [ql, ol, pages, block, per, page, pages.stride(0), 0, pages.stride(2), None, sinks, H, 1, R, R, R, window, 0],
+        ms = timed(op("sb_op_masked_attention_tiles", [ql, ol, pages, block, per, page, pages.stride(0), 0, pages.stride(2), None, sinks, H, 1, R, R, R, window, 0, 0, 0, pages.shape[0]],
                       [0.09]), 5, clear=True)
         record("latent_attention_" + label, ms, moved, 4.0 * keys * H * R)
         pql = rand(n, H * row).to(bf)
