@@ -1136,7 +1136,8 @@ SB_EXPORT int sb_gemm_tc_gated(const void* x, int64_t ldx, const void* w, int64_
   if (!multi && (p.tiles_n > 65535 || splits > 65535)) return sb::fail("sb_gemm_tc: grid too large");
   const dim3 grid(static_cast<unsigned>(multi ? resident : total_tiles));
   CUtensorMap map_out;
-  // (Few tokens leave a tile so few strips that the detour through shared memory costs what it saves.)
+  // (Few tokens leave a tile so few strips that the detour through shared memory costs what it saves. From 129 to 512 tokens, twelve weights of 512 to
+  // 6,144 rows: 0.83 to 1.01 of the time with stores a token at a time.)
   if (!multi && epilogue == kStore && n > 128 && p.block_n >= 32 && p.stages * stage_bytes >= 512 * p.block_n && map_rows_out(splits, &map_out)) {
     static sb::DeviceOnce once;
     if (once.needed()) {

@@ -1,5 +1,5 @@
-// Attention over latent rows of 512 elements whose values are the rows themselves, for prompts: the tile kernel of masked_attention.cu
-// on tcgen05, in the same arithmetic and the same bits.
+// Attention over latent rows of 512 elements whose values are the rows themselves, for prompts and for steps of few entries (launch_latent has the
+// lines): the tile kernel of masked_attention.cu on tcgen05, in the same arithmetic and the same bits.
 //
 // One CTA per (tile of 128 query rows of an entry and key/value head, half of the 512 value columns). A row is a (position, head), the heads
 // of the group side by side: 128 / (H / G) positions. The CTA walks the tiles of 64 keys, cut by absolute position, that any row sees:
@@ -22,10 +22,11 @@
 // of the tile sees are zeroed in shared memory; a key that some rows see and others do not, with a value that is not finite, is zeroed too
 // and added by ordinary multiply-adds to the rows that see it.
 //
-// Measured (16 heads, window 1,024, a sink): prompts of 333, 584 and 1,025 tokens 278 us on mma.sync, 102 here; one of 2,048 tokens 522 and
-// 171. Of the 5,650 cycles a tile takes, the tensor cores' products are about 3,700 (scores 2,400, bound by the operands' reads from shared
-// memory: both halves' CTAs make all scores, since 512 columns of values and the scores do not fit one SM's tensor memory); the rest is the
-// wait for the pieces whose place the tile in front leaves last, and the softmax warps' 2,870 cycles where the products do not cover them.
+// Measured (16 heads, window 1,024, a sink; within a step): prompts of 333, 584 and 1,025 tokens 282 us a layer on mma.sync, 103 here; one of 2,048
+// tokens 176 (alone behind a flush of L2 604 and 182). Of the 5,650 cycles a tile takes (by the clock, in a block that walks many), the products take
+// about 3,700 from issue to completion (scores 2,400: operands from shared memory; both halves' CTAs make all scores, since 512 columns of values
+// and the scores do not fit one SM's tensor memory), of which the tensor pipe works 2,100 (counters: 29% of a launch's active cycles); the rest is the wait for
+// the pieces whose place the tile in front leaves last, and the softmax warps' 2,870 cycles where the products do not cover them.
 #pragma once
 
 #include "tc5.cuh"
