@@ -70,8 +70,9 @@ __global__ void __launch_bounds__(128) expert_choose_kernel(const float* __restr
 
 // order [pairs]; tiles: [0] = how many, then (expert, first row, end row) each. What bounds it with 2,000 tokens is latency: a token's expert is two
 // loads one after the other, so those of up to kHeld pairs a thread are made once and, where table and tokens are the step's inputs, before the
-// wait for the kernels in front; lanes with the same expert count, and take their places, together.
-// Per launch, three prompts of 2,000 tokens in all: 11 us, here 6.1.
+// wait for the kernels in front. With the gather behind it, us, every pair looked up twice and after the wait / here: 2,048 tokens, one of eight
+// experts by table 9.2 / 5.5, chosen by the step 5.6 / 5.5; 4,096 tokens, eight of 512 experts 120 / 118 and 76 / 75.5. (Lanes of the same expert counted
+// together by a match of the warp instead of the atomic additions, a round of it an expert that the warp has: 6.3 and 6.4, 132 and 128.)
 constexpr int kHeld = 4;
 __global__ void __launch_bounds__(kSortThreads) expert_sort_kernel(const int32_t* __restrict__ tokens, const int32_t* __restrict__ slots,
                                                                    const int32_t* __restrict__ sampled, const int32_t* __restrict__ table, int vocab,      // vocab 0: the table's rows are the step's tokens
@@ -80,7 +81,7 @@ __global__ void __launch_bounds__(kSortThreads) expert_sort_kernel(const int32_t
   __shared__ int count[kMaxExperts], place[kMaxExperts], tile_at[kMaxExperts + 1];
   sb::grid_launch_dependents();
   for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
-  const int pairs = n * top, lane = threadIdx.x & 31;
+  const int pairs = n * top;
   auto expert_of = [&](int p) {
     const int row = p % n;
     if (vocab == 0) return min(max(table[static_cast<int64_t>(row) * top + p / n], 0), E - 1);
@@ -89,32 +90,28 @@ __global__ void __launch_bounds__(kSortThreads) expert_sort_kernel(const int32_t
     if (tok < 0 || tok >= vocab) tok = 0;
     return min(max(table[static_cast<int64_t>(tok) * top + p / n], 0), E - 1);
   };
-  // all lanes of a warp: their experts' counters moved on by as many lanes, and each lane's own number before (e < 0: no pair)
-  auto take = [&](int* counters, int e) {
-    const unsigned same = __match_any_sync(0xffffffffu, e);
-    const int leader = __ffs(same) - 1;
-    int at = 0;
-    if (lane == leader && e >= 0) at = atomicAdd(&counters[e], __popc(same));
-    return __shfl_sync(0xffffffffu, at, leader) + __popc(same & ((1u << lane) - 1));
-  };
   int held[kHeld];
   bool open[kHeld];                // (a token that an earlier kernel chooses: known after the wait)
 #pragma unroll
   for (int i = 0; i < kHeld; ++i) {
     const int p = threadIdx.x + i * blockDim.x;
-    open[i] = p < pairs && (vocab == 0 || tokens[p % n] == -1);
-    held[i] = p < pairs && !open[i] ? expert_of(p) : -1;
+    open[i] = false, held[i] = -1;
+    if (p < pairs) {
+      open[i] = vocab == 0 || tokens[p % n] == -1;
+      if (!open[i]) held[i] = expert_of(p);
+    }
   }
   __syncthreads();
   sb::grid_dependency_wait();
 #pragma unroll
   for (int i = 0; i < kHeld; ++i) {
     if (open[i]) held[i] = expert_of(threadIdx.x + i * blockDim.x);
-    if (i * static_cast<int>(blockDim.x) < pairs) take(count, held[i]);
+    if (held[i] >= 0) atomicAdd(&count[held[i]], 1);
   }
-  for (int p = kHeld * blockDim.x + threadIdx.x; p - static_cast<int>(threadIdx.x) < pairs; p += blockDim.x) take(count, p < pairs ? expert_of(p) : -1);
+  for (int p = kHeld * blockDim.x + threadIdx.x; p < pairs; p += blockDim.x) atomicAdd(&count[expert_of(p)], 1);
   __syncthreads();
   if (threadIdx.x < 32) {          // one warp: running sums of the counts and of the tiles, 32 experts at a time
+    const int lane = threadIdx.x;
     int rows_before = 0, tiles_before = 0;
     for (int e0 = 0; e0 < E; e0 += 32) {
       const int e = e0 + lane, c = e < E ? count[e] : 0, t = (c + tile - 1) / tile;
@@ -138,15 +135,9 @@ __global__ void __launch_bounds__(kSortThreads) expert_sort_kernel(const int32_t
   }
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < kHeld; ++i) {
-    if (i * static_cast<int>(blockDim.x) >= pairs) break;
-    const int at = take(place, held[i]);
-    if (held[i] >= 0) order[at] = threadIdx.x + i * blockDim.x;
-  }
-  for (int p = kHeld * blockDim.x + threadIdx.x; p - static_cast<int>(threadIdx.x) < pairs; p += blockDim.x) {
-    const int at = take(place, p < pairs ? expert_of(p) : -1);
-    if (p < pairs) order[at] = p;
-  }
+  for (int i = 0; i < kHeld; ++i)
+    if (held[i] >= 0) order[atomicAdd(&place[held[i]], 1)] = threadIdx.x + i * blockDim.x;
+  for (int p = kHeld * blockDim.x + threadIdx.x; p < pairs; p += blockDim.x) order[atomicAdd(&place[expert_of(p)], 1)] = p;
 }
 
 // out[i] = x[order[i] % n], rows of `chunks` pieces of T.
