@@ -930,23 +930,32 @@ bool latent_shape(const TileParams& p, int pages) {
          ((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.pages)) & 15) == 0;
 }
 
-// From two tiles of 128 rows an entry on; and any entries, single tokens too, whose blocks are few. Microseconds, tile kernel / here, window
-// 1,024, 1,743 points of 1 to 128 heads a latent, 1 to 100 entries, 0 to 3,000 tokens in front: 16 heads, 700 tokens in front: 16 entries of 16
-// tokens 140 / 46, four of 64 tokens 140 / 45, eight of 256 tokens 566 / 193; eight of one token 65 / 47, behind 3,000 tokens 98 / 68.
-// Few blocks: where some request has 128 keys or more in its window, three quarters of the SMs (150 tokens in front: 64 blocks 0.64 to 0.90 of
-// the other's time, 110 blocks 0.69 to 0.98, 128 blocks 0.63 to 1.05; from 160 blocks on with few heads 1.4 and more). Where all have fewer, or
-// the host does not know, a CTA's time is mostly its beginning and its end: with 32 heads and more the same line (110 blocks 0.67 to 0.76), with
-// 8 and 16 heads half the SMs (up to 60 tokens in front: 64 blocks 0.88 to 1.02, 80 blocks 0.92 to 1.04, 110 blocks 1.05 to 1.19), with fewer
-// none (1.00 to 1.12 at 2 to 64 blocks).
-// Slower all the same: what a recorded step takes as known, half of the keys that it is planned for, is 128 in the shortest of them: a step of
-// requests with up to 64 keys and four heads or fewer a latent then takes up to 1 us longer (8.6 / 9.6), one with more takes 2 to 7 us less.
+// From two tiles of 128 rows an entry on; and any entries, single tokens too, whose blocks are few. Microseconds, tile kernel / here, 4,592
+// points of 1 to 128 heads a latent, 1 to 100 entries, 0 to 3,000 tokens in front, windows of 16 to 1,024 and none, pages of 8 to 256: 16 heads,
+// 700 tokens in front: 16 entries of 16 tokens 140 / 46, four of 64 tokens 140 / 45, eight of 256 tokens 566 / 193; eight of one token 65 / 47,
+// behind 3,000 tokens 98 / 68.
+// Few blocks: where some request has 128 keys or more in its window (`far`), three quarters of the SMs (150 tokens in front: 64 blocks 0.64 to
+// 0.90 of the other's time, 110 blocks 0.69 to 0.98, 128 blocks 0.63 to 1.05; from 160 blocks on with few heads 1.4 and more). Where all have
+// fewer, or the host does not know, a CTA's time is mostly its beginning and its end: with 32 heads and more the same line (110 blocks 0.67 to
+// 0.76), with 8 and 16 heads half the SMs (up to 60 tokens in front: 64 blocks 0.88 to 1.02, 80 blocks 0.92 to 1.04, 110 blocks 1.05 to 1.19),
+// with fewer none (1.00 to 1.12 at 2 to 64 blocks); and of the entries of two tiles only those of four heads and more (one head, 256 tokens,
+// windows of 16 to 100: 15 to 21 / 19 to 28), until the tile kernel's blocks of 16 rows are more than the SMs (`many`).
+// Pages of 8, eight loads for one: with 8 heads and more where the requests are far (150 tokens in front 0.78 to 0.95, up to 60 tokens 1.04 to
+// 1.13), or with many blocks (0.4 to 0.7).
+// Slower all the same: a window of 64, or of little less, of several tokens an entry, where a tile of 128 rows happens to lie over three tiles of
+// keys and the tile kernel's 16 rows over two: one or four entries 15.7 / 17.3 (16 heads; elsewhere in the sequence 15.6 / 13.8), 15.8 / 18.1
+// with four heads; pages of 16, four heads, a prompt of 64 tokens 10.3 / 10.8. What a recorded step takes as known, half of the keys that it is
+// planned for, is 128 in the shortest of them: a step of requests with up to 64 keys and four heads or fewer a latent then takes up to 1 us
+// longer (8.6 / 9.6), one with more takes 2 to 7 us less.
 int launch_latent(const TileParams& p, int pages, int n, int longest, cudaStream_t stream, bool* done) {
   using namespace sb::latent5;
   const int Hg = p.H / p.G, ppt = kRows / Hg;
   const int64_t sms = sb::sm_count();
   const int64_t tiles = static_cast<int64_t>(n - p.entries) / ppt + p.entries, blocks = 2 * tiles * p.G;      // (the most: an entry has ceil(its tokens / ppt))
   const bool far = (p.window > 0 ? std::min(p.window, longest) : longest) >= 128;
-  *done = n >= 2 * static_cast<int64_t>(ppt) * p.entries || (far || Hg >= 32 ? 4 * blocks <= 3 * sms : Hg >= 8 && 2 * blocks <= sms);
+  const bool many = static_cast<int64_t>(n) * p.H > 16 * sms;
+  const bool few = far || Hg >= 32 ? 4 * blocks <= 3 * sms : Hg >= 8 && 2 * blocks <= sms;
+  *done = (p.page_size >= 16 || many || (far && Hg >= 8)) && (n >= 2 * static_cast<int64_t>(ppt) * p.entries ? far || many || Hg >= 4 : few);
   if (!*done) return 0;
   int* status = sb::tc5::status_word();
   if (!status) return sb::fail("sb_masked_attention_tiles: no status word");
